@@ -172,6 +172,7 @@ int hc_ctx_destroy(hc_ctx *ctx)
     cudaFree(ctx->qs.d_order);
     cudaFree(ctx->qs.d_fitstart);
     cudaFree(ctx->d_phase);
+    cudaFree(ctx->d_grad_part);
     cudaFree(ctx->d_log10);
     cudaFree(ctx->qs.d_in);
     cudaFree(ctx->qs.d_outbuf);

@@ -218,6 +218,8 @@ struct hc_ctx
     cudaGraphExec_t graph_exec = nullptr;
     hc::GraphKey graph_key{};
     int graph_launches = 0;
+    float *d_grad_part = nullptr;  // training: the CTAs' shares of a minibatch's gradients (hc_mlp.cu)
+    uint32_t grad_part_cap = 0;
     hc::StreamStage *stage = nullptr;  // kept between streaming calls, grown on demand
 };
 

@@ -58,8 +58,6 @@ struct hc_mlp
     float *d_params = nullptr;  // W1 b1 W2 b2 W3 b3
     float *d_grads = nullptr;
     float *d_m = nullptr, *d_v = nullptr;
-    float *d_act = nullptr;     // activations for one minibatch: h1 | h2 | out | dout | dh2 | dh1
-    size_t act_cap = 0;
     float *d_loss = nullptr;
     int step = 0;
     // gate of the learned tail: largest predicted RMS residual (log10 units),
@@ -115,106 +113,356 @@ __global__ void k_features(const uint32_t *__restrict__ hist, const hc_result *_
     for (int b = hyp + lane; b < kIn; b += 32) x[b] = last;
 }
 
-// ---- dense layers for training (row-major: Y[n,N] = X[n,K] W[K,N] + b) ----
-constexpr int TB = 32;
+// ---- training: forward, backward and the weights' gradients of a minibatch ----
+// One CTA takes R rows through all three layers and back without leaving
+// shared memory, and writes the rows' share of every parameter's gradient;
+// k_grad_reduce then adds the CTAs' shares in a fixed order (and, in training,
+// applies Adam), so a step is two launches with no intermediate activations
+// in global memory and its result does not vary from run to run. All sums are FP32.
+// What bounds it: FMA issue and shared-memory reads while the CTAs' rows are
+// worked off (about 90 k FMA a row), the shares' traffic (164 KB a CTA, L2)
+// when rows are few. R is the smallest of 8, 16 and 32 that still gives at
+// most one tile per SM, so small minibatches use most SMs and large ones reuse
+// each weight read for 32 rows.
+constexpr int kGradThreads = 512;
+constexpr int kW2Pitch = kH2 + 4;  // rows 16 bytes apart modulo the banks: a warp reads 32 rows' float4 without conflicts
+constexpr size_t kPartStride = (kParams + 1 + 3) / 4 * 4;  // a CTA's share: gradients, then its loss
 
-__global__ void k_linear(const float *__restrict__ X, const float *__restrict__ W, const float *__restrict__ b,
-                         float *__restrict__ Y, int n, int K, int N, int relu)
+template <int R>
+struct GradSmem
 {
-    __shared__ float xs[TB][TB + 1], ws[TB][TB + 1];
-    const int r = blockIdx.y * TB + threadIdx.y, c = blockIdx.x * TB + threadIdx.x;
-    float acc = 0.0f;
-    for (int k0 = 0; k0 < K; k0 += TB)
+    float xs[R][kIn];
+    float w2[kH1][kW2Pitch];
+    float w3[kH2][kOut];
+    float h1[R][kH1];
+    float h2[R][kH2];
+    float dout[R][kOut];
+    float loss[kGradThreads / 32];
+    union
     {
-        xs[threadIdx.y][threadIdx.x] = (r < n && k0 + threadIdx.x < K) ? X[(size_t)r * K + k0 + threadIdx.x] : 0.0f;
-        ws[threadIdx.y][threadIdx.x] = (k0 + threadIdx.y < K && c < N) ? W[(size_t)(k0 + threadIdx.y) * N + c] : 0.0f;
-        __syncthreads();
-#pragma unroll
-        for (int k = 0; k < TB; k++) acc += xs[threadIdx.y][k] * ws[k][threadIdx.x];
-        __syncthreads();
-    }
-    if (r < n && c < N)
-    {
-        float v = acc + b[c];
-        Y[(size_t)r * N + c] = relu ? fmaxf(v, 0.0f) : v;
-    }
-}
-
-// dX[n,K] = (dY[n,N] W^T) * (X > 0)   (X = the layer input after its ReLU)
-__global__ void k_linear_bwd_x(const float *__restrict__ dY, const float *__restrict__ W,
-                               const float *__restrict__ Xin, float *__restrict__ dX, int n, int K, int N)
-{
-    __shared__ float ds[TB][TB + 1], ws[TB][TB + 1];
-    const int r = blockIdx.y * TB + threadIdx.y, c = blockIdx.x * TB + threadIdx.x;  // c indexes K
-    float acc = 0.0f;
-    for (int j0 = 0; j0 < N; j0 += TB)
-    {
-        ds[threadIdx.y][threadIdx.x] = (r < n && j0 + threadIdx.x < N) ? dY[(size_t)r * N + j0 + threadIdx.x] : 0.0f;
-        const int wc = blockIdx.x * TB + threadIdx.y;  // row of W (a K index)
-        ws[threadIdx.y][threadIdx.x] = (wc < K && j0 + threadIdx.x < N) ? W[(size_t)wc * N + j0 + threadIdx.x] : 0.0f;
-        __syncthreads();
-#pragma unroll
-        for (int j = 0; j < TB; j++) acc += ds[threadIdx.y][j] * ws[threadIdx.x][j];
-        __syncthreads();
-    }
-    if (r < n && c < K) dX[(size_t)r * K + c] = Xin[(size_t)r * K + c] > 0.0f ? acc : 0.0f;
-}
-
-// dW[K,N] = X^T dY, db[N] = sum_rows dY   (one thread per output, rows tiled)
-__global__ void k_linear_bwd_w(const float *__restrict__ X, const float *__restrict__ dY, float *__restrict__ dW,
-                               float *__restrict__ db, int n, int K, int N)
-{
-    __shared__ float xs[TB][TB + 1], ds[TB][TB + 1];
-    const int k = blockIdx.y * TB + threadIdx.y, c = blockIdx.x * TB + threadIdx.x;
-    float acc = 0.0f, accb = 0.0f;
-    for (int r0 = 0; r0 < n; r0 += TB)
-    {
-        const int rx = r0 + threadIdx.x;  // row index for the transposed X tile
-        xs[threadIdx.y][threadIdx.x] = (rx < n && blockIdx.y * TB + threadIdx.y < K)
-                                           ? X[(size_t)rx * K + blockIdx.y * TB + threadIdx.y] : 0.0f;
-        ds[threadIdx.y][threadIdx.x] = (r0 + threadIdx.y < n && c < N) ? dY[(size_t)(r0 + threadIdx.y) * N + c] : 0.0f;
-        __syncthreads();
-#pragma unroll
-        for (int r = 0; r < TB; r++)
+        float red1[4][R][kH1];  // layer 1, a quarter of the inputs each
+        float red2[4][R][kH2];  // layer 2 the same
+        struct
         {
-            acc += xs[threadIdx.y][r] * ds[r][threadIdx.x];
-            accb += ds[r][threadIdx.x];
+            float dh2[R][kH2];
+            float dh1[R][kH1];
+        } d;
+    } u;
+};
+
+__device__ __forceinline__ void fma4(float4 &a, float x, const float4 &w)
+{
+    a.x = fmaf(x, w.x, a.x);
+    a.y = fmaf(x, w.y, a.y);
+    a.z = fmaf(x, w.z, a.z);
+    a.w = fmaf(x, w.w, a.w);
+}
+
+// writes v, or adds it to what an earlier tile of this CTA left there
+__device__ __forceinline__ void put4(float *p, float4 v, bool add)
+{
+    float4 *q = reinterpret_cast<float4 *>(p);
+    if (add)
+    {
+        const float4 o = *q;
+        v = make_float4(o.x + v.x, o.y + v.y, o.z + v.z, o.w + v.w);
+    }
+    *q = v;
+}
+
+template <int R>
+__global__ void __launch_bounds__(kGradThreads, 1) k_grad_tile(const float *__restrict__ P, const float *__restrict__ X,
+                                                               const float *__restrict__ Y, int n, int ntiles,
+                                                               float *__restrict__ part)
+{
+    extern __shared__ __align__(16) unsigned char gsm[];
+    GradSmem<R> &S = *reinterpret_cast<GradSmem<R> *>(gsm);
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    float *mine = part + (size_t)blockIdx.x * kPartStride;
+    for (int i = tid; i < kH1 * kH2 / 4; i += kGradThreads)
+    {
+        const int k = i / (kH2 / 4), j = i % (kH2 / 4);
+        *reinterpret_cast<float4 *>(&S.w2[k][4 * j]) = __ldg(reinterpret_cast<const float4 *>(P + kOffW2) + i);
+    }
+    for (int i = tid; i < kH2 * kOut / 4; i += kGradThreads)
+        reinterpret_cast<float4 *>(&S.w3[0][0])[i] = __ldg(reinterpret_cast<const float4 *>(P + kOffW3) + i);
+    float loss = 0.0f;
+    bool add = false;
+    for (int tile = blockIdx.x; tile < ntiles; tile += gridDim.x, add = true)
+    {
+        const int r0 = tile * R;
+        // rows past the end: zero inputs and, below, zero output gradients
+        for (int i = tid; i < R * kIn / 4; i += kGradThreads)
+        {
+            const int r = i / (kIn / 4), c = i % (kIn / 4);
+            reinterpret_cast<float4 *>(&S.xs[r][0])[c] =
+                r0 + r < n ? __ldg(reinterpret_cast<const float4 *>(X + (size_t)(r0 + r) * kIn) + c)
+                           : make_float4(0.f, 0.f, 0.f, 0.f);
+        }
+        __syncthreads();
+        // layer 1: warps 4q .. 4q+3 take inputs [64q, 64q + 64), each R/4 rows; lane l units 4l .. 4l+3
+        {
+            constexpr int RT = R / 4;
+            const int q = warp >> 2, rb = (warp & 3) * RT;
+            float4 acc[RT];
+#pragma unroll
+            for (int r = 0; r < RT; r++) acc[r] = make_float4(0.f, 0.f, 0.f, 0.f);
+            const float4 *w1 = reinterpret_cast<const float4 *>(P + kOffW1) + lane;
+#pragma unroll 2
+            for (int k = 64 * q; k < 64 * q + 64; k += 4)
+            {
+                float4 w[4];
+#pragma unroll
+                for (int i = 0; i < 4; i++) w[i] = __ldg(w1 + (k + i) * (kH1 / 4));
+#pragma unroll
+                for (int r = 0; r < RT; r++)
+                {
+                    const float4 x = *reinterpret_cast<const float4 *>(&S.xs[rb + r][k]);
+                    fma4(acc[r], x.x, w[0]);
+                    fma4(acc[r], x.y, w[1]);
+                    fma4(acc[r], x.z, w[2]);
+                    fma4(acc[r], x.w, w[3]);
+                }
+            }
+#pragma unroll
+            for (int r = 0; r < RT; r++) *reinterpret_cast<float4 *>(&S.u.red1[q][rb + r][4 * lane]) = acc[r];
+        }
+        __syncthreads();
+        for (int i = tid; i < R * kH1; i += kGradThreads)
+        {
+            const int r = i / kH1, c = i % kH1;
+            const float v = (S.u.red1[0][r][c] + S.u.red1[1][r][c]) + (S.u.red1[2][r][c] + S.u.red1[3][r][c]) +
+                            __ldg(P + kOffB1 + c);
+            S.h1[r][c] = fmaxf(v, 0.0f);
+        }
+        __syncthreads();
+        // layer 2: the same quarters of its 128 inputs; 16 groups of 4 units x 8 groups of R/8 rows
+        {
+            constexpr int RT = R / 8;
+            const int q = warp >> 2, t = tid & 127, cg = t & 15, rb = (t >> 4) * RT;
+            float4 acc[RT];
+#pragma unroll
+            for (int r = 0; r < RT; r++) acc[r] = make_float4(0.f, 0.f, 0.f, 0.f);
+#pragma unroll 2
+            for (int k = 32 * q; k < 32 * q + 32; k += 4)
+            {
+                float4 w[4];
+#pragma unroll
+                for (int i = 0; i < 4; i++) w[i] = *reinterpret_cast<const float4 *>(&S.w2[k + i][4 * cg]);
+#pragma unroll
+                for (int r = 0; r < RT; r++)
+                {
+                    const float4 x = *reinterpret_cast<const float4 *>(&S.h1[rb + r][k]);
+                    fma4(acc[r], x.x, w[0]);
+                    fma4(acc[r], x.y, w[1]);
+                    fma4(acc[r], x.z, w[2]);
+                    fma4(acc[r], x.w, w[3]);
+                }
+            }
+#pragma unroll
+            for (int r = 0; r < RT; r++) *reinterpret_cast<float4 *>(&S.u.red2[q][rb + r][4 * cg]) = acc[r];
+        }
+        __syncthreads();
+        for (int i = tid; i < R * kH2; i += kGradThreads)
+        {
+            const int r = i / kH2, c = i % kH2;
+            const float v = (S.u.red2[0][r][c] + S.u.red2[1][r][c]) + (S.u.red2[2][r][c] + S.u.red2[3][r][c]) +
+                            __ldg(P + kOffB2 + c);
+            S.h2[r][c] = fmaxf(v, 0.0f);
+        }
+        __syncthreads();
+        // outputs (four lanes each, 16 inputs a lane), the mean squared error on
+        // the scaled targets (NaN targets and rows past the end excluded) and its
+        // gradient 2 (out - t) / (n * 4)
+        if (tid < R * 16)
+        {
+            const int r = tid >> 4, c = (tid >> 2) & 3, q = tid & 3;
+            float v = 0.0f;
+#pragma unroll
+            for (int k = 0; k < 16; k++) v = fmaf(S.h2[r][4 * k + q], S.w3[4 * k + q][c], v);
+            v += __shfl_xor_sync(0xFFFFFFFFu, v, 1);
+            v += __shfl_xor_sync(0xFFFFFFFFu, v, 2);
+            if (q == 0)
+            {
+                const float y = r0 + r < n ? Y[(size_t)(r0 + r) * kOut + c] : __int_as_float(0x7FC00000);
+                const float d = isnan(y) ? 0.0f : v + __ldg(P + kOffB3 + c) - y * tscale(c);
+                S.dout[r][c] = 2.0f * d / (float)(n * kOut);
+                loss += d * d / (float)(n * kOut);
+            }
+        }
+        __syncthreads();
+        // back through layer 3
+        for (int i = tid; i < R * kH2; i += kGradThreads)
+        {
+            const int r = i / kH2, j = i % kH2;
+            const float4 g = *reinterpret_cast<const float4 *>(&S.dout[r][0]);
+            const float4 w = *reinterpret_cast<const float4 *>(&S.w3[j][0]);
+            const float v = fmaf(g.w, w.w, fmaf(g.z, w.z, fmaf(g.y, w.y, g.x * w.x)));
+            S.u.d.dh2[r][j] = S.h2[r][j] > 0.0f ? v : 0.0f;
+        }
+        if (tid < kH2 * kOut)
+        {
+            const int j = tid / kOut, c = tid % kOut;
+            float v = 0.0f;
+#pragma unroll 8
+            for (int r = 0; r < R; r++) v = fmaf(S.h2[r][j], S.dout[r][c], v);
+            float *p = mine + kOffW3 + tid;
+            *p = add ? *p + v : v;
+        }
+        else if (tid < kH2 * kOut + kOut)
+        {
+            float v = 0.0f;
+            for (int r = 0; r < R; r++) v += S.dout[r][tid - kH2 * kOut];
+            float *p = mine + kOffB3 + tid - kH2 * kOut;
+            *p = add ? *p + v : v;
+        }
+        __syncthreads();
+        // back through layer 2: a warp takes RB rows and 32 KB units, lane l units l, l + 32 ..
+        {
+            constexpr int RB = R == 8 ? 2 : 4, KB = R == 32 ? 2 : 1, NG = R / RB;
+            const int rb = (warp % NG) * RB, kb = (warp / NG) * 32 * KB + lane;
+            float acc[RB][KB];
+#pragma unroll
+            for (int r = 0; r < RB; r++)
+#pragma unroll
+                for (int i = 0; i < KB; i++) acc[r][i] = 0.0f;
+#pragma unroll 4
+            for (int j = 0; j < kH2; j += 4)
+            {
+                float4 w[KB];
+#pragma unroll
+                for (int i = 0; i < KB; i++) w[i] = *reinterpret_cast<const float4 *>(&S.w2[kb + 32 * i][j]);
+#pragma unroll
+                for (int r = 0; r < RB; r++)
+                {
+                    const float4 g = *reinterpret_cast<const float4 *>(&S.u.d.dh2[rb + r][j]);
+#pragma unroll
+                    for (int i = 0; i < KB; i++)
+                        acc[r][i] = fmaf(g.w, w[i].w, fmaf(g.z, w[i].z, fmaf(g.y, w[i].y, fmaf(g.x, w[i].x, acc[r][i]))));
+                }
+            }
+#pragma unroll
+            for (int r = 0; r < RB; r++)
+#pragma unroll
+                for (int i = 0; i < KB; i++)
+                    S.u.d.dh1[rb + r][kb + 32 * i] = S.h1[rb + r][kb + 32 * i] > 0.0f ? acc[r][i] : 0.0f;
+        }
+        // layer 2's weights: 4 x 4 outputs a thread
+        const int kq = tid >> 4, cq = tid & 15;
+        {
+            float4 acc[4];
+#pragma unroll
+            for (int i = 0; i < 4; i++) acc[i] = make_float4(0.f, 0.f, 0.f, 0.f);
+#pragma unroll 4
+            for (int r = 0; r < R; r++)
+            {
+                const float4 h = *reinterpret_cast<const float4 *>(&S.h1[r][4 * kq]);
+                const float4 g = *reinterpret_cast<const float4 *>(&S.u.d.dh2[r][4 * cq]);
+                fma4(acc[0], h.x, g);
+                fma4(acc[1], h.y, g);
+                fma4(acc[2], h.z, g);
+                fma4(acc[3], h.w, g);
+            }
+#pragma unroll
+            for (int i = 0; i < 4; i++) put4(mine + kOffW2 + (4 * kq + i) * kH2 + 4 * cq, acc[i], add);
+        }
+        __syncthreads();
+        // layer 1's weights: 8 x 8 outputs a thread (inputs 4kq.., 128 + 4kq..; units 4cq.., 64 + 4cq..)
+        {
+            float4 acc[8][2];
+#pragma unroll
+            for (int i = 0; i < 8; i++) acc[i][0] = acc[i][1] = make_float4(0.f, 0.f, 0.f, 0.f);
+#pragma unroll 2
+            for (int r = 0; r < R; r++)
+            {
+                const float4 x0 = *reinterpret_cast<const float4 *>(&S.xs[r][4 * kq]);
+                const float4 x1 = *reinterpret_cast<const float4 *>(&S.xs[r][kIn / 2 + 4 * kq]);
+                const float xv[8] = {x0.x, x0.y, x0.z, x0.w, x1.x, x1.y, x1.z, x1.w};
+#pragma unroll
+                for (int h = 0; h < 2; h++)
+                {
+                    const float4 g = *reinterpret_cast<const float4 *>(&S.u.d.dh1[r][64 * h + 4 * cq]);
+#pragma unroll
+                    for (int i = 0; i < 8; i++) fma4(acc[i][h], xv[i], g);
+                }
+            }
+#pragma unroll
+            for (int i = 0; i < 8; i++)
+#pragma unroll
+                for (int h = 0; h < 2; h++)
+                    put4(mine + kOffW1 + ((i >> 2) * (kIn / 2) + 4 * kq + (i & 3)) * kH1 + 64 * h + 4 * cq, acc[i][h],
+                         add);
+        }
+        // the biases' gradients: column sums
+        if (tid < kH1 + kH2)
+        {
+            float v = 0.0f;
+            if (tid < kH1)
+                for (int r = 0; r < R; r++) v += S.u.d.dh1[r][tid];
+            else
+                for (int r = 0; r < R; r++) v += S.u.d.dh2[r][tid - kH1];
+            float *p = mine + (tid < kH1 ? kOffB1 + tid : kOffB2 + tid - kH1);
+            *p = add ? *p + v : v;
         }
         __syncthreads();
     }
-    if (k < K && c < N) dW[(size_t)k * N + c] = acc;
-    if (blockIdx.y == 0 && threadIdx.y == 0 && c < N) db[c] = accb;
-}
-
-// MSE on scaled targets, NaN targets excluded: dOut = 2 (out - t) / (n * 4)
-__global__ void k_mse(const float *__restrict__ out, const float *__restrict__ Y, int n, float *__restrict__ dOut,
-                      float *__restrict__ loss)
-{
-    const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    float l = 0.0f;
-    if (i < n * kOut)
+    for (int o = 16; o > 0; o >>= 1) loss += __shfl_xor_sync(0xFFFFFFFFu, loss, o);
+    if (lane == 0) S.loss[warp] = loss;
+    __syncthreads();
+    if (tid == 0)
     {
-        const float y = Y[i];
-        float d = 0.0f;
-        if (!isnan(y)) d = out[i] - y * tscale(i % kOut);
-        dOut[i] = 2.0f * d / (float)(n * kOut);
-        l = d * d / (float)(n * kOut);
+        float v = 0.0f;
+        for (int w = 0; w < kGradThreads / 32; w++) v += S.loss[w];
+        mine[kParams] = v;
     }
-    for (int o = 16; o > 0; o >>= 1) l += __shfl_down_sync(0xFFFFFFFFu, l, o);
-    if ((threadIdx.x & 31) == 0) atomicAdd(loss, l);
 }
 
-__global__ void k_adam(float *__restrict__ p, const float *__restrict__ g, float *__restrict__ m, float *__restrict__ v,
-                       size_t n, float lr, float b1t, float b2t)
+struct AdamStep
 {
-    const size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= n) return;
-    const float gi = g[i];
-    const float mi = 0.9f * m[i] + 0.1f * gi;
-    const float vi = 0.999f * v[i] + 0.001f * gi * gi;
-    m[i] = mi;
-    v[i] = vi;
-    p[i] -= lr * (mi / (1.0f - b1t)) / (sqrtf(vi / (1.0f - b2t)) + 1e-8f);
+    float *p, *m, *v;  // null p: gradients only
+    float lr, c1, c2;  // bias corrections 1 - 0.9^t and 1 - 0.999^t
+};
+
+// The CTAs' shares added up, four parameters per thread column and eight
+// threads per column (share c, c + 8, ..): the gradient, or Adam's update from
+// it. Block 0 adds the minibatch's loss to *loss.
+__global__ void __launch_bounds__(256) k_grad_reduce(const float *__restrict__ part, int nparts, float *__restrict__ g,
+                                                     AdamStep ad, float *__restrict__ loss)
+{
+    __shared__ float4 s[8][32];
+    const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+    const size_t i4 = (size_t)blockIdx.x * 32 + lane;  // float4 of the parameters
+    float4 a = make_float4(0.f, 0.f, 0.f, 0.f);
+    if (i4 < kParams / 4)
+#pragma unroll 8
+        for (int c = w; c < nparts; c += 8)
+        {
+            const float4 x = __ldg(reinterpret_cast<const float4 *>(part + (size_t)c * kPartStride) + i4);
+            a = make_float4(a.x + x.x, a.y + x.y, a.z + x.z, a.w + x.w);
+        }
+    s[w][lane] = a;
+    __syncthreads();
+    if (w == 1 && blockIdx.x == 0)
+    {
+        float l = 0.0f;
+        for (int c = lane; c < nparts; c += 32) l += part[(size_t)c * kPartStride + kParams];
+        for (int o = 16; o > 0; o >>= 1) l += __shfl_xor_sync(0xFFFFFFFFu, l, o);
+        if (lane == 0) *loss += l;
+    }
+    if (threadIdx.x >= 128 || (size_t)blockIdx.x * 128 + threadIdx.x >= kParams) return;
+    const size_t i = (size_t)blockIdx.x * 128 + threadIdx.x;
+    const float *c = &s[0][0].x + threadIdx.x;
+    const float gi = ((c[0] + c[128]) + (c[256] + c[384])) + ((c[512] + c[640]) + (c[768] + c[896]));
+    if (!ad.p)
+    {
+        g[i] = gi;
+        return;
+    }
+    const float mi = 0.9f * ad.m[i] + 0.1f * gi;
+    const float vi = 0.999f * ad.v[i] + 0.001f * gi * gi;
+    ad.m[i] = mi;
+    ad.v[i] = vi;
+    ad.p[i] -= ad.lr * (mi / ad.c1) / (sqrtf(vi / ad.c2) + 1e-8f);
 }
 
 // ---- inference: the three layers fused, weights resident in shared memory ----
@@ -529,17 +777,6 @@ __global__ void __launch_bounds__(kLtWarps * 32) k_learned_tail(const uint32_t *
 
 }  // namespace
 
-static int mlp_forward(hc_mlp *m, const float *X, uint32_t n, float *h1, float *h2, float *out, cudaStream_t st)
-{
-    const float *P = m->d_params;
-    dim3 blk(TB, TB);
-    k_linear<<<dim3((kH1 + TB - 1) / TB, (n + TB - 1) / TB), blk, 0, st>>>(X, P + kOffW1, P + kOffB1, h1, n, kIn, kH1, 1);
-    k_linear<<<dim3((kH2 + TB - 1) / TB, (n + TB - 1) / TB), blk, 0, st>>>(h1, P + kOffW2, P + kOffB2, h2, n, kH1, kH2, 1);
-    k_linear<<<dim3((kOut + TB - 1) / TB, (n + TB - 1) / TB), blk, 0, st>>>(h2, P + kOffW3, P + kOffB3, out, n, kH2, kOut, 0);
-    HC_CUDA(m->ctx, cudaGetLastError());
-    return HC_SUCCESS;
-}
-
 // the fused inference kernel (no activations kept)
 static int mlp_infer(hc_mlp *m, const float *X, uint32_t n, float *out, cudaStream_t st)
 {
@@ -553,35 +790,41 @@ static int mlp_infer(hc_mlp *m, const float *X, uint32_t n, float *out, cudaStre
     return HC_SUCCESS;
 }
 
-static int ensure_act(hc_mlp *m, uint32_t n)
+template <int R>
+static cudaError_t grad_tile(const float *P, const float *X, const float *Y, uint32_t n, uint32_t ntiles, uint32_t grid,
+                             float *part, cudaStream_t st)
 {
-    const size_t need = (size_t)n * (kH1 + kH2 + kOut) * 2;
-    if (m->act_cap >= need) return HC_SUCCESS;
-    cudaFree(m->d_act);
-    m->d_act = nullptr;
-    m->act_cap = 0;
-    HC_CUDA(m->ctx, cudaMalloc((void **)&m->d_act, sizeof(float) * need));
-    m->act_cap = need;
-    return HC_SUCCESS;
+    const cudaError_t e =
+        cudaFuncSetAttribute(k_grad_tile<R>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(GradSmem<R>));
+    if (e != cudaSuccess) return e;
+    k_grad_tile<R><<<grid, kGradThreads, sizeof(GradSmem<R>), st>>>(P, X, Y, (int)n, (int)ntiles, part);
+    return cudaGetLastError();
 }
 
-// forward + backward of one minibatch; gradients land in d_grads
-static int mlp_fwd_bwd(hc_mlp *m, const float *X, const float *Y, uint32_t n, cudaStream_t st)
+// forward + backward of one minibatch; the gradients land in d_grads, or Adam
+// is applied to the parameters. d_loss grows by the minibatch's loss.
+static int mlp_step(hc_mlp *m, const float *X, const float *Y, uint32_t n, const AdamStep &ad, cudaStream_t st)
 {
-    int rc = ensure_act(m, n);
-    if (rc) return rc;
-    float *h1 = m->d_act, *h2 = h1 + (size_t)n * kH1, *out = h2 + (size_t)n * kH2;
-    float *dout = out + (size_t)n * kOut, *dh2 = dout + (size_t)n * kOut, *dh1 = dh2 + (size_t)n * kH2;
-    if ((rc = mlp_forward(m, X, n, h1, h2, out, st))) return rc;
+    const uint32_t sms = (uint32_t)m->ctx->sm_count;
+    const uint32_t R = n <= 8 * sms ? 8u : (n <= 16 * sms ? 16u : 32u);
+    const uint32_t ntiles = (n + R - 1) / R, grid = std::min(ntiles, sms);
+    // the shares: scratch of the context (training runs on its stream only), at
+    // most one per SM, 25 MB
+    hc_ctx *ctx = m->ctx;
+    if (ctx->grad_part_cap < grid)
+    {
+        cudaFree(ctx->d_grad_part);
+        ctx->d_grad_part = nullptr;
+        ctx->grad_part_cap = 0;
+        HC_CUDA(ctx, cudaMalloc((void **)&ctx->d_grad_part, sizeof(float) * kPartStride * grid));
+        ctx->grad_part_cap = grid;
+    }
     const float *P = m->d_params;
-    float *G = m->d_grads;
-    k_mse<<<(n * kOut + 255) / 256, 256, 0, st>>>(out, Y, (int)n, dout, m->d_loss);
-    dim3 blk(TB, TB);
-    k_linear_bwd_w<<<dim3((kOut + TB - 1) / TB, (kH2 + TB - 1) / TB), blk, 0, st>>>(h2, dout, G + kOffW3, G + kOffB3, n, kH2, kOut);
-    k_linear_bwd_x<<<dim3((kH2 + TB - 1) / TB, (n + TB - 1) / TB), blk, 0, st>>>(dout, P + kOffW3, h2, dh2, n, kH2, kOut);
-    k_linear_bwd_w<<<dim3((kH2 + TB - 1) / TB, (kH1 + TB - 1) / TB), blk, 0, st>>>(h1, dh2, G + kOffW2, G + kOffB2, n, kH1, kH2);
-    k_linear_bwd_x<<<dim3((kH1 + TB - 1) / TB, (n + TB - 1) / TB), blk, 0, st>>>(dh2, P + kOffW2, h1, dh1, n, kH1, kH2);
-    k_linear_bwd_w<<<dim3((kH1 + TB - 1) / TB, (kIn + TB - 1) / TB), blk, 0, st>>>(X, dh1, G + kOffW1, G + kOffB1, n, kIn, kH1);
+    float *part = ctx->d_grad_part;
+    HC_CUDA(m->ctx, R == 8    ? grad_tile<8>(P, X, Y, n, ntiles, grid, part, st)
+                    : R == 16 ? grad_tile<16>(P, X, Y, n, ntiles, grid, part, st)
+                              : grad_tile<32>(P, X, Y, n, ntiles, grid, part, st));
+    k_grad_reduce<<<(unsigned)((kParams + 127) / 128), 256, 0, st>>>(part, (int)grid, m->d_grads, ad, m->d_loss);
     HC_CUDA(m->ctx, cudaGetLastError());
     return HC_SUCCESS;
 }
@@ -717,7 +960,6 @@ int hc_mlp_destroy(hc_mlp *m)
     cudaFree(m->d_grads);
     cudaFree(m->d_m);
     cudaFree(m->d_v);
-    cudaFree(m->d_act);
     cudaFree(m->d_loss);
     cudaFree(m->d_X);
     cudaFree(m->d_net);
@@ -788,7 +1030,7 @@ int hc_mlp_gradients(hc_mlp *m, const float *d_X, const float *d_Y, uint32_t n, 
     if (!m || !d_X || !d_Y) return HC_ERR_INVLD_PTR;
     cudaStream_t st = m->ctx->stream;
     HC_CUDA(m->ctx, cudaMemsetAsync(m->d_loss, 0, 4, st));
-    int rc = mlp_fwd_bwd(m, d_X, d_Y, n, st);
+    int rc = mlp_step(m, d_X, d_Y, n, AdamStep{}, st);
     if (rc) return rc;
     if (host_grads) HC_CUDA(m->ctx, cudaMemcpyAsync(host_grads, m->d_grads, 4 * kParams, cudaMemcpyDeviceToHost, st));
     if (loss) HC_CUDA(m->ctx, cudaMemcpyAsync(loss, m->d_loss, 4, cudaMemcpyDeviceToHost, st));
@@ -809,12 +1051,12 @@ int hc_mlp_train(hc_mlp *m, const float *d_X, const float *d_Y, uint32_t n, uint
         for (uint32_t s0 = 0; s0 < n; s0 += batch)
         {
             const uint32_t b = std::min(batch, n - s0);
-            int rc = mlp_fwd_bwd(m, d_X + (size_t)s0 * kIn, d_Y + (size_t)s0 * kOut, b, st);
-            if (rc) return rc;
             m->step++;
-            const float b1t = std::pow(0.9f, (float)m->step), b2t = std::pow(0.999f, (float)m->step);
-            k_adam<<<(unsigned)((kParams + 255) / 256), 256, 0, st>>>(m->d_params, m->d_grads, m->d_m, m->d_v, kParams,
-                                                                       lr, b1t, b2t);
+            // in double: 1 - 0.999f alone is 5e-5 off 0.001
+            const float c1 = (float)(1.0 - std::pow(0.9, m->step)), c2 = (float)(1.0 - std::pow(0.999, m->step));
+            int rc = mlp_step(m, d_X + (size_t)s0 * kIn, d_Y + (size_t)s0 * kOut, b,
+                              AdamStep{m->d_params, m->d_m, m->d_v, lr, c1, c2}, st);
+            if (rc) return rc;
             nb++;
         }
         HC_CUDA(m->ctx, cudaMemcpyAsync(&loss, m->d_loss, 4, cudaMemcpyDeviceToHost, st));
