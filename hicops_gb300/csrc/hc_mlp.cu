@@ -150,12 +150,19 @@ struct GradSmem
     } u;
 };
 
+// a += x * w, each product and sum one FP32 FMA, two to an instruction
 __device__ __forceinline__ void fma4(float4 &a, float x, const float4 &w)
 {
-    a.x = fmaf(x, w.x, a.x);
-    a.y = fmaf(x, w.y, a.y);
-    a.z = fmaf(x, w.z, a.z);
-    a.w = fmaf(x, w.w, a.w);
+    uint64_t xx, lo, hi, wl, wh;
+    asm("mov.b64 %0, {%1, %1};" : "=l"(xx) : "f"(x));
+    asm("mov.b64 %0, {%1, %2};" : "=l"(lo) : "f"(a.x), "f"(a.y));
+    asm("mov.b64 %0, {%1, %2};" : "=l"(hi) : "f"(a.z), "f"(a.w));
+    asm("mov.b64 %0, {%1, %2};" : "=l"(wl) : "f"(w.x), "f"(w.y));
+    asm("mov.b64 %0, {%1, %2};" : "=l"(wh) : "f"(w.z), "f"(w.w));
+    asm("fma.rn.f32x2 %0, %1, %2, %0;" : "+l"(lo) : "l"(xx), "l"(wl));
+    asm("fma.rn.f32x2 %0, %1, %2, %0;" : "+l"(hi) : "l"(xx), "l"(wh));
+    asm("mov.b64 {%0, %1}, %2;" : "=f"(a.x), "=f"(a.y) : "l"(lo));
+    asm("mov.b64 {%0, %1}, %2;" : "=f"(a.z), "=f"(a.w) : "l"(hi));
 }
 
 // writes v, or adds it to what an earlier tile of this CTA left there
@@ -186,6 +193,7 @@ __global__ void __launch_bounds__(kGradThreads, 1) k_grad_tile(const float *__re
     }
     for (int i = tid; i < kH2 * kOut / 4; i += kGradThreads)
         reinterpret_cast<float4 *>(&S.w3[0][0])[i] = __ldg(reinterpret_cast<const float4 *>(P + kOffW3) + i);
+    const bool aligned = ((uintptr_t)X & 15) == 0;  // a caller's buffer may start anywhere a float does
     float loss = 0.0f;
     bool add = false;
     for (int tile = blockIdx.x; tile < ntiles; tile += gridDim.x, add = true)
@@ -195,9 +203,12 @@ __global__ void __launch_bounds__(kGradThreads, 1) k_grad_tile(const float *__re
         for (int i = tid; i < R * kIn / 4; i += kGradThreads)
         {
             const int r = i / (kIn / 4), c = i % (kIn / 4);
-            reinterpret_cast<float4 *>(&S.xs[r][0])[c] =
-                r0 + r < n ? __ldg(reinterpret_cast<const float4 *>(X + (size_t)(r0 + r) * kIn) + c)
-                           : make_float4(0.f, 0.f, 0.f, 0.f);
+            const float *x = X + (size_t)(r0 + r) * kIn + 4 * c;
+            float4 v = make_float4(0.f, 0.f, 0.f, 0.f);
+            if (r0 + r < n)
+                v = aligned ? __ldg(reinterpret_cast<const float4 *>(x))
+                            : make_float4(__ldg(x), __ldg(x + 1), __ldg(x + 2), __ldg(x + 3));
+            reinterpret_cast<float4 *>(&S.xs[r][0])[c] = v;
         }
         __syncthreads();
         // layer 1: warps 4q .. 4q+3 take inputs [64q, 64q + 64), each R/4 rows; lane l units 4l .. 4l+3
@@ -465,91 +476,329 @@ __global__ void __launch_bounds__(256) k_grad_reduce(const float *__restrict__ p
     ad.p[i] -= ad.lr * (mi / ad.c1) / (sqrtf(vi / ad.c2) + 1e-8f);
 }
 
-// ---- inference: the three layers fused, weights resident in shared memory ----
-// A CTA stages all parameters (about 162 KB) once and its warps then walk the
-// spectra, two per warp at a time: lane j computes hidden units 4j..4j+3 of
-// layer 1 (one 16-byte weight load per input serves both spectra) and 2j,
-// 2j+1 of layer 2; the four outputs are warp sums. Activations stay in the
-// warp's own shared-memory rows.
-constexpr int kInferWarps = 8;
-constexpr size_t kInferWeights = kParams;  // floats
-constexpr size_t kInferSmem = 4 * (kInferWeights + (size_t)kInferWarps * 2 * (kIn + kH1 + kH2));
+// ---- inference: the three layers fused ----
+// Two kernels, both FP32 FMA throughout (41 k FMA a spectrum; the batch's FMA
+// issue bounds them, not its 1 KB a spectrum of input; two FMAs to an
+// instruction where a thread holds neighbouring outputs).
+//
+// k_infer_tile, for batches that fill the chip: a persistent CTA per SM stages
+// all parameters (162 KB) in shared memory once and takes 64 spectra at a
+// time, inputs arriving in chunks of 64 through cp.async. A thread of layer 1
+// holds 8 x 8 outputs (one shared-memory read of 16 bytes for 16 FMAs), two
+// groups of four warps take half of each layer's inputs. 100,000 spectra: 176 us,
+// against 344 us with two spectra per warp, where a weight read served 8 FMAs,
+// and 202 us with one FMA to an instruction.
+//
+// k_infer_rows, for the rest: a CTA takes 8 spectra and its 16 warps 1/16 of
+// each layer's inputs, so every weight is read once per CTA, straight from L2
+// with no staging. 1,000 spectra: 8.2 us, against 14.3 us.
+//
+// The line between them: a tile takes 20.5 us up to 64 spectra per SM, rows
+// 12.3 us at 16 per SM, 20.5 us at 32 and 36.9 us at 64.
+constexpr int kTileThreads = 256, kRowsThreads = 512;
+constexpr int kInferTile = 64, kInferChunk = 64, kInferRows = 8;
+constexpr uint32_t kInferRowsPerSm = 32;
 
-__global__ void __launch_bounds__(kInferWarps * 32) k_mlp_infer(const float *__restrict__ P,
-                                                                const float *__restrict__ X, uint32_t n,
-                                                                float *__restrict__ out)
+struct InferSmem
 {
-    extern __shared__ __align__(16) float sm[];
-    float *W = sm;
-    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-    for (size_t i = tid; i < kParams / 4; i += blockDim.x)
-        reinterpret_cast<float4 *>(W)[i] = __ldg(reinterpret_cast<const float4 *>(P) + i);
-    __syncthreads();
-    const float *W1 = W + kOffW1, *b1 = W + kOffB1, *W2 = W + kOffW2, *b2 = W + kOffB2, *W3 = W + kOffW3,
-                *b3 = W + kOffB3;
-    float *xs = sm + kInferWeights + (size_t)warp * 2 * (kIn + kH1 + kH2);  // x[2][256] | h1[2][128] | h2[2][64]
-    float *h1s = xs + 2 * kIn, *h2s = h1s + 2 * kH1;
-    const uint32_t npair = (n + 1) / 2;
-    for (uint32_t pr = blockIdx.x * kInferWarps + warp; pr < npair; pr += gridDim.x * kInferWarps)
+    float w1[kIn][kH1];
+    float w2[kH1][kH2];
+    float w3[kH2][kOut];
+    float b[kH1 + kH2 + kOut];
+    float xs[2][kInferTile][kInferChunk];
+    float h1[kInferTile][kH1];
+};
+
+__device__ __forceinline__ void cp_async16(void *dst, const void *src, bool in)
+{
+    // out of range: 16 zero bytes, nothing read
+    asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"((uint32_t)__cvta_generic_to_shared(dst)), "l"(src),
+                 "r"(in ? 16 : 0));
+}
+
+__device__ __forceinline__ float4 relu4(const float4 &a, const float4 &p, const float4 &b)
+{
+    return make_float4(fmaxf(a.x + p.x + b.x, 0.f), fmaxf(a.y + p.y + b.y, 0.f), fmaxf(a.z + p.z + b.z, 0.f),
+                       fmaxf(a.w + p.w + b.w, 0.f));
+}
+
+__global__ void __launch_bounds__(kTileThreads, 1) k_infer_tile(const float *__restrict__ P, const float *__restrict__ X,
+                                                                uint32_t n, float *__restrict__ out)
+{
+    extern __shared__ __align__(16) unsigned char ism[];
+    InferSmem &S = *reinterpret_cast<InferSmem *>(ism);
+    const int tid = threadIdx.x;
+    // group q of 128 threads takes half of the inputs; a thread 8 rows from rb
+    const int q = tid >> 7, cg = tid & 15, rb = 8 * ((tid >> 4) & 7);
+    const uint32_t ntiles = (n + kInferTile - 1) / kInferTile;
+    // chunk c of a tile's inputs, four 16-byte copies a thread
+    auto load = [&](uint32_t tile, int c) {
+#pragma unroll
+        for (int i = 0; i < 4; i++)
+        {
+            const int r = (tid >> 4) + 16 * i, j = 4 * (tid & 15);
+            const uint32_t row = tile * kInferTile + (uint32_t)r;
+            cp_async16(&S.xs[c & 1][r][j], X + (size_t)min(row, n - 1) * kIn + c * kInferChunk + j, row < n);
+        }
+    };
+    auto commit = [] { asm volatile("cp.async.commit_group;"); };
+    auto copy = [&](float *dst, const float *src, int words) {
+        for (int i = 4 * tid; i < words; i += 4 * kTileThreads) cp_async16(dst + i, src + i, true);
+    };
+    // the first tile's first chunk with the weights it meets, then the other weights under it
+    load(blockIdx.x, 0);
+    copy(&S.w1[0][0], P + kOffW1, kInferChunk * kH1);
+    commit();
+    copy(&S.w1[kInferChunk][0], P + kOffW1 + kInferChunk * kH1, (kIn - kInferChunk) * kH1);
+    copy(&S.w2[0][0], P + kOffW2, kH1 * kH2);
+    copy(&S.w3[0][0], P + kOffW3, kH2 * kOut);
+    commit();
+    for (int i = tid; i < kH1 + kH2 + kOut; i += kTileThreads)
+        S.b[i] = __ldg(P + (i < kH1 ? kOffB1 + i : (i < kH1 + kH2 ? kOffB2 + i - kH1 : kOffB3 + i - kH1 - kH2)));
+    bool first = true;
+    for (uint32_t tile = blockIdx.x; tile < ntiles; tile += gridDim.x)
     {
-        const uint32_t s0 = 2 * pr, s1 = min(s0 + 1, n - 1);
-        // inputs: 64 float4 per spectrum
-        for (int i = lane; i < 2 * kIn / 4; i += 32)
+        // layer 1: 8 x 8 outputs a thread (units 4cg.., 64 + 4cg..), half of each chunk
         {
-            const uint32_t sp = i < kIn / 4 ? s0 : s1;
-            const int k = i % (kIn / 4);
-            reinterpret_cast<float4 *>(xs)[i] = __ldg(reinterpret_cast<const float4 *>(X + (size_t)sp * kIn) + k);
-        }
-        __syncwarp();
-        // layer 1: units 4*lane .. 4*lane + 3
-        float4 a0 = reinterpret_cast<const float4 *>(b1)[lane], a1 = a0;
-#pragma unroll 8
-        for (int k = 0; k < kIn; k++)
-        {
-            const float4 w = reinterpret_cast<const float4 *>(W1 + (size_t)k * kH1)[lane];
-            const float x0 = xs[k], x1 = xs[kIn + k];
-            a0.x = fmaf(x0, w.x, a0.x); a0.y = fmaf(x0, w.y, a0.y); a0.z = fmaf(x0, w.z, a0.z); a0.w = fmaf(x0, w.w, a0.w);
-            a1.x = fmaf(x1, w.x, a1.x); a1.y = fmaf(x1, w.y, a1.y); a1.z = fmaf(x1, w.z, a1.z); a1.w = fmaf(x1, w.w, a1.w);
-        }
-        reinterpret_cast<float4 *>(h1s)[lane] =
-            make_float4(fmaxf(a0.x, 0.f), fmaxf(a0.y, 0.f), fmaxf(a0.z, 0.f), fmaxf(a0.w, 0.f));
-        reinterpret_cast<float4 *>(h1s + kH1)[lane] =
-            make_float4(fmaxf(a1.x, 0.f), fmaxf(a1.y, 0.f), fmaxf(a1.z, 0.f), fmaxf(a1.w, 0.f));
-        __syncwarp();
-        // layer 2: units 2*lane, 2*lane + 1
-        float2 c0 = reinterpret_cast<const float2 *>(b2)[lane], c1 = c0;
-#pragma unroll 8
-        for (int k = 0; k < kH1; k++)
-        {
-            const float2 w = reinterpret_cast<const float2 *>(W2 + (size_t)k * kH2)[lane];
-            const float x0 = h1s[k], x1 = h1s[kH1 + k];
-            c0.x = fmaf(x0, w.x, c0.x); c0.y = fmaf(x0, w.y, c0.y);
-            c1.x = fmaf(x1, w.x, c1.x); c1.y = fmaf(x1, w.y, c1.y);
-        }
-        reinterpret_cast<float2 *>(h2s)[lane] = make_float2(fmaxf(c0.x, 0.f), fmaxf(c0.y, 0.f));
-        reinterpret_cast<float2 *>(h2s + kH2)[lane] = make_float2(fmaxf(c1.x, 0.f), fmaxf(c1.y, 0.f));
-        __syncwarp();
-        // layer 3: inputs lane and lane + 32, warp sums
-        float o0[kOut], o1[kOut];
+            float4 acc[8][2];
 #pragma unroll
-        for (int j = 0; j < kOut; j++)
-        {
-            const float wa = W3[lane * kOut + j], wb = W3[(lane + 32) * kOut + j];
-            o0[j] = h2s[lane] * wa + h2s[lane + 32] * wb;
-            o1[j] = h2s[kH2 + lane] * wa + h2s[kH2 + lane + 32] * wb;
-        }
-#pragma unroll
-        for (int j = 0; j < kOut; j++)
-        {
-            for (int o = 16; o > 0; o >>= 1)
+            for (int r = 0; r < 8; r++) acc[r][0] = acc[r][1] = make_float4(0.f, 0.f, 0.f, 0.f);
+            for (int c = 0; c < kIn / kInferChunk; c++)
             {
-                o0[j] += __shfl_xor_sync(0xFFFFFFFFu, o0[j], o);
-                o1[j] += __shfl_xor_sync(0xFFFFFFFFu, o1[j], o);
+                if (first) asm volatile("cp.async.wait_group 1;" ::: "memory");
+                else asm volatile("cp.async.wait_group 0;" ::: "memory");
+                first = false;
+                __syncthreads();  // chunk c is here; every thread is done with chunk c - 1
+                if (c + 1 < kIn / kInferChunk)
+                {
+                    load(tile, c + 1);
+                    commit();
+                }
+                const float *xc = &S.xs[c & 1][rb][0];
+#pragma unroll 1
+                for (int k = 32 * q; k < 32 * q + 32; k += 4)
+                {
+                    float4 x[8];
+#pragma unroll
+                    for (int r = 0; r < 8; r++) x[r] = *reinterpret_cast<const float4 *>(xc + r * kInferChunk + k);
+#pragma unroll
+                    for (int i = 0; i < 4; i++)
+                    {
+                        const float *w = &S.w1[c * kInferChunk + k + i][4 * cg];
+                        const float4 wa = *reinterpret_cast<const float4 *>(w);
+                        const float4 wb = *reinterpret_cast<const float4 *>(w + kH1 / 2);
+#pragma unroll
+                        for (int r = 0; r < 8; r++)
+                        {
+                            const float xv = i == 0 ? x[r].x : i == 1 ? x[r].y : i == 2 ? x[r].z : x[r].w;
+                            fma4(acc[r][0], xv, wa);
+                            fma4(acc[r][1], xv, wb);
+                        }
+                    }
+                }
+            }
+            if (q == 1)
+#pragma unroll
+                for (int r = 0; r < 8; r++)
+#pragma unroll
+                    for (int h = 0; h < 2; h++)
+                        *reinterpret_cast<float4 *>(&S.h1[rb + r][64 * h + 4 * cg]) = acc[r][h];
+            __syncthreads();
+            // the first chunk's buffer is free: the next tile's first chunk arrives under layers 2 and 3
+            if (tile + gridDim.x < ntiles)
+            {
+                load(tile + gridDim.x, 0);
+                commit();
+            }
+            if (q == 0)
+#pragma unroll
+                for (int h = 0; h < 2; h++)
+                {
+                    const float4 b = *reinterpret_cast<const float4 *>(&S.b[64 * h + 4 * cg]);
+#pragma unroll
+                    for (int r = 0; r < 8; r++)
+                    {
+                        float4 *p = reinterpret_cast<float4 *>(&S.h1[rb + r][64 * h + 4 * cg]);
+                        *p = relu4(acc[r][h], *p, b);
+                    }
+                }
+            __syncthreads();
+        }
+        // layer 2: 8 x 4 outputs a thread, half of the inputs; its sums and then
+        // its result take the second chunk's buffer
+        float(*h2)[kH2] = S.xs[1];
+        {
+            float4 acc[8];
+#pragma unroll
+            for (int r = 0; r < 8; r++) acc[r] = make_float4(0.f, 0.f, 0.f, 0.f);
+#pragma unroll 2
+            for (int k = 64 * q; k < 64 * q + 64; k += 4)
+            {
+                float4 w[4];
+#pragma unroll
+                for (int i = 0; i < 4; i++) w[i] = *reinterpret_cast<const float4 *>(&S.w2[k + i][4 * cg]);
+#pragma unroll
+                for (int r = 0; r < 8; r++)
+                {
+                    const float4 x = *reinterpret_cast<const float4 *>(&S.h1[rb + r][k]);
+                    fma4(acc[r], x.x, w[0]);
+                    fma4(acc[r], x.y, w[1]);
+                    fma4(acc[r], x.z, w[2]);
+                    fma4(acc[r], x.w, w[3]);
+                }
+            }
+            if (q == 1)
+#pragma unroll
+                for (int r = 0; r < 8; r++) *reinterpret_cast<float4 *>(&h2[rb + r][4 * cg]) = acc[r];
+            __syncthreads();
+            if (q == 0)
+            {
+                const float4 b = *reinterpret_cast<const float4 *>(&S.b[kH1 + 4 * cg]);
+#pragma unroll
+                for (int r = 0; r < 8; r++)
+                {
+                    float4 *p = reinterpret_cast<float4 *>(&h2[rb + r][4 * cg]);
+                    *p = relu4(acc[r], *p, b);
+                }
+            }
+            __syncthreads();
+        }
+        // layer 3: four lanes a row
+        {
+            const int r = tid >> 2, i = tid & 3;
+            // short sums added pairwise: they round less than one long one
+            float4 o4[4];
+#pragma unroll
+            for (int j = 0; j < kH2 / 16; j++)
+            {
+                o4[j] = make_float4(0.f, 0.f, 0.f, 0.f);
+                const float4 x = *reinterpret_cast<const float4 *>(&h2[r][4 * (i + 4 * j)]);
+                const float4 *w = reinterpret_cast<const float4 *>(&S.w3[4 * (i + 4 * j)][0]);
+                fma4(o4[j], x.x, w[0]);
+                fma4(o4[j], x.y, w[1]);
+                fma4(o4[j], x.z, w[2]);
+                fma4(o4[j], x.w, w[3]);
+            }
+            float4 o = make_float4((o4[0].x + o4[1].x) + (o4[2].x + o4[3].x), (o4[0].y + o4[1].y) + (o4[2].y + o4[3].y),
+                                   (o4[0].z + o4[1].z) + (o4[2].z + o4[3].z), (o4[0].w + o4[1].w) + (o4[2].w + o4[3].w));
+#pragma unroll
+            for (int d = 1; d < 4; d <<= 1)
+            {
+                o.x += __shfl_xor_sync(0xFFFFFFFFu, o.x, d);
+                o.y += __shfl_xor_sync(0xFFFFFFFFu, o.y, d);
+                o.z += __shfl_xor_sync(0xFFFFFFFFu, o.z, d);
+                o.w += __shfl_xor_sync(0xFFFFFFFFu, o.w, d);
+            }
+            const uint32_t row = tile * kInferTile + (uint32_t)r;
+            if (row < n)
+                out[(size_t)row * kOut + i] = (i == 0 ? o.x : i == 1 ? o.y : i == 2 ? o.z : o.w) + S.b[kH1 + kH2 + i];
+        }
+    }
+}
+
+struct InferRowsSmem
+{
+    float xs[kInferRows][kIn];
+    float red[16][kInferRows][kH1];  // a warp's sums (layer 2's in the first half)
+    float h1[kInferRows][kH1];
+    float h2[kInferRows][kH2];
+};
+
+__global__ void __launch_bounds__(kRowsThreads, 2) k_infer_rows(const float *__restrict__ P, const float *__restrict__ X,
+                                                                 uint32_t n, float *__restrict__ out)
+{
+    extern __shared__ __align__(16) unsigned char ism[];
+    InferRowsSmem &S = *reinterpret_cast<InferRowsSmem *>(ism);
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    const uint32_t r0 = blockIdx.x * kInferRows;
+    {
+        const uint32_t row = r0 + (uint32_t)(tid >> 6);
+        reinterpret_cast<float4 *>(&S.xs[0][0])[tid] =
+            row < n ? __ldg(reinterpret_cast<const float4 *>(X + (size_t)row * kIn) + (tid & 63))
+                    : make_float4(0.f, 0.f, 0.f, 0.f);
+    }
+    __syncthreads();
+    {
+        const float4 *w1 = reinterpret_cast<const float4 *>(P + kOffW1) + lane;
+        float4 acc[kInferRows];
+#pragma unroll
+        for (int r = 0; r < kInferRows; r++) acc[r] = make_float4(0.f, 0.f, 0.f, 0.f);
+#pragma unroll 1
+        for (int k = 16 * warp; k < 16 * warp + 16; k += 4)
+        {
+            float4 w[4];
+#pragma unroll
+            for (int i = 0; i < 4; i++) w[i] = __ldg(w1 + (k + i) * (kH1 / 4));
+#pragma unroll
+            for (int r = 0; r < kInferRows; r++)
+            {
+                const float4 x = *reinterpret_cast<const float4 *>(&S.xs[r][k]);
+                fma4(acc[r], x.x, w[0]);
+                fma4(acc[r], x.y, w[1]);
+                fma4(acc[r], x.z, w[2]);
+                fma4(acc[r], x.w, w[3]);
             }
         }
-        if (lane < kOut) out[(size_t)s0 * kOut + lane] = o0[lane] + b3[lane];
-        if (lane < kOut && s1 != s0) out[(size_t)s1 * kOut + lane] = o1[lane] + b3[lane];
-        __syncwarp();
+#pragma unroll
+        for (int r = 0; r < kInferRows; r++) *reinterpret_cast<float4 *>(&S.red[warp][r][4 * lane]) = acc[r];
+    }
+    // this warp's eighth rows of layer 2's weights, loaded ahead of the sums
+    float2 w2[8];
+#pragma unroll
+    for (int i = 0; i < 8; i++) w2[i] = __ldg(reinterpret_cast<const float2 *>(P + kOffW2 + (8 * warp + i) * kH2) + lane);
+    __syncthreads();
+#pragma unroll
+    for (int j = 0; j < kInferRows * kH1 / kRowsThreads; j++)
+    {
+        const int i = tid + j * kRowsThreads;
+        const float *p = &S.red[0][0][0] + i;
+        float v = 0.0f;
+#pragma unroll
+        for (int w = 0; w < 16; w++) v += p[w * kInferRows * kH1];
+        (&S.h1[0][0])[i] = fmaxf(v + __ldg(P + kOffB1 + i % kH1), 0.0f);
+    }
+    __syncthreads();
+    float *red2 = &S.red[0][0][0];  // [16][rows][kH2]
+#pragma unroll
+    for (int r = 0; r < kInferRows; r++)
+    {
+        float2 a = make_float2(0.f, 0.f);
+#pragma unroll
+        for (int i = 0; i < 8; i++)
+        {
+            const float x = S.h1[r][8 * warp + i];
+            a.x = fmaf(x, w2[i].x, a.x);
+            a.y = fmaf(x, w2[i].y, a.y);
+        }
+        reinterpret_cast<float2 *>(red2 + (warp * kInferRows + r) * kH2)[lane] = a;
+    }
+    __syncthreads();
+    {
+        float v = 0.0f;
+#pragma unroll
+        for (int w = 0; w < 16; w++) v += red2[w * kInferRows * kH2 + tid];
+        (&S.h2[0][0])[tid] = fmaxf(v + __ldg(P + kOffB2 + tid % kH2), 0.0f);
+    }
+    __syncthreads();
+    // layer 3: a warp's lanes per row, two inputs each
+    if (warp < kInferRows)
+    {
+        float4 o = make_float4(0.f, 0.f, 0.f, 0.f);
+#pragma unroll
+        for (int j = 0; j < 2; j++)
+            fma4(o, S.h2[warp][lane + 32 * j], __ldg(reinterpret_cast<const float4 *>(P + kOffW3) + lane + 32 * j));
+#pragma unroll
+        for (int d = 1; d < 32; d <<= 1)
+        {
+            o.x += __shfl_xor_sync(0xFFFFFFFFu, o.x, d);
+            o.y += __shfl_xor_sync(0xFFFFFFFFu, o.y, d);
+            o.z += __shfl_xor_sync(0xFFFFFFFFu, o.z, d);
+            o.w += __shfl_xor_sync(0xFFFFFFFFu, o.w, d);
+        }
+        const uint32_t row = r0 + (uint32_t)warp;
+        if (lane < kOut && row < n)
+            out[(size_t)row * kOut + lane] =
+                (lane == 0 ? o.x : lane == 1 ? o.y : lane == 2 ? o.z : o.w) + __ldg(P + kOffB3 + lane);
     }
 }
 
@@ -777,15 +1026,25 @@ __global__ void __launch_bounds__(kLtWarps * 32) k_learned_tail(const uint32_t *
 
 }  // namespace
 
-// the fused inference kernel (no activations kept)
+// the fused inference kernels (no activations kept)
 static int mlp_infer(hc_mlp *m, const float *X, uint32_t n, float *out, cudaStream_t st)
 {
     if (n == 0) return HC_SUCCESS;
-    static_assert(kParams % 4 == 0, "parameters are staged as float4");
-    HC_CUDA(m->ctx, cudaFuncSetAttribute(k_mlp_infer, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kInferSmem));
-    const uint32_t pairs = (n + 1) / 2;
-    const uint32_t blocks = std::min<uint32_t>((pairs + kInferWarps - 1) / kInferWarps, (uint32_t)m->ctx->sm_count);
-    k_mlp_infer<<<blocks, kInferWarps * 32, kInferSmem, st>>>(m->d_params, X, n, out);
+    if (n <= kInferRowsPerSm * (uint32_t)m->ctx->sm_count)
+    {
+        HC_CUDA(m->ctx, cudaFuncSetAttribute(k_infer_rows, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                             (int)sizeof(InferRowsSmem)));
+        k_infer_rows<<<(n + kInferRows - 1) / kInferRows, kRowsThreads, sizeof(InferRowsSmem), st>>>(m->d_params, X, n,
+                                                                                                     out);
+    }
+    else
+    {
+        HC_CUDA(m->ctx, cudaFuncSetAttribute(k_infer_tile, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                             (int)sizeof(InferSmem)));
+        const uint32_t tiles = (n + kInferTile - 1) / kInferTile;
+        k_infer_tile<<<std::min(tiles, (uint32_t)m->ctx->sm_count), kTileThreads, sizeof(InferSmem), st>>>(m->d_params,
+                                                                                                             X, n, out);
+    }
     HC_CUDA(m->ctx, cudaGetLastError());
     return HC_SUCCESS;
 }

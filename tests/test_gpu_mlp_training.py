@@ -66,3 +66,46 @@ def test_training_follows_float64_adam(n, batch):
     assert abs(loss - np.mean(losses)) <= 1e-3 * max(1.0, abs(np.mean(losses)))
     m.close()
     ix.close()
+
+
+@pytest.mark.parametrize("n", [1, 7, 8, 9, 4864, 4865, 9728, 9791, 10001])
+def test_inference_at_tile_edges(n):
+    """Both inference kernels at the edges of their tiles and of the line between them
+    (32 spectra per SM of a 152-SM part), and nothing written past the last spectrum.
+    256 + 128 + 64 FP32 terms: within 448 * 2^-24 of the largest output."""
+    import torch
+    from hicops_gb300 import dslim
+    ix = dslim.Index(S.SearchParams(maxz=2))
+    m = dslim.MLP(ix, seed=13)
+    X, Y = _data(n, n + 2)
+    dX = torch.from_numpy(X).cuda()
+    out = torch.full((n * 4 + 65,), 7.0, dtype=torch.float32, device="cuda")
+    torch.cuda.synchronize()
+    for at in (0, 1):  # the outputs may start at any float
+        m.forward(dX.data_ptr(), n, out.data_ptr() + 4 * at)
+        torch.cuda.synchronize()
+        o = out.cpu().numpy()
+        _, _, o64 = _np_forward_backward(m.params().astype(np.float64), X.astype(np.float64), Y.astype(np.float64))
+        assert np.abs(o[at:at + 4 * n].reshape(n, 4) - o64).max() <= 448 * 2.0 ** -24 * np.abs(o64).max()
+        assert (o[at + 4 * n:] == 7.0).all()
+    m.close()
+    ix.close()
+
+
+def test_gradients_of_inputs_at_any_float():
+    """Inputs that start 4 bytes past a 16-byte boundary give the same gradients."""
+    import torch
+    from hicops_gb300 import dslim
+    ix = dslim.Index(S.SearchParams(maxz=2))
+    m = dslim.MLP(ix, seed=9)
+    X, Y = _data(70, 1)
+    dY = torch.from_numpy(Y).cuda()
+    buf = torch.zeros(70 * 256 + 4, dtype=torch.float32, device="cuda")
+    g = []
+    for at in (0, 1):
+        buf[at:at + 70 * 256] = torch.from_numpy(X).reshape(-1).cuda()
+        torch.cuda.synchronize()
+        g.append(m.gradients(buf.data_ptr() + 4 * at, dY.data_ptr(), 70)[0])
+    assert np.array_equal(g[0], g[1])
+    m.close()
+    ix.close()
