@@ -59,4 +59,61 @@ __device__ __forceinline__ int tail_bins(const uint32_t *__restrict__ yy, int hy
     return n;
 }
 
+// The same bins and, in cum[q], the cumulative counts of bins 0 .. q for every
+// bin up to the last point (the bins before the first point are empty, so
+// these are its cumulative counts too). One pass over the bins up to the top
+// hit's, four groups of 32 in flight.
+__device__ __forceinline__ int tail_curve(const uint32_t *__restrict__ yy, int hyp, int nbins, int lane, uint32_t *cum,
+                                          int &stt1, int &end1)
+{
+    const int lim = hyp < nbins ? hyp + 1 : nbins;  // the bin after a single one may be the top hit's own
+    int first = -1, last = -1;
+    uint32_t carry = 0;
+    for (int q0 = 0; q0 < lim; q0 += 128)
+    {
+        uint32_t v[4];
+#pragma unroll
+        for (int j = 0; j < 4; j++)
+        {
+            const int q = q0 + 32 * j + lane;
+            v[j] = q < lim ? __ldg(yy + q) : 0u;
+        }
+#pragma unroll
+        for (int j = 0; j < 4; j++)
+        {
+            const int q = q0 + 32 * j + lane;
+            const uint32_t b = __ballot_sync(0xFFFFFFFFu, q < hyp && v[j] != 0u);
+            if (b)
+            {
+                if (first < 0) first = q0 + 32 * j + __ffs(b) - 1;
+                last = q0 + 32 * j + 31 - __clz(b);
+            }
+        }
+#pragma unroll
+        for (int o = 1; o < 32; o <<= 1)
+#pragma unroll
+            for (int j = 0; j < 4; j++)
+            {
+                const uint32_t t = __shfl_up_sync(0xFFFFFFFFu, v[j], o);
+                if (lane >= o) v[j] += t;
+            }
+#pragma unroll
+        for (int j = 0; j < 4; j++)
+        {
+            const int q = q0 + 32 * j + lane;
+            v[j] += carry;
+            if (q < lim) cum[q] = v[j];
+            carry = __shfl_sync(0xFFFFFFFFu, v[j], 31);
+        }
+    }
+    __syncwarp();
+    stt1 = first < 0 ? 0 : first;
+    end1 = last < 0 ? hyp - 1 : last;
+    if (stt1 == end1) end1 += 1;
+    int n = end1 - stt1 + 1;
+    if (n < 0) n = 0;
+    if (stt1 + n > nbins) n = nbins - stt1;
+    return n;
+}
+
 }  // namespace hc

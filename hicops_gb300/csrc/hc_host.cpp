@@ -195,6 +195,12 @@ void make_query_const(QueryConst *q)
         q->lgfact[i] = std::log10((double)i) + q->lgfact[i - 1];
     for (int i = 0; i < kLgTable; i++)
         q->lgfact_f[i] = (float)q->lgfact[i];
+    for (int i = 0; i < kLgTab; i++)
+    {
+        const double inv = 1.0 / (1.0 + (i + 0.5) / kLgTab);
+        q->lg_tab[2 * i] = inv;
+        q->lg_tab[2 * i + 1] = (double)-std::log10((long double)inv);
+    }
     q->log10_tab = nullptr;
 }
 

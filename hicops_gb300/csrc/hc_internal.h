@@ -96,10 +96,15 @@ struct IonTables
 
 constexpr uint32_t kLog10Tab = 1u << 24;  // log10(n) for every n the packed sums can reach
 
+// Table of the tail fit's logarithm: for 128 intervals of the mantissa the
+// reciprocal of the midpoint and minus its log10.
+constexpr int kLgTab = 128;
+
 struct QueryConst
 {
     double lgfact[kLgTable];   // log10(n!) exactly as utils.h:115-131 builds it
     float lgfact_f[kLgTable];  // the same, rounded to float (fast path)
+    double lg_tab[2 * kLgTab];
     const double *log10_tab;   // device table: log10_tab[n] = log10(n), n < kLog10Tab (host libm values)
 };
 

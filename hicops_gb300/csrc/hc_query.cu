@@ -1327,9 +1327,8 @@ __global__ void k_windows(const LenDev *__restrict__ lens, uint32_t nlen, const 
 }
 
 // ---- tail fit + e-value ------------------------------------------------------
-constexpr int kTfWarps = 4;
-
-// expeRT::ModelTailFit (expeRT.cpp:572-718) and e(x) (dslim_query.cpp:773-799)
+// The plain form, for the spectra whose result k_tailfit's shorter arithmetic
+// leaves open: expeRT::ModelTailFit (expeRT.cpp:572-718) and e(x) (dslim_query.cpp:773-799)
 // of spectrum s, by one warp. Elementwise steps run across lanes; the sums
 // whose rounding depends on order (ybar, top, bot of LinearFit) run on lane 0
 // in the reference's order. Cumulative sums are exact integers either way.
@@ -1485,23 +1484,320 @@ __device__ void tailfit_one(uint32_t s, hc_result *__restrict__ out, const uint3
     }
 }
 
-// One warp per spectrum: every spectrum of [0, nspec), or those of `list`
-// (its length *nlist read on the device) when a list is given.
-__global__ void __launch_bounds__(kTfWarps * 32) k_tailfit(hc_result *__restrict__ out,
-                                                          const uint32_t *__restrict__ hist,
-                                                          uint32_t nspec, uint32_t min_cpsm,
-                                                          double expect_max, int32_t *__restrict__ fitstart,
-                                                          const uint32_t *__restrict__ list,
-                                                          const uint32_t *__restrict__ nlist)
+// k_tailfit. This part's FP64 rate is 1/64 of its FP32 rate (a warp's FP64
+// instruction takes the SM's pipe 16 clocks, whatever its active lanes), so
+// the fit is arranged around it:
+//   - the regression window is found on an FP32 curve; FP64 decides only the
+//     points that lie within kTfNear of a level;
+//   - FP64 logarithms are taken of the window's points alone, with a table
+//     and a degree-6 polynomial (P. T. P. Tang, "Table-driven implementation of
+//     the logarithm function in IEEE floating-point arithmetic", 1990), and the
+//     quotients by one reciprocal per spectrum and a corrected product
+//     (P. Markstein, "Computation of elementary functions on the IBM RISC
+//     System/6000 processor", 1990: the correctly rounded quotient);
+//   - the abscissae are consecutive integers, so their sums are closed forms,
+//     and the two sums left run across the lanes;
+//   - what follows once per spectrum (the quotients, the power) runs with a
+//     lane per spectrum, sixteen spectra at a time.
+// The line is (mu, beta) x 1e6 truncated to integers, so a result that differs
+// in its last bits is the same result unless a value lies near an integer (or
+// a point on a level): those spectra, about 1 in 10^4, are fitted again by
+// tailfit_one, in the reference's own order of operations. Results are therefore
+// tailfit_one's, bit for bit. 2,000 spectra of an open search: 23 us,
+// against 183 us with every point in FP64 and the sums on one lane.
+constexpr int kTfWarps = 16;
+constexpr float kTfNear = 5e-5f;      // FP32 curve and level: together within 5e-6 of FP64's
+constexpr double kTfLevel = 1e-9;     // the short FP64 logarithm: within 1e-14
+constexpr double kTfInteger = 1e-5;   // mu, beta x 1e6: within 5e-6 of tailfit_one's
+
+struct TfJob
 {
-    __shared__ double sxs[kTfWarps][HC_HIST_BINS + 2];
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    double *sx = sxs[warp];  // sx[0] stands for index -1; element i is sx[i + 1]
-    const uint32_t cnt = list ? min(*nlist, nspec) : nspec;
-    for (uint32_t w = blockIdx.x * kTfWarps + warp; w < cnt; w += gridDim.x * kTfWarps)
+    double sy, sxy, yf;   // sums of y - yf and of (x - xbar) y over the window, yf its first point
+    uint32_t s, fl;
+    int status, m, first, stt1, end1, hyp;
+};
+
+enum TfStatus
+{
+    kTfNone = 0,   // nothing (left) to do
+    kTfFit = 1,    // the window's sums are there
+    kTfAgain = 2,  // to be fitted by tailfit_one
+    kTfEmpty = 3,  // no point
+};
+
+struct TfSmem
+{
+    double sx[HC_HIST_BINS + 2];  // tailfit_one's
+    double2 tab[kLgTab];
+    TfJob job[kTfWarps];
+    uint32_t cum[kTfWarps][HC_HIST_BINS];
+};
+
+// log10 of a positive normal double up to 1, within 4e-15
+__device__ __forceinline__ double lg10_short(double d, const double2 *tab)
+{
+    const int hi = __double2hiint(d);
+    const double2 t = tab[(hi >> 13) & (kLgTab - 1)];
+    const double mant = __hiloint2double((hi & 0x000FFFFF) | 0x3FF00000, __double2loint(d));
+    const double r = fma(mant, t.x, -1.0);  // |r| < 2^-8 (1 + 2^-7)
+    double p = fma(r, -0.07238241365054197128, 0.08685889638065036553);
+    p = fma(r, p, -0.10857362047581295691);
+    p = fma(r, p, 0.14476482730108394255);
+    p = fma(r, p, -0.21714724095162591383);
+    p = fma(r, p, 0.43429448190325182765);
+    return fma(r, p, fma((double)((hi >> 20) - 1023), 0.30102999566398119521, t.y));
+}
+
+// A spectrum's survival curve, s(i) = 1 - cum / cpsms (expeRT.cpp:625-636), its
+// values of 0 replaced by the last one of 1e-4 or more (639-640).
+struct TfCurve
+{
+    const uint32_t *c;  // cumulative counts of the points
+    uint32_t cps, crep; // crep: the count whose value replaces those at or past cps
+    float invf;
+    double cd, inv;
+    __device__ __forceinline__ double value(uint32_t x) const
     {
-        tailfit_one(list ? list[w] : w, out, hist, min_cpsm, expect_max, fitstart, sx, lane);
-        __syncwarp();
+        const double xd = (double)x;
+        double q = __dmul_rn(xd, inv);
+        q = fma(fma(-q, cd, xd), inv, q);  // the correctly rounded x / cps
+        return __dadd_rn(1.0, -q);
+    }
+    __device__ __forceinline__ uint32_t count(int i) const { return c[i] < cps ? c[i] : crep; }
+    __device__ __forceinline__ float lgf(int i) const
+    {
+        return __log2f((float)(cps - count(i)) * invf) * 0.30102999566f;
+    }
+    __device__ __forceinline__ double lg(int i, const double2 *tab) const { return lg10_short(value(count(i)), tab); }
+};
+
+// The sums of spectrum s's regression window, by one warp (see k_tailfit).
+__device__ __forceinline__ void tailfit_sums(uint32_t s, const hc_result &r, const uint32_t *__restrict__ hist, int hyp,
+                                             uint32_t *cum, const double2 *tab, TfJob &job, int lane)
+{
+    int stt1, end1;
+    const int n = tail_curve(hist + (size_t)s * HC_HIST_BINS, hyp, HC_HIST_BINS, lane, cum, stt1, end1);
+    int status = kTfFit, mark = 0, mark2 = n - 1, m = 0;
+    double sy = 0.0, sxy = 0.0, yf = 0.0;
+    if (n == 0) status = kTfEmpty;
+    else
+    {
+        TfCurve cv;
+        cv.c = cum + stt1;
+        cv.cps = r.cpsms;
+        cv.crep = 0;
+        cv.invf = 1.0f / (float)r.cpsms;
+        cv.cd = (double)r.cpsms;
+        cv.inv = __drcp_rn(cv.cd);
+        if (cv.c[n - 1] >= cv.cps)  // the counts ascend: the only case with a value of 0 (or below)
+        {
+            status = kTfAgain;
+            for (int q0 = n - 1; q0 >= 0; q0 -= 32)
+            {
+                const int q = q0 - lane;
+                const uint32_t b = __ballot_sync(0xFFFFFFFFu, q >= 0 && cv.c[q] < cv.cps && cv.value(cv.c[q]) >= 1e-4);
+                if (b)
+                {
+                    cv.crep = cv.c[q0 - (__ffs(b) - 1)];
+                    status = kTfFit;
+                    break;
+                }
+            }
+        }
+        // regression window (expeRT.cpp:646-684)
+        if (status == kTfFit && n >= 3)
+        {
+            const double ye = lane < 2 ? cv.lg(lane ? n - 1 : 0, tab) : 0.0;
+            const double y0 = __shfl_sync(0xFFFFFFFFu, ye, 0), hgt = __dadd_rn(__shfl_sync(0xFFFFFFFFu, ye, 1), -y0);
+            const double t1 = __dadd_rn(y0, __dmul_rn(hgt, 0.22));
+            const float t1f = (float)t1;
+            bool open = false;
+            int lm = 0;
+            for (int q0 = 0; q0 < n; q0 += 32)
+            {
+                const int q = q0 + lane;
+                const float y = q < n ? cv.lgf(q) : 1.0f;
+                bool in = y <= t1f;
+                if (__any_sync(0xFFFFFFFFu, fabsf(y - t1f) < kTfNear) && fabsf(y - t1f) < kTfNear)
+                {
+                    const double yd = cv.lg(q, tab);
+                    in = yd <= t1;
+                    open |= fabs(yd - t1) < kTfLevel;
+                }
+                const uint32_t b = __ballot_sync(0xFFFFFFFFu, q < n && in);
+                if (b)
+                {
+                    lm = q0 + __ffs(b) - 1;
+                    break;
+                }
+            }
+            mark = lm - 1;
+            if (n > 3)
+            {
+                const double t2 = __dadd_rn(y0, __dmul_rn(hgt, 0.87));
+                const float t2f = (float)t2;
+                for (int q0 = n - 1; q0 >= 0; q0 -= 32)
+                {
+                    const int q = q0 - lane;
+                    const float y = q >= 0 ? cv.lgf(q) : -1e9f;
+                    bool in = y >= t2f;
+                    if (fabsf(y - t2f) < kTfNear)
+                    {
+                        const double yd = cv.lg(q, tab);
+                        in = yd >= t2;
+                        open |= fabs(yd - t2) < kTfLevel;
+                    }
+                    const uint32_t b = __ballot_sync(0xFFFFFFFFu, q >= 0 && in);
+                    if (b)
+                    {
+                        mark2 = q0 - (__ffs(b) - 1);
+                        break;
+                    }
+                }
+            }
+            if (mark >= mark2) mark = mark2 - 1;
+            if (__any_sync(0xFFFFFFFFu, open)) status = kTfAgain;
+        }
+        m = mark2 - mark + 1;
+        if (status == kTfFit)
+        {
+            // element -1 reads as 0 (see tailfit_one)
+            double dx = (double)(2 * lane - (m - 1)) * 0.5;
+            for (int j0 = 0; j0 < m; j0 += 32)
+            {
+                const int j = j0 + lane;
+                const double y = j < m && mark + j >= 0 ? cv.lg(mark + j, tab) : 0.0;
+                if (j0 == 0) yf = __shfl_sync(0xFFFFFFFFu, y, 0);
+                if (j < m)
+                {
+                    const double v = y - yf;
+                    sy += v;
+                    sxy = fma(dx, v, sxy);
+                }
+                dx += 32.0;
+            }
+#pragma unroll
+            for (int o = 16; o > 0; o >>= 1)
+            {
+                sy += __shfl_xor_sync(0xFFFFFFFFu, sy, o);
+                sxy += __shfl_xor_sync(0xFFFFFFFFu, sxy, o);
+            }
+        }
+    }
+    if (lane == 0)
+    {
+        job.sy = sy;
+        job.sxy = sxy;
+        job.yf = yf;
+        job.s = s;
+        job.fl = status == kTfEmpty ? HC_FLAG_TAILFIT_EMPTY : (mark < 0 ? HC_FLAG_TAILFIT_OOB : 0u);
+        job.status = status;
+        job.m = m;
+        job.first = n ? stt1 + mark : -1;
+        job.stt1 = stt1;
+        job.end1 = end1;
+        job.hyp = hyp;
+    }
+}
+
+// The line and the e-value of a job, one lane each; false when a value's
+// truncation is left open (nothing is written then).
+__device__ __forceinline__ bool tailfit_line(const TfJob &j, hc_result *__restrict__ out, double expect_max,
+                                             int32_t *__restrict__ fitstart)
+{
+    double mu_t, beta_t;  // x 1e6
+    if (j.status == kTfEmpty) mu_t = beta_t = __longlong_as_double(0x7FF8000000000000ll);  // LinearFit of 0 points: 0/0
+    else
+    {
+        const double m = (double)j.m, xbar = (double)j.first + 0.5 * (m - 1.0);
+        const double ybar = j.yf + j.sy / m;
+        // sum of (x - xbar)^2 over m consecutive integers: m (m^2 - 1) / 12
+        const double bot = 0.25 * (double)(((uint32_t)j.m * ((uint32_t)j.m * (uint32_t)j.m - 1u)) / 3u);
+        const double mu = j.m == 1 ? 0.0 : j.sxy / bot;
+        mu_t = mu * 1e6;
+        beta_t = (ybar - mu * xbar) * 1e6;
+        // (a value that truncates to 0 from either side is not open)
+        const bool open = !(fabs(mu_t) < 1e9) || !(fabs(beta_t) < 1e9) ||
+                          (fabs(mu_t) > 0.5 && fabs(mu_t - rint(mu_t)) < kTfInteger) ||
+                          (fabs(beta_t) > 0.5 && fabs(beta_t - rint(beta_t)) < kTfInteger);
+        if (open) return false;
+    }
+    hc_result r = out[j.s];
+    fitstart[j.s] = j.first;
+    r.flags |= j.fl;
+    r.mu = x86_d2i(mu_t);
+    r.beta = x86_d2i(beta_t);
+    r.minhyp = j.stt1;
+    r.nexthyp = j.end1;
+    r.maxhyp = j.hyp;
+    // e(x) = 10^(w*maxhyp + b) * cpsms (dslim_query.cpp:786-799)
+    const double wv = __ddiv_rn((double)r.mu, 1e6), bv = __ddiv_rn((double)r.beta, 1e6);
+    const double lgs = __dadd_rn(__dmul_rn(wv, (double)j.hyp), bv);
+    double e = pow(10.0, lgs);
+    e = __dmul_rn(e, (double)r.cpsms);
+    r.evalue = e;
+    r.reported = e < expect_max ? 1u : 0u;
+    out[j.s] = r;
+    return true;
+}
+
+// One warp per spectrum, then one lane per spectrum: every spectrum of
+// [0, nspec), or those of `list` (its length *nlist read on the device) when a
+// list is given.
+__global__ void __launch_bounds__(kTfWarps * 32, 2) k_tailfit(const QueryConst *__restrict__ qc,
+                                                             hc_result *__restrict__ out,
+                                                             const uint32_t *__restrict__ hist, uint32_t nspec,
+                                                             uint32_t min_cpsm, double expect_max,
+                                                             int32_t *__restrict__ fitstart,
+                                                             const uint32_t *__restrict__ list,
+                                                             const uint32_t *__restrict__ nlist)
+{
+    extern __shared__ __align__(16) unsigned char tsm[];
+    TfSmem &S = *reinterpret_cast<TfSmem *>(tsm);
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const uint32_t cnt = list ? min(*nlist, nspec) : nspec;
+    if (blockIdx.x * kTfWarps >= cnt) return;
+    for (int i = threadIdx.x; i < kLgTab; i += kTfWarps * 32) S.tab[i] = make_double2(qc->lg_tab[2 * i], qc->lg_tab[2 * i + 1]);
+    __syncthreads();
+    for (uint32_t w0 = blockIdx.x * kTfWarps; w0 < cnt; w0 += gridDim.x * kTfWarps)
+    {
+        TfJob &job = S.job[warp];
+        if (lane == 0) job.status = kTfNone;
+        if (w0 + warp < cnt)
+        {
+            const uint32_t s = list ? list[w0 + warp] : w0 + warp;
+            hc_result r = out[s];
+            if (r.cpsms < min_cpsm || r.cpsms == 0)
+            {
+                if (lane == 0)
+                {
+                    r.mu = r.beta = r.minhyp = r.nexthyp = r.maxhyp = 0;
+                    r.evalue = 0.0;
+                    r.reported = 0;
+                    out[s] = r;
+                    fitstart[s] = -1;
+                }
+            }
+            else
+                tailfit_sums(s, r, hist, hist_bin(r.hyperscore), S.cum[warp], S.tab, job, lane);
+        }
+        __syncthreads();
+        if (warp == 0)
+        {
+            bool again = false;
+            if (lane < kTfWarps)
+            {
+                const TfJob &j = S.job[lane];
+                again = j.status == kTfAgain;
+                if (j.status == kTfFit || j.status == kTfEmpty) again = !tailfit_line(j, out, expect_max, fitstart);
+            }
+            for (uint32_t b = __ballot_sync(0xFFFFFFFFu, again); b; b &= b - 1)
+            {
+                tailfit_one(S.job[__ffs(b) - 1].s, out, hist, min_cpsm, expect_max, fitstart, S.sx, lane);
+                __syncwarp();
+            }
+        }
+        __syncthreads();
     }
 }
 
@@ -1749,6 +2045,18 @@ static int launch_packed(hc_ctx *ctx, SearchArgs &a, uint32_t sched, uint32_t ns
                                 search_smem(small_tile, s.dF, false, kSmallThreads), 2, st);
 }
 
+// the tail fit of spectra [0, n), or of a list of at most n
+static int launch_tailfit(hc_ctx *ctx, hc_result *out, const uint32_t *hist, uint32_t n, int32_t *fitstart,
+                          const uint32_t *list, const uint32_t *nlist, cudaStream_t st)
+{
+    HC_CUDA(ctx, cudaFuncSetAttribute(k_tailfit, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(TfSmem)));
+    const uint32_t blocks = std::min<uint32_t>((n + kTfWarps - 1) / kTfWarps, 2u * (uint32_t)ctx->sm_count);
+    k_tailfit<<<blocks, kTfWarps * 32, sizeof(TfSmem), st>>>(ctx->d_qconst, out, hist, n, ctx->p.min_cpsm,
+                                                             ctx->p.expect_max, fitstart, list, nlist);
+    HC_CUDA(ctx, cudaGetLastError());
+    return HC_SUCCESS;
+}
+
 int query_device(hc_ctx *ctx, const uint32_t *d_idx, const uint32_t *d_moz, const uint32_t *d_int,
                  const float *d_prec, const double *d_dM, uint32_t nspec, uint32_t npeaks,
                  hc_result *d_out, uint32_t *d_hist, cudaStream_t st, bool tailfit)
@@ -1823,9 +2131,7 @@ int query_device(hc_ctx *ctx, const uint32_t *d_idx, const uint32_t *d_moz, cons
     if (ctx->profiling) HC_CUDA(ctx, record_stage(ctx, 3, st));
     if (tailfit)
     {
-        k_tailfit<<<(nspec + kTfWarps - 1) / kTfWarps, kTfWarps * 32, 0, st>>>(
-            d_out, d_hist, nspec, ctx->p.min_cpsm, ctx->p.expect_max, q.d_fitstart, nullptr, nullptr);
-        HC_CUDA(ctx, cudaGetLastError());
+        if ((rc2 = launch_tailfit(ctx, d_out, d_hist, nspec, q.d_fitstart, nullptr, nullptr, st))) return rc2;
     }
     else
         launches--;
@@ -1889,11 +2195,7 @@ int tailfit_list(hc_ctx *ctx, hc_result *d_out, const uint32_t *d_hist, const ui
     QueryScratch &q = ctx->qs;
     int rc = grow(ctx, &q.d_fitstart, &q.fit_cap, (size_t)nmax);
     if (rc) return rc;
-    const uint32_t blocks = std::min<uint32_t>((nmax + kTfWarps - 1) / kTfWarps, (uint32_t)ctx->sm_count * 16);
-    k_tailfit<<<blocks, kTfWarps * 32, 0, st>>>(d_out, d_hist, nmax, ctx->p.min_cpsm, ctx->p.expect_max,
-                                                q.d_fitstart, list, d_nlist);
-    HC_CUDA(ctx, cudaGetLastError());
-    return HC_SUCCESS;
+    return launch_tailfit(ctx, d_out, d_hist, nmax, q.d_fitstart, list, d_nlist, st);
 }
 
 // The query pipeline of query_device with every scratch buffer supplied by
@@ -1959,10 +2261,7 @@ int launch_query_scratch(hc_ctx *ctx, const uint32_t *d_idx, const uint32_t *d_m
     b.tile = std::max(kRowG, ctx->tuning.tile / 2 / kRowG * kRowG);  // same shared memory, 16-byte words
     rc = launch_search<true>(ctx, b, ctx->sm_count, ctx->tuning.threads, search_smem(b.tile, b.dF, true, ctx->tuning.threads), 2, st);
     if (rc) return rc;
-    k_tailfit<<<(nspec + kTfWarps - 1) / kTfWarps, kTfWarps * 32, 0, st>>>(d_out, d_hist, nspec, ctx->p.min_cpsm,
-                                                                            ctx->p.expect_max, s.fitstart, nullptr,
-                                                                            nullptr);
-    HC_CUDA(ctx, cudaGetLastError());
+    if ((rc = launch_tailfit(ctx, d_out, d_hist, nspec, s.fitstart, nullptr, nullptr, st))) return rc;
     ctx->last_launches = launches + 1;
     return HC_SUCCESS;
 }
