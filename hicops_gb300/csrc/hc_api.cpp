@@ -316,7 +316,7 @@ int hc_dslim_load(hc_ctx *ctx, uint32_t L, const uint8_t *seqs, uint32_t npep, c
     HC_CUDA(ctx, cudaMalloc((void **)&d_ids, 4 * M + 4));
     HC_CUDA(ctx, cudaMemcpy(d_ids, iA, 4 * M, cudaMemcpyHostToDevice));
     lh->npost = M;
-    const int rq = build_query_postings(ctx, *lh, M ? d_ids : nullptr);
+    const int rq = build_query_postings(ctx, *lh, M ? d_ids : nullptr, nullptr);
     cudaFree(d_ids);
     if (rq) return rq;
     lh->built = true;

@@ -494,20 +494,98 @@ __global__ void k_pad_counts(const uint32_t *__restrict__ bA, uint32_t nb, uint3
         pc[b] = b < nb ? ((bA[b + 1] - bA[b] + 3u) & ~3u) : 0u;
 }
 
-// ids (entry*speclen + ion, bucket order) -> query postings and their ions, one thread per bucket
-__global__ void k_qpost(const uint32_t *__restrict__ bA, const uint32_t *__restrict__ ids,
-                        const uint32_t *__restrict__ qA, uint32_t nb, uint32_t speclen, uint32_t half,
-                        uint32_t *__restrict__ qp, uint16_t *__restrict__ qion)
+// Division of the ids by the postings of an entry: multiply and shift below
+// 2^31 ids (division_magic), the plain quotient past it.
+struct IdDiv
+{
+    uint32_t d, magic, sh;
+    bool fast;
+    __device__ __forceinline__ uint32_t operator()(uint32_t x) const { return fast ? __umulhi(x, magic) >> sh : x / d; }
+};
+
+// the charge of a query posting's ion when it is a y1 ion, else -1;
+// ion = series * half + charge * (L - 1) + position
+__device__ __forceinline__ int y1_charge(uint32_t ion, uint32_t Lm1, uint32_t half)
+{
+    int z = -1;
+    for (uint32_t y = half, k = 0; y < 2 * half; y += Lm1, k++)
+        if (ion == y) z = (int)k;
+    return z;
+}
+
+// The query postings, a thread per posting: `ids` (entry * speclen + ion) and
+// their buckets `keys` in bucket order; posting j of the order goes to
+// qA[b] + (j - bA[b]). Bound by its bytes (8 read, 6 written a posting): the
+// same with a thread per bucket took 24 ms for 115 M postings (the buckets of the
+// y1 ions hold a large share each, walked by one thread), 0.6 ms so.
+// Every y1 posting of a classed entry must lie in its class's key bucket;
+// bad[e] = 1 marks the entries where one does not (they lose their class).
+// A padding id (kQpostPad) is skipped. qp null: the check only.
+__global__ void k_qpost(const uint32_t *__restrict__ ids, const uint32_t *__restrict__ keys, uint32_t total,
+                        const uint32_t *__restrict__ bA, const uint32_t *__restrict__ qA, IdDiv div, uint32_t half,
+                        uint32_t Lm1, const uint8_t *__restrict__ cls, const ClassKeys *__restrict__ ck,
+                        uint8_t *__restrict__ bad, uint32_t *__restrict__ qp, uint16_t *__restrict__ qion)
+{
+    for (uint64_t j = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; j < total; j += (uint64_t)gridDim.x * blockDim.x)
+    {
+        const uint32_t id = ids[j];
+        if (id == kQpostPad) continue;
+        const uint32_t b = keys[j], entry = div(id), ion = id - entry * div.d;
+        if (qp)
+        {
+            const uint32_t q = qA[b] + ((uint32_t)j - bA[b]);
+            qp[q] = (entry << kQpEntryShift) | ((ion >= half ? 1u : 0u) << 2);
+            qion[q] = (uint16_t)ion;
+        }
+        const int z = y1_charge(ion, Lm1, half);
+        if (z >= 0)
+        {
+            const uint32_t c = cls[entry];
+            if (c != kClassNone && ck->key[c][z] != b) bad[entry] = 1;
+        }
+    }
+}
+
+// the padding after each bucket's postings
+__global__ void k_qpost_pads(const uint32_t *__restrict__ bA, const uint32_t *__restrict__ qA, uint32_t nb,
+                             uint32_t *__restrict__ qp, uint16_t *__restrict__ qion)
 {
     for (uint32_t b = blockIdx.x * blockDim.x + threadIdx.x; b < nb; b += gridDim.x * blockDim.x)
-    {
-        const uint32_t s = bA[b], e = bA[b + 1], q = qA[b];
-        for (uint32_t i = s; i < e; i++)
+        for (uint32_t q = qA[b] + (bA[b + 1] - bA[b]); q < qA[b + 1]; q++)
         {
-            const uint32_t id = ids[i], entry = id / speclen, ion = id - entry * speclen;
-            qp[q + (i - s)] = (entry << kQpEntryShift) | ((ion >= half ? 1u : 0u) << 2);
-            qion[q + (i - s)] = (uint16_t)ion;
+            qp[q] = kQpostPad;
+            qion[q] = 0;
         }
+}
+
+// The last bucket that starts at or before i: start[b] <= i < start[b + 1].
+__device__ __forceinline__ uint32_t bucket_of(const uint32_t *__restrict__ start, uint32_t nb, uint32_t i)
+{
+    uint32_t lo = 0, hi = nb - 1;
+    while (lo < hi)
+    {
+        const uint32_t m = (lo + hi + 1) >> 1;
+        if (__ldg(start + m) <= i) lo = m;
+        else hi = m - 1;
+    }
+    return lo;
+}
+
+// the bucket of every posting (postings that were not sorted here)
+__global__ void k_bucket_keys(const uint32_t *__restrict__ start, uint32_t nb, uint32_t total, uint32_t *__restrict__ keys)
+{
+    for (uint64_t j = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; j < total; j += (uint64_t)gridDim.x * blockDim.x)
+        keys[j] = bucket_of(start, nb, (uint32_t)j);
+}
+
+// query postings -> ids, position by position (padding: kQpostPad)
+__global__ void k_qpost_to_ids(const uint32_t *__restrict__ qp, const uint16_t *__restrict__ qion, uint32_t total,
+                               uint32_t speclen, uint32_t *__restrict__ ids)
+{
+    for (uint64_t j = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; j < total; j += (uint64_t)gridDim.x * blockDim.x)
+    {
+        const uint32_t x = qp[j];
+        ids[j] = x == kQpostPad ? kQpostPad : (x >> kQpEntryShift) * speclen + qion[j];
     }
 }
 
@@ -527,16 +605,16 @@ __global__ void k_check_qpost(const uint32_t *__restrict__ qp, const uint16_t *_
     if (b) atomicAdd(bad, b);
 }
 
-// query postings -> ids (the reference's iA), one thread per bucket
+// query postings -> ids (the reference's iA), one thread per posting
 __global__ void k_qpost_ids(const uint32_t *__restrict__ bA, const uint32_t *__restrict__ qA,
                             const uint32_t *__restrict__ qp, const uint16_t *__restrict__ qion, uint32_t nb,
-                            uint32_t speclen, uint32_t *__restrict__ ids)
+                            uint32_t npost, uint32_t speclen, uint32_t *__restrict__ ids)
 {
-    for (uint32_t b = blockIdx.x * blockDim.x + threadIdx.x; b < nb; b += gridDim.x * blockDim.x)
+    const uint32_t qtotal = qA[nb];
+    for (uint64_t j = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; j < npost; j += (uint64_t)gridDim.x * blockDim.x)
     {
-        const uint32_t s = bA[b], e = bA[b + 1], q = qA[b];
-        for (uint32_t i = s; i < e; i++)
-            ids[i] = (qp[q + (i - s)] >> kQpEntryShift) * speclen + qion[q + (i - s)];
+        const uint32_t b = bucket_of(bA, nb, (uint32_t)j), q = qA[b] + ((uint32_t)j - bA[b]);
+        if (q < qtotal) ids[j] = (qp[q] >> kQpEntryShift) * speclen + qion[q];
     }
 }
 
@@ -587,103 +665,85 @@ __global__ void k_entry_classes(const uint16_t *__restrict__ code, uint32_t n, c
     cls[k] = class_of[code[k]];
 }
 
-// the charge of a query posting's ion when it is a y1 ion, else -1;
-// ion = series * half + charge * (L - 1) + position
-__device__ __forceinline__ int y1_charge(uint32_t ion, uint32_t Lm1, uint32_t half)
-{
-    if (ion < half || (ion - half) % Lm1) return -1;
-    return (int)((ion - half) / Lm1);
-}
-
-constexpr uint32_t kPosChunk = 64;  // postings per thread in the flat kernels below
-
-// The bucket holding position i of the query postings, from a bucket b with
-// qA[b] <= i: b itself while i is inside it, else the last bucket starting at
-// or before i (a binary search, so runs of empty buckets cost no walk).
-__device__ __forceinline__ uint32_t bucket_at(const uint32_t *__restrict__ qA, uint32_t nb, uint32_t i, uint32_t b)
-{
-    if (qA[b + 1] > i) return b;
-    uint32_t lo = b + 1, hi = nb;
-    while (lo < hi)
-    {
-        const uint32_t m = (lo + hi + 1) >> 1;
-        if (qA[m] <= i) lo = m;
-        else hi = m - 1;
-    }
-    return lo;
-}
-
-// kPosChunk postings per thread: every y1 posting of a classed entry must lie
-// in its class's key bucket; bad[e] = 1 marks the entries where one does not
-// (they lose their class).
-__global__ void k_class_check(const uint32_t *__restrict__ qA, const uint32_t *__restrict__ qp,
-                              const uint16_t *__restrict__ qion, uint32_t nb, uint32_t total, uint32_t Lm1,
-                              uint32_t half, const uint8_t *__restrict__ cls, const ClassKeys *__restrict__ ck,
-                              uint8_t *__restrict__ bad)
-{
-    const uint64_t i0 = ((uint64_t)blockIdx.x * blockDim.x + threadIdx.x) * kPosChunk;
-    if (i0 >= total) return;
-    const uint32_t i1 = (uint32_t)min((uint64_t)total, i0 + kPosChunk);
-    uint32_t b = bucket_at(qA, nb, (uint32_t)i0, 0);
-    for (uint32_t i = (uint32_t)i0; i < i1; i++)
-    {
-        const uint32_t x = qp[i];
-        if (x == kQpostPad) continue;
-        const int z = y1_charge(qion[i], Lm1, half);
-        if (z < 0) continue;
-        b = bucket_at(qA, nb, i, b);
-        const uint32_t e = x >> kQpEntryShift, c = cls[e];
-        if (c != kClassNone && ck->key[c][z] != b) bad[e] = 1;
-    }
-}
-
 __global__ void k_class_fix(uint8_t *__restrict__ cls, const uint8_t *__restrict__ bad, uint32_t n)
 {
     const uint32_t k = blockIdx.x * blockDim.x + threadIdx.x;
     if (k < n && bad[k]) cls[k] = (uint8_t)kClassNone;
 }
 
-// a query posting stays in the search postings unless it is padding or the
-// y1 posting of a classed entry
-__device__ __forceinline__ bool search_kept(uint32_t x, uint32_t ion, uint32_t Lm1, uint32_t half,
-                                            const uint8_t *__restrict__ cls)
+// Which postings stay in the search postings (all but padding and the y1
+// postings of classed entries): a bit each, in words of 32, and each word's
+// count. With the counts scanned, the kept postings before position i are one
+// word's sum and a population count, so the flags cost a thirty-second of a
+// scan over the postings themselves (three passes of 4 bytes a posting).
+__global__ void k_spost_mask(const uint32_t *__restrict__ ids, uint32_t total, IdDiv div, uint32_t half, uint32_t Lm1,
+                             const uint8_t *__restrict__ cls, uint32_t nwords, uint32_t *__restrict__ mask,
+                             uint32_t *__restrict__ sum)
 {
-    if (x == kQpostPad) return false;
-    return y1_charge(ion, Lm1, half) < 0 || cls[x >> kQpEntryShift] == kClassNone;
+    const int lane = threadIdx.x & 31;
+    for (uint64_t w = ((uint64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5; w < nwords;
+         w += ((uint64_t)gridDim.x * blockDim.x) >> 5)
+    {
+        const uint64_t j = 32 * w + (uint64_t)lane;
+        const uint32_t id = j < total ? ids[j] : kQpostPad;
+        bool keep = false;
+        if (id != kQpostPad)
+        {
+            const uint32_t entry = div(id), ion = id - entry * div.d;
+            keep = y1_charge(ion, Lm1, half) < 0 || cls[entry] == kClassNone;
+        }
+        const uint32_t m = __ballot_sync(0xFFFFFFFFu, keep);
+        if (lane == 0)
+        {
+            mask[w] = m;
+            sum[w] = (uint32_t)__popc(m);
+        }
+    }
 }
 
-// keep[i] = 1 for a query posting that stays in the search postings, else 0
-__global__ void k_spost_keep(const uint32_t *__restrict__ qp, const uint16_t *__restrict__ qion, uint32_t total,
-                              uint32_t Lm1, uint32_t half, const uint8_t *__restrict__ cls, uint32_t *__restrict__ keep)
+// kept postings before position i (sum scanned)
+__device__ __forceinline__ uint32_t kept_before(const uint32_t *__restrict__ mask, const uint32_t *__restrict__ sum,
+                                                uint32_t i)
 {
-    for (uint64_t i = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; i < total; i += (uint64_t)gridDim.x * blockDim.x)
-        keep[i] = search_kept(qp[i], qion[i], Lm1, half, cls) ? 1u : 0u;
+    return sum[i >> 5] + (uint32_t)__popc(mask[i >> 5] & ((1u << (i & 31u)) - 1u));
 }
 
-// the padded size of each bucket's search postings, from the exclusive scan S
-// of the keep flags; entry nb is 0 (the scan makes it the total)
-__global__ void k_spost_counts(const uint32_t *__restrict__ qA, const uint32_t *__restrict__ S, uint32_t nb,
-                                uint32_t *__restrict__ qAs)
+// the padded size of each bucket's search postings; entry nb is 0 (the scan
+// makes it the total)
+__global__ void k_spost_counts(const uint32_t *__restrict__ start, const uint32_t *__restrict__ mask,
+                               const uint32_t *__restrict__ sum, uint32_t nb, uint32_t *__restrict__ qAs)
 {
     for (uint32_t b = blockIdx.x * blockDim.x + threadIdx.x; b <= nb; b += gridDim.x * blockDim.x)
-        qAs[b] = b < nb ? ((S[qA[b + 1]] - S[qA[b]] + 3u) & ~3u) : 0u;
+        qAs[b] = b < nb ? ((kept_before(mask, sum, start[b + 1]) - kept_before(mask, sum, start[b]) + 3u) & ~3u) : 0u;
 }
 
-// kPosChunk postings per thread: each kept posting to its place, bucket b's
-// at qAs[b] in their order.
-__global__ void k_spost_scatter(const uint32_t *__restrict__ qA, const uint32_t *__restrict__ qp,
-                                 const uint32_t *__restrict__ S, uint32_t nb, uint32_t total,
-                                 const uint32_t *__restrict__ qAs, uint32_t *__restrict__ qps)
+// per bucket: what takes a kept posting's rank to its place (off), and the
+// padding after the bucket's postings
+__global__ void k_spost_pads(const uint32_t *__restrict__ start, const uint32_t *__restrict__ mask,
+                             const uint32_t *__restrict__ sum, uint32_t nb, const uint32_t *__restrict__ qAs,
+                             uint32_t *__restrict__ off, uint32_t *__restrict__ qps)
 {
-    const uint64_t i0 = ((uint64_t)blockIdx.x * blockDim.x + threadIdx.x) * kPosChunk;
-    if (i0 >= total) return;
-    const uint32_t i1 = (uint32_t)min((uint64_t)total, i0 + kPosChunk);
-    uint32_t b = bucket_at(qA, nb, (uint32_t)i0, 0);
-    for (uint32_t i = (uint32_t)i0; i < i1; i++)
+    for (uint32_t b = blockIdx.x * blockDim.x + threadIdx.x; b < nb; b += gridDim.x * blockDim.x)
     {
-        if (S[i + 1] == S[i]) continue;  // not kept
-        b = bucket_at(qA, nb, i, b);
-        qps[qAs[b] + S[i] - S[qA[b]]] = qp[i];
+        const uint32_t k0 = kept_before(mask, sum, start[b]), k1 = kept_before(mask, sum, start[b + 1]);
+        off[b] = qAs[b] - k0;
+        for (uint32_t q = qAs[b] + (k1 - k0); q < qAs[b + 1]; q++) qps[q] = kQpostPad;
+    }
+}
+
+// every kept posting to its place, a thread per posting
+__global__ void k_spost_scatter(const uint32_t *__restrict__ ids, const uint32_t *__restrict__ keys, uint32_t total,
+                                IdDiv div, uint32_t half, const uint32_t *__restrict__ mask,
+                                const uint32_t *__restrict__ sum, const uint32_t *__restrict__ off,
+                                uint32_t *__restrict__ qps)
+{
+    for (uint64_t j = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; j < total; j += (uint64_t)gridDim.x * blockDim.x)
+    {
+        const uint32_t m = mask[j >> 5];
+        if (!((m >> (j & 31u)) & 1u)) continue;
+        const uint32_t rank = sum[j >> 5] + (uint32_t)__popc(m & ((1u << (j & 31u)) - 1u));
+        const uint32_t id = ids[j], entry = div(id), ion = id - entry * div.d;
+        qps[off[keys[j]] + rank] = (entry << kQpEntryShift) | ((ion >= half ? 1u : 0u) << 2);
     }
 }
 
@@ -713,6 +773,9 @@ struct Scratch
 };
 
 }  // namespace
+
+static int build_search(hc_ctx *ctx, LenHost &lh, const uint32_t *d_ids, const uint32_t *d_keys, uint32_t total,
+                        const uint32_t *start, bool write);
 
 // The entries of one length enumerated on the device (k_enum_entries, two
 // passes around a scan of the per-peptide variant counts) into fresh SoA
@@ -871,7 +934,7 @@ int build_length_device(hc_ctx *ctx, LenHost &lh, const hc_entry *h_entries, boo
                           st>>>(skeys, M, nb, lh.d_bA);
         launches += 1;
         lh.npost = M;
-        const int rq = build_query_postings(ctx, lh, svals);
+        const int rq = build_query_postings(ctx, lh, svals, skeys);
         if (rq) return rq;
         launches += 4;
     }
@@ -879,7 +942,7 @@ int build_length_device(hc_ctx *ctx, LenHost &lh, const hc_entry *h_entries, boo
     {
         HC_CUDA(ctx, cudaMemsetAsync(lh.d_bA, 0, 4ull * (nb + 1), st));
         lh.npost = 0;
-        const int rq = build_query_postings(ctx, lh, nullptr);
+        const int rq = build_query_postings(ctx, lh, nullptr, nullptr);
         if (rq) return rq;
     }
     uint32_t h_uninit = 0;
@@ -891,41 +954,57 @@ int build_length_device(hc_ctx *ctx, LenHost &lh, const hc_entry *h_entries, boo
     return HC_SUCCESS;
 }
 
-// The query postings (padded buckets), their bucket starts and the row table,
+static IdDiv id_div(uint32_t speclen, uint64_t ids)
+{
+    IdDiv d{speclen, 0, 0, ids < 0x80000000ull};
+    if (d.fast) division_magic(speclen, &d.magic, &d.sh);
+    return d;
+}
+
+static unsigned flat_blocks(const hc_ctx *ctx, uint64_t items)
+{
+    return (unsigned)std::max<uint64_t>(1, std::min<uint64_t>((items + 255) / 256, (uint64_t)ctx->sm_count * 64));
+}
+
+// The query postings (padded buckets), their bucket starts and the search side,
 // from bA (on the device) and the ids in bucket order (d_ids; null when the
-// length has no postings). Leaves d_ids untouched.
-int build_query_postings(hc_ctx *ctx, LenHost &lh, const uint32_t *d_ids)
+// length has no postings) with their buckets (d_keys; null: found here).
+// Leaves d_ids untouched.
+int build_query_postings(hc_ctx *ctx, LenHost &lh, const uint32_t *d_ids, const uint32_t *d_keys)
 {
     cudaStream_t st = ctx->stream;
     const uint32_t nb = ctx->p.max_mass * ctx->p.scale;
-    const uint32_t speclen = 2 * ctx->p.maxz * (lh.L - 1);
     // entry << 3 must stay below 2^32 and below the padding word
     if (lh.n > kQpMaxEntries)
         return set_error(ctx, HC_ERR_INVLD_SIZE, "too many entries of one length for the query postings");
     cudaFree(lh.d_qA);
     cudaFree(lh.d_qp);
     cudaFree(lh.d_qion);
-    cudaFree(lh.d_rows);
-    lh.d_qA = lh.d_qp = lh.d_rows = nullptr;
+    lh.d_qA = lh.d_qp = nullptr;
     lh.d_qion = nullptr;
     HC_CUDA(ctx, dalloc(&lh.d_qA, (size_t)nb + 1));
-    uint32_t *stmp = nullptr;
+    uint32_t *stmp = nullptr, *keys = nullptr;
     Scratch scr;
     HC_CUDA(ctx, scr.alloc(&stmp, scan_tmp_words((size_t)nb + 1)));
-    const unsigned bblocks = (unsigned)std::min<uint64_t>((nb + 256) / 256, (uint64_t)ctx->sm_count * 16);
-    k_pad_counts<<<bblocks, 256, 0, st>>>(lh.d_bA, nb, lh.d_qA);
+    const uint32_t npost = d_ids ? (uint32_t)lh.npost : 0u;
+    if (npost && !d_keys)
+    {
+        HC_CUDA(ctx, scr.alloc(&keys, npost));
+        k_bucket_keys<<<flat_blocks(ctx, npost), 256, 0, st>>>(lh.d_bA, nb, npost, keys);
+        d_keys = keys;
+    }
+    k_pad_counts<<<flat_blocks(ctx, (uint64_t)nb + 1), 256, 0, st>>>(lh.d_bA, nb, lh.d_qA);
     HC_CUDA(ctx, scan_exclusive(lh.d_qA, (size_t)nb + 1, stmp, st));
     uint32_t total = 0;
     HC_CUDA(ctx, cudaMemcpyAsync(&total, lh.d_qA + nb, 4, cudaMemcpyDeviceToHost, st));
     HC_CUDA(ctx, cudaStreamSynchronize(st));
     HC_CUDA(ctx, dalloc(&lh.d_qp, (size_t)total + kIaPad));
     HC_CUDA(ctx, dalloc(&lh.d_qion, (size_t)total + kIaPad));
-    HC_CUDA(ctx, cudaMemsetAsync(lh.d_qp, 0xFF, 4 * ((size_t)total + kIaPad), st));
-    HC_CUDA(ctx, cudaMemsetAsync(lh.d_qion, 0, 2 * ((size_t)total + kIaPad), st));
-    if (d_ids && lh.npost)
-        k_qpost<<<bblocks, 256, 0, st>>>(lh.d_bA, d_ids, lh.d_qA, nb, speclen, speclen / 2, lh.d_qp, lh.d_qion);
+    HC_CUDA(ctx, cudaMemsetAsync(lh.d_qp + total, 0xFF, 4 * kIaPad, st));
+    HC_CUDA(ctx, cudaMemsetAsync(lh.d_qion + total, 0, 2 * kIaPad, st));
+    k_qpost_pads<<<flat_blocks(ctx, nb), 256, 0, st>>>(lh.d_bA, lh.d_qA, nb, lh.d_qp, lh.d_qion);
     HC_CUDA(ctx, cudaGetLastError());
-    return build_rows(ctx, lh);
+    return build_search(ctx, lh, d_ids, d_keys, npost, lh.d_bA, true);
 }
 
 // Classes for the codes seen in `used` that have none yet (ids are only ever
@@ -958,15 +1037,18 @@ static int add_classes(hc_ctx *ctx, const std::vector<uint8_t> &used)
     return HC_SUCCESS;
 }
 
-// The search side of a length from its query postings (qA, qp, qion and the
-// entries set): each entry's class (checked against its own y1 postings),
-// the search postings (the query postings less the y1 postings of classed
-// entries, buckets padded to 4 words) and their row table.
-int build_rows(hc_ctx *ctx, LenHost &lh)
+// The search side of a length: each entry's class (checked against its own y1
+// postings), the search postings (the query postings less the y1 postings of
+// classed entries, buckets padded to 4 words) and their row table. From `total`
+// ids (entry * speclen + ion, kQpostPad: none) in bucket order, their buckets
+// and the buckets' starts among them; `write`: the query postings too.
+static int build_search(hc_ctx *ctx, LenHost &lh, const uint32_t *d_ids, const uint32_t *d_keys, uint32_t total,
+                        const uint32_t *start, bool write)
 {
     cudaStream_t st = ctx->stream;
     const uint32_t nb = ctx->p.max_mass * ctx->p.scale, n = lh.n, Lm1 = lh.L - 1;
     const uint32_t half = ctx->p.maxz * Lm1;
+    const IdDiv div = id_div(2 * half, (uint64_t)n * 2 * half);
     cudaFree(lh.d_rows);
     cudaFree(lh.d_qAs);
     cudaFree(lh.d_qps);
@@ -976,11 +1058,8 @@ int build_rows(hc_ctx *ctx, LenHost &lh)
     HC_CUDA(ctx, dalloc(&lh.d_cls, (size_t)n + 4));  // +4: the search reads class bytes in fours
     HC_CUDA(ctx, dalloc(&lh.d_qAs, (size_t)nb + 1));
     HC_CUDA(ctx, cudaMemsetAsync(lh.d_cls, (int)kClassNone, (size_t)n + 4, st));
-    const unsigned eblocks = (n + 255) / 256;
-    uint32_t qtotal = 0;  // query postings with padding
-    HC_CUDA(ctx, cudaMemcpyAsync(&qtotal, lh.d_qA + nb, 4, cudaMemcpyDeviceToHost, st));
-    HC_CUDA(ctx, cudaStreamSynchronize(st));
-    const unsigned pblocks = (unsigned)(((uint64_t)qtotal + 256ull * kPosChunk - 1) / (256ull * kPosChunk));
+    const unsigned eblocks = (n + 255) / 256, bblocks = flat_blocks(ctx, (uint64_t)nb + 1);
+    const unsigned pblocks = flat_blocks(ctx, total);
     Scratch scr;
     if (n > 0)
     {
@@ -1000,37 +1079,36 @@ int build_rows(hc_ctx *ctx, LenHost &lh)
         const int rc = add_classes(ctx, hused);
         if (rc) return rc;
         k_entry_classes<<<eblocks, 256, 0, st>>>(code, n, ctx->d_class_of, lh.d_cls);
-        if (qtotal)
-            k_class_check<<<pblocks, 256, 0, st>>>(lh.d_qA, lh.d_qp, lh.d_qion, nb, qtotal, Lm1, half, lh.d_cls,
-                                                   ctx->d_classes, bad);
+        if (total)
+            k_qpost<<<pblocks, 256, 0, st>>>(d_ids, d_keys, total, start, lh.d_qA, div, half, Lm1, lh.d_cls, ctx->d_classes,
+                                             bad, write ? lh.d_qp : nullptr, write ? lh.d_qion : nullptr);
         k_class_fix<<<eblocks, 256, 0, st>>>(lh.d_cls, bad, n);
         HC_CUDA(ctx, cudaGetLastError());
     }
-    // keep flags of the query postings, their exclusive scan S (S[qtotal] =
-    // postings kept), the padded bucket sizes from S and their scan (qAs),
-    // then every kept posting to its place
-    uint32_t *keep = nullptr, *stmp = nullptr, *btmp = nullptr;
-    HC_CUDA(ctx, scr.alloc(&keep, (size_t)qtotal + 1));
-    HC_CUDA(ctx, scr.alloc(&stmp, scan_tmp_words((size_t)qtotal + 1)));
-    HC_CUDA(ctx, scr.alloc(&btmp, scan_tmp_words((size_t)nb + 1)));
-    HC_CUDA(ctx, cudaMemsetAsync(keep + qtotal, 0, 4, st));
-    if (qtotal)
-        k_spost_keep<<<(unsigned)std::min<uint64_t>((qtotal + 255) / 256, (uint64_t)ctx->sm_count * 64), 256, 0, st>>>(
-            lh.d_qp, lh.d_qion, qtotal, Lm1, half, lh.d_cls, keep);
+    // the kept postings' bits and counts, the padded bucket sizes from them and
+    // their scan (qAs), then every kept posting to its place
+    const uint32_t nwords = total / 32 + 1;  // (position `total` has one too)
+    uint32_t *mask = nullptr, *sum = nullptr, *stmp = nullptr, *off = nullptr;
+    HC_CUDA(ctx, scr.alloc(&mask, nwords));
+    HC_CUDA(ctx, scr.alloc(&sum, nwords));
+    HC_CUDA(ctx, scr.alloc(&off, (size_t)nb));
+    HC_CUDA(ctx, scr.alloc(&stmp, scan_tmp_words(std::max<size_t>(nwords, (size_t)nb + 1))));
+    k_spost_mask<<<flat_blocks(ctx, 32ull * nwords), 256, 0, st>>>(d_ids, total, div, half, Lm1, lh.d_cls, nwords, mask,
+                                                                   sum);
     HC_CUDA(ctx, cudaGetLastError());
-    HC_CUDA(ctx, scan_exclusive(keep, (size_t)qtotal + 1, stmp, st));
-    k_spost_counts<<<(unsigned)std::min<uint64_t>((nb + 256) / 256, (uint64_t)ctx->sm_count * 16), 256, 0, st>>>(
-        lh.d_qA, keep, nb, lh.d_qAs);
+    HC_CUDA(ctx, scan_exclusive(sum, nwords, stmp, st));
+    k_spost_counts<<<bblocks, 256, 0, st>>>(start, mask, sum, nb, lh.d_qAs);
     HC_CUDA(ctx, cudaGetLastError());
-    HC_CUDA(ctx, scan_exclusive(lh.d_qAs, (size_t)nb + 1, btmp, st));
-    uint32_t total = 0;
-    HC_CUDA(ctx, cudaMemcpyAsync(&total, lh.d_qAs + nb, 4, cudaMemcpyDeviceToHost, st));
+    HC_CUDA(ctx, scan_exclusive(lh.d_qAs, (size_t)nb + 1, stmp, st));
+    uint32_t stotal = 0;
+    HC_CUDA(ctx, cudaMemcpyAsync(&stotal, lh.d_qAs + nb, 4, cudaMemcpyDeviceToHost, st));
     HC_CUDA(ctx, cudaStreamSynchronize(st));
-    lh.nsearch = total;
-    HC_CUDA(ctx, dalloc(&lh.d_qps, (size_t)total + kIaPad));
-    HC_CUDA(ctx, cudaMemsetAsync(lh.d_qps, 0xFF, 4 * ((size_t)total + kIaPad), st));
-    if (qtotal)
-        k_spost_scatter<<<pblocks, 256, 0, st>>>(lh.d_qA, lh.d_qp, keep, nb, qtotal, lh.d_qAs, lh.d_qps);
+    lh.nsearch = stotal;
+    HC_CUDA(ctx, dalloc(&lh.d_qps, (size_t)stotal + kIaPad));
+    HC_CUDA(ctx, cudaMemsetAsync(lh.d_qps + stotal, 0xFF, 4 * kIaPad, st));
+    k_spost_pads<<<bblocks, 256, 0, st>>>(start, mask, sum, nb, lh.d_qAs, off, lh.d_qps);
+    if (total)
+        k_spost_scatter<<<pblocks, 256, 0, st>>>(d_ids, d_keys, total, div, half, mask, sum, off, lh.d_qps);
     HC_CUDA(ctx, cudaGetLastError());
     lh.stride = (n + kRowG - 1) / kRowG + 1;
     HC_CUDA(ctx, dalloc(&lh.d_rows, (size_t)nb * lh.stride));
@@ -1040,6 +1118,28 @@ int build_rows(hc_ctx *ctx, LenHost &lh)
     HC_CUDA(ctx, cudaGetLastError());
     HC_CUDA(ctx, cudaStreamSynchronize(st));
     return HC_SUCCESS;
+}
+
+// The same from query postings that are there already (an index file's, in
+// padded order): qA, qp, qion and the entries set and checked.
+int build_rows(hc_ctx *ctx, LenHost &lh)
+{
+    const uint32_t nb = ctx->p.max_mass * ctx->p.scale;
+    uint32_t qtotal = 0;
+    HC_CUDA(ctx, cudaMemcpyAsync(&qtotal, lh.d_qA + nb, 4, cudaMemcpyDeviceToHost, ctx->stream));
+    HC_CUDA(ctx, cudaStreamSynchronize(ctx->stream));
+    Scratch scr;
+    uint32_t *ids = nullptr, *keys = nullptr;
+    HC_CUDA(ctx, scr.alloc(&ids, qtotal));
+    HC_CUDA(ctx, scr.alloc(&keys, qtotal));
+    if (qtotal)
+    {
+        k_qpost_to_ids<<<flat_blocks(ctx, qtotal), 256, 0, ctx->stream>>>(lh.d_qp, lh.d_qion, qtotal,
+                                                                          2 * ctx->p.maxz * (lh.L - 1), ids);
+        k_bucket_keys<<<flat_blocks(ctx, qtotal), 256, 0, ctx->stream>>>(lh.d_qA, nb, qtotal, keys);
+        HC_CUDA(ctx, cudaGetLastError());
+    }
+    return build_search(ctx, lh, ids, keys, qtotal, lh.d_qA, false);
 }
 
 // Checks query postings read from outside (an index file): bucket starts
@@ -1080,9 +1180,9 @@ int export_ids(hc_ctx *ctx, const LenHost &lh, uint32_t *d_ids)
 {
     const uint32_t nb = ctx->p.max_mass * ctx->p.scale;
     const uint32_t speclen = 2 * ctx->p.maxz * (lh.L - 1);
-    const unsigned bblocks = (unsigned)std::min<uint64_t>((nb + 255) / 256, (uint64_t)ctx->sm_count * 16);
     if (lh.npost)
-        k_qpost_ids<<<bblocks, 256, 0, ctx->stream>>>(lh.d_bA, lh.d_qA, lh.d_qp, lh.d_qion, nb, speclen, d_ids);
+        k_qpost_ids<<<flat_blocks(ctx, lh.npost), 256, 0, ctx->stream>>>(lh.d_bA, lh.d_qA, lh.d_qp, lh.d_qion, nb,
+                                                                         (uint32_t)lh.npost, speclen, d_ids);
     HC_CUDA(ctx, cudaGetLastError());
     HC_CUDA(ctx, cudaStreamSynchronize(ctx->stream));
     return HC_SUCCESS;

@@ -262,8 +262,8 @@ void division_magic(uint32_t d, uint32_t *magic, uint32_t *sh);
 
 // hc_index.cu
 int build_length_device(hc_ctx *ctx, LenHost &lh, const hc_entry *h_entries, bool sort_by_mass);
-int build_query_postings(hc_ctx *ctx, LenHost &lh, const uint32_t *d_ids);
-int build_rows(hc_ctx *ctx, LenHost &lh);  // entry classes, search postings and their row table
+int build_query_postings(hc_ctx *ctx, LenHost &lh, const uint32_t *d_ids, const uint32_t *d_keys);
+int build_rows(hc_ctx *ctx, LenHost &lh);  // from query postings: entry classes, search postings and their row table
 void class_keys_of(const hc_params &p, const IonTables &t, uint32_t code, uint32_t *keys);
 int check_query_postings(hc_ctx *ctx, const LenHost &lh, uint64_t qtotal);
 void free_len(LenHost &lh);
