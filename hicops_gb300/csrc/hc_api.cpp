@@ -23,21 +23,30 @@ int cuda_check(hc_ctx *ctx, cudaError_t e, const char *what)
     return set_error(ctx, e == cudaErrorMemoryAllocation ? HC_ERR_BAD_MEM_ALLOC : HC_ERR_CUDA, m);
 }
 
-void free_len(LenHost &lh)
+cudaError_t pool_alloc(hc_ctx *ctx, void **p, size_t bytes)
 {
-    cudaFree(lh.d_mass);
-    cudaFree(lh.d_seqid);
-    cudaFree(lh.d_sites);
-    cudaFree(lh.d_modnum);
-    cudaFree(lh.d_seqs);
-    cudaFree(lh.d_bA);
-    cudaFree(lh.d_qA);
-    cudaFree(lh.d_qp);
-    cudaFree(lh.d_qion);
-    cudaFree(lh.d_qAs);
-    cudaFree(lh.d_qps);
-    cudaFree(lh.d_cls);
-    cudaFree(lh.d_rows);
+    *p = nullptr;
+    return cudaMallocFromPoolAsync(p, bytes, ctx->pool, ctx->stream);
+}
+
+// Frees a length's arrays. A search of them may still run on any stream (the
+// frees are ordered on the context's), so a length in use is waited for.
+void free_len(hc_ctx *ctx, LenHost &lh)
+{
+    if (lh.built) cudaDeviceSynchronize();
+    dfree(ctx, lh.d_mass);
+    dfree(ctx, lh.d_seqid);
+    dfree(ctx, lh.d_sites);
+    dfree(ctx, lh.d_modnum);
+    dfree(ctx, lh.d_seqs);
+    dfree(ctx, lh.d_bA);
+    dfree(ctx, lh.d_qA);
+    dfree(ctx, lh.d_qp);
+    dfree(ctx, lh.d_qion);
+    dfree(ctx, lh.d_qAs);
+    dfree(ctx, lh.d_qps);
+    dfree(ctx, lh.d_cls);
+    dfree(ctx, lh.d_rows);
     const uint32_t L = lh.L;
     lh = LenHost();
     lh.L = L;
@@ -117,6 +126,20 @@ int hc_ctx_create(int device, const hc_params *p, hc_ctx **out)
         delete ctx;
         return HC_ERR_CUDA;
     }
+    {
+        cudaMemPoolProps pp{};
+        pp.allocType = cudaMemAllocationTypePinned;
+        pp.location.type = cudaMemLocationTypeDevice;
+        pp.location.id = device;
+        uint64_t keep = kPoolKeep;
+        if (cudaMemPoolCreate(&ctx->pool, &pp) != cudaSuccess ||
+            cudaMemPoolSetAttribute(ctx->pool, cudaMemPoolAttrReleaseThreshold, &keep) != cudaSuccess ||
+            cudaMallocHost(&ctx->h_read, kReadBytes) != cudaSuccess)
+        {
+            hc_ctx_destroy(ctx);
+            return HC_ERR_BAD_MEM_ALLOC;
+        }
+    }
     make_ion_tables(ctx->p, &ctx->tables);
     ctx->class_of.assign(kCodes, (uint8_t)kClassNone);
     QueryConst qc;
@@ -160,7 +183,13 @@ int hc_ctx_destroy(hc_ctx *ctx)
 {
     if (!ctx) return HC_ERR_INVLD_PTR;
     cudaSetDevice(ctx->device);
-    for (auto &lh : ctx->lens) free_len(lh);
+    for (auto &lh : ctx->lens) free_len(ctx, lh);
+    if (ctx->pool)
+    {
+        cudaStreamSynchronize(ctx->stream);
+        cudaMemPoolDestroy(ctx->pool);
+    }
+    cudaFreeHost(ctx->h_read);
     cudaFree(ctx->d_lens);
     cudaFree(ctx->d_tables);
     cudaFree(ctx->d_classes);
@@ -241,8 +270,8 @@ static int upload_seqs(hc_ctx *ctx, LenHost &lh, const uint8_t *seqs, uint32_t n
 {
     for (size_t i = 0; i < (size_t)npep * lh.L; i++)
         if (seqs[i] < 'A' || seqs[i] > 'Z') return set_error(ctx, HC_ERR_INVLD_PARAM, "residue outside A-Z");
-    HC_CUDA(ctx, cudaMalloc((void **)&lh.d_seqs, (size_t)npep * lh.L + 1));
-    HC_CUDA(ctx, cudaMemcpy(lh.d_seqs, seqs, (size_t)npep * lh.L, cudaMemcpyHostToDevice));
+    HC_CUDA(ctx, dalloc(ctx, &lh.d_seqs, (size_t)npep * lh.L + 1));
+    HC_CUDA(ctx, cudaMemcpyAsync(lh.d_seqs, seqs, (size_t)npep * lh.L, cudaMemcpyHostToDevice, ctx->stream));
     lh.npep = npep;
     return HC_SUCCESS;
 }
@@ -254,7 +283,7 @@ int hc_dslim_construct(hc_ctx *ctx, uint32_t L, const uint8_t *seqs, uint32_t np
     LenHost *lh = find_len(ctx, L);
     if (!lh) return set_error(ctx, HC_ERR_INVLD_PARAM, "length outside [min_len, max_len]");
     cudaSetDevice(ctx->device);
-    free_len(*lh);
+    free_len(ctx, *lh);
     int rc = upload_seqs(ctx, *lh, seqs, npep);
     if (rc) return rc;
     if (!order) return build_length_device(ctx, *lh, nullptr, true);  // entries enumerated on the device
@@ -273,7 +302,7 @@ int hc_dslim_load(hc_ctx *ctx, uint32_t L, const uint8_t *seqs, uint32_t npep, c
     if (!lh) return set_error(ctx, HC_ERR_INVLD_PARAM, "length outside [min_len, max_len]");
     if (n >= (1u << 24)) return set_error(ctx, HC_ERR_INVLD_SIZE, "more than 2^24 entries in one length");
     cudaSetDevice(ctx->device);
-    free_len(*lh);
+    free_len(ctx, *lh);
     int rc = upload_seqs(ctx, *lh, seqs, npep);
     if (rc) return rc;
     const uint32_t speclen = 2 * ctx->p.maxz * (L - 1);
@@ -302,22 +331,25 @@ int hc_dslim_load(hc_ctx *ctx, uint32_t L, const uint8_t *seqs, uint32_t npep, c
         si[i] = entries[i].sites;
         mo[i] = entries[i].modnum;
     }
-    HC_CUDA(ctx, cudaMalloc((void **)&lh->d_mass, 4ull * n + 4));
-    HC_CUDA(ctx, cudaMalloc((void **)&lh->d_seqid, 4ull * n + 4));
-    HC_CUDA(ctx, cudaMalloc((void **)&lh->d_modnum, 4ull * n + 4));
-    HC_CUDA(ctx, cudaMalloc((void **)&lh->d_sites, 8ull * n + 8));
-    HC_CUDA(ctx, cudaMalloc((void **)&lh->d_bA, 4ull * (nb + 1)));
-    HC_CUDA(ctx, cudaMemcpy(lh->d_mass, m.data(), 4ull * n, cudaMemcpyHostToDevice));
-    HC_CUDA(ctx, cudaMemcpy(lh->d_seqid, s.data(), 4ull * n, cudaMemcpyHostToDevice));
-    HC_CUDA(ctx, cudaMemcpy(lh->d_modnum, mo.data(), 4ull * n, cudaMemcpyHostToDevice));
-    HC_CUDA(ctx, cudaMemcpy(lh->d_sites, si.data(), 8ull * n, cudaMemcpyHostToDevice));
-    HC_CUDA(ctx, cudaMemcpy(lh->d_bA, bA, 4ull * (nb + 1), cudaMemcpyHostToDevice));
+    cudaStream_t st = ctx->stream;
+    HC_CUDA(ctx, dalloc(ctx, &lh->d_mass, (size_t)n + 1));
+    HC_CUDA(ctx, dalloc(ctx, &lh->d_seqid, (size_t)n + 1));
+    HC_CUDA(ctx, dalloc(ctx, &lh->d_modnum, (size_t)n + 1));
+    HC_CUDA(ctx, dalloc(ctx, &lh->d_sites, (size_t)n + 1));
+    HC_CUDA(ctx, dalloc(ctx, &lh->d_bA, (size_t)nb + 1));
+    HC_CUDA(ctx, cudaMemcpyAsync(lh->d_mass, m.data(), 4ull * n, cudaMemcpyHostToDevice, st));
+    HC_CUDA(ctx, cudaMemcpyAsync(lh->d_seqid, s.data(), 4ull * n, cudaMemcpyHostToDevice, st));
+    HC_CUDA(ctx, cudaMemcpyAsync(lh->d_modnum, mo.data(), 4ull * n, cudaMemcpyHostToDevice, st));
+    HC_CUDA(ctx, cudaMemcpyAsync(lh->d_sites, si.data(), 8ull * n, cudaMemcpyHostToDevice, st));
+    HC_CUDA(ctx, cudaMemcpyAsync(lh->d_bA, bA, 4ull * (nb + 1), cudaMemcpyHostToDevice, st));
     uint32_t *d_ids = nullptr;
-    HC_CUDA(ctx, cudaMalloc((void **)&d_ids, 4 * M + 4));
-    HC_CUDA(ctx, cudaMemcpy(d_ids, iA, 4 * M, cudaMemcpyHostToDevice));
+    HC_CUDA(ctx, dalloc(ctx, &d_ids, M + 1));
+    cudaError_t e = cudaMemcpyAsync(d_ids, iA, 4 * M, cudaMemcpyHostToDevice, st);
+    if (e == cudaSuccess) e = cudaStreamSynchronize(st);  // the host vectors above go with this call
     lh->npost = M;
-    const int rq = build_query_postings(ctx, *lh, M ? d_ids : nullptr, nullptr);
-    cudaFree(d_ids);
+    const int rq = e == cudaSuccess ? build_query_postings(ctx, *lh, M ? d_ids : nullptr, nullptr)
+                                    : cuda_check(ctx, e, "hc_dslim_load");
+    dfree(ctx, d_ids);
     if (rq) return rq;
     lh->built = true;
     ctx->lens_dirty = true;

@@ -238,7 +238,7 @@ cudaError_t radix_sort(uint32_t *keys0, uint32_t *keys1, uint32_t *vals0, uint32
 // (mods.cpp:333-384): at each modifiable position the branch that modifies it
 // comes before the one that skips it, and a variant is emitted as each mod is
 // added. Here the walk is a loop over a stack of chosen positions. The first
-// pass (out == nullptr) counts the variants per peptide; the second writes
+// pass (mass == nullptr) counts the variants per peptide; the second writes
 // them at npep + voff[i].
 __global__ void k_enum_entries(const uint8_t *__restrict__ seqs, uint32_t L, uint32_t npep, EnumConst ec,
                                const uint32_t *__restrict__ voff, uint32_t *__restrict__ vcount,
@@ -246,6 +246,7 @@ __global__ void k_enum_entries(const uint8_t *__restrict__ seqs, uint32_t L, uin
                                uint64_t *__restrict__ sites, uint32_t *__restrict__ modnum)
 {
     const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
+    if (i == npep && vcount) vcount[i] = 0;  // the scan makes it the total
     if (i >= npep) return;
     const uint8_t *s = seqs + (size_t)i * L;
     // UTILS_CalculatePepMass: two float additions per residue, in order
@@ -255,7 +256,7 @@ __global__ void k_enum_entries(const uint8_t *__restrict__ seqs, uint32_t L, uin
         pm += ec.aa[s[l] - 'A'];
         pm += ec.stat[s[l] - 'A'];
     }
-    const bool write = voff != nullptr;
+    const bool write = mass != nullptr;
     if (write)
     {
         mass[i] = pm;
@@ -272,7 +273,7 @@ __global__ void k_enum_entries(const uint8_t *__restrict__ seqs, uint32_t L, uin
         uint32_t d = 0, mn = 0;
         uint64_t st = 0;
         uint32_t start = 0;
-        const uint64_t at = write ? (uint64_t)npep + voff[i] : 0;
+        const uint64_t at = write ? (uint64_t)npep + voff[i] : 0;  // (read only with mods)
         for (;;)
         {
             // virtual positions: q = 0 is the N-terminus (a '^' mod, an
@@ -357,8 +358,7 @@ __global__ void k_gather_entries(const uint32_t *__restrict__ perm, uint32_t n, 
 __global__ void k_ion_keys(const IonTables *__restrict__ gt, uint32_t L, uint32_t n,
                            const float *__restrict__ mass, const uint32_t *__restrict__ seqid,
                            const uint64_t *__restrict__ sites, const uint32_t *__restrict__ modnum,
-                           const uint8_t *__restrict__ seqs, uint32_t *__restrict__ keys,
-                           uint32_t *__restrict__ nuninit)
+                           const uint8_t *__restrict__ seqs, uint32_t *__restrict__ keys)
 {
     __shared__ IonTables t;
     for (int i = threadIdx.x; i < (int)(sizeof(IonTables) / 4); i += blockDim.x)
@@ -378,11 +378,8 @@ __global__ void k_ion_keys(const IonTables *__restrict__ gt, uint32_t L, uint32_
     const uint32_t top = t.max_mass * t.scale;
     const uint32_t mn = modnum[k];
     bool legal = (m >= minm && m <= maxm);
-    if (mn != 0 && legal && !(m > minm && m < maxm))
-    {   // mass exactly on a bound: the reference reads an uninitialised spectrum
-        if (s == 0) atomicAdd(nuninit, 1u);
-        legal = false;
-    }
+    // mass exactly on a bound: the reference reads an uninitialised spectrum
+    if (mn != 0 && legal && !(m > minm && m < maxm)) legal = false;
     if (!legal)
     {
         for (uint32_t l = 0; l < Lm1; l++) out[l] = 0;
@@ -546,16 +543,19 @@ __global__ void k_qpost(const uint32_t *__restrict__ ids, const uint32_t *__rest
     }
 }
 
-// the padding after each bucket's postings
+// the padding after each bucket's postings and after the last bucket
 __global__ void k_qpost_pads(const uint32_t *__restrict__ bA, const uint32_t *__restrict__ qA, uint32_t nb,
                              uint32_t *__restrict__ qp, uint16_t *__restrict__ qion)
 {
-    for (uint32_t b = blockIdx.x * blockDim.x + threadIdx.x; b < nb; b += gridDim.x * blockDim.x)
-        for (uint32_t q = qA[b] + (bA[b + 1] - bA[b]); q < qA[b + 1]; q++)
+    for (uint32_t b = blockIdx.x * blockDim.x + threadIdx.x; b <= nb; b += gridDim.x * blockDim.x)
+    {
+        const uint32_t q0 = b < nb ? qA[b] + (bA[b + 1] - bA[b]) : qA[nb], q1 = b < nb ? qA[b + 1] : qA[nb] + (uint32_t)kIaPad;
+        for (uint32_t q = q0; q < q1; q++)
         {
             qp[q] = kQpostPad;
             qion[q] = 0;
         }
+    }
 }
 
 // The last bucket that starts at or before i: start[b] <= i < start[b + 1].
@@ -648,21 +648,22 @@ __device__ __forceinline__ uint32_t entry_code(double minm, double maxm, uint32_
 __global__ void k_entry_codes(double minm, double maxm, uint32_t L, uint32_t n, const float *__restrict__ mass,
                               const uint32_t *__restrict__ seqid, const uint64_t *__restrict__ sites,
                               const uint32_t *__restrict__ modnum, const uint8_t *__restrict__ seqs,
-                              uint16_t *__restrict__ code, uint8_t *__restrict__ used)
+                              uint16_t *__restrict__ code, uint8_t *__restrict__ used, uint8_t *__restrict__ bad)
 {
     const uint32_t k = blockIdx.x * blockDim.x + threadIdx.x;
     if (k >= n) return;
     const uint32_t c = entry_code(minm, maxm, L, seqs + (size_t)seqid[k] * L, (double)mass[k], modnum[k], sites[k]);
     code[k] = (uint16_t)c;
     used[c] = 1;
+    bad[k] = 0;
 }
 
+// (and the 4 bytes past the last entry, which the search reads in fours)
 __global__ void k_entry_classes(const uint16_t *__restrict__ code, uint32_t n, const uint8_t *__restrict__ class_of,
                                 uint8_t *__restrict__ cls)
 {
     const uint32_t k = blockIdx.x * blockDim.x + threadIdx.x;
-    if (k >= n) return;
-    cls[k] = class_of[code[k]];
+    if (k < n + 4) cls[k] = k < n ? class_of[code[k]] : (uint8_t)kClassNone;
 }
 
 __global__ void k_class_fix(uint8_t *__restrict__ cls, const uint8_t *__restrict__ bad, uint32_t n)
@@ -718,13 +719,18 @@ __global__ void k_spost_counts(const uint32_t *__restrict__ start, const uint32_
 }
 
 // per bucket: what takes a kept posting's rank to its place (off), and the
-// padding after the bucket's postings
+// padding after the bucket's postings (and after the last bucket)
 __global__ void k_spost_pads(const uint32_t *__restrict__ start, const uint32_t *__restrict__ mask,
                              const uint32_t *__restrict__ sum, uint32_t nb, const uint32_t *__restrict__ qAs,
                              uint32_t *__restrict__ off, uint32_t *__restrict__ qps)
 {
-    for (uint32_t b = blockIdx.x * blockDim.x + threadIdx.x; b < nb; b += gridDim.x * blockDim.x)
+    for (uint32_t b = blockIdx.x * blockDim.x + threadIdx.x; b <= nb; b += gridDim.x * blockDim.x)
     {
+        if (b == nb)
+        {
+            for (uint32_t q = 0; q < kIaPad; q++) qps[qAs[nb] + q] = kQpostPad;
+            break;
+        }
         const uint32_t k0 = kept_before(mask, sum, start[b]), k1 = kept_before(mask, sum, start[b + 1]);
         off[b] = qAs[b] - k0;
         for (uint32_t q = qAs[b] + (k1 - k0); q < qAs[b + 1]; q++) qps[q] = kQpostPad;
@@ -747,35 +753,37 @@ __global__ void k_spost_scatter(const uint32_t *__restrict__ ids, const uint32_t
     }
 }
 
-template <class T>
-cudaError_t dalloc(T **p, size_t n)
-{
-    return cudaMalloc((void **)p, sizeof(T) * (n ? n : 1));
-}
-
 // Device scratch of one build step, freed when the step returns (also on its
 // error paths).
 struct Scratch
 {
+    hc_ctx *ctx;
     std::vector<void *> ptrs;
+    explicit Scratch(hc_ctx *c) : ctx(c) {}
     template <class T>
     cudaError_t alloc(T **p, size_t n)
     {
-        const cudaError_t e = dalloc(p, n);
+        const cudaError_t e = dalloc(ctx, p, n);
         if (e == cudaSuccess) ptrs.push_back(*p);
-        else *p = nullptr;
         return e;
     }
     ~Scratch()
     {
-        for (void *p : ptrs) cudaFree(p);
+        for (void *p : ptrs) dfree(ctx, p);
     }
 };
 
 }  // namespace
 
-static int build_search(hc_ctx *ctx, LenHost &lh, const uint32_t *d_ids, const uint32_t *d_keys, uint32_t total,
-                        const uint32_t *start, bool write);
+// The class code of every entry, and room for a mark on those that lose their class.
+struct EntryCodes
+{
+    uint16_t *code;
+    uint8_t *bad;
+};
+
+static int build_search(hc_ctx *ctx, LenHost &lh, const EntryCodes &ec, const uint32_t *d_ids, const uint32_t *d_keys,
+                        uint32_t total, const uint32_t *start, bool write);
 
 // The entries of one length enumerated on the device (k_enum_entries, two
 // passes around a scan of the per-peptide variant counts) into fresh SoA
@@ -787,22 +795,22 @@ static int enumerate_entries(hc_ctx *ctx, LenHost &lh, Scratch &out, float **d_m
     const uint32_t npep = lh.npep, L = lh.L;
     EnumConst ec;
     make_enum_const(ctx->p, &ec);
-    Scratch tmp;
+    Scratch tmp(ctx);
     uint32_t *cnt = nullptr, *stmp = nullptr;
-    HC_CUDA(ctx, tmp.alloc(&cnt, (size_t)npep + 1));
-    HC_CUDA(ctx, tmp.alloc(&stmp, scan_tmp_words((size_t)npep + 1)));
-    HC_CUDA(ctx, cudaMemsetAsync(cnt, 0, 4ull * (npep + 1), st));
-    const unsigned grid = (npep + 127) / 128;
-    if (npep)
+    uint32_t nvar = 0;
+    const unsigned grid = npep / 128 + 1;
+    if (ec.vmods > 0 && ec.nmods > 0 && npep)  // without variable mods there is nothing to count
     {
+        HC_CUDA(ctx, tmp.alloc(&cnt, (size_t)npep + 1));
+        HC_CUDA(ctx, tmp.alloc(&stmp, scan_tmp_words((size_t)npep + 1)));
         k_enum_entries<<<grid, 128, 0, st>>>(lh.d_seqs, L, npep, ec, nullptr, cnt, nullptr, nullptr, nullptr,
                                               nullptr);
         (*launches)++;
+        HC_CUDA(ctx, scan_exclusive(cnt, (size_t)npep + 1, stmp, st));
+        HC_CUDA(ctx, cudaMemcpyAsync(ctx->h_read, cnt + npep, 4, cudaMemcpyDeviceToHost, st));
+        HC_CUDA(ctx, cudaStreamSynchronize(st));
+        nvar = *static_cast<const uint32_t *>(ctx->h_read);
     }
-    HC_CUDA(ctx, scan_exclusive(cnt, (size_t)npep + 1, stmp, st));
-    uint32_t nvar = 0;
-    HC_CUDA(ctx, cudaMemcpyAsync(&nvar, cnt + npep, 4, cudaMemcpyDeviceToHost, st));
-    HC_CUDA(ctx, cudaStreamSynchronize(st));
     const uint64_t n = (uint64_t)npep + nvar;
     if (n >= (1u << 24)) return set_error(ctx, HC_ERR_INVLD_SIZE, "more than 2^24 entries in one length");
     lh.n = (uint32_t)n;
@@ -816,7 +824,6 @@ static int enumerate_entries(hc_ctx *ctx, LenHost &lh, Scratch &out, float **d_m
         (*launches)++;
     }
     HC_CUDA(ctx, cudaGetLastError());
-    HC_CUDA(ctx, cudaStreamSynchronize(st));
     return HC_SUCCESS;
 }
 
@@ -825,7 +832,7 @@ int build_length_device(hc_ctx *ctx, LenHost &lh, const hc_entry *h_entries, boo
     cudaStream_t st = ctx->stream;
     int launches = 0;
     // entries in generation order: enumerated here, or uploaded from the host
-    Scratch scr;
+    Scratch scr(ctx);
     float *d_m0 = nullptr;
     uint32_t *d_s0 = nullptr, *d_mod0 = nullptr;
     uint64_t *d_site0 = nullptr;
@@ -855,29 +862,28 @@ int build_length_device(hc_ctx *ctx, LenHost &lh, const hc_entry *h_entries, boo
         HC_CUDA(ctx, scr.alloc(&d_s0, n));
         HC_CUDA(ctx, scr.alloc(&d_mod0, n));
         HC_CUDA(ctx, scr.alloc(&d_site0, n));
-        HC_CUDA(ctx, cudaMemcpy(d_m0, hm.data(), 4ull * n, cudaMemcpyHostToDevice));
-        HC_CUDA(ctx, cudaMemcpy(d_s0, hs.data(), 4ull * n, cudaMemcpyHostToDevice));
-        HC_CUDA(ctx, cudaMemcpy(d_mod0, hmod.data(), 4ull * n, cudaMemcpyHostToDevice));
-        HC_CUDA(ctx, cudaMemcpy(d_site0, hsite.data(), 8ull * n, cudaMemcpyHostToDevice));
+        HC_CUDA(ctx, cudaMemcpyAsync(d_m0, hm.data(), 4ull * n, cudaMemcpyHostToDevice, st));
+        HC_CUDA(ctx, cudaMemcpyAsync(d_s0, hs.data(), 4ull * n, cudaMemcpyHostToDevice, st));
+        HC_CUDA(ctx, cudaMemcpyAsync(d_mod0, hmod.data(), 4ull * n, cudaMemcpyHostToDevice, st));
+        HC_CUDA(ctx, cudaMemcpyAsync(d_site0, hsite.data(), 8ull * n, cudaMemcpyHostToDevice, st));
+        HC_CUDA(ctx, cudaStreamSynchronize(st));
     }
-    HC_CUDA(ctx, dalloc(&lh.d_mass, n));
-    HC_CUDA(ctx, dalloc(&lh.d_seqid, n));
-    HC_CUDA(ctx, dalloc(&lh.d_sites, n));
-    HC_CUDA(ctx, dalloc(&lh.d_modnum, n));
-    HC_CUDA(ctx, dalloc(&lh.d_bA, (size_t)nb + 1));
+    HC_CUDA(ctx, dalloc(ctx, &lh.d_mass, n));
+    HC_CUDA(ctx, dalloc(ctx, &lh.d_seqid, n));
+    HC_CUDA(ctx, dalloc(ctx, &lh.d_sites, n));
+    HC_CUDA(ctx, dalloc(ctx, &lh.d_modnum, n));
+    HC_CUDA(ctx, dalloc(ctx, &lh.d_bA, (size_t)nb + 1));
 
     // scratch: keys/vals ping-pong, radix histograms, scan temp
     const size_t items = M > n ? M : n;
     const size_t ntiles = (items + kRsTile - 1) / kRsTile;
-    uint32_t *k0, *k1, *v0, *v1, *hist, *stmp, *d_uninit;
+    uint32_t *k0, *k1, *v0, *v1, *hist, *stmp;
     HC_CUDA(ctx, scr.alloc(&k0, items));
     HC_CUDA(ctx, scr.alloc(&k1, items));
     HC_CUDA(ctx, scr.alloc(&v0, items));
     HC_CUDA(ctx, scr.alloc(&v1, items));
     HC_CUDA(ctx, scr.alloc(&hist, ntiles * kRadix));
     HC_CUDA(ctx, scr.alloc(&stmp, scan_tmp_words(ntiles * kRadix)));
-    HC_CUDA(ctx, scr.alloc(&d_uninit, 1));
-    HC_CUDA(ctx, cudaMemsetAsync(d_uninit, 0, 4, st));
 
     if (sort_by_mass && n > 1)
     {
@@ -910,10 +916,11 @@ int build_length_device(hc_ctx *ctx, LenHost &lh, const hc_entry *h_entries, boo
             hsite[i] = h_entries[i].sites;
             hmod[i] = h_entries[i].modnum;
         }
-        HC_CUDA(ctx, cudaMemcpy(lh.d_mass, hm.data(), 4ull * n, cudaMemcpyHostToDevice));
-        HC_CUDA(ctx, cudaMemcpy(lh.d_seqid, hs.data(), 4ull * n, cudaMemcpyHostToDevice));
-        HC_CUDA(ctx, cudaMemcpy(lh.d_modnum, hmod.data(), 4ull * n, cudaMemcpyHostToDevice));
-        HC_CUDA(ctx, cudaMemcpy(lh.d_sites, hsite.data(), 8ull * n, cudaMemcpyHostToDevice));
+        HC_CUDA(ctx, cudaMemcpyAsync(lh.d_mass, hm.data(), 4ull * n, cudaMemcpyHostToDevice, st));
+        HC_CUDA(ctx, cudaMemcpyAsync(lh.d_seqid, hs.data(), 4ull * n, cudaMemcpyHostToDevice, st));
+        HC_CUDA(ctx, cudaMemcpyAsync(lh.d_modnum, hmod.data(), 4ull * n, cudaMemcpyHostToDevice, st));
+        HC_CUDA(ctx, cudaMemcpyAsync(lh.d_sites, hsite.data(), 8ull * n, cudaMemcpyHostToDevice, st));
+        HC_CUDA(ctx, cudaStreamSynchronize(st));
     }
 
     // ion keys -> (k0), sorted with ids -> iA, bucket bounds -> bA
@@ -921,8 +928,7 @@ int build_length_device(hc_ctx *ctx, LenHost &lh, const hc_entry *h_entries, boo
     {
         const uint64_t threads = (uint64_t)n * 2 * ctx->p.maxz;
         k_ion_keys<<<(unsigned)((threads + 127) / 128), 128, 0, st>>>(
-            ctx->d_tables, L, n, lh.d_mass, lh.d_seqid, lh.d_sites, lh.d_modnum, lh.d_seqs, k0,
-            d_uninit);
+            ctx->d_tables, L, n, lh.d_mass, lh.d_seqid, lh.d_sites, lh.d_modnum, lh.d_seqs, k0);
         launches++;
         int bits = 1;
         while ((1ull << bits) < nb) bits++;
@@ -945,9 +951,6 @@ int build_length_device(hc_ctx *ctx, LenHost &lh, const hc_entry *h_entries, boo
         const int rq = build_query_postings(ctx, lh, nullptr, nullptr);
         if (rq) return rq;
     }
-    uint32_t h_uninit = 0;
-    HC_CUDA(ctx, cudaMemcpyAsync(&h_uninit, d_uninit, 4, cudaMemcpyDeviceToHost, st));
-    HC_CUDA(ctx, cudaStreamSynchronize(st));
     lh.built = true;
     ctx->lens_dirty = true;
     ctx->last_launches = launches + 1;
@@ -959,6 +962,35 @@ static IdDiv id_div(uint32_t speclen, uint64_t ids)
     IdDiv d{speclen, 0, 0, ids < 0x80000000ull};
     if (d.fast) division_magic(speclen, &d.magic, &d.sh);
     return d;
+}
+
+// Where the build reads back to, in pinned memory: the codes seen, a total.
+static uint8_t *read_used(hc_ctx *ctx) { return static_cast<uint8_t *>(ctx->h_read); }
+static uint32_t *read_total(hc_ctx *ctx) { return reinterpret_cast<uint32_t *>(read_used(ctx) + kCodes); }
+static_assert(kCodes + 4 <= kReadBytes, "read-back words");
+
+// The entries' class codes; waits for the codes seen and for the query
+// postings' total (qA scanned), read back together.
+static int entry_codes(hc_ctx *ctx, LenHost &lh, Scratch &scr, EntryCodes *ec)
+{
+    cudaStream_t st = ctx->stream;
+    const uint32_t nb = ctx->p.max_mass * ctx->p.scale, n = lh.n;
+    if (n > 0)
+    {
+        uint8_t *used;
+        HC_CUDA(ctx, scr.alloc(&ec->code, n));
+        HC_CUDA(ctx, scr.alloc(&used, (size_t)kCodes));
+        HC_CUDA(ctx, scr.alloc(&ec->bad, (size_t)n));
+        HC_CUDA(ctx, cudaMemsetAsync(used, 0, kCodes, st));
+        k_entry_codes<<<(n + 255) / 256, 256, 0, st>>>((double)ctx->p.min_mass, (double)ctx->p.max_mass, lh.L, n, lh.d_mass,
+                                                       lh.d_seqid, lh.d_sites, lh.d_modnum, lh.d_seqs, ec->code, used,
+                                                       ec->bad);
+        HC_CUDA(ctx, cudaGetLastError());
+        HC_CUDA(ctx, cudaMemcpyAsync(read_used(ctx), used, kCodes, cudaMemcpyDeviceToHost, st));
+    }
+    HC_CUDA(ctx, cudaMemcpyAsync(read_total(ctx), lh.d_qA + nb, 4, cudaMemcpyDeviceToHost, st));
+    HC_CUDA(ctx, cudaStreamSynchronize(st));
+    return HC_SUCCESS;
 }
 
 static unsigned flat_blocks(const hc_ctx *ctx, uint64_t items)
@@ -977,14 +1009,14 @@ int build_query_postings(hc_ctx *ctx, LenHost &lh, const uint32_t *d_ids, const 
     // entry << 3 must stay below 2^32 and below the padding word
     if (lh.n > kQpMaxEntries)
         return set_error(ctx, HC_ERR_INVLD_SIZE, "too many entries of one length for the query postings");
-    cudaFree(lh.d_qA);
-    cudaFree(lh.d_qp);
-    cudaFree(lh.d_qion);
+    dfree(ctx, lh.d_qA);
+    dfree(ctx, lh.d_qp);
+    dfree(ctx, lh.d_qion);
     lh.d_qA = lh.d_qp = nullptr;
     lh.d_qion = nullptr;
-    HC_CUDA(ctx, dalloc(&lh.d_qA, (size_t)nb + 1));
+    HC_CUDA(ctx, dalloc(ctx, &lh.d_qA, (size_t)nb + 1));
     uint32_t *stmp = nullptr, *keys = nullptr;
-    Scratch scr;
+    Scratch scr(ctx);
     HC_CUDA(ctx, scr.alloc(&stmp, scan_tmp_words((size_t)nb + 1)));
     const uint32_t npost = d_ids ? (uint32_t)lh.npost : 0u;
     if (npost && !d_keys)
@@ -995,21 +1027,20 @@ int build_query_postings(hc_ctx *ctx, LenHost &lh, const uint32_t *d_ids, const 
     }
     k_pad_counts<<<flat_blocks(ctx, (uint64_t)nb + 1), 256, 0, st>>>(lh.d_bA, nb, lh.d_qA);
     HC_CUDA(ctx, scan_exclusive(lh.d_qA, (size_t)nb + 1, stmp, st));
-    uint32_t total = 0;
-    HC_CUDA(ctx, cudaMemcpyAsync(&total, lh.d_qA + nb, 4, cudaMemcpyDeviceToHost, st));
-    HC_CUDA(ctx, cudaStreamSynchronize(st));
-    HC_CUDA(ctx, dalloc(&lh.d_qp, (size_t)total + kIaPad));
-    HC_CUDA(ctx, dalloc(&lh.d_qion, (size_t)total + kIaPad));
-    HC_CUDA(ctx, cudaMemsetAsync(lh.d_qp + total, 0xFF, 4 * kIaPad, st));
-    HC_CUDA(ctx, cudaMemsetAsync(lh.d_qion + total, 0, 2 * kIaPad, st));
-    k_qpost_pads<<<flat_blocks(ctx, nb), 256, 0, st>>>(lh.d_bA, lh.d_qA, nb, lh.d_qp, lh.d_qion);
+    EntryCodes ec{};
+    const int rc = entry_codes(ctx, lh, scr, &ec);
+    if (rc) return rc;
+    const uint32_t total = *read_total(ctx);
+    HC_CUDA(ctx, dalloc(ctx, &lh.d_qp, (size_t)total + kIaPad));
+    HC_CUDA(ctx, dalloc(ctx, &lh.d_qion, (size_t)total + kIaPad));
+    k_qpost_pads<<<flat_blocks(ctx, (uint64_t)nb + 1), 256, 0, st>>>(lh.d_bA, lh.d_qA, nb, lh.d_qp, lh.d_qion);
     HC_CUDA(ctx, cudaGetLastError());
-    return build_search(ctx, lh, d_ids, d_keys, npost, lh.d_bA, true);
+    return build_search(ctx, lh, ec, d_ids, d_keys, npost, lh.d_bA, true);
 }
 
 // Classes for the codes seen in `used` that have none yet (ids are only ever
 // added, so the lengths built before keep theirs), and the device copies.
-static int add_classes(hc_ctx *ctx, const std::vector<uint8_t> &used)
+static int add_classes(hc_ctx *ctx, const uint8_t *used)
 {
     bool changed = false;
     for (uint32_t code = 0; code < kCodes; code++)
@@ -1042,47 +1073,33 @@ static int add_classes(hc_ctx *ctx, const std::vector<uint8_t> &used)
 // classed entries, buckets padded to 4 words) and their row table. From `total`
 // ids (entry * speclen + ion, kQpostPad: none) in bucket order, their buckets
 // and the buckets' starts among them; `write`: the query postings too.
-static int build_search(hc_ctx *ctx, LenHost &lh, const uint32_t *d_ids, const uint32_t *d_keys, uint32_t total,
-                        const uint32_t *start, bool write)
+static int build_search(hc_ctx *ctx, LenHost &lh, const EntryCodes &ec, const uint32_t *d_ids, const uint32_t *d_keys,
+                        uint32_t total, const uint32_t *start, bool write)
 {
     cudaStream_t st = ctx->stream;
     const uint32_t nb = ctx->p.max_mass * ctx->p.scale, n = lh.n, Lm1 = lh.L - 1;
     const uint32_t half = ctx->p.maxz * Lm1;
     const IdDiv div = id_div(2 * half, (uint64_t)n * 2 * half);
-    cudaFree(lh.d_rows);
-    cudaFree(lh.d_qAs);
-    cudaFree(lh.d_qps);
-    cudaFree(lh.d_cls);
+    dfree(ctx, lh.d_rows);
+    dfree(ctx, lh.d_qAs);
+    dfree(ctx, lh.d_qps);
+    dfree(ctx, lh.d_cls);
     lh.d_rows = lh.d_qAs = lh.d_qps = nullptr;
     lh.d_cls = nullptr;
-    HC_CUDA(ctx, dalloc(&lh.d_cls, (size_t)n + 4));  // +4: the search reads class bytes in fours
-    HC_CUDA(ctx, dalloc(&lh.d_qAs, (size_t)nb + 1));
-    HC_CUDA(ctx, cudaMemsetAsync(lh.d_cls, (int)kClassNone, (size_t)n + 4, st));
+    HC_CUDA(ctx, dalloc(ctx, &lh.d_cls, (size_t)n + 4));  // +4: the search reads class bytes in fours
+    HC_CUDA(ctx, dalloc(ctx, &lh.d_qAs, (size_t)nb + 1));
     const unsigned eblocks = (n + 255) / 256, bblocks = flat_blocks(ctx, (uint64_t)nb + 1);
     const unsigned pblocks = flat_blocks(ctx, total);
-    Scratch scr;
+    Scratch scr(ctx);
     if (n > 0)
     {
-        uint16_t *code;
-        uint8_t *used, *bad;
-        HC_CUDA(ctx, scr.alloc(&code, n));
-        HC_CUDA(ctx, scr.alloc(&used, (size_t)kCodes));
-        HC_CUDA(ctx, scr.alloc(&bad, (size_t)n));
-        HC_CUDA(ctx, cudaMemsetAsync(used, 0, kCodes, st));
-        HC_CUDA(ctx, cudaMemsetAsync(bad, 0, n, st));
-        k_entry_codes<<<eblocks, 256, 0, st>>>((double)ctx->p.min_mass, (double)ctx->p.max_mass, lh.L, n, lh.d_mass,
-                                              lh.d_seqid, lh.d_sites, lh.d_modnum, lh.d_seqs, code, used);
-        HC_CUDA(ctx, cudaGetLastError());
-        std::vector<uint8_t> hused(kCodes);
-        HC_CUDA(ctx, cudaMemcpyAsync(hused.data(), used, kCodes, cudaMemcpyDeviceToHost, st));
-        HC_CUDA(ctx, cudaStreamSynchronize(st));
-        const int rc = add_classes(ctx, hused);
+        const int rc = add_classes(ctx, read_used(ctx));
         if (rc) return rc;
-        k_entry_classes<<<eblocks, 256, 0, st>>>(code, n, ctx->d_class_of, lh.d_cls);
+        k_entry_classes<<<n / 256 + 2, 256, 0, st>>>(ec.code, n, ctx->d_class_of, lh.d_cls);
         if (total)
             k_qpost<<<pblocks, 256, 0, st>>>(d_ids, d_keys, total, start, lh.d_qA, div, half, Lm1, lh.d_cls, ctx->d_classes,
-                                             bad, write ? lh.d_qp : nullptr, write ? lh.d_qion : nullptr);
-        k_class_fix<<<eblocks, 256, 0, st>>>(lh.d_cls, bad, n);
+                                             ec.bad, write ? lh.d_qp : nullptr, write ? lh.d_qion : nullptr);
+        k_class_fix<<<eblocks, 256, 0, st>>>(lh.d_cls, ec.bad, n);
         HC_CUDA(ctx, cudaGetLastError());
     }
     // the kept postings' bits and counts, the padded bucket sizes from them and
@@ -1100,18 +1117,16 @@ static int build_search(hc_ctx *ctx, LenHost &lh, const uint32_t *d_ids, const u
     k_spost_counts<<<bblocks, 256, 0, st>>>(start, mask, sum, nb, lh.d_qAs);
     HC_CUDA(ctx, cudaGetLastError());
     HC_CUDA(ctx, scan_exclusive(lh.d_qAs, (size_t)nb + 1, stmp, st));
-    uint32_t stotal = 0;
-    HC_CUDA(ctx, cudaMemcpyAsync(&stotal, lh.d_qAs + nb, 4, cudaMemcpyDeviceToHost, st));
+    HC_CUDA(ctx, cudaMemcpyAsync(read_total(ctx), lh.d_qAs + nb, 4, cudaMemcpyDeviceToHost, st));
     HC_CUDA(ctx, cudaStreamSynchronize(st));
-    lh.nsearch = stotal;
-    HC_CUDA(ctx, dalloc(&lh.d_qps, (size_t)stotal + kIaPad));
-    HC_CUDA(ctx, cudaMemsetAsync(lh.d_qps + stotal, 0xFF, 4 * kIaPad, st));
+    lh.nsearch = *read_total(ctx);
+    HC_CUDA(ctx, dalloc(ctx, &lh.d_qps, (size_t)lh.nsearch + kIaPad));
     k_spost_pads<<<bblocks, 256, 0, st>>>(start, mask, sum, nb, lh.d_qAs, off, lh.d_qps);
     if (total)
         k_spost_scatter<<<pblocks, 256, 0, st>>>(d_ids, d_keys, total, div, half, mask, sum, off, lh.d_qps);
     HC_CUDA(ctx, cudaGetLastError());
     lh.stride = (n + kRowG - 1) / kRowG + 1;
-    HC_CUDA(ctx, dalloc(&lh.d_rows, (size_t)nb * lh.stride));
+    HC_CUDA(ctx, dalloc(ctx, &lh.d_rows, (size_t)nb * lh.stride));
     const uint64_t rt = (uint64_t)nb * lh.stride;
     const unsigned blocks = (unsigned)std::min<uint64_t>((rt + 255) / 256, (uint64_t)ctx->sm_count * 64);
     k_row_table<<<blocks, 256, 0, st>>>(lh.d_qAs, lh.d_qps, nb, lh.stride, n, lh.d_rows);
@@ -1125,10 +1140,11 @@ static int build_search(hc_ctx *ctx, LenHost &lh, const uint32_t *d_ids, const u
 int build_rows(hc_ctx *ctx, LenHost &lh)
 {
     const uint32_t nb = ctx->p.max_mass * ctx->p.scale;
-    uint32_t qtotal = 0;
-    HC_CUDA(ctx, cudaMemcpyAsync(&qtotal, lh.d_qA + nb, 4, cudaMemcpyDeviceToHost, ctx->stream));
-    HC_CUDA(ctx, cudaStreamSynchronize(ctx->stream));
-    Scratch scr;
+    Scratch scr(ctx);
+    EntryCodes ec{};
+    const int rc = entry_codes(ctx, lh, scr, &ec);
+    if (rc) return rc;
+    const uint32_t qtotal = *read_total(ctx);
     uint32_t *ids = nullptr, *keys = nullptr;
     HC_CUDA(ctx, scr.alloc(&ids, qtotal));
     HC_CUDA(ctx, scr.alloc(&keys, qtotal));
@@ -1139,7 +1155,7 @@ int build_rows(hc_ctx *ctx, LenHost &lh)
         k_bucket_keys<<<flat_blocks(ctx, qtotal), 256, 0, ctx->stream>>>(lh.d_qA, nb, qtotal, keys);
         HC_CUDA(ctx, cudaGetLastError());
     }
-    return build_search(ctx, lh, ids, keys, qtotal, lh.d_qA, false);
+    return build_search(ctx, lh, ec, ids, keys, qtotal, lh.d_qA, false);
 }
 
 // Checks query postings read from outside (an index file): bucket starts

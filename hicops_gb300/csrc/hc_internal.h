@@ -193,6 +193,12 @@ struct Launch
 struct hc_ctx
 {
     int device = 0;
+    // Index arrays and build scratch come from this pool, ordered on `stream`:
+    // building a length takes some 25 buffers, and cudaMalloc / cudaFree at 10-25 us
+    // each were two thirds of a build. What a build gives back is kept for the
+    // next one up to kPoolKeep bytes; the pool goes with the context.
+    cudaMemPool_t pool = nullptr;
+    void *h_read = nullptr;  // pinned words the build reads counts back through
     int sm_count = 0;
     size_t smem_optin = 0;     // per CTA, opt-in maximum
     size_t smem_sm = 0;        // per SM
@@ -266,7 +272,7 @@ int build_query_postings(hc_ctx *ctx, LenHost &lh, const uint32_t *d_ids, const 
 int build_rows(hc_ctx *ctx, LenHost &lh);  // from query postings: entry classes, search postings and their row table
 void class_keys_of(const hc_params &p, const IonTables &t, uint32_t code, uint32_t *keys);
 int check_query_postings(hc_ctx *ctx, const LenHost &lh, uint64_t qtotal);
-void free_len(LenHost &lh);
+void free_len(hc_ctx *ctx, LenHost &lh);
 int export_ids(hc_ctx *ctx, const LenHost &lh, uint32_t *d_ids);
 
 // hc_query.cu
@@ -293,6 +299,23 @@ int learned_prepare(hc_mlp *m, uint32_t n);
 void learned_gate(const hc_mlp *m, float *max_resid, uint32_t *radius);
 int learned_pipeline(hc_mlp *m, const uint32_t *d_hist, hc_result *d_res, uint32_t n, float *lg, cudaStream_t st,
                      int *launches);
+
+constexpr uint64_t kPoolKeep = 1ull << 30;
+constexpr size_t kReadBytes = 4096;  // hc_ctx::h_read
+
+// hc_api.cpp: device memory of the index and its builds, n elements (at least one)
+cudaError_t pool_alloc(hc_ctx *ctx, void **p, size_t bytes);
+template <class T>
+cudaError_t dalloc(hc_ctx *ctx, T **p, size_t n)
+{
+    return pool_alloc(ctx, (void **)p, sizeof(T) * (n ? n : 1));
+}
+template <class T>
+void dfree(hc_ctx *ctx, T *&p)
+{
+    if (p) cudaFreeAsync(p, ctx->stream);
+    p = nullptr;
+}
 
 int set_error(hc_ctx *ctx, int code, const std::string &msg);
 int cuda_check(hc_ctx *ctx, cudaError_t e, const char *what);

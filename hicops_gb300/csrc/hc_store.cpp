@@ -147,23 +147,25 @@ extern "C" int hc_dslim_restore(hc_ctx *ctx, const char *path)
             shift != kQpEntryShift)
             return set_error(ctx, HC_ERR_FILE_ERROR, "index file does not match this context");
         LenHost &lh = ctx->lens[L - ctx->p.min_len];
-        free_len(lh);
+        free_len(ctx, lh);
         lh.npep = npep;
         lh.n = n;
         lh.npost = npost;
-        cudaError_t e = cudaMalloc((void **)&lh.d_seqs, (size_t)npep * L + 1);
-        if (e == cudaSuccess) e = cudaMalloc((void **)&lh.d_mass, 4ull * n + 4);
-        if (e == cudaSuccess) e = cudaMalloc((void **)&lh.d_seqid, 4ull * n + 4);
-        if (e == cudaSuccess) e = cudaMalloc((void **)&lh.d_sites, 8ull * n + 8);
-        if (e == cudaSuccess) e = cudaMalloc((void **)&lh.d_modnum, 4ull * n + 4);
-        if (e == cudaSuccess) e = cudaMalloc((void **)&lh.d_bA, 4ull * (nb + 1));
-        if (e == cudaSuccess) e = cudaMalloc((void **)&lh.d_qA, 4ull * (nb + 1));
-        if (e == cudaSuccess) e = cudaMalloc((void **)&lh.d_qp, 4ull * (qtotal + kIaPad));
-        if (e == cudaSuccess) e = cudaMemset(lh.d_qp + qtotal, 0xFF, 4ull * kIaPad);
-        if (e == cudaSuccess) e = cudaMalloc((void **)&lh.d_qion, 2ull * (qtotal + kIaPad));
+        cudaError_t e = dalloc(ctx, &lh.d_seqs, (size_t)npep * L + 1);
+        if (e == cudaSuccess) e = dalloc(ctx, &lh.d_mass, (size_t)n + 1);
+        if (e == cudaSuccess) e = dalloc(ctx, &lh.d_seqid, (size_t)n + 1);
+        if (e == cudaSuccess) e = dalloc(ctx, &lh.d_sites, (size_t)n + 1);
+        if (e == cudaSuccess) e = dalloc(ctx, &lh.d_modnum, (size_t)n + 1);
+        if (e == cudaSuccess) e = dalloc(ctx, &lh.d_bA, (size_t)nb + 1);
+        if (e == cudaSuccess) e = dalloc(ctx, &lh.d_qA, (size_t)nb + 1);
+        if (e == cudaSuccess) e = dalloc(ctx, &lh.d_qp, (size_t)qtotal + kIaPad);
+        if (e == cudaSuccess) e = cudaMemsetAsync(lh.d_qp + qtotal, 0xFF, 4ull * kIaPad, ctx->stream);
+        if (e == cudaSuccess) e = dalloc(ctx, &lh.d_qion, (size_t)qtotal + kIaPad);
+        // the file's arrays are copied on the default stream: the buffers are there first
+        if (e == cudaSuccess) e = cudaStreamSynchronize(ctx->stream);
         if (e != cudaSuccess)
         {
-            free_len(lh);
+            free_len(ctx, lh);
             return set_error(ctx, HC_ERR_BAD_MEM_ALLOC, cudaGetErrorString(e));
         }
         bool ok = get_dev(f, lh.d_seqs, (size_t)npep * L, buf);
@@ -173,7 +175,7 @@ extern "C" int hc_dslim_restore(hc_ctx *ctx, const char *path)
         ok = ok && get_dev(f, lh.d_qp, 4ull * qtotal, buf) && get_dev(f, lh.d_qion, 2ull * qtotal, buf);
         if (!ok)
         {
-            free_len(lh);
+            free_len(ctx, lh);
             return set_error(ctx, HC_ERR_FILE_ERROR, "truncated index file");
         }
         lh.L = L;
@@ -190,7 +192,7 @@ extern "C" int hc_dslim_restore(hc_ctx *ctx, const char *path)
         if (rc == HC_SUCCESS) rc = build_rows(ctx, lh);
         if (rc)
         {
-            free_len(lh);
+            free_len(ctx, lh);
             return rc;
         }
         lh.built = true;
