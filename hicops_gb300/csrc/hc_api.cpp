@@ -230,6 +230,7 @@ int hc_ctx_set_tuning(hc_ctx *ctx, const hc_tuning *t)
     if (t->ctas_per_sm * (need + ctx->smem_reserved) > ctx->smem_sm || need > ctx->smem_optin)
         return set_error(ctx, HC_ERR_INVLD_PARAM, "tile does not fit in shared memory");
     ctx->tuning = *t;
+    ctx->auto_shape = false;
     return HC_SUCCESS;
 }
 

@@ -62,6 +62,7 @@ static GraphKey make_key(const hc_ctx *ctx, const uint32_t *d_idx, const uint32_
     key.nspec = nspec;
     key.npeaks = npeaks;
     key.tuning = ctx->tuning;
+    key.auto_shape = ctx->auto_shape ? 1u : 0u;
     key.profiling = ctx->profiling ? 1u : 0u;
     return key;
 }
@@ -131,6 +132,7 @@ int hc_tune(hc_ctx *ctx, const uint32_t *d_idx, const uint32_t *d_moz, const uin
     cudaSetDevice(ctx->device);
     cudaStream_t st = ctx->stream;
     const hc_tuning saved = ctx->tuning;
+    const bool saved_auto = ctx->auto_shape;
     // stage 1: schedule x CTAs per SM x block size x chunks in flight, each with
     // the largest scorecard tile that fits (small windows in the same launch)
     std::vector<hc_tuning> cand;
@@ -210,7 +212,7 @@ int hc_tune(hc_ctx *ctx, const uint32_t *d_idx, const uint32_t *d_moz, const uin
         if (best2 != timed.end() && best2->second.schedule == 2)
         {
             const hc_tuning base = best2->second;
-            for (uint32_t lg : {12u, 15u, 18u})
+            for (uint32_t lg : {13u, 15u, 16u})
             {
                 hc_tuning t = base;
                 t.small_log2 = lg;
@@ -225,6 +227,7 @@ int hc_tune(hc_ctx *ctx, const uint32_t *d_idx, const uint32_t *d_moz, const uin
     if (rc || timed.empty())
     {
         ctx->tuning = saved;
+        ctx->auto_shape = saved_auto;
         return rc ? rc : set_error(ctx, HC_ERR_INVLD_PARAM, "no launch shape could be timed");
     }
     const auto bestp = *std::min_element(timed.begin(), timed.end(),

@@ -175,6 +175,7 @@ struct GraphKey
     uint32_t gate_radius;
     uint32_t nspec, npeaks;
     hc_tuning tuning;
+    uint32_t auto_shape;
     uint32_t profiling;  // stage events captured or not
 };
 
@@ -206,6 +207,7 @@ struct hc_ctx
     hc_params p{};
     cudaStream_t stream = nullptr;
     hc_tuning tuning{};
+    bool auto_shape = true;  // nobody chose a launch shape: picked by what is searched (launch_packed)
     std::vector<hc::LenHost> lens;
     hc::LenDev *d_lens = nullptr;
     hc::IonTables tables{};

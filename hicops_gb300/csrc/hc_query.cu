@@ -13,6 +13,8 @@
 //               qualifying list the moment its shared-peak count reaches
 //               min_shp; listed candidates are scored (dslim_query.cpp:679-725)
 //               into the 1002-bin histogram, cpsms and the top hit.
+//   k_search_small the same for spectra whose windows hold few candidates: all
+//               their windows in one scorecard.
 //   k_search<WIDE> the same for spectra whose packed words could overflow
 //               (a count past 127): 2 x 64-bit words per candidate, exact FP64.
 //   k_tailfit   one thread per spectrum: expeRT::ModelTailFit (expeRT.cpp:572-718)
@@ -76,7 +78,8 @@ struct SearchArgs
     const uint32_t *order;  // optional processing order (longest first)
     const uint32_t *obase;  // optional (device word): the first position of the order this launch takes
     const uint32_t *olim;   // optional (device word): the position it stops at (else nspec)
-    uint32_t always_return; // the stream's atomics always return the old words (no all-pairs peak test)
+    uint32_t wsplit;        // optional: k_search leaves the spectra whose windows hold fewer candidates
+                            // in all, k_search_small those whose windows hold as many or more
     uint32_t persistent;    // 1: CTAs loop over a work counter; 0: one spectrum per CTA
     uint32_t maxz;
     const ClassKeys *classes;   // entry classes (null: none built)
@@ -447,6 +450,37 @@ __device__ __forceinline__ uint32_t find_list(const uint32_t *off, uint32_t n, u
     return lo;
 }
 
+// a spectrum's result, its e-value left open
+__device__ __forceinline__ void write_result(const SearchArgs &a, uint32_t s, uint32_t cpsms, uint32_t flags,
+                                             unsigned long long bytes, unsigned long long best, uint32_t best_shp)
+{
+    hc_result r;
+    r.cpsms = cpsms;
+    r.flags = flags;
+    r.post_bytes = bytes;
+    if (cpsms > 0 && best != 0)
+    {
+        const uint32_t tie = ~(uint32_t)(best & 0xFFFFFFFFu);
+        r.idxoffset = (int32_t)(tie >> 24);
+        r.psid = (int32_t)(tie & 0xFFFFFF);
+        r.hyperscore = __uint_as_float((uint32_t)(best >> 32));
+        r.sharedions = (uint16_t)best_shp;
+        r.totalions = (uint16_t)a.lens[r.idxoffset].speclen;
+    }
+    else
+    {
+        r.idxoffset = -1;
+        r.psid = -1;
+        r.hyperscore = 0.0f;
+        r.sharedions = 0;
+        r.totalions = 0;
+    }
+    r.mu = r.beta = r.minhyp = r.nexthyp = r.maxhyp = 0;
+    r.reported = 0;
+    r.evalue = 0.0;
+    a.out[s] = r;
+}
+
 template <bool WIDE, int G>
 __global__ void __launch_bounds__(G >= 4 ? 512 : 1024, G == 4 ? 2 : 1) k_search(SearchArgs a)
 {
@@ -482,6 +516,8 @@ __global__ void __launch_bounds__(G >= 4 ? 512 : 1024, G == 4 ? 2 : 1) k_search(
     const uint32_t sink_s = (uint32_t)__cvta_generic_to_shared(smem + L.sink) + 4u * (uint32_t)lane;
     uint16_t *wq = reinterpret_cast<uint16_t *>(smem + L.wq) + wid * kWQ;  // this warp's candidate ring (tile < 2^16)
 
+    // k_search_small, launched after this kernel, may take SMs as they fall free
+    if constexpr (!WIDE) asm volatile("griddepcontrol.launch_dependents;");
     for (uint32_t i = tid; i < tile * NW; i += nthr) card[i] = 0;
     if (tid == 0)
     {
@@ -582,7 +618,6 @@ __global__ void __launch_bounds__(G >= 4 ? 512 : 1024, G == 4 ? 2 : 1) k_search(
         __syncthreads();
         const uint32_t s = T.spec;
         if (s == 0xFFFFFFFFu) break;
-        for (int i = kHistSm + tid; i < HC_HIST_BINS; i += nthr) a.hist[(size_t)s * HC_HIST_BINS + i] = 0;
         if (tid == 0)
         {
             T.best = 0;
@@ -600,6 +635,14 @@ __global__ void __launch_bounds__(G >= 4 ? 512 : 1024, G == 4 ? 2 : 1) k_search(
         for (uint32_t l = tid; l < a.nlen; l += nthr) T.win[l] = a.win[(size_t)s * a.nlen + l];
         for (uint32_t i = tid; i < kMaxClasses + 1; i += nthr) ucls[i] = 0ull;
         __syncthreads();
+        if (!WIDE && a.wsplit)
+        {
+            uint32_t c = 0;
+            for (uint32_t l = lane; l < a.nlen; l += 32)
+                if (T.win[l].x <= T.win[l].y) c += (uint32_t)(T.win[l].y - T.win[l].x) + 1u;
+            if (__reduce_add_sync(0xFFFFFFFFu, c) < a.wsplit) continue;  // k_search_small's
+        }
+        for (int i = kHistSm + tid; i < HC_HIST_BINS; i += nthr) a.hist[(size_t)s * HC_HIST_BINS + i] = 0;
         // valid peaks (dslim_query.cpp:625): dF < qion < max*scale - 1 - dF
         {
             const uint32_t lowlim = a.classes ? __ldg(&a.classes->maxkey) + a.dF : 0u;
@@ -628,13 +671,7 @@ __global__ void __launch_bounds__(G >= 4 ? 512 : 1024, G == 4 ? 2 : 1) k_search(
         // its own (valid peaks more than 2*dF bins apart), a candidate's b (y)
         // count is at most its number of b (y) ions, (L-1)*maxz, below 128 for
         // every length; with intensities below 2^17 the sums stay below 2^24.
-        // (The small-window launch skips the all-pairs test: its spectra visit
-        // few postings, so returning atomics cost less than the test.)
-        if (!WIDE && a.always_return)
-        {
-            if (tid == 0) T.noret = 0u;
-        }
-        else if constexpr (!WIDE)
+        if constexpr (!WIDE)
         {
             // warp w takes peaks i = w, w + nw, ...; its lanes the peaks j > i
             bool close = false;
@@ -1218,40 +1255,477 @@ __global__ void __launch_bounds__(G >= 4 ? 512 : 1024, G == 4 ? 2 : 1) k_search(
             continue;
         }
         for (int i = tid; i < kHistSm; i += nthr) a.hist[(size_t)s * HC_HIST_BINS + i] = T.u.run.hist[i];
-        if (tid == 0)
-        {
-            hc_result r;
-            r.cpsms = T.cpsms;
-            r.flags = T.flags;
-            r.post_bytes = T.bytes;
-            if (T.cpsms > 0 && T.best != 0)
-            {
-                const uint32_t tie = ~(uint32_t)(T.best & 0xFFFFFFFFu);
-                r.idxoffset = (int32_t)(tie >> 24);
-                r.psid = (int32_t)(tie & 0xFFFFFF);
-                r.hyperscore = __uint_as_float((uint32_t)(T.best >> 32));
-                r.sharedions = (uint16_t)T.best_shp;
-                r.totalions = (uint16_t)a.lens[r.idxoffset].speclen;
-            }
-            else
-            {
-                r.idxoffset = -1;
-                r.psid = -1;
-                r.hyperscore = 0.0f;
-                r.sharedions = 0;
-                r.totalions = 0;
-            }
-            r.mu = r.beta = r.minhyp = r.nexthyp = r.maxhyp = 0;
-            r.reported = 0;
-            r.evalue = 0.0;
-            a.out[s] = r;
-        }
+        if (tid == 0) write_result(a, s, T.cpsms, T.flags, T.bytes, T.best, T.best_shp);
     }
     if (a.phase && tid == 0)
     {
         for (int k = 0; k < kPhases; k++) atomicAdd(&a.phase[k], T.ph[k]);
         for (int k = 0; k < 4; k++) atomicAdd(&a.phase[kPhases + k], T.cnt[k]);
     }
+}
+
+// ---- the search of small windows ------------------------------------------------
+// k_search gives a length of a spectrum's windows a job of its own: list bounds,
+// chunk offsets, two barriers, whatever the window holds. Where windows hold a few
+// hundred candidates (a small database, a narrow tolerance) that fixed work is all
+// there is: 34 jobs a spectrum, most of their lists empty, some 2,500 warp
+// instructions each. k_search_small packs the windows of all lengths into one
+// scorecard instead (each from a multiple of 128 candidates on, so that a step of the
+// scan lies in one length) and walks the (length, list) pairs flat, a thread a
+// pair: its two row-table words say whether the list holds anything; the non-empty
+// ones (a tenth, in a database of 20,000 peptides) go through a ring of the warp's
+// and are read 32 at a time, a lane a list, long ones by the whole warp. A spectrum
+// whose windows together exceed the scorecard takes it as often as it needs.
+// The same results as k_search: the same words, the same scoring.
+constexpr int kSmThreads = 256;      // threads of a CTA
+constexpr uint32_t kSmTile = 3584;   // candidates of the scorecard (a multiple of 128, < 2^16): four CTAs an SM
+                                     // then leave it the 60 KB of L1 (see kSmemKeepL1)
+constexpr uint32_t kSmRing = 64;     // lists waiting per warp (a power of two, >= 31 + 32)
+constexpr uint32_t kSmLong = 8;      // chunks from which the warp reads a list together
+constexpr uint32_t kSmStep = 128;
+constexpr uint32_t kSmCtas = 4;
+// launch shapes picked for a context that chose none (see launch_packed)
+constexpr uint32_t kAutoSmallLog2 = 15, kAutoAllSmall = 1u << 16, kAutoOrder = 1024;
+
+struct SmSeg
+{
+    const uint32_t *rows;  // of the first bucket, at the segment's first row-table entry
+    const uint32_t *qp;
+    uint32_t stride, drow;  // ... and how far its last one is
+    uint32_t off, lim;      // byte offset of its first entry's words, bytes of its words
+    uint32_t card;          // where they lie in the scorecard (shared-window address)
+};
+
+struct SmSmem
+{
+    uint32_t card[2 * kSmTile];
+    uint2 ring[kSmThreads / 32][kSmRing];
+    uint16_t wq[kSmThreads / 32][kWQ];
+    uint2 defer[kDefer];
+    unsigned long long ucls[kMaxClasses + 1];
+    SmSeg seg[HC_MAX_LENGTHS];
+    uint32_t low[HC_QALEN];
+    uint32_t pmoz[HC_QALEN], pint[HC_QALEN];
+    uint32_t upk[kMaxClasses + 1];
+    float lgf[kLgTable];  // (all of it: an overflowing count, redone wide, reads inside)
+    uint32_t hist[kHistSm];
+    int2 win[HC_MAX_LENGTHS];
+    uint32_t vbase[HC_MAX_LENGTHS + 1];  // first packed candidate of each length
+    uint32_t sink[32];
+    uint8_t stepl[kSmTile / kSmStep];    // the length a step of the scan lies in (0xFF: none)
+    unsigned long long best, bytes;
+    uint32_t best_shp, maxbits, cpsms, flags, overflow, spec, nv, nlow, ndefer, nseg, cand;
+};
+
+static size_t small_smem(uint32_t dF) { return sizeof(SmSmem) + 4 * (size_t)HC_QALEN * (2 * dF + 1); }
+
+__global__ void __launch_bounds__(kSmThreads, 4) k_search_small(SearchArgs a)
+{
+    extern __shared__ __align__(16) unsigned char smem[];
+    SmSmem &S = *reinterpret_cast<SmSmem *>(smem);
+    uint32_t *lbkt = reinterpret_cast<uint32_t *>(smem + sizeof(SmSmem));  // bucket of each list
+    const int tid = threadIdx.x, lane = tid & 31, wid = tid >> 5;
+    constexpr int nthr = kSmThreads;
+    const uint32_t nbin = 2 * a.dF + 1;
+    const uint32_t card_s = (uint32_t)__cvta_generic_to_shared(S.card);
+    const uint32_t sink_s = (uint32_t)__cvta_generic_to_shared(S.sink) + 4u * (uint32_t)lane;
+    uint16_t *wq = S.wq[wid];
+    uint2 *ring = S.ring[wid];
+    for (int i = tid; i < kLgTable; i += nthr) S.lgf[i] = a.qc->lgfact_f[i];
+
+    uint32_t my_cps = 0, my_fl = 0, my_shp = 0;
+    unsigned long long my_best = 0;
+    auto hist_add = [&](int bin) {
+        if (bin < kHistSm) atomicAdd(&S.hist[bin], 1u);
+        else atomicAdd(&a.hist[(size_t)S.spec * HC_HIST_BINS + (uint32_t)bin], 1u);
+    };
+    auto count_psm = [&](uint32_t bc, uint32_t yc, int bin) {
+        my_cps++;
+        if (bc >= (uint32_t)kRefMaxShp || yc >= (uint32_t)kRefMaxShp) my_fl |= HC_FLAG_LGFACT_OOB;
+        if (bin >= HC_HIST_BINS || bin < 0) { my_fl |= HC_FLAG_HIST_OOB; bin = bin < 0 ? 0 : HC_HIST_BINS - 1; }
+        hist_add(bin);
+    };
+    // one candidate, as k_search scores it
+    auto score_one = [&](uint32_t wb, uint32_t wy, uint32_t key_lo) {
+        uint32_t bc, yc, shp;
+        uint64_t ib, iy;
+        decode_packed(wb, wy, bc, yc, shp, ib, iy);
+        const float ha = approx_h(S.lgf, bc, yc, ib, iy);
+        const float runmax = __uint_as_float(*(volatile uint32_t *)&S.maxbits);
+        if (ha >= runmax - kNear)
+        {
+            if (ha > runmax) atomicMax(&S.maxbits, __float_as_uint(ha));
+            const float he = exact_h(a.qc, bc, yc, ib, iy);
+            if (he > 0.0f)
+            {
+                const unsigned long long key = ((unsigned long long)__float_as_uint(he) << 32) | key_lo;
+                if (key > my_best)
+                {
+                    my_best = key;
+                    my_shp = shp;
+                }
+                atomicMax(&S.best, key);
+            }
+        }
+        const float tt = ha * 10.0f + 0.5f;
+        const float fr = tt - floorf(tt);
+        if (fabsf(ha) <= kApproxErr * 4.0f || fr < kBinMargin || fr > 1.0f - kBinMargin)
+        {
+            const uint32_t di = atomicAdd(&S.ndefer, 1u);
+            if (di < a.defer_cap)
+            {
+                S.defer[di] = make_uint2(wb, wy);
+                return;
+            }
+            const float h = exact_h(a.qc, bc, yc, ib, iy);
+            if (h > 0.0f) count_psm(bc, yc, hist_bin(h));
+        }
+        else if (ha > 0.0f) count_psm(bc, yc, (int)floorf(tt));
+    };
+
+    for (uint32_t iter = 0;; iter++)
+    {
+        __syncthreads();
+        if (tid == 0)
+        {
+            const uint32_t w = atomicAdd(a.work, 1u);
+            const uint32_t o = (a.obase ? *a.obase : 0u) + w;
+            S.spec = w < a.nspec && o < a.nspec ? (a.order ? a.order[o] : o) : 0xFFFFFFFFu;
+            S.best = 0;
+            S.best_shp = 0;
+            S.maxbits = 0;
+            S.cpsms = 0;
+            S.ndefer = 0;
+            S.flags = 0;
+            S.overflow = 0;
+            S.bytes = 0;
+            S.nv = 0;
+            S.nlow = 0;
+        }
+        for (uint32_t i = tid; i < kMaxClasses + 1; i += nthr) S.ucls[i] = 0ull;
+        __syncthreads();
+        const uint32_t s = S.spec;
+        if (s == 0xFFFFFFFFu) break;
+        // the windows' places in the packed candidates, by warp 0 (two lengths a lane)
+        if (wid == 0)
+        {
+            uint32_t sz[2], tot = 0, cand = 0;
+#pragma unroll
+            for (int h = 0; h < 2; h++)
+            {
+                const uint32_t l = 2 * (uint32_t)lane + h;
+                const int2 w = l < a.nlen ? a.win[(size_t)s * a.nlen + l] : make_int2(1, 0);
+                S.win[l] = w;
+                sz[h] = w.x <= w.y ? ((uint32_t)(w.y - w.x) + kSmStep) / kSmStep * kSmStep : 0u;
+                tot += sz[h];
+                cand += w.x <= w.y ? (uint32_t)(w.y - w.x) + 1u : 0u;
+            }
+            cand = __reduce_add_sync(0xFFFFFFFFu, cand);
+            if (lane == 0) S.cand = cand;
+            uint32_t x = tot;
+#pragma unroll
+            for (int o = 1; o < 32; o <<= 1)
+            {
+                const uint32_t y = __shfl_up_sync(0xFFFFFFFFu, x, o);
+                if (lane >= o) x += y;
+            }
+            S.vbase[2 * lane] = x - tot;
+            S.vbase[2 * lane + 1] = x - tot + sz[0];
+            if (lane == 31) S.vbase[HC_MAX_LENGTHS] = x;
+        }
+        // valid peaks (dslim_query.cpp:625): dF < qion < max*scale - 1 - dF
+        else
+        {
+            const uint32_t lowlim = a.classes ? __ldg(&a.classes->maxkey) + a.dF : 0u;
+            const uint32_t p1 = a.idx[s + 1];
+            for (uint32_t k = a.idx[s] + tid - 32; k < p1; k += nthr - 32)
+            {
+                const uint32_t q = a.moz[k];
+                if (q > a.dF && (uint64_t)q + 1 + a.dF < a.maxbin)
+                {
+                    const uint32_t in = a.inten[k];
+                    // packed sums stay exact only for intensities below 2^17
+                    if (in >= (1u << 17)) S.overflow = 1;
+                    const uint32_t slot = atomicAdd(&S.nv, 1u);
+                    if (slot < HC_QALEN)
+                    {
+                        S.pmoz[slot] = q;
+                        S.pint[slot] = in;
+                        if (q <= lowlim) S.low[atomicAdd(&S.nlow, 1u)] = slot;
+                    }
+                }
+            }
+        }
+        __syncthreads();
+        if (a.wsplit && S.cand >= a.wsplit) continue;  // k_search's
+        for (int i = tid; i < HC_HIST_BINS; i += nthr)
+        {
+            if (i < kHistSm) S.hist[i] = 0;
+            else a.hist[(size_t)s * HC_HIST_BINS + i] = 0;
+        }
+        const uint32_t nv = S.nv < HC_QALEN ? S.nv : HC_QALEN;
+        const uint32_t np = nv * nbin, vtot = S.vbase[HC_MAX_LENGTHS];
+        // the class adds (see k_search), the lists' buckets
+        if (a.classes)
+        {
+            const uint32_t nz = a.maxz, tot = a.classes->n * nz, nlow = S.nlow;
+            for (uint32_t i = tid; i < tot; i += nthr)
+            {
+                const uint32_t c = i / nz, z = i - c * nz;
+                const uint32_t key = a.classes->key[c][z];
+                unsigned long long acc = 0;
+                for (uint32_t t = 0; t < nlow; t++)
+                {
+                    const uint32_t sl = S.low[t], q = S.pmoz[sl];
+                    if (q <= key + a.dF && q + a.dF >= key) acc += (1ull << 40) | S.pint[sl];
+                }
+                if (acc) atomicAdd(&S.ucls[c], acc);
+            }
+        }
+        for (uint32_t i = tid; i < np; i += nthr)
+        {
+            const uint32_t k = i / nbin;
+            lbkt[i] = S.pmoz[k] - a.dF + (i - k * nbin);
+        }
+        __syncthreads();
+        for (uint32_t i = tid; i < kMaxClasses + 1; i += nthr)
+        {
+            // packed: a count of 64 or more from a class alone is redone wide
+            const unsigned long long u = S.ucls[i];
+            if ((u >> 40) >= 64u) S.overflow = 1;
+            S.upk[i] = ((uint32_t)(u >> 40) << 24) | (uint32_t)(u & 0xFFFFFFull);
+        }
+        if (tid < (int)a.nlen && S.win[tid].x <= S.win[tid].y)
+            atomicAdd(&S.bytes, 4ull * (2 * a.dF + 2) * nv);  // the reference's bA reads
+        my_best = 0;
+        my_shp = my_cps = my_fl = 0;
+        uint32_t npass = 0, ovf = 0;
+        for (uint32_t v0 = 0; v0 < vtot; v0 += kSmTile)
+        {
+            const uint32_t v1 = min(vtot, v0 + kSmTile), used = v1 - v0;
+            // the steps' lengths and the lengths' pieces of this scorecard
+            if (tid < (int)(kSmTile / kSmStep))
+            {
+                const uint32_t v = v0 + kSmStep * (uint32_t)tid;
+                uint32_t l = 0xFFu;
+                if (v < v1)
+                {
+                    uint32_t lo = 0, hi = HC_MAX_LENGTHS - 1;  // the last length with vbase <= v
+                    while (lo < hi)
+                    {
+                        const uint32_t m = (lo + hi + 1) >> 1;
+                        if (S.vbase[m] <= v) lo = m;
+                        else hi = m - 1;
+                    }
+                    l = lo;
+                }
+                S.stepl[tid] = (uint8_t)l;
+            }
+            // (lengths in order: the pieces' list is the range [l0, l1] of those not empty here)
+            if (wid == kSmThreads / 32 - 1)
+            {
+                uint32_t n = 0;
+                for (int h = 0; h < 2; h++)
+                {
+                    const uint32_t l = 32 * h + (uint32_t)lane;
+                    const uint32_t b0 = S.vbase[l], b1 = S.vbase[l + 1];
+                    const bool in = b0 < b1 && b0 < v1 && b1 > v0;
+                    const uint32_t bal = __ballot_sync(0xFFFFFFFFu, in);
+                    if (in)
+                    {
+                        const int2 w = S.win[l];
+                        const uint32_t skip = v0 > b0 ? v0 - b0 : 0u;  // candidates of earlier scorecards
+                        const uint32_t c0 = (uint32_t)w.x + skip, c1 = min((uint32_t)w.y + 1u, c0 + (v1 - max(b0, v0)));
+                        const LenS d = a.len[l];
+                        SmSeg g;
+                        g.rows = d.rows + c0 / kRowG;
+                        g.qp = d.qp;
+                        g.stride = d.stride;
+                        g.drow = (c1 + kRowG - 1) / kRowG - c0 / kRowG;
+                        g.off = c0 << kQpEntryShift;
+                        g.lim = (c1 - c0) << kQpEntryShift;
+                        g.card = card_s + 8u * (max(b0, v0) - v0);
+                        S.seg[n + (uint32_t)__popc(bal & ((1u << lane) - 1u))] = g;
+                    }
+                    n += (uint32_t)__popc(bal);
+                }
+                if (lane == 0) S.nseg = n;
+            }
+            __syncthreads();
+            const uint32_t nseg = S.nseg;
+            // every candidate's start: b word zero, y word its class's adds (zero past its window)
+            for (uint32_t c = 4 * (uint32_t)tid; c < used; c += 4 * nthr)
+            {
+                const uint32_t l = S.stepl[c / kSmStep];
+                const int2 w = S.win[l];
+                const uint32_t e = (uint32_t)w.x + (v0 + c - S.vbase[l]);  // entry of the first of four
+                const uint8_t *cl = a.len[l].cls + e;
+                const uint32_t left = (uint32_t)w.y + 1u > e ? (uint32_t)w.y + 1u - e : 0u;
+                uint32_t y[4];
+#pragma unroll
+                for (int i = 0; i < 4; i++)
+                {
+                    y[i] = (uint32_t)i < left ? S.upk[__ldg(cl + i)] : 0u;
+                    npass += y[i] >> 24;
+                }
+                uint4 *z4 = reinterpret_cast<uint4 *>(S.card);
+                z4[c >> 1] = make_uint4(0u, y[0], 0u, y[1]);
+                z4[(c >> 1) + 1] = make_uint4(0u, y[2], 0u, y[3]);
+            }
+            __syncthreads();
+            // ---- the lists: (piece, list) pairs, a thread a pair ----
+            auto add4 = [&](const uint4 v, const SmSeg &g, uint32_t inten) {
+                const uint32_t add = (1u << 24) | inten;
+                const uint32_t xs[4] = {v.x, v.y, v.z, v.w};
+#pragma unroll
+                for (int e = 0; e < 4; e++)
+                {
+                    const uint32_t o = xs[e] - g.off;
+                    const bool in = o < g.lim;
+                    const uint32_t old = atom_shared_add(in ? g.card + o : sink_s, add);
+                    ovf |= in ? old : 0u;
+                    npass += in ? 1u : 0u;
+                }
+            };
+            uint32_t qn = 0, qh = 0;  // ring fill and head (warp-uniform)
+            auto drain = [&](uint32_t cnt) {
+                __syncwarp();
+                if ((uint32_t)lane < cnt)
+                {
+                    const uint2 r = ring[(qh + (uint32_t)lane) & (kSmRing - 1)];
+                    const SmSeg g = S.seg[r.y >> 20];
+                    const uint32_t pr = (r.y >> 4) & 0xFFFFu, nch = r.y & 0xFu;
+                    const uint4 *p = reinterpret_cast<const uint4 *>(g.qp) + r.x;
+                    const uint32_t inten = S.pint[pr / nbin];
+                    uint4 v = __ldg(p);
+                    for (uint32_t c = 1; c < nch; c++)
+                    {
+                        const uint4 nx = __ldg(p + c);
+                        add4(v, g, inten);
+                        v = nx;
+                    }
+                    add4(v, g, inten);
+                }
+                __syncwarp();
+                qh += cnt;
+                qn -= cnt;
+            };
+            constexpr int U = 4;  // pairs whose row-table words are in flight
+            uint32_t sg = np ? (uint32_t)tid / np : 0u, pr = (uint32_t)tid - sg * np;
+            const uint32_t dsg = np ? nthr / np : 0u, dpr = nthr - dsg * np;
+            const uint32_t pairs = nseg * np, iters = (pairs + nthr * U - 1) / (nthr * U);
+            for (uint32_t it = 0; it < iters; it++)
+            {
+                uint32_t st[U], en[U], id[U];
+#pragma unroll
+                for (int u = 0; u < U; u++)
+                {
+                    st[u] = en[u] = 0;
+                    id[u] = (sg << 20) | (pr << 4);
+                    if (sg < nseg)
+                    {
+                        const SmSeg &g = S.seg[sg];
+                        const uint32_t *col = g.rows + (size_t)lbkt[pr] * g.stride;
+                        st[u] = __ldg(col);
+                        en[u] = __ldg(col + g.drow);
+                    }
+                    sg += dsg;
+                    pr += dpr;
+                    if (pr >= np) { pr -= np; sg++; }
+                }
+#pragma unroll
+                for (int u = 0; u < U; u++)
+                {
+                    const uint32_t nch = st[u] < en[u] ? ((en[u] + 3) >> 2) - (st[u] >> 2) : 0u;
+                    const bool shrt = nch != 0u && nch < kSmLong;
+                    const uint32_t b = __ballot_sync(0xFFFFFFFFu, shrt);
+                    if (shrt)
+                        ring[(qh + qn + (uint32_t)__popc(b & ((1u << lane) - 1u))) & (kSmRing - 1)] =
+                            make_uint2(st[u] >> 2, id[u] | nch);
+                    qn += (uint32_t)__popc(b);
+                    if (qn >= 32) drain(32);
+                    for (uint32_t lb = __ballot_sync(0xFFFFFFFFu, nch >= kSmLong); lb; lb &= lb - 1)
+                    {
+                        const int src = __ffs(lb) - 1;
+                        const uint32_t q0 = __shfl_sync(0xFFFFFFFFu, st[u] >> 2, src);
+                        const uint32_t n = __shfl_sync(0xFFFFFFFFu, nch, src), i = __shfl_sync(0xFFFFFFFFu, id[u], src);
+                        const SmSeg g = S.seg[i >> 20];
+                        const uint32_t inten = S.pint[((i >> 4) & 0xFFFFu) / nbin];
+                        for (uint32_t c = (uint32_t)lane; c < n; c += 32)
+                            add4(__ldg(reinterpret_cast<const uint4 *>(g.qp) + q0 + c), g, inten);
+                    }
+                }
+            }
+            if (qn) drain(qn);
+            __syncthreads();
+            // ---- every candidate that reached min_shp (see k_search's scan) ----
+            const uint4 *c4 = reinterpret_cast<const uint4 *>(S.card);
+            uint32_t fill = 0, head = 0;
+            auto pop_score = [&](uint32_t cnt) {
+                __syncwarp();
+                if ((uint32_t)lane < cnt)
+                {
+                    const uint32_t loc = wq[(head + (uint32_t)lane) & (kWQ - 1)];
+                    const uint32_t l = S.stepl[loc / kSmStep];
+                    const uint32_t e = (uint32_t)S.win[l].x + (v0 + loc - S.vbase[l]);
+                    const uint2 w = reinterpret_cast<const uint2 *>(S.card)[loc];
+                    score_one(w.x, w.y, ~((l << 24) | (e & 0xFFFFFFu)));
+                }
+                __syncwarp();
+                head += cnt;
+                fill -= cnt;
+            };
+            for (uint32_t base = 64 * (uint32_t)wid; base < used; base += 64 * (nthr / 32))
+            {
+                const uint32_t c = base + 2 * (uint32_t)lane;
+                const uint4 w = c4[c >> 1];
+                const uint32_t s0 = (w.x >> 24) + (w.y >> 24), s1 = (w.z >> 24) + (w.w >> 24);
+                const bool q0 = s0 >= a.thr, q1 = s1 >= a.thr;  // (words past a window are zero; thr >= 1)
+                const uint32_t b0 = __ballot_sync(0xFFFFFFFFu, q0), b1 = __ballot_sync(0xFFFFFFFFu, q1);
+                if ((b0 | b1) == 0) continue;
+                const uint32_t lt = (1u << lane) - 1u;
+                const uint32_t r = head + fill + (uint32_t)(__popc(b0 & lt) + __popc(b1 & lt));
+                if (q0) wq[r & (kWQ - 1)] = (uint16_t)c;
+                if (q1) wq[(r + (q0 ? 1u : 0u)) & (kWQ - 1)] = (uint16_t)(c + 1);
+                fill += (uint32_t)(__popc(b0) + __popc(b1));
+                while (fill >= 32) pop_score(32);
+            }
+            if (fill) pop_score(fill);
+            __syncthreads();
+        }
+        if ((__reduce_or_sync(0xFFFFFFFFu, ovf) & 0x80000000u) && lane == 0) S.overflow = 1;
+        // ---- candidates whose sign or bin the float estimate left open ----
+        for (uint32_t i = tid; i < min(S.ndefer, a.defer_cap); i += nthr)
+        {
+            uint32_t bc, yc, shp;
+            uint64_t ib, iy;
+            const uint2 w = S.defer[i];
+            decode_packed(w.x, w.y, bc, yc, shp, ib, iy);
+            const float h = exact_h(a.qc, bc, yc, ib, iy);
+            if (h > 0.0f) count_psm(bc, yc, hist_bin(h));
+        }
+        my_cps = __reduce_add_sync(0xFFFFFFFFu, my_cps);
+        my_fl = __reduce_or_sync(0xFFFFFFFFu, my_fl);
+        npass = __reduce_add_sync(0xFFFFFFFFu, npass);
+        if (lane == 0)
+        {
+            if (my_cps) atomicAdd(&S.cpsms, my_cps);
+            if (my_fl) atomicOr(&S.flags, my_fl);
+            if (npass) atomicAdd(&S.bytes, 4ull * npass);  // postings visited: those of entries inside the windows
+        }
+        // the top hit's shared ions come from the thread that found it
+        if (my_best != 0 && my_best == S.best) S.best_shp = my_shp;
+        __syncthreads();
+        if (S.overflow)
+        {
+            if (tid == 0) a.wide_list[atomicAdd(a.nwide, 1u)] = s;
+            continue;
+        }
+        for (int i = tid; i < kHistSm; i += nthr) a.hist[(size_t)s * HC_HIST_BINS + i] = S.hist[i];
+        if (tid == 0) write_result(a, s, S.cpsms, S.flags, S.bytes, S.best, S.best_shp);
+    }
+    // what follows this kernel follows the k_search it may have overlapped too
+    asm volatile("griddepcontrol.wait;" ::: "memory");
 }
 
 // ---- windows: DSLIM_BinarySearch (dslim_query.cpp:854-994) -----------------
@@ -2002,22 +2476,79 @@ static int grow(hc_ctx *ctx, T **p, size_t *cap, size_t need)
     return HC_SUCCESS;
 }
 
-// The packed search of a batch: with schedule 2 the longest-first order first,
-// then one launch of the tuned shape or, when small windows have their own
-// launch, two: the tuned shape takes the order up to the split point and
-// 128-thread CTAs, kSmallCtas per SM, the rest (spectra that are mostly
-// fixed per-job latency gain from more of them in flight per SM). Both read
-// their range of the order on the device.
-constexpr uint32_t kSmallThreads = 128, kSmallCtas = 6;
-
-static int launch_packed(hc_ctx *ctx, SearchArgs &a, uint32_t sched, uint32_t nspec, uint32_t nlen, const int2 *win,
-                         uint32_t *order, uint32_t *work, cudaStream_t st, int &launches, bool stages)
+// The search of small windows: the spectra of the order from *obase on (null: all, in
+// batch order). `after`: it was preceded by k_search on the same order, which it
+// does not depend on; its CTAs start as k_search's leave SMs free.
+static int launch_small(hc_ctx *ctx, SearchArgs s, uint32_t nspec, const uint32_t *obase, uint32_t *work, bool after,
+                        cudaStream_t st)
 {
-    const hc_tuning &t = ctx->tuning;
-    const uint32_t small_tile = max_tile_for(ctx, a.dF, kSmallCtas, kSmallThreads);
-    const bool split = sched == 2 && t.small_log2 != 0 && small_tile >= kRowG;
+    s.obase = obase;
+    s.olim = nullptr;
+    s.work = work + kWkSmall;
+    const size_t smem = small_smem(s.dF);
+    HC_CUDA(ctx, cudaFuncSetAttribute(k_search_small, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+    cudaLaunchAttribute at{};
+    at.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    at.val.programmaticStreamSerializationAllowed = 1;
+    cudaLaunchConfig_t lc{};
+    lc.gridDim = dim3(std::min<uint32_t>(nspec, (uint32_t)ctx->sm_count * kSmCtas));
+    lc.blockDim = dim3(kSmThreads);
+    lc.dynamicSmemBytes = smem;
+    lc.stream = st;
+    lc.attrs = &at;
+    lc.numAttrs = after ? 1 : 0;
+    HC_CUDA(ctx, cudaLaunchKernelEx(&lc, k_search_small, s));
+    return HC_SUCCESS;
+}
+
+// The packed search of a batch: with schedule 2 the longest-first order first,
+// then the tuned shape, or, when small windows have their own launch, two: the
+// tuned shape takes the order up to the split point and k_search_small the rest.
+// Both read their range of the order on the device.
+//
+// A context whose launch shape nobody chose (neither hc_tune nor
+// hc_ctx_set_tuning) gets one by what is searched. k_search_small takes the
+// spectra whose windows hold fewer than 2^15 candidates: search times of 3,000
+// spectra, all in k_search_small / all in two 512-thread k_search CTAs per SM, at
+// about 2 k candidates a spectrum 191 / 455 us, 9 k 358 / 692, 45 k 908 / 926 and,
+// in a larger index, 1,013 / 862, 220 k 3,833 / 2,377. An index of fewer than 2^16
+// entries has next to no others. Else both kernels are launched: up to kAutoOrder
+// spectra each passes over the other's (the order's two kernels take longer than
+// that), beyond it the order splits the batch. k_search runs as one 1024-thread CTA
+// per SM while a CTA has at most one spectrum (8 spectra of 220 k candidates 199 us
+// against 257), as two of 512 beyond that (3,000 spectra 2,380 us against 2,946).
+static int launch_packed(hc_ctx *ctx, SearchArgs &a, uint32_t nspec, uint32_t nlen, const int2 *win, uint32_t *order,
+                         uint32_t *work, cudaStream_t st, int &launches, bool stages)
+{
+    hc_tuning t = ctx->tuning;
+    bool all_small = false;
+    a.wsplit = 0;
+    if (ctx->auto_shape)
+    {
+        uint64_t entries = 0;
+        for (const LenHost &lh : ctx->lens) entries += lh.built ? lh.n : 0u;
+        all_small = entries < kAutoAllSmall;
+        const uint32_t tile = max_tile_for(ctx, a.dF, 2, 512);
+        if (nspec > (uint32_t)ctx->sm_count && tile >= kRowG)
+        {
+            t.threads = 512;
+            t.ctas_per_sm = 2;
+            t.pairs_per_warp = 4;
+            t.tile = tile;
+        }
+        if (nspec > kAutoOrder)
+        {
+            t.schedule = 2;
+            t.small_log2 = kAutoSmallLog2;
+        }
+        else
+            a.wsplit = 1u << kAutoSmallLog2;
+    }
+    a.tile = t.tile;
+    a.persistent = t.schedule != 1;
     a.obase = a.olim = nullptr;
-    if (sched == 2)
+    const bool split = t.schedule == 2 && t.small_log2 != 0;
+    if (t.schedule == 2 && !all_small)
     {
         uint32_t *cls = order + nspec;
         k_cost<<<(nspec + 255) / 256, 256, 0, st>>>(win, nspec, nlen, cls, work + kWkCnt);
@@ -2030,19 +2561,17 @@ static int launch_packed(hc_ctx *ctx, SearchArgs &a, uint32_t sched, uint32_t ns
     }
     // the search stage: the packed launches
     if (stages) HC_CUDA(ctx, record_stage(ctx, 1, st));
-    const size_t smem = search_smem(a.tile, a.dF, false, t.threads);
-    const int grid = sched == 1 ? (int)nspec : ctx->sm_count * (int)t.ctas_per_sm;
-    int rc = launch_search<false>(ctx, a, grid, t.threads, smem, t.pairs_per_warp, st);
-    if (rc || !split) return rc;
-    SearchArgs s = a;
-    s.obase = work + kWkSplit;
-    s.olim = nullptr;
-    s.work = work + kWkSmall;
-    s.tile = small_tile;
-    s.always_return = 1;
+    if (all_small)
+    {
+        a.wsplit = 0;
+        return launch_small(ctx, a, nspec, nullptr, work, false, st);
+    }
+    const size_t smem = search_smem(t.tile, a.dF, false, t.threads);
+    const int grid = t.schedule == 1 ? (int)nspec : ctx->sm_count * (int)t.ctas_per_sm;
+    const int rc = launch_search<false>(ctx, a, grid, t.threads, smem, t.pairs_per_warp, st);
+    if (rc || !(split || a.wsplit)) return rc;
     launches++;
-    return launch_search<false>(ctx, s, ctx->sm_count * (int)kSmallCtas, kSmallThreads,
-                                search_smem(small_tile, s.dF, false, kSmallThreads), 2, st);
+    return launch_small(ctx, a, nspec, split ? work + kWkSplit : nullptr, work, true, st);
 }
 
 // the tail fit of spectra [0, n), or of a list of at most n
@@ -2071,8 +2600,8 @@ int query_device(hc_ctx *ctx, const uint32_t *d_idx, const uint32_t *d_moz, cons
     QueryScratch &q = ctx->qs;
     if ((rc = grow(ctx, &q.d_win, &q.win_cap, (size_t)nspec * nlen))) return rc;
     if ((rc = grow(ctx, &q.d_wide, &q.wide_cap, (size_t)nspec + 4))) return rc;
-    const uint32_t sched = ctx->tuning.schedule;
-    if (sched == 2 && (rc = grow(ctx, &q.d_order, &q.order_cap, 2 * (size_t)nspec))) return rc;
+    if ((ctx->tuning.schedule == 2 || ctx->auto_shape) && (rc = grow(ctx, &q.d_order, &q.order_cap, 2 * (size_t)nspec)))
+        return rc;
     if ((rc = grow(ctx, &q.d_fitstart, &q.fit_cap, (size_t)nspec))) return rc;
     if (!q.d_work) HC_CUDA(ctx, cudaMalloc((void **)&q.d_work, 4 * kWorkWords));
     q.d_nwide = q.d_work + kWkNwide;
@@ -2104,14 +2633,12 @@ int query_device(hc_ctx *ctx, const uint32_t *d_idx, const uint32_t *d_moz, cons
     a.wide_list = q.d_wide;
     a.nwide = q.d_nwide;
     a.work = q.d_work;
-    a.tile = ctx->tuning.tile;
     a.defer_cap = ctx->tuning.defer_cap;
-    a.persistent = sched != 1;
     a.maxz = ctx->p.maxz;
     a.classes = ctx->d_classes;
     a.phase = ctx->d_phase;
     int launches = 4;
-    int rc2 = launch_packed(ctx, a, sched, nspec, nlen, q.d_win, q.d_order, q.d_work, st, launches, ctx->profiling);
+    int rc2 = launch_packed(ctx, a, nspec, nlen, q.d_win, q.d_order, q.d_work, st, launches, ctx->profiling);
     if (rc2) return rc2;
     if (ctx->profiling) HC_CUDA(ctx, record_stage(ctx, 2, st));
     // spectra whose packed scorecard could overflow are redone wide; the
@@ -2182,6 +2709,7 @@ int preload_query_kernels(hc_ctx *ctx)
     chk(load_one(k_search<false, 4>));
     chk(load_one(k_search<false, 8>));
     chk(load_one(k_search<true, 2>));
+    chk(load_one(k_search_small));
     HC_CUDA(ctx, e);
     return HC_SUCCESS;
 }
@@ -2242,14 +2770,11 @@ int launch_query_scratch(hc_ctx *ctx, const uint32_t *d_idx, const uint32_t *d_m
     a.wide_list = s.wide;
     a.nwide = nwide;
     a.work = s.work;
-    a.tile = ctx->tuning.tile;
     a.defer_cap = ctx->tuning.defer_cap;
-    const uint32_t sched = ctx->tuning.schedule;
-    a.persistent = sched != 1;
     a.maxz = ctx->p.maxz;
     a.classes = ctx->d_classes;
     int launches = 4;
-    int rc = launch_packed(ctx, a, sched, nspec, nlen, s.win, s.order, s.work, st, launches, false);
+    int rc = launch_packed(ctx, a, nspec, nlen, s.win, s.order, s.work, st, launches, false);
     if (rc) return rc;
     SearchArgs b = a;
     b.persistent = 1;

@@ -123,9 +123,9 @@ typedef struct hc_tuning
                               evaluation at the spectrum's end (<= HC_DEFER_MAX; 0: each
                               is evaluated in place). Results do not depend on it. */
     uint32_t small_log2;   /* schedule 2: spectra whose windows hold fewer than
-                              2^small_log2 candidates in all run in a second launch of
-                              128-thread CTAs, several per SM, after the others (0: none;
-                              at most 40). Results do not depend on it. */
+                              2^small_log2 candidates in all run in a launch of their
+                              own, with all their windows in one scorecard (0: none; at
+                              most 40). Results do not depend on it. */
 } hc_tuning;
 #define HC_DEFER_MAX 128
 
