@@ -41,7 +41,7 @@ namespace hc {
 namespace {
 
 constexpr int kDefer = HC_DEFER_MAX;  // undecided candidates per spectrum, resolved at its end
-constexpr uint32_t kWQ = 128;        // per-warp ring of qualifying candidates (power of two, >= 32 + 64)
+constexpr uint32_t kWQ = 64;         // per-warp ring of qualifying candidates' words (power of two, >= 31 + 32)
 constexpr uint32_t kNoJob = 0xFFFFFFFFu;
 constexpr float kApproxErr = 1.1e-4f;
 constexpr float kBinMargin = 2.5e-3f;  // on the x10 scale: 10*(1.1e-4) + float product slack
@@ -179,7 +179,6 @@ struct SmemTail
     unsigned long long ph_last;
     unsigned long long cnt[4];  // tiles | tiles scanned whole | listed candidates | exact evaluations
     int2 win[HC_MAX_LENGTHS];  // the spectrum's window per length
-    uint32_t wtail[32];        // per warp: candidates appended to its ring so far (this job)
     // per entry class: what its y1 keys collect from the spectrum's valid
     // peaks, packed [count:8 | sum:24]; entry kClassNone stays zero
     uint32_t upk[kMaxClasses + 1];
@@ -225,7 +224,7 @@ __host__ __device__ inline SmemLayout smem_layout(uint32_t tile, uint32_t dF, bo
     o.pmoz = (o.kinfo + 8 * maxpairs + 15) & ~(size_t)15;
     o.pint = o.pmoz + 4ull * HC_QALEN;
     o.wq = (o.pint + 4ull * HC_QALEN + 15) & ~(size_t)15;
-    size_t end = o.wq + 2ull * kWQ * nwarps;
+    size_t end = o.wq + 4ull * kWQ * nwarps;
     // wide words: the class adds, read by every job's scorecard start
     o.ucls = (end + 15) & ~(size_t)15;
     if (wide) end = o.ucls + 8ull * (kMaxClasses + 1);
@@ -514,7 +513,7 @@ __global__ void __launch_bounds__(G >= 4 ? 512 : 1024, G == 4 ? 2 : 1) k_search(
     // the stream addresses the scorecard and the sinks as shared-window offsets
     const uint32_t card_s = (uint32_t)__cvta_generic_to_shared(smem);
     const uint32_t sink_s = (uint32_t)__cvta_generic_to_shared(smem + L.sink) + 4u * (uint32_t)lane;
-    uint16_t *wq = reinterpret_cast<uint16_t *>(smem + L.wq) + wid * kWQ;  // this warp's candidate ring (tile < 2^16)
+    uint32_t *wq = reinterpret_cast<uint32_t *>(smem + L.wq) + wid * kWQ;  // this warp's candidate ring
 
     // k_search_small, launched after this kernel, may take SMs as they fall free
     if constexpr (!WIDE) asm volatile("griddepcontrol.launch_dependents;");
@@ -534,10 +533,23 @@ __global__ void __launch_bounds__(G >= 4 ? 512 : 1024, G == 4 ? 2 : 1) k_search(
     // reference's double hyperscore and competes for the top hit. The true top
     // hit's estimate is within 2*kApproxErr < kNear of the final maximum, so it
     // is always among them, whatever the order candidates are scored in.
-    uint32_t my_cps = 0, my_fl = 0, my_exact = 0;
-    auto hist_add = [&](int bin) {
+    // (cpsms is the histogram's sum: T.cpsms counts only what goes past kHistSm)
+    auto count_psm = [&](uint32_t bc, uint32_t yc, int bin) {
+        if (bc >= (uint32_t)kRefMaxShp || yc >= (uint32_t)kRefMaxShp) atomicOr(&T.flags, HC_FLAG_LGFACT_OOB);
+        if (bin >= HC_HIST_BINS || bin < 0)
+        {
+            atomicOr(&T.flags, HC_FLAG_HIST_OOB);
+            bin = bin < 0 ? 0 : HC_HIST_BINS - 1;
+        }
         if (bin < kHistSm) atomicAdd(&T.u.run.hist[bin], 1u);
-        else atomicAdd(&a.hist[(size_t)T.spec * HC_HIST_BINS + (uint32_t)bin], 1u);
+        else
+        {
+            atomicAdd(&T.cpsms, 1u);
+            atomicAdd(&a.hist[(size_t)T.spec * HC_HIST_BINS + (uint32_t)bin], 1u);
+        }
+    };
+    auto exact_done = [&]() {
+        if (a.phase) atomicAdd(&T.cnt[3], 1ull);
     };
     unsigned long long my_best = 0;
     uint32_t my_shp = 0;
@@ -575,7 +587,7 @@ __global__ void __launch_bounds__(G >= 4 ? 512 : 1024, G == 4 ? 2 : 1) k_search(
                     defer[di] = make_uint2((uint32_t)ib | (bc << 24), (uint32_t)iy | (yc << 24));
                     return;
                 }
-                my_exact++;  // queue full: exact now
+                exact_done();  // queue full: exact now
                 h = exact_h(a.qc, bc, yc, ib, iy);
                 bin = hist_bin(h);
                 if (!(h > 0.0f)) return;
@@ -589,15 +601,12 @@ __global__ void __launch_bounds__(G >= 4 ? 512 : 1024, G == 4 ? 2 : 1) k_search(
         }
         else
         {
-            my_exact++;
+            exact_done();
             h = ha;
             bin = hist_bin(h);
             if (!(h > 0.0f)) return;
         }
-        my_cps++;
-        if (bc >= (uint32_t)kRefMaxShp || yc >= (uint32_t)kRefMaxShp) my_fl |= HC_FLAG_LGFACT_OOB;
-        if (bin >= HC_HIST_BINS || bin < 0) { my_fl |= HC_FLAG_HIST_OOB; bin = bin < 0 ? 0 : HC_HIST_BINS - 1; }
-        hist_add(bin);
+        count_psm(bc, yc, bin);
     };
 
     for (uint32_t iter = 0;; iter++)
@@ -1023,49 +1032,45 @@ __global__ void __launch_bounds__(G >= 4 ? 512 : 1024, G == 4 ? 2 : 1) k_search(
             }
             // ---- every candidate that reached min_shp ----
             // cpsms, histogram and the top hit (see score_one). The packed tile
-            // is scanned two candidates per lane and step; a warp collects its
+            // is scanned four candidates per lane and step; a warp collects its
             // qualifying candidates in its own ring and scores them 32 at a
             // time (all lanes busy), then clears the words it scanned.
-            my_cps = my_fl = my_exact = 0;
             const uint32_t key_l = jb.l << 24;
             if constexpr (!WIDE)
             {
                 const uint4 *c4 = reinterpret_cast<const uint4 *>(card);
-                uint32_t qh = 0, qhead = 0;  // ring fill and head (warp-uniform)
-                if (lane == 0) T.wtail[wid] = 0;
-                __syncwarp();
+                // the warp's ring: an entry is one lane's four candidates of a
+                // step, (first candidate << 4) | the ones that qualify, so a step
+                // takes one ballot and one store whatever it finds (an entry a
+                // candidate, placed by a returning shared-memory atomic and a
+                // loop over the lane's candidates, took 27 instructions more a
+                // step). A pop scores one candidate of each of 32 entries and
+                // puts back those that hold another (one in eight).
+                uint32_t fill = 0, head = 0;  // warp-uniform
+                const uint32_t lt = (1u << lane) - 1u;
+                auto put = [&](bool any, uint32_t e) {
+                    const uint32_t b = __ballot_sync(0xFFFFFFFFu, any);
+                    if (any) wq[(head + fill + (uint32_t)__popc(b & lt)) & (kWQ - 1)] = e;
+                    fill += (uint32_t)__popc(b);
+                };
                 auto pop_score = [&](uint32_t cnt) {
                     __syncwarp();
+                    uint32_t rest = 0;
                     if ((uint32_t)lane < cnt)
                     {
-                        const uint32_t loc = wq[(qhead + lane) & (kWQ - 1)];
+                        const uint32_t e = wq[(head + lane) & (kWQ - 1)];
+                        const uint32_t k = (uint32_t)__ffs(e) - 1u;
+                        rest = e & (e - 1u);
+                        const uint32_t loc = (e >> 4) + (k & 1u) + ((k & 2u) << 5);
                         uint32_t bc, yc, shp;
                         uint64_t ib, iy;
                         decode<false>(card, loc, bc, yc, shp, ib, iy);
                         score_one(bc, yc, ib, iy, shp, ~(key_l | ((c0 + loc) & 0xFFFFFF)));
                     }
+                    head += cnt;
+                    fill -= cnt;
+                    put((rest & 15u) != 0u, rest);
                     __syncwarp();
-                };
-                // a warp covers 128 consecutive candidates per step, as two
-                // halves of 64 (two per lane) whose loads are issued together;
-                // the ring is drained after each half (it never holds more than
-                // 31 + 64 entries)
-                auto push = [&](const uint4 w, uint32_t c) {
-                    const uint32_t s0 = (w.x >> 24) + (w.y >> 24), s1 = (w.z >> 24) + (w.w >> 24);
-                    const bool q0 = s0 >= a.thr && c < ntile, q1 = s1 >= a.thr && c + 1 < ntile;  // thr = max(min_shp, 1)
-                    const uint32_t b0 = __ballot_sync(0xFFFFFFFFu, q0), b1 = __ballot_sync(0xFFFFFFFFu, q1);
-                    if ((b0 | b1) == 0) return;
-                    const uint32_t lt = (1u << lane) - 1u;
-                    const uint32_t r = qhead + qh + (uint32_t)(__popc(b0 & lt) + __popc(b1 & lt));
-                    if (q0) wq[r & (kWQ - 1)] = (uint16_t)c;
-                    if (q1) wq[(r + (q0 ? 1u : 0u)) & (kWQ - 1)] = (uint16_t)(c + 1);
-                    qh += (uint32_t)(__popc(b0) + __popc(b1));
-                    while (qh >= 32)
-                    {
-                        pop_score(32);
-                        qhead += 32;
-                        qh -= 32;
-                    }
                 };
                 const uint32_t first = 4 * (tid - (uint32_t)lane), step = 4 * nthr;
                 const uint32_t thr4 = min(a.thr, 255u) * 0x01010101u;
@@ -1095,40 +1100,13 @@ __global__ void __launch_bounds__(G >= 4 ? 512 : 1024, G == 4 ? 2 : 1) k_search(
                     if (base + 128u > ntile)  // warp-uniform
                         m &= (ca < ntile ? 0x80u : 0u) | (ca + 1u < ntile ? 0x8000u : 0u) |
                              (cb < ntile ? 0x800000u : 0u) | (cb + 1u < ntile ? 0x80000000u : 0u);
-                    // this lane's place in the warp's ring: from the warp's
-                    // append counter (T.wtail = qhead + qh; lanes in any order)
-                    const uint32_t n4 = __popc(m);
-                    const uint32_t tot = __reduce_add_sync(0xFFFFFFFFu, n4);
-                    if (tot == 0) continue;
-                    if (qh + tot <= kWQ)
-                    {
-                        uint32_t r = n4 ? atomicAdd(&T.wtail[wid], n4) : 0u;
-                        while (m)
-                        {
-                            const int k = (__ffs(m) - 1) >> 3;
-                            m &= m - 1;
-                            wq[r & (kWQ - 1)] = (uint16_t)((k < 2 ? ca : cb) + (uint32_t)(k & 1));
-                            r++;
-                        }
-                        qh += tot;
-                        while (qh >= 32)
-                        {
-                            pop_score(32);
-                            qhead += 32;
-                            qh -= 32;
-                        }
-                    }
-                    else
-                    {
-                        // the ring would overflow: the two halves one after the other
-                        push(wa, ca);
-                        push(wb, cb);
-                        __syncwarp();
-                        if (lane == 0) T.wtail[wid] = qhead + qh;
-                        __syncwarp();
-                    }
+                    // bytes' top bits to bits 0..3 (the products land apart)
+                    const uint32_t nib = ((m >> 7) * 0x01020408u) >> 24;
+                    if (!__any_sync(0xFFFFFFFFu, m)) continue;
+                    put(m != 0u, (ca << 4) | nib);
+                    while (fill >= 32) pop_score(32);
                 }
-                if (qh) pop_score(qh);
+                while (fill) pop_score(min(fill, 32u));
                 // the next job's candidates and their classes (its scorecard start)
                 const uint32_t nn = nj.l != kNoJob ? nj.c1 - nj.c0 : 0u;
                 const uint8_t *ncls = nn ? a.len[nj.l].cls + nj.c0 : nullptr;
@@ -1161,7 +1139,8 @@ __global__ void __launch_bounds__(G >= 4 ? 512 : 1024, G == 4 ? 2 : 1) k_search(
                         z4[c >> 1] = make_uint4(0u, y0, 0u, y1);
                         z4[(c >> 1) + 1] = make_uint4(0u, y2, 0u, y3);
                     }
-                    npass += (y0 >> 24) + (y1 >> 24) + (y2 >> 24) + (y3 >> 24);
+                    npass = __dp4a(__byte_perm(__byte_perm(y0, y1, 0x0073u), __byte_perm(y2, y3, 0x0073u), 0x5410u),
+                                   0x01010101u, npass);  // + the four counts (top bytes)
                 }
             }
             else
@@ -1191,17 +1170,7 @@ __global__ void __launch_bounds__(G >= 4 ? 512 : 1024, G == 4 ? 2 : 1) k_search(
                     card[2 * c + 1] = wy;
                 }
             }
-            {
-                my_cps = __reduce_add_sync(0xFFFFFFFFu, my_cps);
-                my_fl = __reduce_or_sync(0xFFFFFFFFu, my_fl);
-                if (lane == 0)
-                {
-                    if (my_cps) atomicAdd(&T.cpsms, my_cps);
-                    if (my_fl) atomicOr(&T.flags, my_fl);
-                }
-                if (a.phase && my_exact) atomicAdd(&T.cnt[3], (unsigned long long)my_exact);
-                if (a.phase && tid == 0) T.cnt[0] += 1;
-            }
+            if (a.phase && tid == 0) T.cnt[0] += 1;
             HC_PHASE(2);
             if (tid == 0) T.pnext = 0;
             __syncthreads();
@@ -1212,30 +1181,16 @@ __global__ void __launch_bounds__(G >= 4 ? 512 : 1024, G == 4 ? 2 : 1) k_search(
         if (!WIDE)
         {
             const uint32_t nd = min(T.ndefer, a.defer_cap);
-            uint32_t cps = 0, fl = 0, nex = 0;
             for (uint32_t i = tid; i < nd; i += nthr)
             {
                 uint32_t bc, yc, shp;
                 uint64_t ib, iy;
                 const uint2 w = defer[i];
                 decode_packed(w.x, w.y, bc, yc, shp, ib, iy);
-                nex++;
+                exact_done();
                 const float h = exact_h(a.qc, bc, yc, ib, iy);
-                if (!(h > 0.0f)) continue;
-                int bin = hist_bin(h);
-                cps++;
-                if (bc >= (uint32_t)kRefMaxShp || yc >= (uint32_t)kRefMaxShp) fl |= HC_FLAG_LGFACT_OOB;
-                if (bin >= HC_HIST_BINS || bin < 0) { fl |= HC_FLAG_HIST_OOB; bin = bin < 0 ? 0 : HC_HIST_BINS - 1; }
-                hist_add(bin);
+                if (h > 0.0f) count_psm(bc, yc, hist_bin(h));
             }
-            cps = __reduce_add_sync(0xFFFFFFFFu, cps);
-            fl = __reduce_or_sync(0xFFFFFFFFu, fl);
-            if (lane == 0)
-            {
-                if (cps) atomicAdd(&T.cpsms, cps);
-                if (fl) atomicOr(&T.flags, fl);
-            }
-            if (a.phase && nex) atomicAdd(&T.cnt[3], (unsigned long long)nex);
         }
         // postings visited: those of entries inside the window
         npass = __reduce_add_sync(0xFFFFFFFFu, npass);
@@ -1255,7 +1210,14 @@ __global__ void __launch_bounds__(G >= 4 ? 512 : 1024, G == 4 ? 2 : 1) k_search(
             continue;
         }
         for (int i = tid; i < kHistSm; i += nthr) a.hist[(size_t)s * HC_HIST_BINS + i] = T.u.run.hist[i];
-        if (tid == 0) write_result(a, s, T.cpsms, T.flags, T.bytes, T.best, T.best_shp);
+        if (wid == 0)
+        {
+            uint32_t cps = 0;
+#pragma unroll
+            for (int i = 0; i < kHistSm; i += 32) cps += T.u.run.hist[i + lane];
+            cps = __reduce_add_sync(0xFFFFFFFFu, cps) + T.cpsms;
+            if (lane == 0) write_result(a, s, cps, T.flags, T.bytes, T.best, T.best_shp);
+        }
     }
     if (a.phase && tid == 0)
     {
@@ -1283,6 +1245,7 @@ constexpr uint32_t kSmTile = 3584;   // candidates of the scorecard (a multiple 
 constexpr uint32_t kSmRing = 64;     // lists waiting per warp (a power of two, >= 31 + 32)
 constexpr uint32_t kSmLong = 8;      // chunks from which the warp reads a list together
 constexpr uint32_t kSmStep = 128;
+constexpr uint32_t kSmWQ = 128;      // candidates waiting per warp (a power of two, >= 31 + 64)
 constexpr uint32_t kSmCtas = 4;
 // launch shapes picked for a context that chose none (see launch_packed)
 constexpr uint32_t kAutoSmallLog2 = 15, kAutoAllSmall = 1u << 16, kAutoOrder = 1024;
@@ -1300,7 +1263,7 @@ struct SmSmem
 {
     uint32_t card[2 * kSmTile];
     uint2 ring[kSmThreads / 32][kSmRing];
-    uint16_t wq[kSmThreads / 32][kWQ];
+    uint16_t wq[kSmThreads / 32][kSmWQ];
     uint2 defer[kDefer];
     unsigned long long ucls[kMaxClasses + 1];
     SmSeg seg[HC_MAX_LENGTHS];
@@ -1665,7 +1628,7 @@ __global__ void __launch_bounds__(kSmThreads, 4) k_search_small(SearchArgs a)
                 __syncwarp();
                 if ((uint32_t)lane < cnt)
                 {
-                    const uint32_t loc = wq[(head + (uint32_t)lane) & (kWQ - 1)];
+                    const uint32_t loc = wq[(head + (uint32_t)lane) & (kSmWQ - 1)];
                     const uint32_t l = S.stepl[loc / kSmStep];
                     const uint32_t e = (uint32_t)S.win[l].x + (v0 + loc - S.vbase[l]);
                     const uint2 w = reinterpret_cast<const uint2 *>(S.card)[loc];
@@ -1685,8 +1648,8 @@ __global__ void __launch_bounds__(kSmThreads, 4) k_search_small(SearchArgs a)
                 if ((b0 | b1) == 0) continue;
                 const uint32_t lt = (1u << lane) - 1u;
                 const uint32_t r = head + fill + (uint32_t)(__popc(b0 & lt) + __popc(b1 & lt));
-                if (q0) wq[r & (kWQ - 1)] = (uint16_t)c;
-                if (q1) wq[(r + (q0 ? 1u : 0u)) & (kWQ - 1)] = (uint16_t)(c + 1);
+                if (q0) wq[r & (kSmWQ - 1)] = (uint16_t)c;
+                if (q1) wq[(r + (q0 ? 1u : 0u)) & (kSmWQ - 1)] = (uint16_t)(c + 1);
                 fill += (uint32_t)(__popc(b0) + __popc(b1));
                 while (fill >= 32) pop_score(32);
             }
