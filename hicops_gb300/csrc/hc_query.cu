@@ -24,8 +24,11 @@
 // log10(1+ibc) + log10(1+iyc) - 6 in double and stores it as float. Here it is
 // first evaluated in float; the float value lies within 1.1e-4 of the
 // reference's (table rounding 2 x 7.6e-6, three float additions 3 x 1.6e-5,
-// log10f within 2 ulp, the final rounding 4e-6). Wherever that bound leaves a
-// decision open (sign, histogram bin, or a candidate that can still be the
+// log10f within 2 ulp, the final rounding 4e-6), and a score below 50 within
+// 1.5e-5 (its terms and sums stay below 64: table roundings 2 x 1.9e-6, the sums
+// 3 x 1.9e-6, the logarithm 2 ulp of a log2 below 48, x 0.301: 2.3e-6, its factor
+// and product 1.2e-6, the reference's rounding 1.9e-6). Wherever that bound leaves
+// a decision open (sign, histogram bin, or a candidate that can still be the
 // top hit) the reference's double expression is evaluated, so cpsms, the
 // histogram and the top hit equal the reference's double evaluation.
 #include <algorithm>
@@ -44,7 +47,16 @@ constexpr int kDefer = HC_DEFER_MAX;  // undecided candidates per spectrum, reso
 constexpr uint32_t kWQ = 64;         // per-warp ring of qualifying candidates' words (power of two, >= 31 + 32)
 constexpr uint32_t kNoJob = 0xFFFFFFFFu;
 constexpr float kApproxErr = 1.1e-4f;
-constexpr float kBinMargin = 2.5e-3f;  // on the x10 scale: 10*(1.1e-4) + float product slack
+// A score this close to a bin's edge (on the x10 scale) is open: 10 x the bound
+// above and the roundings of the two products (3e-5 and 6e-5 below 512; 2.4e-4 in all
+// for scores below 50). The wider margin took in 420 candidates of an open-search
+// spectrum, more than its queue holds, and the rest were evaluated on the spot, some
+// warp of almost every job waiting on double arithmetic; the narrow one takes in 60.
+constexpr float kBinMargin = 4e-4f, kBinMarginHigh = 2.5e-3f, kLowScore = 50.0f;
+__device__ __forceinline__ bool bin_open(float ha, float fr)
+{
+    return fabsf(fr - 0.5f) > 0.5f - (ha < kLowScore ? kBinMargin : kBinMarginHigh);
+}
 constexpr float kNear = 3.5e-4f;       // > 2 * kApproxErr: candidates that may be the top
 static_assert(HC_DEFER_MAX >= 128, "the scan's last step may read 127 packed words past the tile, into the queue");
 
@@ -279,32 +291,6 @@ __device__ __forceinline__ void decode(const typename Card<WIDE>::word *card, ui
     shp = (uint32_t)(uint16_t)(bc + yc);
 }
 
-// Hyperscore of one candidate: returns false unless h > 0; h is the float
-// estimate (or the reference's value where the estimate's bound leaves the
-// sign or the histogram bin undecided), bin its histogram bin.
-template <bool WIDE>
-__device__ __forceinline__ bool score(const QueryConst *__restrict__ qc, const float *lgf, uint32_t bc, uint32_t yc,
-                                      uint64_t ib, uint64_t iy, float &h, int &bin, uint32_t &nexact)
-{
-    if (!WIDE)
-    {
-        const float ha = approx_h(lgf, bc, yc, ib, iy);
-        const float t = ha * 10.0f + 0.5f;
-        const float fr = t - floorf(t);
-        if (!(fabsf(ha) <= kApproxErr * 4.0f || fr < kBinMargin || fr > 1.0f - kBinMargin))
-        {
-            h = ha;
-            bin = (int)floorf(t);
-            return ha > 0.0f;
-        }
-    }
-    nexact++;
-    const float hf = exact_h(qc, bc, yc, ib, iy);
-    h = hf;
-    bin = hist_bin(hf);
-    return hf > 0.0f;
-}
-
 // 32-bit adds to a shared-memory word given by its shared-window address.
 // No memory clobber: the scorecard is read only after a block barrier.
 __device__ __forceinline__ void red_shared_add(uint32_t addr, uint32_t v)
@@ -535,15 +521,15 @@ __global__ void __launch_bounds__(G >= 4 ? 512 : 1024, G == 4 ? 2 : 1) k_search(
     // is always among them, whatever the order candidates are scored in.
     // (cpsms is the histogram's sum: T.cpsms counts only what goes past kHistSm)
     auto count_psm = [&](uint32_t bc, uint32_t yc, int bin) {
-        if (bc >= (uint32_t)kRefMaxShp || yc >= (uint32_t)kRefMaxShp) atomicOr(&T.flags, HC_FLAG_LGFACT_OOB);
-        if (bin >= HC_HIST_BINS || bin < 0)
-        {
-            atomicOr(&T.flags, HC_FLAG_HIST_OOB);
-            bin = bin < 0 ? 0 : HC_HIST_BINS - 1;
-        }
-        if (bin < kHistSm) atomicAdd(&T.u.run.hist[bin], 1u);
+        if (max(bc, yc) >= (uint32_t)kRefMaxShp) atomicOr(&T.flags, HC_FLAG_LGFACT_OOB);
+        if ((uint32_t)bin < (uint32_t)kHistSm) atomicAdd(&T.u.run.hist[bin], 1u);
         else
         {
+            if (bin >= HC_HIST_BINS || bin < 0)
+            {
+                atomicOr(&T.flags, HC_FLAG_HIST_OOB);
+                bin = bin < 0 ? 0 : HC_HIST_BINS - 1;
+            }
             atomicAdd(&T.cpsms, 1u);
             atomicAdd(&a.hist[(size_t)T.spec * HC_HIST_BINS + (uint32_t)bin], 1u);
         }
@@ -579,7 +565,7 @@ __global__ void __launch_bounds__(G >= 4 ? 512 : 1024, G == 4 ? 2 : 1) k_search(
         {
             const float tt = ha * 10.0f + 0.5f;
             const float fr = tt - floorf(tt);
-            if (fabsf(ha) <= kApproxErr * 4.0f || fr < kBinMargin || fr > 1.0f - kBinMargin)
+            if (fabsf(ha) <= kApproxErr * 4.0f || bin_open(ha, fr))
             {
                 const uint32_t di = atomicAdd(&T.ndefer, 1u);
                 if (di < a.defer_cap)
@@ -1332,7 +1318,7 @@ __global__ void __launch_bounds__(kSmThreads, 4) k_search_small(SearchArgs a)
         }
         const float tt = ha * 10.0f + 0.5f;
         const float fr = tt - floorf(tt);
-        if (fabsf(ha) <= kApproxErr * 4.0f || fr < kBinMargin || fr > 1.0f - kBinMargin)
+        if (fabsf(ha) <= kApproxErr * 4.0f || bin_open(ha, fr))
         {
             const uint32_t di = atomicAdd(&S.ndefer, 1u);
             if (di < a.defer_cap)
