@@ -753,26 +753,6 @@ __global__ void k_spost_scatter(const uint32_t *__restrict__ ids, const uint32_t
     }
 }
 
-// Device scratch of one build step, freed when the step returns (also on its
-// error paths).
-struct Scratch
-{
-    hc_ctx *ctx;
-    std::vector<void *> ptrs;
-    explicit Scratch(hc_ctx *c) : ctx(c) {}
-    template <class T>
-    cudaError_t alloc(T **p, size_t n)
-    {
-        const cudaError_t e = dalloc(ctx, p, n);
-        if (e == cudaSuccess) ptrs.push_back(*p);
-        return e;
-    }
-    ~Scratch()
-    {
-        for (void *p : ptrs) dfree(ctx, p);
-    }
-};
-
 }  // namespace
 
 // The class code of every entry, and room for a mark on those that lose their class.
@@ -788,14 +768,14 @@ static int build_search(hc_ctx *ctx, LenHost &lh, const EntryCodes &ec, const ui
 // The entries of one length enumerated on the device (k_enum_entries, two
 // passes around a scan of the per-peptide variant counts) into fresh SoA
 // arrays in generation order; sets lh.n.
-static int enumerate_entries(hc_ctx *ctx, LenHost &lh, Scratch &out, float **d_m, uint32_t **d_s,
+static int enumerate_entries(hc_ctx *ctx, LenHost &lh, PoolScratch &out, float **d_m, uint32_t **d_s,
                              uint64_t **d_si, uint32_t **d_mo, int *launches)
 {
     cudaStream_t st = ctx->stream;
     const uint32_t npep = lh.npep, L = lh.L;
     EnumConst ec;
     make_enum_const(ctx->p, &ec);
-    Scratch tmp(ctx);
+    PoolScratch tmp(ctx);
     uint32_t *cnt = nullptr, *stmp = nullptr;
     uint32_t nvar = 0;
     const unsigned grid = npep / 128 + 1;
@@ -832,7 +812,7 @@ int build_length_device(hc_ctx *ctx, LenHost &lh, const hc_entry *h_entries, boo
     cudaStream_t st = ctx->stream;
     int launches = 0;
     // entries in generation order: enumerated here, or uploaded from the host
-    Scratch scr(ctx);
+    PoolScratch scr(ctx);
     float *d_m0 = nullptr;
     uint32_t *d_s0 = nullptr, *d_mod0 = nullptr;
     uint64_t *d_site0 = nullptr;
@@ -971,7 +951,7 @@ static_assert(kCodes + 4 <= kReadBytes, "read-back words");
 
 // The entries' class codes; waits for the codes seen and for the query
 // postings' total (qA scanned), read back together.
-static int entry_codes(hc_ctx *ctx, LenHost &lh, Scratch &scr, EntryCodes *ec)
+static int entry_codes(hc_ctx *ctx, LenHost &lh, PoolScratch &scr, EntryCodes *ec)
 {
     cudaStream_t st = ctx->stream;
     const uint32_t nb = ctx->p.max_mass * ctx->p.scale, n = lh.n;
@@ -1016,7 +996,7 @@ int build_query_postings(hc_ctx *ctx, LenHost &lh, const uint32_t *d_ids, const 
     lh.d_qion = nullptr;
     HC_CUDA(ctx, dalloc(ctx, &lh.d_qA, (size_t)nb + 1));
     uint32_t *stmp = nullptr, *keys = nullptr;
-    Scratch scr(ctx);
+    PoolScratch scr(ctx);
     HC_CUDA(ctx, scr.alloc(&stmp, scan_tmp_words((size_t)nb + 1)));
     const uint32_t npost = d_ids ? (uint32_t)lh.npost : 0u;
     if (npost && !d_keys)
@@ -1090,7 +1070,7 @@ static int build_search(hc_ctx *ctx, LenHost &lh, const EntryCodes &ec, const ui
     HC_CUDA(ctx, dalloc(ctx, &lh.d_qAs, (size_t)nb + 1));
     const unsigned eblocks = (n + 255) / 256, bblocks = flat_blocks(ctx, (uint64_t)nb + 1);
     const unsigned pblocks = flat_blocks(ctx, total);
-    Scratch scr(ctx);
+    PoolScratch scr(ctx);
     if (n > 0)
     {
         const int rc = add_classes(ctx, read_used(ctx));
@@ -1140,7 +1120,7 @@ static int build_search(hc_ctx *ctx, LenHost &lh, const EntryCodes &ec, const ui
 int build_rows(hc_ctx *ctx, LenHost &lh)
 {
     const uint32_t nb = ctx->p.max_mass * ctx->p.scale;
-    Scratch scr(ctx);
+    PoolScratch scr(ctx);
     EntryCodes ec{};
     const int rc = entry_codes(ctx, lh, scr, &ec);
     if (rc) return rc;

