@@ -267,10 +267,22 @@ int64_t hc_make_entries(const hc_params *p, uint32_t L, const uint8_t *seqs, uin
     return make_entries(*p, L, seqs, npep, out, out ? cap : 0);
 }
 
+// (no early exit inside a block, so that the compiler can compare many at once)
+__attribute__((optimize("O3"))) static bool residues_ok(const uint8_t *seqs, size_t n)
+{
+    for (size_t a = 0; a < n; a += 4096)
+    {
+        const size_t b = std::min(n, a + 4096);
+        uint8_t bad = 0;
+        for (size_t i = a; i < b; i++) bad |= (uint8_t)((uint8_t)(seqs[i] - 'A') > 25);
+        if (bad) return false;
+    }
+    return true;
+}
+
 static int upload_seqs(hc_ctx *ctx, LenHost &lh, const uint8_t *seqs, uint32_t npep)
 {
-    for (size_t i = 0; i < (size_t)npep * lh.L; i++)
-        if (seqs[i] < 'A' || seqs[i] > 'Z') return set_error(ctx, HC_ERR_INVLD_PARAM, "residue outside A-Z");
+    if (!residues_ok(seqs, (size_t)npep * lh.L)) return set_error(ctx, HC_ERR_INVLD_PARAM, "residue outside A-Z");
     HC_CUDA(ctx, dalloc(ctx, &lh.d_seqs, (size_t)npep * lh.L + 1));
     HC_CUDA(ctx, cudaMemcpyAsync(lh.d_seqs, seqs, (size_t)npep * lh.L, cudaMemcpyHostToDevice, ctx->stream));
     lh.npep = npep;

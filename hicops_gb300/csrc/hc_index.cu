@@ -240,21 +240,41 @@ cudaError_t radix_sort(uint32_t *keys0, uint32_t *keys1, uint32_t *vals0, uint32
 // added. Here the walk is a loop over a stack of chosen positions. The first
 // pass (mass == nullptr) counts the variants per peptide; the second writes
 // them at npep + voff[i].
-__global__ void k_enum_entries(const uint8_t *__restrict__ seqs, uint32_t L, uint32_t npep, EnumConst ec,
+constexpr int kEnumThreads = 128;
+
+__global__ void __launch_bounds__(kEnumThreads) k_enum_entries(const uint8_t *__restrict__ seqs, uint32_t L, uint32_t npep, EnumConst ec,
                                const uint32_t *__restrict__ voff, uint32_t *__restrict__ vcount,
                                float *__restrict__ mass, uint32_t *__restrict__ seqid,
                                uint64_t *__restrict__ sites, uint32_t *__restrict__ modnum)
 {
-    const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
+    // the block's sequences, read together (a thread's own are L bytes apart)
+    __shared__ uint8_t sh[kEnumThreads * 64];
+    const size_t at0 = (size_t)blockIdx.x * kEnumThreads * L, all = (size_t)npep * L;
+    const uint32_t bytes = at0 < all ? (uint32_t)min((size_t)kEnumThreads * L, all - at0) : 0u;
+    for (uint32_t b = threadIdx.x; b < bytes; b += kEnumThreads) sh[b] = __ldg(seqs + at0 + b);
+    // the residue tables too: lanes index them apart, which kernel parameters serialise
+    __shared__ float2 mtab[26];  // residue, static mod
+    __shared__ int8_t cond[26];
+    if (threadIdx.x < 26)
+    {
+        mtab[threadIdx.x] = make_float2(ec.aa[threadIdx.x], ec.stat[threadIdx.x]);
+        cond[threadIdx.x] = ec.cond_of[threadIdx.x];
+    }
+    __syncthreads();
+    const uint32_t i = blockIdx.x * kEnumThreads + threadIdx.x;
     if (i == npep && vcount) vcount[i] = 0;  // the scan makes it the total
     if (i >= npep) return;
-    const uint8_t *s = seqs + (size_t)i * L;
+    const uint8_t *s = sh + threadIdx.x * L;
     // UTILS_CalculatePepMass: two float additions per residue, in order
+    // (and a bit per modifiable virtual position, see below)
     float pm = ec.h2o;
+    uint64_t can = ec.nterm >= 0 ? 1ull : 0ull;
     for (uint32_t l = 0; l < L; l++)
     {
-        pm += ec.aa[s[l] - 'A'];
-        pm += ec.stat[s[l] - 'A'];
+        can |= (uint64_t)(cond[s[l] - 'A'] >= 0) << (l + 1);
+        const float2 m = mtab[s[l] - 'A'];
+        pm += m.x;
+        pm += m.y;
     }
     const bool write = mass != nullptr;
     if (write)
@@ -280,18 +300,18 @@ __global__ void k_enum_entries(const uint8_t *__restrict__ seqs, uint32_t L, uin
             // extension; site bit kNtermBit), q >= 1 is residue q - 1
             int p = -1;
             if (d < ec.vmods && d < 64)
-                for (uint32_t q = start; q <= L; q++)
+                for (uint64_t t = can & (~0ull << start); t; t &= t - 1)
                 {
-                    const int c = q == 0 ? ec.nterm : ec.cond_of[s[q - 1] - 'A'];
-                    if (c >= 0 && cap[c] > 0)
+                    const int q = __ffsll((long long)t) - 1;
+                    if (cap[q == 0 ? ec.nterm : cond[s[q - 1] - 'A']] > 0)
                     {
-                        p = (int)q;
+                        p = q;
                         break;
                     }
                 }
             if (p >= 0)
             {
-                const int c = p == 0 ? ec.nterm : ec.cond_of[s[p - 1] - 'A'];
+                const int c = p == 0 ? ec.nterm : cond[s[p - 1] - 'A'];
                 cap[c] -= 1;
                 pos[d] = (uint8_t)p;
                 mn += (1u << ((4u * d) & 31u)) * (uint32_t)(1 + c);  // shift count taken mod 32, as the CPU does
@@ -314,7 +334,7 @@ __global__ void k_enum_entries(const uint8_t *__restrict__ seqs, uint32_t L, uin
                 if (d == 0) break;
                 d--;
                 const uint32_t q = pos[d];
-                const int c = q == 0 ? ec.nterm : ec.cond_of[s[q - 1] - 'A'];
+                const int c = q == 0 ? ec.nterm : cond[s[q - 1] - 'A'];
                 cap[c] += 1;
                 mn -= (1u << ((4u * d) & 31u)) * (uint32_t)(1 + c);
                 st &= ~(1ull << (q == 0 ? kNtermBit : q - 1));
@@ -778,12 +798,12 @@ static int enumerate_entries(hc_ctx *ctx, LenHost &lh, PoolScratch &out, float *
     PoolScratch tmp(ctx);
     uint32_t *cnt = nullptr, *stmp = nullptr;
     uint32_t nvar = 0;
-    const unsigned grid = npep / 128 + 1;
+    const unsigned grid = npep / kEnumThreads + 1;
     if (ec.vmods > 0 && ec.nmods > 0 && npep)  // without variable mods there is nothing to count
     {
         HC_CUDA(ctx, tmp.alloc(&cnt, (size_t)npep + 1));
         HC_CUDA(ctx, tmp.alloc(&stmp, scan_tmp_words((size_t)npep + 1)));
-        k_enum_entries<<<grid, 128, 0, st>>>(lh.d_seqs, L, npep, ec, nullptr, cnt, nullptr, nullptr, nullptr,
+        k_enum_entries<<<grid, kEnumThreads, 0, st>>>(lh.d_seqs, L, npep, ec, nullptr, cnt, nullptr, nullptr, nullptr,
                                               nullptr);
         (*launches)++;
         HC_CUDA(ctx, scan_exclusive(cnt, (size_t)npep + 1, stmp, st));
@@ -800,7 +820,7 @@ static int enumerate_entries(hc_ctx *ctx, LenHost &lh, PoolScratch &out, float *
     HC_CUDA(ctx, out.alloc(d_mo, n));
     if (npep)
     {
-        k_enum_entries<<<grid, 128, 0, st>>>(lh.d_seqs, L, npep, ec, cnt, nullptr, *d_m, *d_s, *d_si, *d_mo);
+        k_enum_entries<<<grid, kEnumThreads, 0, st>>>(lh.d_seqs, L, npep, ec, cnt, nullptr, *d_m, *d_s, *d_si, *d_mo);
         (*launches)++;
     }
     HC_CUDA(ctx, cudaGetLastError());
