@@ -40,3 +40,24 @@ def test_build_load_restore_at_word_edges(npep, tmp_path):
     for x in (a, b, c):
         compare(*x.query(q), ores, ohist)
         x.close()
+
+
+@pytest.mark.parametrize("npep", [2, 3, 1024, 1025, 8191, 8192, 8193, 16400])
+def test_entry_order_at_sort_edges(npep):
+    """The entries' order where the mass sort changes (one CTA up to 8192 entries, digit
+    passes and their 8192-item tiles past it): ascending, equal masses (the sequences have
+    four residues, so most masses repeat) in file order; and the postings sorted from them."""
+    from hicops_gb300 import dslim
+    from oracle import oracle as O
+    p = S.SearchParams(min_len=9, max_len=9, maxz=1, dF=1, dM=300.0, threads=8)
+    rng = np.random.default_rng(npep)
+    seqs = rng.choice(np.frombuffer(b"AGLK", np.uint8), size=(npep, 9))
+    ix = dslim.Index(p)
+    ix.construct(9, seqs)
+    e, bA, iA = ix.export(9)
+    mass = S.pep_mass_f32(seqs)
+    order = np.argsort(mass, kind="stable")
+    assert np.array_equal(e["seqid"], order) and np.array_equal(e["mass"], mass[order])
+    obA, oiA = O.build_index(seqs, 9, e, p)
+    assert np.array_equal(bA, obA) and np.array_equal(iA, oiA)
+    ix.close()
