@@ -3,8 +3,36 @@
 #pragma once
 
 #include <cstdint>
+#include <cuda_runtime.h>
 
 namespace hc {
+
+// Kernels that follow one another in a stream, the launch and the set-up of each under
+// the end of the one before: each lets its successor's CTAs start once all of its own
+// have (release_successor), and each waits for its predecessor's end, and sees
+// what it wrote, before it reads any of it, writes anything or ends itself
+// (after_predecessor; nothing to wait for in a launch without the attribute, or behind
+// a copy). So when a kernel ends, all before it have.
+__device__ __forceinline__ void after_predecessor() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+__device__ __forceinline__ void release_successor() { asm volatile("griddepcontrol.launch_dependents;"); }
+
+// Launches k, which calls after_predecessor, where its CTAs may start before the
+// kernel in front of it has ended.
+template <class... P, class... A>
+cudaError_t launch_after(void (*k)(P...), unsigned grid, unsigned threads, size_t smem, cudaStream_t st, A... args)
+{
+    cudaLaunchAttribute at{};
+    at.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    at.val.programmaticStreamSerializationAllowed = 1;
+    cudaLaunchConfig_t lc{};
+    lc.gridDim = dim3(grid);
+    lc.blockDim = dim3(threads);
+    lc.dynamicSmemBytes = smem;
+    lc.stream = st;
+    lc.attrs = &at;
+    lc.numAttrs = 1;
+    return cudaLaunchKernelEx(&lc, k, static_cast<P>(args)...);
+}
 
 // histogram bin of a hyperscore, (int)(h * 10 + 0.5) as the reference writes
 // it (dslim_query.cpp:712, 778): a float product, then a double sum

@@ -92,6 +92,7 @@ struct SearchArgs
     const uint32_t *olim;   // optional (device word): the position it stops at (else nspec)
     uint32_t wsplit;        // optional: k_search leaves the spectra whose windows hold fewer candidates
                             // in all, k_search_small those whose windows hold as many or more
+    uint32_t follows;       // k_search_small: 1 when the launch before it writes what it reads
     uint32_t persistent;    // 1: CTAs loop over a work counter; 0: one spectrum per CTA
     uint32_t maxz;
     const ClassKeys *classes;   // entry classes (null: none built)
@@ -501,9 +502,21 @@ __global__ void __launch_bounds__(G >= 4 ? 512 : 1024, G == 4 ? 2 : 1) k_search(
     const uint32_t sink_s = (uint32_t)__cvta_generic_to_shared(smem + L.sink) + 4u * (uint32_t)lane;
     uint32_t *wq = reinterpret_cast<uint32_t *>(smem + L.wq) + wid * kWQ;  // this warp's candidate ring
 
-    // k_search_small, launched after this kernel, may take SMs as they fall free
-    if constexpr (!WIDE) asm volatile("griddepcontrol.launch_dependents;");
+    // The next launch's CTAs may take SMs as they fall free: the tail fit's, which
+    // wait for this one's end, or k_search_small's, which read only what was
+    // complete before this kernel's wait.
+    if constexpr (WIDE)
+    {
+        after_predecessor();
+        release_successor();
+        if (blockIdx.x >= *a.nonly_dev) return;  // most batches list no spectrum
+    }
     for (uint32_t i = tid; i < tile * NW; i += nthr) card[i] = 0;
+    if constexpr (!WIDE)
+    {
+        after_predecessor();
+        release_successor();
+    }
     if (tid == 0)
     {
         for (int k = 0; k < kPhases; k++) T.ph[k] = 0;
@@ -1281,6 +1294,8 @@ __global__ void __launch_bounds__(kSmThreads, 4) k_search_small(SearchArgs a)
     uint16_t *wq = S.wq[wid];
     uint2 *ring = S.ring[wid];
     for (int i = tid; i < kLgTable; i += nthr) S.lgf[i] = a.qc->lgfact_f[i];
+    if (a.follows) after_predecessor();
+    release_successor();
 
     uint32_t my_cps = 0, my_fl = 0, my_shp = 0;
     unsigned long long my_best = 0;
@@ -1674,52 +1689,46 @@ __global__ void __launch_bounds__(kSmThreads, 4) k_search_small(SearchArgs a)
         if (tid == 0) write_result(a, s, S.cpsms, S.flags, S.bytes, S.best, S.best_shp);
     }
     // what follows this kernel follows the k_search it may have overlapped too
-    asm volatile("griddepcontrol.wait;" ::: "memory");
+    after_predecessor();
 }
 
 // ---- windows: DSLIM_BinarySearch (dslim_query.cpp:854-994) -----------------
-__device__ int find_min(const float *__restrict__ m, float pm, int mn, int mx)
+// The first of m's n sorted masses that is not below x1, and the first that is
+// above x2: one four-way search for each, three loads of either in flight at a time.
+// The limits are the reference's (its binary search and the walks at its end find the
+// same places), and a NaN limit finds no window.
+//
+// A batch waits for this kernel before it can search anything, and what bounds it is
+// the chain of dependent loads: two halving searches one after the other, with a walk
+// over the last 20 masses each, took 9 us for 8 spectra against 34 lengths of 600 masses;
+// this takes 6 us for 2,000. With the launches' overlap the device's part of such a
+// search fell from 47 to 34 us for 8 spectra and from 132 to 117 us for 2,000.
+__device__ __forceinline__ int2 find_limits(const float *__restrict__ m, int n, float x1, float x2)
 {
-    for (;;)
+    int b1 = 0, b2 = 0, n1 = n, n2 = n;
+    while (n1 > 0 || n2 > 0)
     {
-        int half = (mn + mx) / 2;
-        if (mx - mn < 20)
+        const int s1 = (n1 + 3) >> 2, s2 = (n2 + 3) >> 2;
+        int c1 = 0, c2 = 0;
+#pragma unroll
+        for (int k = 1; k <= 3; k++)
         {
-            int cur = mn;
-            while (__ldg(m + cur) < pm) cur++;
-            return cur;
+            if (k * s1 <= n1 && n1 > 0) c1 += __ldg(m + b1 + k * s1 - 1) < x1;
+            if (k * s2 <= n2 && n2 > 0) c2 += __ldg(m + b2 + k * s2 - 1) <= x2;
         }
-        const float v = __ldg(m + half);
-        if (pm > v) { mn = half; continue; }
-        if (pm < v) { mx = half; continue; }
-        while (half >= 0 && pm == __ldg(m + half)) half--;
-        return half + 1;
+        b1 += c1 * s1;
+        b2 += c2 * s2;
+        // a probe that fails ends the range before it
+        n1 = c1 == 3 ? n1 - 3 * s1 : min(n1 - c1 * s1, s1 - 1);
+        n2 = c2 == 3 ? n2 - 3 * s2 : min(n2 - c2 * s2, s2 - 1);
     }
-}
-
-__device__ int find_max(const float *__restrict__ m, int n, float pm, int mn, int mx)
-{
-    for (;;)
-    {
-        int half = (mn + mx) / 2;
-        if (mx - mn < 20)
-        {
-            int cur = mx;
-            while (__ldg(m + cur) > pm) cur--;
-            return cur;
-        }
-        const float v = __ldg(m + half);
-        if (pm > v) { mn = half; continue; }
-        if (pm < v) { mx = half; continue; }
-        half++;
-        while (half < n && pm == __ldg(m + half)) half++;
-        return half - 1;
-    }
+    return make_int2(b1, b2);
 }
 
 __global__ void k_windows(const LenDev *__restrict__ lens, uint32_t nlen, const float *__restrict__ prec,
                           const double *__restrict__ dMs, double dM0, uint32_t nspec, int2 *__restrict__ win)
 {
+    release_successor();
     const uint64_t g = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x;
     if (g >= (uint64_t)nspec * nlen) return;
     const uint32_t s = (uint32_t)(g / nlen), l = (uint32_t)(g % nlen);
@@ -1733,18 +1742,8 @@ __global__ void k_windows(const LenDev *__restrict__ lens, uint32_t nlen, const 
     int2 r = make_int2(1, 0);
     if (n > 0 && !(dM < 0.0))
     {
-        int mn = 0, mx = n - 1, lo, hi;
-        bool ok = true;
-        if (pm1 < __ldg(m + mn)) lo = mn;
-        else if (pm1 > __ldg(m + mx)) ok = false;
-        else lo = find_min(m, pm1, mn, mx);
-        if (ok)
-        {
-            if (pm2 > __ldg(m + mx)) hi = mx;
-            else if (pm2 < __ldg(m + mn)) ok = false;
-            else hi = find_max(m, n, pm2, mn, mx);
-        }
-        if (ok && __ldg(m + hi) <= pm2 && __ldg(m + lo) >= pm1 && hi >= lo) r = make_int2(lo, hi);
+        const int2 f = find_limits(m, n, pm1, pm2);
+        if (f.x < f.y) r = make_int2(f.x, f.y - 1);
     }
     win[g] = r;
 }
@@ -2178,9 +2177,10 @@ __global__ void __launch_bounds__(kTfWarps * 32, 2) k_tailfit(const QueryConst *
     extern __shared__ __align__(16) unsigned char tsm[];
     TfSmem &S = *reinterpret_cast<TfSmem *>(tsm);
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    for (int i = threadIdx.x; i < kLgTab; i += kTfWarps * 32) S.tab[i] = make_double2(qc->lg_tab[2 * i], qc->lg_tab[2 * i + 1]);
+    after_predecessor();
     const uint32_t cnt = list ? min(*nlist, nspec) : nspec;
     if (blockIdx.x * kTfWarps >= cnt) return;
-    for (int i = threadIdx.x; i < kLgTab; i += kTfWarps * 32) S.tab[i] = make_double2(qc->lg_tab[2 * i], qc->lg_tab[2 * i + 1]);
     __syncthreads();
     for (uint32_t w0 = blockIdx.x * kTfWarps; w0 < cnt; w0 += gridDim.x * kTfWarps)
     {
@@ -2344,8 +2344,7 @@ int launch_g(hc_ctx *ctx, const SearchArgs &a, int grid, uint32_t threads, size_
 {
     if (G >= 4 && threads > 512) threads = 512;
     HC_CUDA(ctx, cudaFuncSetAttribute(k_search<WIDE, G>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-    k_search<WIDE, G><<<grid, threads, smem, st>>>(a);
-    HC_CUDA(ctx, cudaGetLastError());
+    HC_CUDA(ctx, launch_after(k_search<WIDE, G>, (unsigned)grid, threads, smem, st, a));
     return HC_SUCCESS;
 }
 
@@ -2434,19 +2433,11 @@ static int launch_small(hc_ctx *ctx, SearchArgs s, uint32_t nspec, const uint32_
     s.obase = obase;
     s.olim = nullptr;
     s.work = work + kWkSmall;
+    s.follows = after ? 0u : 1u;
     const size_t smem = small_smem(s.dF);
     HC_CUDA(ctx, cudaFuncSetAttribute(k_search_small, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-    cudaLaunchAttribute at{};
-    at.id = cudaLaunchAttributeProgrammaticStreamSerialization;
-    at.val.programmaticStreamSerializationAllowed = 1;
-    cudaLaunchConfig_t lc{};
-    lc.gridDim = dim3(std::min<uint32_t>(nspec, (uint32_t)ctx->sm_count * kSmCtas));
-    lc.blockDim = dim3(kSmThreads);
-    lc.dynamicSmemBytes = smem;
-    lc.stream = st;
-    lc.attrs = &at;
-    lc.numAttrs = after ? 1 : 0;
-    HC_CUDA(ctx, cudaLaunchKernelEx(&lc, k_search_small, s));
+    HC_CUDA(ctx, launch_after(k_search_small, std::min<uint32_t>(nspec, (uint32_t)ctx->sm_count * kSmCtas), kSmThreads,
+                              smem, st, s));
     return HC_SUCCESS;
 }
 
@@ -2529,9 +2520,8 @@ static int launch_tailfit(hc_ctx *ctx, hc_result *out, const uint32_t *hist, uin
 {
     HC_CUDA(ctx, cudaFuncSetAttribute(k_tailfit, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(TfSmem)));
     const uint32_t blocks = std::min<uint32_t>((n + kTfWarps - 1) / kTfWarps, 2u * (uint32_t)ctx->sm_count);
-    k_tailfit<<<blocks, kTfWarps * 32, sizeof(TfSmem), st>>>(ctx->d_qconst, out, hist, n, ctx->p.min_cpsm,
-                                                             ctx->p.expect_max, fitstart, list, nlist);
-    HC_CUDA(ctx, cudaGetLastError());
+    HC_CUDA(ctx, launch_after(k_tailfit, blocks, kTfWarps * 32, sizeof(TfSmem), st, ctx->d_qconst, out, hist, n,
+                              ctx->p.min_cpsm, ctx->p.expect_max, fitstart, list, nlist));
     return HC_SUCCESS;
 }
 
