@@ -30,8 +30,7 @@ namespace hc {
 namespace {
 
 constexpr int kRsThreads = 512;
-constexpr int kRsItems = 16;
-constexpr int kRsTile = kRsThreads * kRsItems;  // 8192 items per CTA
+constexpr int kRsLong = 16, kRsShort = 4;  // items a thread of a long and of a short sort
 constexpr int kRsMaxBits = 11;
 constexpr int kRsWarps = kRsThreads / 32;
 
@@ -47,23 +46,24 @@ __device__ __forceinline__ uint32_t lanemask_lt()
 // ion keys' 19 bits take two passes of 10 instead of three of 8, and a CTA puts
 // its 8192 items in digit order in shared memory before it writes them, so that a
 // digit's items leave as one run (32 bytes on average at 10 bits) instead of a
-// 4-byte write each. Sorting the ion keys of a 500,000-peptide database (115 M
-// postings in 34 lengths, entries' masses included): 7.0 ms, against 10.6 ms with 8-bit
-// digits written item by item and a scan of three launches.
+// 4-byte write each: 7.0 ms of sorting for a 500,000-peptide database (115 M postings
+// in 34 lengths, entries' masses included), against 10.6 ms with 8-bit digits written
+// item by item and a scan of three launches. With the ranking and the tile sizes below
+// its build takes 21.8 ms against 22.7.
 
-template <int BITS>
+template <int BITS, int ITEMS>
 __global__ void __launch_bounds__(kRsThreads) k_rs_upsweep(const uint32_t *__restrict__ keys, size_t n, int shift,
                                                           uint32_t *__restrict__ tile_hist, uint32_t ntiles)
 {
     after_predecessor();
     release_successor();
-    constexpr int R = 1 << BITS;
+    constexpr int R = 1 << BITS, kTile = kRsThreads * ITEMS;
     __shared__ uint32_t h[R];
     for (int i = threadIdx.x; i < R; i += kRsThreads) h[i] = 0;
     __syncthreads();
-    const size_t base = (size_t)blockIdx.x * kRsTile;
+    const size_t base = (size_t)blockIdx.x * kTile;
 #pragma unroll
-    for (int i = 0; i < kRsItems; i++)
+    for (int i = 0; i < ITEMS; i++)
     {
         size_t idx = base + (size_t)i * kRsThreads + threadIdx.x;
         if (idx < n) atomicAdd(&h[(keys[idx] >> shift) & (R - 1)], 1u);
@@ -72,20 +72,21 @@ __global__ void __launch_bounds__(kRsThreads) k_rs_upsweep(const uint32_t *__res
     for (int d = threadIdx.x; d < R; d += kRsThreads) tile_hist[(size_t)d * ntiles + blockIdx.x] = h[d];
 }
 
-template <int BITS>
+template <int BITS, int ITEMS>
 struct RsSmem
 {
     uint16_t whist[kRsWarps][1 << BITS];  // a warp's items per digit so far, then what precedes them in the tile
     uint32_t goff[1 << BITS];             // from a place in the tile's digit order to its place in the output
     uint32_t wsum[kRsWarps];
-    uint32_t key[kRsTile], val[kRsTile];  // the tile in digit order
+    uint32_t key[kRsThreads * ITEMS], val[kRsThreads * ITEMS];  // the tile in digit order
 };
 
-// Stable ranking: warp w owns items [w*512, w*512+512) of the tile in order;
-// inside a round of 32 items, lanes with equal digits are ranked by lane id
-// (match.any + lanemask_lt), rounds advance a per-warp digit counter, and the
+// Stable ranking: warp w owns items [w*32*ITEMS, (w+1)*32*ITEMS) of the tile in order;
+// inside a round of 32 items, lanes with equal digits are ranked by lane id (a ballot
+// a bit of the digit; with a match instruction, slow where a warp's 32 digits differ,
+// a pass over 3.4 M ion keys took 47 us against 41), rounds advance a per-warp digit counter, and the
 // warps' counters are scanned per digit, then over the digits.
-template <int BITS>
+template <int BITS, int ITEMS>
 __global__ void __launch_bounds__(kRsThreads) k_rs_downsweep(const uint32_t *__restrict__ keys_in,
                                                             const uint32_t *__restrict__ vals_in,
                                                             uint32_t *__restrict__ keys_out,
@@ -95,20 +96,20 @@ __global__ void __launch_bounds__(kRsThreads) k_rs_downsweep(const uint32_t *__r
 {
     after_predecessor();
     release_successor();
-    constexpr int R = 1 << BITS;
+    constexpr int R = 1 << BITS, kTile = kRsThreads * ITEMS;
     constexpr int kPer = (R + kRsThreads - 1) / kRsThreads;  // digits per thread (consecutive)
     extern __shared__ __align__(16) unsigned char rsm[];
-    RsSmem<BITS> &S = *reinterpret_cast<RsSmem<BITS> *>(rsm);
+    RsSmem<BITS, ITEMS> &S = *reinterpret_cast<RsSmem<BITS, ITEMS> *>(rsm);
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
     for (int i = tid; i < kRsWarps * R / 2; i += kRsThreads) reinterpret_cast<uint32_t *>(&S.whist[0][0])[i] = 0;
     __syncthreads();
-    const size_t tile0 = (size_t)blockIdx.x * kRsTile;
-    const size_t base = tile0 + (size_t)warp * (kRsItems * 32);
-    uint32_t k[kRsItems], v[kRsItems];
-    uint16_t rank[kRsItems];
+    const size_t tile0 = (size_t)blockIdx.x * kTile;
+    const size_t base = tile0 + (size_t)warp * (ITEMS * 32);
+    uint32_t k[ITEMS], v[ITEMS];
+    uint16_t rank[ITEMS];
     const uint32_t lt = lanemask_lt();
 #pragma unroll
-    for (int r = 0; r < kRsItems; r++)
+    for (int r = 0; r < ITEMS; r++)
     {
         const size_t idx = base + (size_t)r * 32 + lane;
         const bool ok = idx < n;
@@ -116,11 +117,17 @@ __global__ void __launch_bounds__(kRsThreads) k_rs_downsweep(const uint32_t *__r
         v[r] = ok ? (vals_in ? vals_in[idx] : (uint32_t)idx) : 0u;
     }
 #pragma unroll
-    for (int r = 0; r < kRsItems; r++)
+    for (int r = 0; r < ITEMS; r++)
     {
         const bool ok = base + (size_t)r * 32 + lane < n;
-        const uint32_t d = ok ? ((k[r] >> shift) & (R - 1)) : (uint32_t)R;
-        const uint32_t peers = __match_any_sync(0xFFFFFFFFu, d);
+        const uint32_t d = (k[r] >> shift) & (R - 1);
+        uint32_t peers = __ballot_sync(0xFFFFFFFFu, ok);
+#pragma unroll
+        for (int b = 0; b < BITS; b++)
+        {
+            const uint32_t m = __ballot_sync(0xFFFFFFFFu, (d >> b) & 1u);
+            peers &= (d >> b) & 1u ? m : ~m;
+        }
         const uint32_t before = ok ? S.whist[warp][d] : 0u;
         rank[r] = (uint16_t)(before + __popc(peers & lt));
         __syncwarp();
@@ -169,7 +176,7 @@ __global__ void __launch_bounds__(kRsThreads) k_rs_downsweep(const uint32_t *__r
     }
     __syncthreads();
 #pragma unroll
-    for (int r = 0; r < kRsItems; r++)
+    for (int r = 0; r < ITEMS; r++)
         if (base + (size_t)r * 32 + lane < n)
         {
             const uint32_t p = (uint32_t)S.whist[warp][(k[r] >> shift) & (R - 1)] + rank[r];
@@ -177,7 +184,7 @@ __global__ void __launch_bounds__(kRsThreads) k_rs_downsweep(const uint32_t *__r
             S.val[p] = v[r];
         }
     __syncthreads();
-    const uint32_t items = (uint32_t)min((size_t)kRsTile, n - tile0);
+    const uint32_t items = (uint32_t)min((size_t)kTile, n - tile0);
     for (uint32_t i = tid; i < items; i += kRsThreads)
     {
         const uint32_t key = S.key[i], dst = S.goff[(key >> shift) & (R - 1)] + i;
@@ -344,34 +351,58 @@ size_t scan_tmp_words(size_t n)
     return t + 16;
 }
 
+// Items a thread sorts. The long sort's 8192-item tiles leave SMs idle below one a
+// SM, and what a CTA does once per digit is then all there is: 45,000 masses are six
+// tiles, 12.7 us a pass against 6.8 in 2048-item tiles, a small database's 34 lengths
+// 7.3 ms against 6.7. Up to a short tile for every SM the sort is short (twice as many,
+// or long tiles of 4096 or 6144: no faster).
+int radix_items(const hc_ctx *ctx, size_t n)
+{
+    return n > (size_t)ctx->sm_count * kRsThreads * kRsShort ? kRsLong : kRsShort;
+}
+
+template <int BITS, int ITEMS>
+cudaError_t radix_pass_of(const uint32_t *kin, const uint32_t *vin, uint32_t *kout, uint32_t *vout, size_t n, int shift,
+                          uint32_t *hist, uint32_t *scan_tmp, int write_keys, cudaStream_t st)
+{
+    const uint32_t ntiles = (uint32_t)((n + kRsThreads * ITEMS - 1) / (kRsThreads * ITEMS));
+    constexpr size_t smem = sizeof(RsSmem<BITS, ITEMS>);
+    cudaError_t e = cudaFuncSetAttribute(k_rs_downsweep<BITS, ITEMS>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                         (int)smem);
+    if (e != cudaSuccess) return e;
+    launch_after(k_rs_upsweep<BITS, ITEMS>, ntiles, kRsThreads, 0, st, kin, n, shift, hist, ntiles);
+    if ((e = scan_exclusive(hist, (size_t)ntiles << BITS, scan_tmp, st)) != cudaSuccess) return e;
+    launch_after(k_rs_downsweep<BITS, ITEMS>, ntiles, kRsThreads, smem, st, kin, vin, kout, vout, n, shift, hist,
+                 ntiles, write_keys);
+    return cudaGetLastError();
+}
+
+template <int BITS, class... A>
+cudaError_t radix_pass(int items, A... args)
+{
+    return items == kRsLong ? radix_pass_of<BITS, kRsLong>(args...) : radix_pass_of<BITS, kRsShort>(args...);
+}
+
+// words of `hist` a sort of up to n items needs
+size_t radix_hist_words(const hc_ctx *ctx, size_t n)
+{
+    const size_t shortest = std::min(n, (size_t)ctx->sm_count * kRsThreads * kRsShort);
+    return std::max((n + kRsThreads * kRsLong - 1) / (kRsThreads * kRsLong),
+                    (shortest + kRsThreads * kRsShort - 1) / (kRsThreads * kRsShort))
+           << kRsMaxBits;
+}
+
 // Sorts (keys, vals) by the low `bits` bits of the keys, stably. Ping-pongs
 // between the given buffers (all four must be valid, n words each); returns
 // which pair holds the result (0 or 1). With positions_as_values the input
 // values are not read: value i is the input position i.
-template <int BITS>
-cudaError_t radix_pass(const uint32_t *kin, const uint32_t *vin, uint32_t *kout, uint32_t *vout, size_t n, int shift,
-                       uint32_t *hist, uint32_t *scan_tmp, int write_keys, cudaStream_t st)
-{
-    const uint32_t ntiles = (uint32_t)((n + kRsTile - 1) / kRsTile);
-    cudaError_t e = cudaFuncSetAttribute(k_rs_downsweep<BITS>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                         (int)sizeof(RsSmem<BITS>));
-    if (e != cudaSuccess) return e;
-    launch_after(k_rs_upsweep<BITS>, ntiles, kRsThreads, 0, st, kin, n, shift, hist, ntiles);
-    if ((e = scan_exclusive(hist, (size_t)ntiles << BITS, scan_tmp, st)) != cudaSuccess) return e;
-    launch_after(k_rs_downsweep<BITS>, ntiles, kRsThreads, sizeof(RsSmem<BITS>), st, kin, vin, kout, vout, n, shift,
-                 hist, ntiles, write_keys);
-    return cudaGetLastError();
-}
-
-// words of `hist` a sort of n items needs
-size_t radix_hist_words(size_t n) { return ((n + kRsTile - 1) / kRsTile) << kRsMaxBits; }
-
-cudaError_t radix_sort(uint32_t *keys0, uint32_t *keys1, uint32_t *vals0, uint32_t *vals1, size_t n,
+cudaError_t radix_sort(const hc_ctx *ctx, uint32_t *keys0, uint32_t *keys1, uint32_t *vals0, uint32_t *vals1, size_t n,
                        int bits, uint32_t *hist, uint32_t *scan_tmp, cudaStream_t st, int *which,
                        int *launches, bool keys_out, bool positions_as_values)
 {
     int cur = 0;
     const uint32_t *vin = positions_as_values ? nullptr : vals0;
+    const int items = radix_items(ctx, n);
     const int passes = (bits + kRsMaxBits - 1) / kRsMaxBits, digit = std::max(8, (bits + passes - 1) / passes);
     for (int shift = 0; shift < bits; shift += digit)
     {
@@ -381,10 +412,10 @@ cudaError_t radix_sort(uint32_t *keys0, uint32_t *keys1, uint32_t *vals0, uint32
         {
             const int write_keys = shift + digit >= bits && !keys_out ? 0 : 1;
             const cudaError_t e =
-                digit == 8    ? radix_pass<8>(kin, vin, kout, vout, n, shift, hist, scan_tmp, write_keys, st)
-                : digit == 9  ? radix_pass<9>(kin, vin, kout, vout, n, shift, hist, scan_tmp, write_keys, st)
-                : digit == 10 ? radix_pass<10>(kin, vin, kout, vout, n, shift, hist, scan_tmp, write_keys, st)
-                              : radix_pass<11>(kin, vin, kout, vout, n, shift, hist, scan_tmp, write_keys, st);
+                digit == 8    ? radix_pass<8>(items, kin, vin, kout, vout, n, shift, hist, scan_tmp, write_keys, st)
+                : digit == 9  ? radix_pass<9>(items, kin, vin, kout, vout, n, shift, hist, scan_tmp, write_keys, st)
+                : digit == 10 ? radix_pass<10>(items, kin, vin, kout, vout, n, shift, hist, scan_tmp, write_keys, st)
+                              : radix_pass<11>(items, kin, vin, kout, vout, n, shift, hist, scan_tmp, write_keys, st);
             if (e != cudaSuccess) return e;
             *launches += 3;
         }
@@ -1085,8 +1116,8 @@ int build_length_device(hc_ctx *ctx, LenHost &lh, const hc_entry *h_entries, boo
     HC_CUDA(ctx, scr.alloc(&k1, items));
     HC_CUDA(ctx, scr.alloc(&v0, items));
     HC_CUDA(ctx, scr.alloc(&v1, items));
-    HC_CUDA(ctx, scr.alloc(&hist, radix_hist_words(items)));
-    HC_CUDA(ctx, scr.alloc(&stmp, scan_tmp_words(radix_hist_words(items))));
+    HC_CUDA(ctx, scr.alloc(&hist, radix_hist_words(ctx, items)));
+    HC_CUDA(ctx, scr.alloc(&stmp, scan_tmp_words(radix_hist_words(ctx, items))));
 
     if (sort_by_mass && n > 1)
     {
@@ -1104,7 +1135,7 @@ int build_length_device(hc_ctx *ctx, LenHost &lh, const hc_entry *h_entries, boo
         {
             launch_after(k_mass_keys, (n + 255) / 256, 256, 0, st, d_m0, n, k0);
             int which = 0;
-            HC_CUDA(ctx, radix_sort(k0, k1, v0, v1, n, 32, hist, stmp, st, &which, &launches, false, true));
+            HC_CUDA(ctx, radix_sort(ctx, k0, k1, v0, v1, n, 32, hist, stmp, st, &which, &launches, false, true));
             perm = which ? v1 : v0;
         }
         launch_after(k_gather_entries, (n + 255) / 256, 256, 0, st, perm, n, d_m0, d_s0, d_site0, d_mod0, lh.d_mass,
@@ -1147,7 +1178,7 @@ int build_length_device(hc_ctx *ctx, LenHost &lh, const hc_entry *h_entries, boo
         int bits = 1;
         while ((1ull << bits) < nb) bits++;
         int which = 0;
-        HC_CUDA(ctx, radix_sort(k0, k1, v0, v1, M, bits, hist, stmp, st, &which, &launches, true, true));
+        HC_CUDA(ctx, radix_sort(ctx, k0, k1, v0, v1, M, bits, hist, stmp, st, &which, &launches, true, true));
         uint32_t *skeys = which ? k1 : k0;
         uint32_t *svals = which ? v1 : v0;
         launch_after(k_bucket_bounds, (unsigned)std::min<uint64_t>((nb + 256) / 256, (uint64_t)ctx->sm_count * 32),

@@ -42,10 +42,11 @@ def test_build_load_restore_at_word_edges(npep, tmp_path):
         x.close()
 
 
-@pytest.mark.parametrize("npep", [2, 3, 1024, 1025, 8191, 8192, 8193, 16400])
+@pytest.mark.parametrize("npep", [2, 3, 1024, 1025, 8191, 8192, 8193, 16400, 19455, 19456, 19457])
 def test_entry_order_at_sort_edges(npep):
     """The entries' order where the mass sort changes (one CTA up to 8192 entries, digit
-    passes and their 8192-item tiles past it): ascending, equal masses (the sequences have
+    passes past it; 16 postings an entry, tiles of 2048 of them up to 152 tiles, of 8192
+    past that): ascending, equal masses (the sequences have
     four residues, so most masses repeat) in file order; and the postings sorted from them."""
     from hicops_gb300 import dslim
     from oracle import oracle as O
