@@ -109,12 +109,86 @@ struct PickScale
     __device__ __forceinline__ uint32_t operator()(uint32_t v) const { return top ? (uint32_t)((double)v * factor) : 0u; }
 };
 
+// A warp's part of the shared memory: a spectrum's raw peaks, the kept ones and
+// those next to them in ascending order, and the work space of the tied ranges.
+constexpr uint32_t kPickTop = 128;  // >= HC_QALEN + 1
+static_assert(HC_QALEN < kPickTop && kPickCap <= 1u << 16, "the cut's neighbour is among the sorted; 16-bit positions");
+struct PickSmem
+{
+    unsigned long long top[kPickTop];  // intensity above m/z
+    uint32_t it[kPickCap], ms[kPickCap];
+    uint16_t lp[kPickCap], rp[kPickCap];
+    uint32_t stk[16];  // ranges left to split, the smaller of two first: at most 10 of 1024 peaks
+};
+
+// The reference's sort splits a range at a pivot: i walks up to the next value not
+// below it, j down to the next not above it, the two are swapped, until they cross. What
+// they stop at does not depend on the swaps before, so the t-th swap is of the t-th
+// such value from the left and from the right, as long as the first lies left of the
+// second. Splits it[l, r] that way, the warp together; i and j as the walk leaves them.
+__device__ __forceinline__ void pick_split(PickSmem &S, int l, int r, int lane, int &i, int &j)
+{
+    const uint32_t pivot = S.it[(l + r) / 2], lt = (1u << lane) - 1u;
+    int totr = 0;
+    for (int b = l; b <= r; b += 32)
+    {
+        const int x = b + lane;
+        totr += __popc(__ballot_sync(0xFFFFFFFFu, x <= r && S.it[x] <= pivot));
+    }
+    int totl = 0, seen = 0;
+    for (int b = l; b <= r; b += 32)
+    {
+        const int x = b + lane;
+        const uint32_t v = x <= r ? S.it[x] : 0u;
+        const bool isl = x <= r && v >= pivot, isr = x <= r && v <= pivot;
+        const uint32_t bl = __ballot_sync(0xFFFFFFFFu, isl), br = __ballot_sync(0xFFFFFFFFu, isr);
+        if (isl) S.lp[totl + __popc(bl & lt)] = (uint16_t)x;
+        if (isr) S.rp[totr - 1 - seen - __popc(br & lt)] = (uint16_t)x;
+        totl += __popc(bl);
+        seen += __popc(br);
+    }
+    __syncwarp();
+    int swaps = 0;
+    const int most = min(totl, totr);
+    for (int b = 0; b < most; b += 32)
+    {
+        const int t = b + lane;
+        const int x = t < most ? S.lp[t] : 1, y = t < most ? S.rp[t] : 0;
+        const bool sw = x <= y;
+        if (sw)
+        {
+            const uint32_t v = S.it[x], m = S.ms[x];
+            S.it[x] = S.it[y];
+            S.ms[x] = S.ms[y];
+            S.it[y] = v;
+            S.ms[y] = m;
+        }
+        const uint32_t k = __ballot_sync(0xFFFFFFFFu, sw);
+        swaps += __popc(k);
+        if (k != 0xFFFFFFFFu) break;
+    }
+    __syncwarp();
+    // (the pivot stops both: at least one swap). The walks end at the next value of
+    // their own or at the other's last one, which the swap left on their side; a
+    // swap of one place with itself ends them at once.
+    const int x = S.lp[swaps - 1], y = S.rp[swaps - 1];
+    i = x == y ? x + 1 : min(swaps < totl ? (int)S.lp[swaps] : y, y);
+    j = x == y ? x - 1 : max(swaps < totr ? (int)S.rp[swaps] : x, x);
+    __syncwarp();
+}
+
 // One warp per spectrum of up to kPickCap raw peaks (the others are left to
 // k_pick_long): its kept peaks, in the order of the reference's sort, at
-// QALEN * s of omz / oint, and their count. Bound by the compare-exchanges of the
-// bitonic sort (45 rounds for 300 peaks); 5,000 spectra of 100-500 peaks take
-// 381 us, against 4,210 us with a thread per spectrum running the quicksort in
-// global memory.
+// QALEN * s of omz / oint, and their count.
+//
+// At most HC_QALEN peaks are kept, so only the largest are sorted: a threshold that
+// at least HC_QALEN + 1 and at most kPickTop peaks reach, found by halving, and a
+// bitonic sort of those. The order of equal intensities is what the reference's
+// quicksort leaves; it runs on the raw peaks only where a range of places holds equal
+// ones among the kept, and there a warp splits the range at once. Two of five
+// spectra of 100-500 log-normal intensities hold some. Bound by the latency of its short
+// steps: 5,000 such spectra take 68 us, against 381 us with a sort of all peaks and the
+// quicksort in one lane, and 4,210 with a thread per spectrum.
 __global__ void __launch_bounds__(kPickWarps * 32) k_pick(const uint64_t *__restrict__ off,
                                                          const uint32_t *__restrict__ mz,
                                                          const uint32_t *__restrict__ intn, uint32_t nspec,
@@ -124,9 +198,9 @@ __global__ void __launch_bounds__(kPickWarps * 32) k_pick(const uint64_t *__rest
 {
     extern __shared__ __align__(16) unsigned char psm[];
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    const uint32_t s = blockIdx.x * kPickWarps + (uint32_t)warp;
+    const uint32_t s = blockIdx.x * kPickWarps + (uint32_t)warp, lt = (1u << lane) - 1u;
     if (s >= nspec) return;
-    unsigned long long *key = reinterpret_cast<unsigned long long *>(psm) + (size_t)warp * kPickCap;
+    PickSmem &S = reinterpret_cast<PickSmem *>(psm)[warp];
     const uint64_t o = off[s] - off[0];
     const uint64_t len = off[s + 1] - off[s];
     if (len > kPickCap) return;
@@ -136,11 +210,53 @@ __global__ void __launch_bounds__(kPickWarps * 32) k_pick(const uint64_t *__rest
         if (lane == 0) count[s] = 0;
         return;
     }
-    // intensity above m/z: equal intensities come out next to each other
+    uint32_t most = 0;
+    for (uint32_t i = (uint32_t)lane; i < n; i += 32)
+    {
+        const uint32_t v = intn[o + i];
+        S.it[i] = v;
+        S.ms[i] = mz[o + i];
+        most = max(most, v);
+    }
+    most = __reduce_max_sync(0xFFFFFFFFu, most);
+    __syncwarp();
+    // more than kPickTop peaks reach `below`, HC_QALEN at most reach `thr`, unless one
+    // is found that a number between reaches
+    unsigned long long thr = 0, below = 0;
+    if (n > kPickTop)
+    {
+        unsigned long long hi = (unsigned long long)most + 1;
+        thr = hi;
+        while (hi - below > 1)
+        {
+            const unsigned long long mid = (below + hi) / 2;
+            uint32_t c = 0;
+            for (uint32_t i = (uint32_t)lane; i < n; i += 32) c += S.it[i] >= mid;
+            c = __reduce_add_sync(0xFFFFFFFFu, c);
+            if (c > kPickTop) below = mid;
+            else
+            {
+                thr = mid;
+                if (c > HC_QALEN) break;
+                hi = mid;
+            }
+        }
+    }
+    uint32_t c = 0;  // sorted peaks
+    for (uint32_t b = 0; b < n; b += 32)
+    {
+        const uint32_t i = b + (uint32_t)lane;
+        const bool in = i < n && S.it[i] >= thr;
+        const uint32_t k = __ballot_sync(0xFFFFFFFFu, in);
+        if (in) S.top[c + __popc(k & lt)] = ((unsigned long long)S.it[i] << 32) | S.ms[i];
+        c += (uint32_t)__popc(k);
+    }
+    // the rest up to the cut's neighbour are some of more than 28 equal ones
+    const uint32_t want = min(n, (uint32_t)HC_QALEN + 1u), take = max(c, want);
     uint32_t P = 32;
-    while (P < n) P <<= 1;
-    for (uint32_t i = (uint32_t)lane; i < P; i += 32)
-        key[i] = i < n ? ((unsigned long long)intn[o + i] << 32) | mz[o + i] : ~0ull;
+    while (P < take) P <<= 1;
+    for (uint32_t i = c + (uint32_t)lane; i < P; i += 32) S.top[i] = i < take ? below << 32 : ~0ull;
+    c = take;
     __syncwarp();
     for (uint32_t k = 2; k <= P; k <<= 1)
         for (uint32_t j = k >> 1; j; j >>= 1)
@@ -148,67 +264,101 @@ __global__ void __launch_bounds__(kPickWarps * 32) k_pick(const uint64_t *__rest
             for (uint32_t t = (uint32_t)lane; t < P / 2; t += 32)
             {
                 const uint32_t a = 2 * t - (t & (j - 1)), b = a + j;
-                const unsigned long long x = key[a], y = key[b];
+                const unsigned long long x = S.top[a], y = S.top[b];
                 if ((x > y) == ((a & k) == 0u))
                 {
-                    key[a] = y;
-                    key[b] = x;
+                    S.top[a] = y;
+                    S.top[b] = x;
                 }
             }
             __syncwarp();
         }
-    // (padding sorts last, as does a peak equal to it: the first n are the peaks)
-    const PickScale sc((uint32_t)(key[n - 1] >> 32), base_int);
+    // (padding sorts last, as does a peak equal to it: the first c are the peaks)
+    const PickScale sc((uint32_t)(S.top[c - 1] >> 32), base_int);
     const uint32_t cand = n < HC_QALEN ? n : HC_QALEN;
     uint32_t keep = 1;
     for (uint32_t b = 1; b < cand; b += 32)
     {
         const uint32_t i = b + (uint32_t)lane;
         keep += (uint32_t)__popc(
-            __ballot_sync(0xFFFFFFFFu, i < cand && sc((uint32_t)(key[n - 1 - i] >> 32)) >= min_int));
+            __ballot_sync(0xFFFFFFFFu, i < cand && sc((uint32_t)(S.top[c - 1 - i] >> 32)) >= min_int));
     }
-    // equal intensities of different m/z among the kept, or across the cut
-    bool tie = false;
+    const uint32_t first = c - keep;  // sorted peak c - keep is the first kept one
     for (uint32_t i = (uint32_t)lane; i < keep; i += 32)
-        if (n - 1 - i > 0)
-        {
-            const unsigned long long x = key[n - 1 - i], y = key[n - 2 - i];
-            tie |= x != y && (x >> 32) == (y >> 32);
-        }
-    if (__any_sync(0xFFFFFFFFu, tie))
     {
-        // the reference's own sort, on the raw order
-        uint32_t *it = reinterpret_cast<uint32_t *>(key), *ms = it + kPickCap;
-        __syncwarp();
-        for (uint32_t i = (uint32_t)lane; i < n; i += 32)
+        const unsigned long long x = S.top[first + i];
+        omz[(size_t)s * HC_QALEN + i] = (uint32_t)x;
+        oint[(size_t)s * HC_QALEN + i] = i == keep - 1 ? base_int : sc((uint32_t)(x >> 32));
+    }
+    if (lane == 0) count[s] = keep;
+    // bit e of the words of lanes 0..3: sorted peaks e and e + 1 are equally intense, and e + 1 is kept
+    uint32_t tied = 0;
+    bool any = false;
+#pragma unroll
+    for (uint32_t w = 0; w < kPickTop / 32; w++)
+    {
+        const uint32_t e = 32 * w + (uint32_t)lane;
+        const bool t = e + 1 < c && e + 1 >= first && (S.top[e] >> 32) == (S.top[e + 1] >> 32);
+        const uint32_t m = __ballot_sync(0xFFFFFFFFu, t);
+        if ((uint32_t)lane == w) tied = m;
+        any |= m != 0u;
+    }
+    if (!any) return;
+    const int base = (int)n - (int)c;  // the place of sorted peak e is base + e
+    auto holds_tie = [&](int l, int r) {  // two equal kept peaks at the places l .. r?
+        const int lo = min(max(l - base - 32 * lane, 0), 32), hi = min(max(r - base - 32 * lane, 0), 32);
+        const uint32_t m = (hi > 31 ? 0xFFFFFFFFu : (1u << hi) - 1u) & ~(lo > 31 ? 0xFFFFFFFFu : (1u << lo) - 1u);
+        return __any_sync(0xFFFFFFFFu, lane < (int)(kPickTop / 32) && (tied & m) != 0u) != 0;
+    };
+    // the peaks of a range without such: each one that equals others elsewhere is the
+    // only one here, at the first of their places that the range has
+    auto settle = [&](int l, int r) {
+        for (int x = l + lane; x <= r; x += 32)
         {
-            it[i] = intn[o + i];
-            ms[i] = mz[o + i];
+            const uint32_t v = S.it[x];
+            uint32_t lo = 0, hi = c;  // the first sorted peak that is not below v
+            while (lo < hi)
+            {
+                const uint32_t mid = (lo + hi) / 2;
+                if ((uint32_t)(S.top[mid] >> 32) < v) lo = mid + 1;
+                else hi = mid;
+            }
+            if (lo + 1 >= c || (uint32_t)(S.top[lo + 1] >> 32) != v) continue;
+            const int e = max((int)lo, l - base);
+            if ((uint32_t)(S.top[lo] >> 32) == v && e >= (int)first) omz[(size_t)s * HC_QALEN + (e - (int)first)] = S.ms[x];
         }
-        __syncwarp();
-        bool ok = true;
-        if (lane == 0) ok = key_sort(it, ms, (int)n);
-        __syncwarp();
-        if (!__shfl_sync(0xFFFFFFFFu, (int)ok, 0))
+    };
+    __syncwarp();
+    int l = 0, r = (int)n - 1, sp = 0;
+    for (;;)
+    {
+        int i, j;
+        pick_split(S, l, r, lane, i, j);
+        if (i - j > 1) settle(j + 1, i - 1);
+        const int keep_from = base + (int)first;
+        const bool ta = holds_tie(l, j), tb = holds_tie(i, r);
+        if (!ta && l <= j && j >= keep_from) settle(l, j);
+        if (!tb && i <= r && r >= keep_from) settle(i, r);
+        if (ta && tb)
         {
-            if (lane == 0) count[s] = 0xFFFFFFFFu;  // cannot happen with its stack bound; reported as an error
-            return;
+            const bool lefts = j - l > r - i;  // the larger one waits
+            if (lane == 0) S.stk[sp] = lefts ? (uint32_t)l << 16 | (uint32_t)j : (uint32_t)i << 16 | (uint32_t)r;
+            sp++;
+            __syncwarp();
+            if (lefts) l = i;
+            else r = j;
         }
-        for (uint32_t i = (uint32_t)lane; i < keep; i += 32)
+        else if (ta) r = j;
+        else if (tb) l = i;
+        else
         {
-            const uint32_t j = n - keep + i;
-            omz[(size_t)s * HC_QALEN + i] = ms[j];
-            oint[(size_t)s * HC_QALEN + i] = j == n - 1 ? base_int : sc(it[j]);
+            if (sp == 0) break;
+            const uint32_t q = S.stk[--sp];
+            __syncwarp();
+            l = (int)(q >> 16);
+            r = (int)(q & 0xFFFFu);
         }
     }
-    else
-        for (uint32_t i = (uint32_t)lane; i < keep; i += 32)
-        {
-            const uint32_t j = n - keep + i;
-            omz[(size_t)s * HC_QALEN + i] = (uint32_t)key[j];
-            oint[(size_t)s * HC_QALEN + i] = j == n - 1 ? base_int : sc((uint32_t)(key[j] >> 32));
-        }
-    if (lane == 0) count[s] = keep;
 }
 
 // The spectra of more than kPickCap raw peaks, a thread each, sorted in place
@@ -1003,7 +1153,7 @@ extern "C" int hc_ms2_extract(hc_ctx *ctx, hc_ms2 *m, uint32_t first, uint32_t c
     }
     const uint32_t *r_mz = there ? m->d_mz + r0 : d_mz, *r_int = there ? m->d_int + r0 : d_int;
     const uint32_t base_int = (uint32_t)ctx->p.base_int, min_int = (uint32_t)ctx->p.min_int;
-    constexpr int kPickSmem = kPickWarps * (int)kPickCap * 8;
+    constexpr int kPickSmem = kPickWarps * (int)sizeof(PickSmem);
     HC_CUDA(ctx, cudaFuncSetAttribute(k_pick, cudaFuncAttributeMaxDynamicSharedMemorySize, kPickSmem));
     k_pick<<<(n + kPickWarps - 1) / kPickWarps, kPickWarps * 32, kPickSmem, st>>>(d_off, r_mz, r_int, n, base_int, min_int,
                                                                                d_idx + 1, d_kmz, d_kint);

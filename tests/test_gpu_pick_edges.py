@@ -1,5 +1,5 @@
 """Peak picking where its sort changes: powers of two of the bitonic sort, the QALEN
-cut, the largest spectrum sorted in shared memory and the ones past it, with
+cut, the most peaks that are sorted without a threshold, the largest spectrum sorted in shared memory and the ones past it, with
 distinct intensities, a few equal ones (among the kept peaks, across the cut, below
 it) and only equal ones; against the reader's restatement."""
 import numpy as np
@@ -13,7 +13,7 @@ pytestmark = pytest.mark.gpu
 SIZES = [0, 1, 2, 3, 31, 32, 33, 99, 100, 101, 102, 127, 128, 129, 512, 513, 1024, 1025, 1500]
 
 
-@pytest.mark.parametrize("kind", ["distinct", "few", "cut", "below", "all", "zero"])
+@pytest.mark.parametrize("kind", ["distinct", "few", "cut", "below", "levels", "steps", "all", "zero"])
 @pytest.mark.parametrize("pick", [(100, 100000, 1000), (10, 5000, 0)])
 def test_pick_at_sort_edges(kind, pick, tmp_path):
     rng = np.random.default_rng(17)
@@ -28,6 +28,10 @@ def test_pick_at_sort_edges(kind, pick, tmp_path):
             it[o[98:102]] = it[o[98]]
         if kind == "below" and n > 128:
             it[o[110:120]] = it[o[110]]
+        if kind == "levels":  # groups of equal ones everywhere
+            it = np.floor(it / (100 if n > 200 else 12))
+        if kind == "steps":  # ... in ascending order, the largest group across the cut
+            it = np.sort(np.floor(it / 40))
         if kind == "all":
             it[:] = 77.5
         if kind == "zero":
