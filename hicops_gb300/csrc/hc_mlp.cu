@@ -516,19 +516,22 @@ __global__ void __launch_bounds__(256) k_grad_reduce(const float *__restrict__ p
 // all parameters (162 KB) in shared memory once and takes 64 spectra at a
 // time, inputs arriving in chunks of 64 through cp.async. A thread of layer 1
 // holds 8 x 8 outputs (one shared-memory read of 16 bytes for 16 FMAs), two
-// groups of four warps take half of each layer's inputs. 100,000 spectra: 176 us,
-// against 344 us with two spectra per warp, where a weight read served 8 FMAs,
-// and 202 us with one FMA to an instruction.
+// groups of four warps take half of each layer's inputs; with two warps a
+// scheduler to cover each other's reads, the loops over the inputs are unrolled
+// whole (176 -> 167 us below). What is left over after whole waves of tiles goes in
+// half tiles of 32 if one wave takes it (167 -> 161 us; 9,800 spectra 34.8 -> 27.9).
+// 100,000 spectra: 161 us, against 344 us with two spectra per warp, where a weight
+// read served 8 FMAs, and 202 us with one FMA to an instruction.
 //
 // k_infer_rows, for the rest: a CTA takes 8 spectra and its 16 warps 1/16 of
 // each layer's inputs, so every weight is read once per CTA, straight from L2
 // with no staging. 1,000 spectra: 8.2 us, against 14.3 us.
 //
-// The line between them: a tile takes 20.5 us up to 64 spectra per SM, rows
-// 12.3 us at 16 per SM, 20.5 us at 32 and 36.9 us at 64.
+// The line between them: half a tile takes 12.3 us up to 32 spectra per SM, rows
+// 8.2 us at 8 per SM, 12.3 us at 16, 16.4 at 20 and 20.5 us at 32.
 constexpr int kTileThreads = 256, kRowsThreads = 512;
 constexpr int kInferTile = 64, kInferChunk = 64, kInferRows = 8;
-constexpr uint32_t kInferRowsPerSm = 32;
+constexpr uint32_t kInferRowsPerSm = 16;
 
 struct InferSmem
 {
@@ -554,21 +557,26 @@ __device__ __forceinline__ float4 relu4(const float4 &a, const float4 &p, const 
 }
 
 __global__ void __launch_bounds__(kTileThreads, 1) k_infer_tile(const float *__restrict__ P, const float *__restrict__ X,
-                                                                uint32_t n, float *__restrict__ out)
+                                                                uint32_t n, uint32_t nfull, uint32_t ntiles,
+                                                                float *__restrict__ out)
 {
     extern __shared__ __align__(16) unsigned char ism[];
     InferSmem &S = *reinterpret_cast<InferSmem *>(ism);
     const int tid = threadIdx.x;
-    // group q of 128 threads takes half of the inputs; a thread 8 rows from rb
-    const int q = tid >> 7, cg = tid & 15, rb = 8 * ((tid >> 4) & 7);
-    const uint32_t ntiles = (n + kInferTile - 1) / kInferTile;
-    // chunk c of a tile's inputs, four 16-byte copies a thread
+    // group q of 128 threads takes half of the inputs; a thread 8 rows (4 of a half tile)
+    const int q = tid >> 7, cg = tid & 15;
+    auto first_row = [&](uint32_t tile) {
+        return tile < nfull ? tile * kInferTile : nfull * kInferTile + (tile - nfull) * (kInferTile / 2);
+    };
+    // chunk c of a tile's inputs, four 16-byte copies a thread (two of a half tile)
     auto load = [&](uint32_t tile, int c) {
+        const uint32_t row0 = first_row(tile);
 #pragma unroll
         for (int i = 0; i < 4; i++)
         {
+            if (i == 2 && tile >= nfull) break;
             const int r = (tid >> 4) + 16 * i, j = 4 * (tid & 15);
-            const uint32_t row = tile * kInferTile + (uint32_t)r;
+            const uint32_t row = row0 + (uint32_t)r;
             cp_async16(&S.xs[c & 1][r][j], X + (size_t)min(row, n - 1) * kIn + c * kInferChunk + j, row < n);
         }
     };
@@ -587,13 +595,15 @@ __global__ void __launch_bounds__(kTileThreads, 1) k_infer_tile(const float *__r
     for (int i = tid; i < kH1 + kH2 + kOut; i += kTileThreads)
         S.b[i] = __ldg(P + (i < kH1 ? kOffB1 + i : (i < kH1 + kH2 ? kOffB2 + i - kH1 : kOffB3 + i - kH1 - kH2)));
     bool first = true;
-    for (uint32_t tile = blockIdx.x; tile < ntiles; tile += gridDim.x)
-    {
-        // layer 1: 8 x 8 outputs a thread (units 4cg.., 64 + 4cg..), half of each chunk
+    // a tile of 8 * RT rows
+    auto run = [&](auto rt, uint32_t tile) {
+        constexpr int RT = decltype(rt)::value;
+        const int rb = RT * ((tid >> 4) & 7);
+        // layer 1: RT x 8 outputs a thread (units 4cg.., 64 + 4cg..), half of each chunk
         {
-            float4 acc[8][2];
+            float4 acc[RT][2];
 #pragma unroll
-            for (int r = 0; r < 8; r++) acc[r][0] = acc[r][1] = make_float4(0.f, 0.f, 0.f, 0.f);
+            for (int r = 0; r < RT; r++) acc[r][0] = acc[r][1] = make_float4(0.f, 0.f, 0.f, 0.f);
             for (int c = 0; c < kIn / kInferChunk; c++)
             {
                 if (first) asm volatile("cp.async.wait_group 1;" ::: "memory");
@@ -606,12 +616,12 @@ __global__ void __launch_bounds__(kTileThreads, 1) k_infer_tile(const float *__r
                     commit();
                 }
                 const float *xc = &S.xs[c & 1][rb][0];
-#pragma unroll 1
+#pragma unroll
                 for (int k = 32 * q; k < 32 * q + 32; k += 4)
                 {
-                    float4 x[8];
+                    float4 x[RT];
 #pragma unroll
-                    for (int r = 0; r < 8; r++) x[r] = *reinterpret_cast<const float4 *>(xc + r * kInferChunk + k);
+                    for (int r = 0; r < RT; r++) x[r] = *reinterpret_cast<const float4 *>(xc + r * kInferChunk + k);
 #pragma unroll
                     for (int i = 0; i < 4; i++)
                     {
@@ -619,7 +629,7 @@ __global__ void __launch_bounds__(kTileThreads, 1) k_infer_tile(const float *__r
                         const float4 wa = *reinterpret_cast<const float4 *>(w);
                         const float4 wb = *reinterpret_cast<const float4 *>(w + kH1 / 2);
 #pragma unroll
-                        for (int r = 0; r < 8; r++)
+                        for (int r = 0; r < RT; r++)
                         {
                             const float xv = i == 0 ? x[r].x : i == 1 ? x[r].y : i == 2 ? x[r].z : x[r].w;
                             fma4(acc[r][0], xv, wa);
@@ -630,7 +640,7 @@ __global__ void __launch_bounds__(kTileThreads, 1) k_infer_tile(const float *__r
             }
             if (q == 1)
 #pragma unroll
-                for (int r = 0; r < 8; r++)
+                for (int r = 0; r < RT; r++)
 #pragma unroll
                     for (int h = 0; h < 2; h++)
                         *reinterpret_cast<float4 *>(&S.h1[rb + r][64 * h + 4 * cg]) = acc[r][h];
@@ -647,7 +657,7 @@ __global__ void __launch_bounds__(kTileThreads, 1) k_infer_tile(const float *__r
                 {
                     const float4 b = *reinterpret_cast<const float4 *>(&S.b[64 * h + 4 * cg]);
 #pragma unroll
-                    for (int r = 0; r < 8; r++)
+                    for (int r = 0; r < RT; r++)
                     {
                         float4 *p = reinterpret_cast<float4 *>(&S.h1[rb + r][64 * h + 4 * cg]);
                         *p = relu4(acc[r][h], *p, b);
@@ -655,21 +665,21 @@ __global__ void __launch_bounds__(kTileThreads, 1) k_infer_tile(const float *__r
                 }
             __syncthreads();
         }
-        // layer 2: 8 x 4 outputs a thread, half of the inputs; its sums and then
+        // layer 2: RT x 4 outputs a thread, half of the inputs; its sums and then
         // its result take the second chunk's buffer
         float(*h2)[kH2] = S.xs[1];
         {
-            float4 acc[8];
+            float4 acc[RT];
 #pragma unroll
-            for (int r = 0; r < 8; r++) acc[r] = make_float4(0.f, 0.f, 0.f, 0.f);
-#pragma unroll 2
+            for (int r = 0; r < RT; r++) acc[r] = make_float4(0.f, 0.f, 0.f, 0.f);
+#pragma unroll
             for (int k = 64 * q; k < 64 * q + 64; k += 4)
             {
                 float4 w[4];
 #pragma unroll
                 for (int i = 0; i < 4; i++) w[i] = *reinterpret_cast<const float4 *>(&S.w2[k + i][4 * cg]);
 #pragma unroll
-                for (int r = 0; r < 8; r++)
+                for (int r = 0; r < RT; r++)
                 {
                     const float4 x = *reinterpret_cast<const float4 *>(&S.h1[rb + r][k]);
                     fma4(acc[r], x.x, w[0]);
@@ -680,13 +690,13 @@ __global__ void __launch_bounds__(kTileThreads, 1) k_infer_tile(const float *__r
             }
             if (q == 1)
 #pragma unroll
-                for (int r = 0; r < 8; r++) *reinterpret_cast<float4 *>(&h2[rb + r][4 * cg]) = acc[r];
+                for (int r = 0; r < RT; r++) *reinterpret_cast<float4 *>(&h2[rb + r][4 * cg]) = acc[r];
             __syncthreads();
             if (q == 0)
             {
                 const float4 b = *reinterpret_cast<const float4 *>(&S.b[kH1 + 4 * cg]);
 #pragma unroll
-                for (int r = 0; r < 8; r++)
+                for (int r = 0; r < RT; r++)
                 {
                     float4 *p = reinterpret_cast<float4 *>(&h2[rb + r][4 * cg]);
                     *p = relu4(acc[r], *p, b);
@@ -695,6 +705,7 @@ __global__ void __launch_bounds__(kTileThreads, 1) k_infer_tile(const float *__r
             __syncthreads();
         }
         // layer 3: four lanes a row
+        if (RT == 8 || tid < 4 * 8 * RT)
         {
             const int r = tid >> 2, i = tid & 3;
             // short sums added pairwise: they round less than one long one
@@ -720,10 +731,15 @@ __global__ void __launch_bounds__(kTileThreads, 1) k_infer_tile(const float *__r
                 o.z += __shfl_xor_sync(0xFFFFFFFFu, o.z, d);
                 o.w += __shfl_xor_sync(0xFFFFFFFFu, o.w, d);
             }
-            const uint32_t row = tile * kInferTile + (uint32_t)r;
+            const uint32_t row = first_row(tile) + (uint32_t)r;
             if (row < n)
                 out[(size_t)row * kOut + i] = (i == 0 ? o.x : i == 1 ? o.y : i == 2 ? o.z : o.w) + S.b[kH1 + kH2 + i];
         }
+    };
+    for (uint32_t tile = blockIdx.x; tile < ntiles; tile += gridDim.x)
+    {
+        if (tile < nfull) run(std::integral_constant<int, 8>{}, tile);
+        else run(std::integral_constant<int, 4>{}, tile);
     }
 }
 
@@ -1097,9 +1113,12 @@ static int mlp_infer(hc_mlp *m, const float *X, uint32_t n, float *out, cudaStre
     {
         HC_CUDA(m->ctx, cudaFuncSetAttribute(k_infer_tile, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                              (int)sizeof(InferSmem)));
-        const uint32_t tiles = (n + kInferTile - 1) / kInferTile;
-        k_infer_tile<<<std::min(tiles, (uint32_t)m->ctx->sm_count), kTileThreads, sizeof(InferSmem), st>>>(m->d_params,
-                                                                                                             X, n, out);
+        // whole waves of full tiles, and what is left over in half tiles where one wave takes it
+        const uint32_t sms = (uint32_t)m->ctx->sm_count;
+        uint32_t nfull = n / (kInferTile * sms) * sms, rest = n - nfull * kInferTile, ntiles;
+        if (rest <= kInferTile / 2 * sms) ntiles = nfull + (rest + kInferTile / 2 - 1) / (kInferTile / 2);
+        else ntiles = nfull = (n - 1) / kInferTile + 1;
+        k_infer_tile<<<std::min(ntiles, sms), kTileThreads, sizeof(InferSmem), st>>>(m->d_params, X, n, nfull, ntiles, out);
     }
     HC_CUDA(m->ctx, cudaGetLastError());
     return HC_SUCCESS;

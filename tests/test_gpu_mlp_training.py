@@ -68,10 +68,11 @@ def test_training_follows_float64_adam(n, batch):
     ix.close()
 
 
-@pytest.mark.parametrize("n", [1, 7, 8, 9, 4864, 4865, 9728, 9791, 10001])
+@pytest.mark.parametrize("n", [1, 7, 8, 9, 2432, 2433, 2465, 4864, 4865, 9728, 9729, 9761, 9791, 10001, 14592,
+                               14593])
 def test_inference_at_tile_edges(n):
-    """Both inference kernels at the edges of their tiles and of the line between them
-    (32 spectra per SM of a 152-SM part), and nothing written past the last spectrum.
+    """Both inference kernels at the edges of their tiles, of the line between them (16
+    spectra per SM of a 152-SM part) and of the last wave's half tiles, and nothing written past the last spectrum.
     256 + 128 + 64 FP32 terms: within 448 * 2^-24 of the largest output."""
     import torch
     from hicops_gb300 import dslim
