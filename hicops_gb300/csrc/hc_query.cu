@@ -195,6 +195,7 @@ struct SmemTail
     // per entry class: what its y1 keys collect from the spectrum's valid
     // peaks, packed [count:8 | sum:24]; entry kClassNone stays zero
     uint32_t upk[kMaxClasses + 1];
+    uint32_t ncu, cu;          // how many of them are not zero; one that is not
     uint32_t nlow;
 };
 
@@ -290,6 +291,15 @@ __device__ __forceinline__ void decode(const typename Card<WIDE>::word *card, ui
     }
     // the reference reads bc/yc through short/ushort (dslim_query.cpp:684-686)
     shp = (uint32_t)(uint16_t)(bc + yc);
+}
+
+// byte k's top bit of x (S = 0x8888 + k * 0x1111) in every bit
+template <uint32_t S>
+__device__ __forceinline__ uint32_t byte_sign(uint32_t x)
+{
+    uint32_t r;
+    asm("prmt.b32 %0, %1, 0, %2;" : "=r"(r) : "r"(x), "n"(S));
+    return r;
 }
 
 // 32-bit adds to a shared-memory word given by its shared-window address.
@@ -639,6 +649,7 @@ __global__ void __launch_bounds__(G >= 4 ? 512 : 1024, G == 4 ? 2 : 1) k_search(
             T.bytes = 0;
             T.nv = 0;
             T.nlow = 0;
+            T.ncu = 0;
         }
         for (uint32_t l = tid; l < a.nlen; l += nthr) T.win[l] = a.win[(size_t)s * a.nlen + l];
         for (uint32_t i = tid; i < kMaxClasses + 1; i += nthr) ucls[i] = 0ull;
@@ -721,6 +732,11 @@ __global__ void __launch_bounds__(G >= 4 ? 512 : 1024, G == 4 ? 2 : 1) k_search(
             const unsigned long long u = ucls[i];
             if (!WIDE && (u >> 40) >= 64u) T.overflow = 1;
             T.upk[i] = ((uint32_t)(u >> 40) << 24) | (uint32_t)(u & 0xFFFFFFull);
+            if (u)
+            {
+                T.cu = i;
+                atomicAdd(&T.ncu, 1u);
+            }
         }
         __syncthreads();
         // the set-up's tables are read: their space takes the scoring's (seen
@@ -1115,7 +1131,36 @@ __global__ void __launch_bounds__(G >= 4 ? 512 : 1024, G == 4 ? 2 : 1) k_search(
                 uint4 *z4 = reinterpret_cast<uint4 *>(card);
                 const uint32_t lim = max(ntile, nn);
                 const bool al4 = (nj.c0 & 3u) == 0u;  // class bytes readable as one word (warp-uniform)
-                for (uint32_t base = first; base < lim; base += step)
+                uint32_t base = first;
+                // The steps that lie in the next job. Most spectra have a peak at the
+                // y1 keys of one class (K or R at the end) or of none: a compare
+                // takes the place of the table, and with none the classes are
+                // not read at all; without the edges' checks, and with stores that
+                // meet no bank twice, a step takes half the instructions
+                // (2,432 open-search spectra: 6.26 -> 6.06 ms).
+                const uint32_t ncu = T.ncu;
+                if (ncu == 0u)
+                    for (; base + 128u <= nn; base += step)
+                        z4[(base >> 1) + (uint32_t)lane] = z4[(base >> 1) + 32u + (uint32_t)lane] =
+                            make_uint4(0u, 0u, 0u, 0u);
+                else if (ncu == 1u && al4)
+                {
+                    const uint32_t cu4 = T.cu * 0x01010101u, cu_y = T.upk[T.cu];
+                    const uint16_t *cp = reinterpret_cast<const uint16_t *>(ncls) + lane;
+                    uint32_t hits = 0;
+                    for (; base + 128u <= nn; base += step)
+                    {
+                        const uint32_t k4 = __ldg(cp + (base >> 1)) | (uint32_t)__ldg(cp + (base >> 1) + 32) << 16;
+                        // class ids stay below 128: a byte's top bit is set where it is the class
+                        const uint32_t e = (0x80808080u - (k4 ^ cu4)) & 0x80808080u;
+                        hits += (uint32_t)__popc(e);
+                        uint4 *z = z4 + (base >> 1) + lane;
+                        z[0] = make_uint4(0u, cu_y & byte_sign<0x8888>(e), 0u, cu_y & byte_sign<0x9999>(e));
+                        z[32] = make_uint4(0u, cu_y & byte_sign<0xAAAA>(e), 0u, cu_y & byte_sign<0xBBBB>(e));
+                    }
+                    npass += hits * (cu_y >> 24);
+                }
+                for (; base < lim; base += step)
                 {
                     const uint32_t c = base + 4 * (uint32_t)lane;
                     uint32_t k4 = kClassNone * 0x01010101u;
