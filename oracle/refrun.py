@@ -40,7 +40,7 @@ def reference_dir() -> str:
 def build(ref_root: str | None = None) -> bool:
     """Compile the reference into oracle/_ref when its sources are present."""
     ref_root = ref_root or reference_dir()
-    if not os.path.isdir(ref_root):
+    if not os.path.isdir(os.path.join(ref_root, "source", "core")):
         return False
     subprocess.run(["make", "-s", "-C", os.path.join(HERE, "ref"), f"REF={ref_root}",
                     f"-j{os.cpu_count() or 4}"], check=True)
