@@ -12,7 +12,11 @@ namespace hc {
 // have (release_successor), and each waits for its predecessor's end, and sees
 // what it wrote, before it reads any of it, writes anything or ends itself
 // (after_predecessor; nothing to wait for in a launch without the attribute, or behind
-// a copy). So when a kernel ends, all before it have.
+// a copy). So when a kernel ends, all before it have. A kernel that waits releases
+// only after its wait: its successor then starts, with an L1 emptied, when all
+// kernels before the two have ended, and lines that could go stale under it are only
+// those that its predecessor both reads and writes. Kernels that do work in
+// place keep each CTA to 128-byte lines of its own, or have no successor launched so.
 __device__ __forceinline__ void after_predecessor() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 __device__ __forceinline__ void release_successor() { asm volatile("griddepcontrol.launch_dependents;"); }
 

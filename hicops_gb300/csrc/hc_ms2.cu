@@ -4,11 +4,11 @@
 // (k_ms2_lines), small ones, and those with a peak line that is not two plain
 // decimal numbers, on the host. hc_ms2_extract then hands out batches the
 // way MSQuery::extractbatch does (msquery.cpp:239-297), with the peak picking
-// of MSQuery::pickpeaks (msquery.cpp:509-569) on the device, one thread per
-// spectrum: sort the peaks by intensity with the reference's quicksort
-// (KeyVal_Parallel_Internal, source/core/include/keyval.h:48-104: Hoare
-// partition around the middle key, which fixes the order of equal
-// intensities), set the top peak to base_int, scale the next QALEN-1 by
+// of MSQuery::pickpeaks (msquery.cpp:509-569) on the device, a warp per
+// spectrum: sort the peaks by intensity, equal ones in the order that the
+// reference's quicksort leaves them in (KeyVal_Parallel_Internal,
+// source/core/include/keyval.h:48-104: Hoare partition around the middle
+// key), set the top peak to base_int, scale the next QALEN-1 by
 // base_int / top (truncated to integers) and keep the highest ones that
 // reach min_int. A second kernel prefix-sums the kept counts and a third
 // copies the kept peaks into the CSR batch.

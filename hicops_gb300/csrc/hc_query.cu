@@ -1,24 +1,24 @@
 // DSLIM query on the device (DSLIM_QuerySpectrum, source/core/dslim_query.cpp:515-842).
 //
-// Kernels, in launch order:
+// Kernels, in launch order (each starts under the end of the one before, see launch_after):
 //   k_windows   one thread per (spectrum, length): the precursor window
 //               [minlimit, maxlimit] of DSLIM_BinarySearch (dslim_query.cpp:854-994).
 //   k_search    persistent CTAs, one spectrum at a time (work stealing):
 //               for every length with a non-empty window, the candidate range
 //               is cut into shared-memory scorecard tiles; the postings of every
 //               (peak, bin) pair (dslim_query.cpp:617-676) are streamed with
-//               coalesced loads from a per-pair cursor, and each posting adds
-//               (count, intensity) to its candidate's packed 64-bit scorecard
-//               word with one shared-memory atomic. A candidate enters the
-//               qualifying list the moment its shared-peak count reaches
-//               min_shp; listed candidates are scored (dslim_query.cpp:679-725)
+//               coalesced loads, and each posting adds (count, intensity) to its
+//               candidate's packed b or y word with one shared-memory atomic. Then
+//               the tile is scanned, and the candidates whose shared-peak count
+//               reaches min_shp are scored (dslim_query.cpp:679-725)
 //               into the 1002-bin histogram, cpsms and the top hit.
 //   k_search_small the same for spectra whose windows hold few candidates: all
 //               their windows in one scorecard.
 //   k_search<WIDE> the same for spectra whose packed words could overflow
 //               (a count past 127): 2 x 64-bit words per candidate, exact FP64.
-//   k_tailfit   one thread per spectrum: expeRT::ModelTailFit (expeRT.cpp:572-718)
-//               and e(x) = 10^(mu*maxhyp + beta) * cpsms (dslim_query.cpp:773-799).
+//   k_tailfit   expeRT::ModelTailFit (expeRT.cpp:572-718) and
+//               e(x) = 10^(mu*maxhyp + beta) * cpsms (dslim_query.cpp:773-799):
+//               a warp per spectrum for its curve, then a lane per spectrum.
 //
 // Hyperscore. The reference evaluates h = lgfact[bc] + lgfact[yc] +
 // log10(1+ibc) + log10(1+iyc) - 6 in double and stores it as float. Here it is
@@ -177,7 +177,6 @@ struct SmemTail
     uint32_t best_shp;
     uint32_t maxbits;          // running max of the float estimate
     uint32_t cpsms;
-    uint32_t qcount;
     uint32_t flags;
     uint32_t overflow;
     uint32_t spec;
@@ -212,7 +211,7 @@ struct SmemTail
 
 struct SmemLayout
 {
-    size_t qual, defer, lnext, lend, loff, coff, kinfo, pmoz, pint, wq, ucls, sink, tail, total;
+    size_t defer, lnext, lend, loff, coff, kinfo, pmoz, pint, wq, ucls, sink, tail, total;
     uint32_t maxpairs;  // lists: valid peaks x bins
 };
 
@@ -223,8 +222,7 @@ __host__ __device__ inline SmemLayout smem_layout(uint32_t tile, uint32_t dF, bo
     // the scorecard, then the undecided queue: the scan reads whole
     // 128-candidate steps, and a window's last step may read up to 127 words
     // past the tile's end (masked), inside the queue
-    o.qual = wide ? (size_t)tile * 16 : (size_t)tile * 8;
-    o.defer = o.qual;
+    o.defer = wide ? (size_t)tile * 16 : (size_t)tile * 8;
     o.maxpairs = (uint32_t)maxpairs;
     // per list (of the next job: written while the job streams): its first
     // posting, the end of its list, its chunk count; per non-empty list of
@@ -533,7 +531,6 @@ __global__ void __launch_bounds__(G >= 4 ? 512 : 1024, G == 4 ? 2 : 1) k_search(
         for (int k = 0; k < 4; k++) T.cnt[k] = 0;
         T.ph_last = clock64();
         T.pnext = 0;   // reset again after every tile
-        T.qcount = 0;
     }
 
     // Scores one candidate (the float estimate; undecided ones are queued):
@@ -642,8 +639,7 @@ __global__ void __launch_bounds__(G >= 4 ? 512 : 1024, G == 4 ? 2 : 1) k_search(
             T.best_shp = 0;
             T.maxbits = 0;
             T.cpsms = 0;
-            T.qcount = 0;
-            T.ndefer = 0;
+                T.ndefer = 0;
             T.flags = WIDE ? HC_FLAG_WIDE : 0u;
             T.overflow = 0;
             T.bytes = 0;
