@@ -877,7 +877,7 @@ struct TailGate
 // quotients and a power, or a logarithm), and an FP64 instruction costs the
 // same for one lane as for 32, so it runs with a lane per spectrum, sixteen
 // spectra at a time, and not at all for the training targets. Targets of 50,000
-// spectra: 46 us, against 215 us with the FP64 part on one lane per spectrum.
+// spectra: 43 us, against 215 us with the FP64 part on one lane per spectrum.
 struct LtJob
 {
     float slope, icpt;
@@ -889,7 +889,7 @@ struct LtJob
 struct LtSmem
 {
     LtJob job[kLtWarps];
-    uint32_t cum[kLtWarps][HC_HIST_BINS];  // cumulative counts, then the curve in their place
+    alignas(16) uint32_t cum[kLtWarps][kCumRow];  // cumulative counts, then the curve in their place
 };
 
 // The e-value of a job, one lane each: e(x) from the line as the reference forms

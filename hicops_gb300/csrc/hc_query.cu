@@ -1993,7 +1993,7 @@ struct TfSmem
     double sx[HC_HIST_BINS + 2];  // tailfit_one's
     double2 tab[kLgTab];
     TfJob job[kTfWarps];
-    uint32_t cum[kTfWarps][HC_HIST_BINS];
+    alignas(16) uint32_t cum[kTfWarps][kCumRow];
 };
 
 // log10 of a positive normal double up to 1, within 4e-15
