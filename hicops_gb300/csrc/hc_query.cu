@@ -1288,6 +1288,7 @@ constexpr uint32_t kSmStep = 128;
 constexpr uint32_t kSmWQ = 128;      // candidates waiting per warp (a power of two, >= 31 + 64)
 constexpr uint32_t kSmCtas = 4;
 // launch shapes picked for a context that chose none (see launch_packed)
+constexpr uint32_t kWideWindows = 512;  // (spectrum, length) pairs per SM up to which windows are searched four ways
 constexpr uint32_t kAutoSmallLog2 = 15, kAutoAllSmall = 1u << 16, kAutoOrder = 1024;
 
 struct SmSeg
@@ -1735,24 +1736,27 @@ __global__ void __launch_bounds__(kSmThreads, 4) k_search_small(SearchArgs a)
 
 // ---- windows: DSLIM_BinarySearch (dslim_query.cpp:854-994) -----------------
 // The first of m's n sorted masses that is not below x1, and the first that is
-// above x2: one four-way search for each, three loads of either in flight at a time.
+// above x2: a search in P + 1 parts for each, P loads of either in flight at a time.
 // The limits are the reference's (its binary search and the walks at its end find the
 // same places), and a NaN limit finds no window.
 //
-// A batch waits for this kernel before it can search anything, and what bounds it is
-// the chain of dependent loads: two halving searches one after the other, with a walk
-// over the last 20 masses each, took 9 us for 8 spectra against 34 lengths of 600 masses;
-// this takes 6 us for 2,000. With the launches' overlap the device's part of such a
-// search fell from 47 to 34 us for 8 spectra and from 132 to 117 us for 2,000.
+// A batch waits for this kernel before it can search anything. What bounds it is
+// the chain of dependent loads while all pairs run at once (two halving searches one
+// after the other, with a walk over the last 20 masses each, took 9 us for 8 spectra
+// against 34 lengths of 600 masses; four ways this takes 4 us), and the loads
+// themselves in larger batches, of which four ways take half as many again. Against 34
+// lengths of up to 60,000 masses, four ways / two: 8 spectra 4.7 / 5.8 us, 2,000 9.1 /
+// 11.3, 6,000 18.9 / 14.3, 60,000 130 / 90.
+template <int P>
 __device__ __forceinline__ int2 find_limits(const float *__restrict__ m, int n, float x1, float x2)
 {
     int b1 = 0, b2 = 0, n1 = n, n2 = n;
     while (n1 > 0 || n2 > 0)
     {
-        const int s1 = (n1 + 3) >> 2, s2 = (n2 + 3) >> 2;
+        const int s1 = (n1 + P) / (P + 1), s2 = (n2 + P) / (P + 1);
         int c1 = 0, c2 = 0;
 #pragma unroll
-        for (int k = 1; k <= 3; k++)
+        for (int k = 1; k <= P; k++)
         {
             if (k * s1 <= n1 && n1 > 0) c1 += __ldg(m + b1 + k * s1 - 1) < x1;
             if (k * s2 <= n2 && n2 > 0) c2 += __ldg(m + b2 + k * s2 - 1) <= x2;
@@ -1760,12 +1764,13 @@ __device__ __forceinline__ int2 find_limits(const float *__restrict__ m, int n, 
         b1 += c1 * s1;
         b2 += c2 * s2;
         // a probe that fails ends the range before it
-        n1 = c1 == 3 ? n1 - 3 * s1 : min(n1 - c1 * s1, s1 - 1);
-        n2 = c2 == 3 ? n2 - 3 * s2 : min(n2 - c2 * s2, s2 - 1);
+        n1 = c1 == P ? n1 - P * s1 : min(n1 - c1 * s1, s1 - 1);
+        n2 = c2 == P ? n2 - P * s2 : min(n2 - c2 * s2, s2 - 1);
     }
     return make_int2(b1, b2);
 }
 
+template <int P>
 __global__ void k_windows(const LenDev *__restrict__ lens, uint32_t nlen, const float *__restrict__ prec,
                           const double *__restrict__ dMs, double dM0, uint32_t nspec, int2 *__restrict__ win)
 {
@@ -1783,7 +1788,7 @@ __global__ void k_windows(const LenDev *__restrict__ lens, uint32_t nlen, const 
     int2 r = make_int2(1, 0);
     if (n > 0 && !(dM < 0.0))
     {
-        const int2 f = find_limits(m, n, pm1, pm2);
+        const int2 f = find_limits<P>(m, n, pm1, pm2);
         if (f.x < f.y) r = make_int2(f.x, f.y - 1);
     }
     win[g] = r;
@@ -2465,6 +2470,21 @@ static int grow(hc_ctx *ctx, T **p, size_t *cap, size_t need)
     return HC_SUCCESS;
 }
 
+// The windows of a batch: four-way searches in small batches, halving ones in large
+// ones; the two meet between 2,000 and 6,000 spectra of 34 lengths (find_limits).
+static int launch_windows(hc_ctx *ctx, const LenDev *lens, uint32_t nlen, const float *d_prec, const double *d_dM,
+                          uint32_t nspec, int2 *win, cudaStream_t st)
+{
+    const uint64_t nw = (uint64_t)nspec * nlen;
+    const unsigned blocks = (unsigned)((nw + 255) / 256);
+    if (nw <= kWideWindows * (uint64_t)ctx->sm_count)
+        k_windows<3><<<blocks, 256, 0, st>>>(lens, nlen, d_prec, d_dM, ctx->p.dM, nspec, win);
+    else
+        k_windows<1><<<blocks, 256, 0, st>>>(lens, nlen, d_prec, d_dM, ctx->p.dM, nspec, win);
+    HC_CUDA(ctx, cudaGetLastError());
+    return HC_SUCCESS;
+}
+
 // The search of small windows: the spectra of the order from *obase on (null: all, in
 // batch order). `after`: it was preceded by k_search on the same order, which it
 // does not depend on; its CTAs start as k_search's leave SMs free.
@@ -2587,11 +2607,8 @@ int query_device(hc_ctx *ctx, const uint32_t *d_idx, const uint32_t *d_moz, cons
     q.d_nwide = q.d_work + kWkNwide;
     HC_CUDA(ctx, cudaMemsetAsync(q.d_work, 0, 4 * kWorkWords, st));
 
-    const uint64_t nw = (uint64_t)nspec * nlen;
     if (ctx->profiling) HC_CUDA(ctx, record_stage(ctx, 0, st));
-    k_windows<<<(unsigned)((nw + 255) / 256), 256, 0, st>>>(ctx->d_lens, nlen, d_prec, d_dM, ctx->p.dM,
-                                                            nspec, q.d_win);
-    HC_CUDA(ctx, cudaGetLastError());
+    if ((rc = launch_windows(ctx, ctx->d_lens, nlen, d_prec, d_dM, nspec, q.d_win, st))) return rc;
 
     SearchArgs a{};
     a.lens = ctx->d_lens;
@@ -2680,7 +2697,8 @@ int preload_query_kernels(hc_ctx *ctx)
     cudaError_t e = cudaSuccess;
     auto chk = [&](cudaError_t x) { if (e == cudaSuccess) e = x; };
     chk(load_one(k_put_lens));
-    chk(load_one(k_windows));
+    chk(load_one(k_windows<1>));
+    chk(load_one(k_windows<3>));
     chk(load_one(k_cost));
     chk(load_one(k_order));
     chk(load_one(k_tailfit));
@@ -2727,9 +2745,8 @@ int launch_query_scratch(hc_ctx *ctx, const uint32_t *d_idx, const uint32_t *d_m
     if (nspec == 0) return HC_SUCCESS;
     uint32_t *nwide = s.work + kWkNwide;
     HC_CUDA(ctx, cudaMemsetAsync(s.work, 0, 4 * kWorkWords, st));
-    const uint64_t nw = (uint64_t)nspec * nlen;
-    k_windows<<<(unsigned)((nw + 255) / 256), 256, 0, st>>>(s.lens, nlen, d_prec, d_dM, ctx->p.dM, nspec, s.win);
-    HC_CUDA(ctx, cudaGetLastError());
+    int rc = launch_windows(ctx, s.lens, nlen, d_prec, d_dM, nspec, s.win, st);
+    if (rc) return rc;
     SearchArgs a{};
     a.lens = s.lens;
     fill_lens(ctx, a);
@@ -2754,7 +2771,7 @@ int launch_query_scratch(hc_ctx *ctx, const uint32_t *d_idx, const uint32_t *d_m
     a.maxz = ctx->p.maxz;
     a.classes = ctx->d_classes;
     int launches = 4;
-    int rc = launch_packed(ctx, a, nspec, nlen, s.win, s.order, s.work, st, launches, false);
+    rc = launch_packed(ctx, a, nspec, nlen, s.win, s.order, s.work, st, launches, false);
     if (rc) return rc;
     SearchArgs b = a;
     b.persistent = 1;

@@ -9,8 +9,10 @@ from tests._util import compare
 pytestmark = pytest.mark.gpu
 
 
+# 216 spectra are searched four ways, 12 times as many in halves
+@pytest.mark.parametrize("times", [1, 12])
 @pytest.mark.parametrize("npep", [1, 4, 40, 600, 6000])
-def test_window_limits_equal_oracle(npep):
+def test_window_limits_equal_oracle(npep, times):
     from hicops_gb300 import dslim
     from oracle import oracle as O
     p = S.SearchParams(maxz=2, dF=2, dM=500.0, threads=8, vmods_per_pep=2, mods=[("M", 15.99, 2)])
@@ -26,6 +28,7 @@ def test_window_limits_equal_oracle(npep):
     dM = rng.choice([0.0, 0.25, 64.0, 500.0, 1e6], 3 * lim.size)
     prec = (np.concatenate([lim, lim, lim]) + dM * np.repeat([0.0, 1.0, -1.0], lim.size)).astype(np.float32)
     prec[-2:] = 0.0, 1e9
+    prec, dM = np.tile(prec, times), np.tile(dM, times)
     q = S.make_queries(db, prec.size, 5600, p)
     q = S.QueryBatch(idx=q.idx, moz=q.moz, intensity=q.intensity, precurse=prec, charges=q.charges, rtimes=q.rtimes,
                      dM=dM)
