@@ -1744,13 +1744,17 @@ __global__ void __launch_bounds__(kSmThreads, 4) k_search_small(SearchArgs a)
 // the chain of dependent loads while all pairs run at once (two halving searches one
 // after the other, with a walk over the last 20 masses each, took 9 us for 8 spectra
 // against 34 lengths of 600 masses; four ways this takes 4 us), and the loads
-// themselves in larger batches, of which four ways take half as many again. Against 34
-// lengths of up to 60,000 masses, four ways / two: 8 spectra 4.7 / 5.8 us, 2,000 9.1 /
-// 11.3, 6,000 18.9 / 14.3, 60,000 130 / 90.
+// themselves in larger batches, of which four ways take half as many again. +-500 Da
+// against 34 lengths of up to 60,000 masses, four ways / two / as it was: 8 spectra 4.4 /
+// 5.2 / 11.6 us, 2,000 8.2 / 11.0 / 19.7, 8,000 23 / 21 / 21, 100,000 189 / 172 / 148;
+// +-1 ppm, 60,000 spectra: 65 / 66 / 99.
 template <int P>
 __device__ __forceinline__ int2 find_limits(const float *__restrict__ m, int n, float x1, float x2)
 {
-    int b1 = 0, b2 = 0, n1 = n, n2 = n;
+    // many windows end at, or miss, the length's masses
+    const float lo = __ldg(m), hi = __ldg(m + n - 1);
+    if (!(x1 <= hi && x2 >= lo)) return make_int2(0, 0);
+    int b1 = 0, b2 = x2 >= hi ? n : 0, n1 = x1 <= lo ? 0 : n, n2 = x2 >= hi ? 0 : n;
     while (n1 > 0 || n2 > 0)
     {
         const int s1 = (n1 + P) / (P + 1), s2 = (n2 + P) / (P + 1);
