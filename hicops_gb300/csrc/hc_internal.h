@@ -154,7 +154,7 @@ struct ScratchPtrs
 {
     int2 *win;          // nspec * nlen
     uint32_t *wide;     // nspec + 4
-    uint32_t *work;     // 4 + 2 * 64
+    uint32_t *work;     // kWorkWords
     uint32_t *order;    // 2 * nspec
     int32_t *fitstart;  // nspec
     LenDev *lens;       // HC_MAX_LENGTHS
@@ -164,7 +164,12 @@ struct ScratchPtrs
 // overflow list's length, the small-window split point of the longest-first
 // order, then its per-class counts and cursors.
 constexpr uint32_t kWkSearch = 0, kWkWide = 1, kWkNwide = 2, kWkSmall = 3, kWkSplit = 4;
-constexpr uint32_t kWkCnt = 8, kWkCur = kWkCnt + 64, kWorkWords = kWkCur + 64;
+constexpr uint32_t kWkCnt = 8, kWkCur = kWkCnt + 64, kWkArrived = kWkCur + 64;
+// spectra searched in parts (k_search): per spectrum the parts that have ended, then
+// (not zeroed) each part's sums
+constexpr uint32_t kMaxPartItems = 256, kPartWords = 8;
+constexpr uint32_t kWkPart = kWkArrived + kMaxPartItems / 2, kWorkWords = kWkPart + kPartWords * kMaxPartItems;
+static_assert(kWkPart % 4 == 0, "16-byte aligned");
 
 // What a captured query graph was recorded with; a call that differs re-captures.
 struct GraphKey

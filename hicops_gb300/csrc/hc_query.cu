@@ -69,6 +69,14 @@ struct LenS
     const uint8_t *cls;         // entry classes (4 bytes of padding past the last entry)
 };
 
+// what one of the CTAs that share a spectrum found
+struct PartSum
+{
+    unsigned long long best, bytes;
+    uint32_t best_shp, flags, cps, overflow;
+};
+static_assert(sizeof(PartSum) == 4 * kPartWords, "kPartWords");
+
 struct SearchArgs
 {
     const LenDev *lens;
@@ -92,6 +100,10 @@ struct SearchArgs
     const uint32_t *olim;   // optional (device word): the position it stops at (else nspec)
     uint32_t wsplit;        // optional: k_search leaves the spectra whose windows hold fewer candidates
                             // in all, k_search_small those whose windows hold as many or more
+    uint32_t parts;         // k_search: CTAs that share a spectrum at most (0, 1: none; else `hist` starts at zero)
+    uint32_t part_min;      // ... candidates of a part at least
+    uint32_t *arrived;      // ... per spectrum, how many of them have ended
+    struct PartSum *psum;   // ... what each found, `parts` a spectrum
     uint32_t follows;       // k_search_small: 1 when the launch before it writes what it reads
     uint32_t persistent;    // 1: CTAs loop over a work counter; 0: one spectrum per CTA
     uint32_t maxz;
@@ -475,7 +487,85 @@ __device__ __forceinline__ void write_result(const SearchArgs &a, uint32_t s, ui
     a.out[s] = r;
 }
 
-template <bool WIDE, int G>
+// the candidates of a spectrum's windows, by one warp
+__device__ __forceinline__ uint32_t window_sum(const int2 *win, uint32_t nlen, int lane)
+{
+    uint32_t c = 0;
+    for (uint32_t l = lane; l < nlen; l += 32)
+        if (win[l].x <= win[l].y) c += (uint32_t)(win[l].y - win[l].x) + 1u;
+    return __reduce_add_sync(0xFFFFFFFFu, c);
+}
+
+// The windows of part `part` of `parts`, by one warp: the row-table steps (kRowG
+// entries) that the spectrum's windows touch, laid end to end, are dealt out in equal runs.
+__device__ __forceinline__ void part_windows(int2 *win, uint32_t nlen, uint32_t part, uint32_t parts, int lane)
+{
+    uint32_t rows[2], sum = 0;
+    int2 w[2];
+#pragma unroll
+    for (int h = 0; h < 2; h++)
+    {
+        const uint32_t l = 2 * (uint32_t)lane + h;
+        w[h] = l < nlen ? win[l] : make_int2(1, 0);
+        rows[h] = w[h].x <= w[h].y ? (uint32_t)w[h].y / kRowG - (uint32_t)w[h].x / kRowG + 1u : 0u;
+        sum += rows[h];
+    }
+    uint32_t x = sum;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1)
+    {
+        const uint32_t y = __shfl_up_sync(0xFFFFFFFFu, x, o);
+        if (lane >= o) x += y;
+    }
+    const unsigned long long total = __shfl_sync(0xFFFFFFFFu, x, 31);
+    const uint32_t g0 = (uint32_t)(total * part / parts), g1 = (uint32_t)(total * (part + 1) / parts);
+    uint32_t base = x - sum;  // of the rows before this length
+#pragma unroll
+    for (int h = 0; h < 2; h++)
+    {
+        const uint32_t l = 2 * (uint32_t)lane + h;
+        const uint32_t r0 = max(base, g0), r1 = min(base + rows[h], g1);  // its rows of this part
+        int2 p = make_int2(1, 0);
+        if (r0 < r1)
+        {
+            const uint32_t first = (uint32_t)w[h].x / kRowG - base;
+            p.x = max(w[h].x, (int)((first + r0) * kRowG));
+            p.y = min(w[h].y, (int)((first + r1) * kRowG) - 1);
+        }
+        if (l < nlen) win[l] = p;
+        base += rows[h];
+    }
+}
+
+// Leaves what a part found; the last of the spectrum's parts writes its result, or
+// lists it for the wide search. By one thread.
+__device__ __forceinline__ void end_part(const SearchArgs &a, uint32_t s, uint32_t part, uint32_t parts,
+                                         const PartSum &mine)
+{
+    PartSum *p = a.psum + (size_t)s * a.parts;
+    p[part] = mine;
+    __threadfence();
+    if (atomicAdd(&a.arrived[s], 1u) + 1u != parts) return;
+    __threadfence();
+    PartSum t{};
+    for (uint32_t i = 0; i < parts; i++)
+    {
+        const unsigned long long best = __ldcg(&p[i].best);
+        if (best > t.best)
+        {
+            t.best = best;
+            t.best_shp = __ldcg(&p[i].best_shp);
+        }
+        t.bytes += __ldcg(&p[i].bytes);
+        t.flags |= __ldcg(&p[i].flags);
+        t.cps += __ldcg(&p[i].cps);
+        t.overflow |= __ldcg(&p[i].overflow);
+    }
+    if (t.overflow) a.wide_list[atomicAdd(a.nwide, 1u)] = s;
+    else write_result(a, s, t.cps, t.flags, t.bytes, t.best, t.best_shp);
+}
+
+template <bool WIDE, int G, bool PARTS = false>
 __global__ void __launch_bounds__(G >= 4 ? 512 : 1024, G == 4 ? 2 : 1) k_search(SearchArgs a)
 {
     using W = typename Card<WIDE>::word;
@@ -520,10 +610,21 @@ __global__ void __launch_bounds__(G >= 4 ? 512 : 1024, G == 4 ? 2 : 1) k_search(
         if (blockIdx.x >= *a.nonly_dev) return;  // most batches list no spectrum
     }
     for (uint32_t i = tid; i < tile * NW; i += nthr) card[i] = 0;
+    [[maybe_unused]] uint32_t parts = 1;  // that the spectrum is searched in
     if constexpr (!WIDE)
     {
         after_predecessor();
         release_successor();
+        if constexpr (PARTS)
+        {
+            // CTA i takes part i % parts of spectrum i / parts, and nothing else; most of a
+            // batch of small windows leave here
+            const uint32_t s = blockIdx.x / a.parts;
+            if (s >= a.nspec) return;
+            const uint32_t c = window_sum(a.win + (size_t)s * a.nlen, a.nlen, lane);
+            parts = min(a.parts, max(c / a.part_min, 1u));
+            if (c < a.wsplit || blockIdx.x % a.parts >= parts) return;
+        }
     }
     if (tid == 0)
     {
@@ -623,6 +724,10 @@ __global__ void __launch_bounds__(G >= 4 ? 512 : 1024, G == 4 ? 2 : 1) k_search(
             const uint32_t w = a.persistent ? atomicAdd(a.work, 1u) : (iter == 0 ? blockIdx.x : 0xFFFFFFFFu);
             uint32_t sp = 0xFFFFFFFFu;
             if (a.only) sp = w < *a.nonly_dev ? a.only[w] : 0xFFFFFFFFu;
+            else if (PARTS)
+            {
+                if (iter == 0) sp = blockIdx.x / a.parts;
+            }
             else
             {
                 const uint32_t o = (a.obase ? *a.obase : 0u) + w;
@@ -650,14 +755,14 @@ __global__ void __launch_bounds__(G >= 4 ? 512 : 1024, G == 4 ? 2 : 1) k_search(
         for (uint32_t l = tid; l < a.nlen; l += nthr) T.win[l] = a.win[(size_t)s * a.nlen + l];
         for (uint32_t i = tid; i < kMaxClasses + 1; i += nthr) ucls[i] = 0ull;
         __syncthreads();
-        if (!WIDE && a.wsplit)
+        if (!WIDE && !PARTS && a.wsplit && window_sum(T.win, a.nlen, lane) < a.wsplit) continue;  // k_search_small's
+        const bool shared = PARTS && parts > 1;
+        if (shared)
         {
-            uint32_t c = 0;
-            for (uint32_t l = lane; l < a.nlen; l += 32)
-                if (T.win[l].x <= T.win[l].y) c += (uint32_t)(T.win[l].y - T.win[l].x) + 1u;
-            if (__reduce_add_sync(0xFFFFFFFFu, c) < a.wsplit) continue;  // k_search_small's
+            if (wid == 0) part_windows(T.win, a.nlen, blockIdx.x % a.parts, parts, lane);
         }
-        for (int i = kHistSm + tid; i < HC_HIST_BINS; i += nthr) a.hist[(size_t)s * HC_HIST_BINS + i] = 0;
+        else
+            for (int i = kHistSm + tid; i < HC_HIST_BINS; i += nthr) a.hist[(size_t)s * HC_HIST_BINS + i] = 0;
         // valid peaks (dslim_query.cpp:625): dF < qion < max*scale - 1 - dF
         {
             const uint32_t lowlim = a.classes ? __ldg(&a.classes->maxkey) + a.dF : 0u;
@@ -744,7 +849,9 @@ __global__ void __launch_bounds__(G >= 4 ? 512 : 1024, G == 4 ? 2 : 1) k_search(
         my_shp = 0;
         if (tid == 0)
             for (uint32_t l = 0; l < a.nlen; l++)
-                if (T.win[l].x <= T.win[l].y) atomicAdd(&T.bytes, 4ull * (2 * a.dF + 2) * nv);  // the reference's bA reads
+                // the reference's bA reads (of a window in parts, with its first)
+                if (T.win[l].x <= T.win[l].y && (!shared || T.win[l].x == a.win[(size_t)s * a.nlen + l].x))
+                    atomicAdd(&T.bytes, 4ull * (2 * a.dF + 2) * nv);
 
         // The spectrum's work is a sequence of jobs (length l, scorecard tile
         // t). Interior tile boundaries are row-table entries; a window's own
@@ -1240,6 +1347,21 @@ __global__ void __launch_bounds__(G >= 4 ? 512 : 1024, G == 4 ? 2 : 1) k_search(
         __syncthreads();
         HC_PHASE(5);
         // ---- write the spectrum's results ----
+        if (shared)
+        {
+            for (int i = tid; i < kHistSm; i += nthr)
+                if (T.u.run.hist[i]) atomicAdd(&a.hist[(size_t)s * HC_HIST_BINS + i], T.u.run.hist[i]);
+            if (wid == 0)
+            {
+                uint32_t cps = 0;
+#pragma unroll
+                for (int i = 0; i < kHistSm; i += 32) cps += T.u.run.hist[i + lane];
+                cps = __reduce_add_sync(0xFFFFFFFFu, cps) + T.cpsms;
+                if (lane == 0)
+                    end_part(a, s, blockIdx.x % a.parts, parts, PartSum{T.best, T.bytes, T.best_shp, T.flags, cps, T.overflow});
+            }
+            continue;
+        }
         if (!WIDE && T.overflow)
         {
             if (tid == 0)
@@ -1289,6 +1411,7 @@ constexpr uint32_t kSmWQ = 128;      // candidates waiting per warp (a power of 
 constexpr uint32_t kSmCtas = 4;
 // launch shapes picked for a context that chose none (see launch_packed)
 constexpr uint32_t kWideWindows = 512;  // (spectrum, length) pairs per SM up to which windows are searched four ways
+constexpr uint32_t kMaxParts = 32, kPartMin = 32768, kPartMinFew = 4096;  // see auto_parts
 constexpr uint32_t kAutoSmallLog2 = 15, kAutoAllSmall = 1u << 16, kAutoOrder = 1024;
 
 struct SmSeg
@@ -1776,10 +1899,13 @@ __device__ __forceinline__ int2 find_limits(const float *__restrict__ m, int n, 
 
 template <int P>
 __global__ void k_windows(const LenDev *__restrict__ lens, uint32_t nlen, const float *__restrict__ prec,
-                          const double *__restrict__ dMs, double dM0, uint32_t nspec, int2 *__restrict__ win)
+                          const double *__restrict__ dMs, double dM0, uint32_t nspec, int2 *__restrict__ win,
+                          uint32_t *__restrict__ zero)
 {
     release_successor();
     const uint64_t g = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x;
+    if (zero)  // the histograms that several CTAs will add to
+        for (uint64_t i = g; i < (uint64_t)nspec * HC_HIST_BINS; i += (uint64_t)gridDim.x * blockDim.x) zero[i] = 0u;
     if (g >= (uint64_t)nspec * nlen) return;
     const uint32_t s = (uint32_t)(g / nlen), l = (uint32_t)(g % nlen);
     const double dM = dMs ? dMs[s] : dM0;
@@ -2389,12 +2515,12 @@ int prepare_query(hc_ctx *ctx, uint32_t nspec)
 
 namespace {
 
-template <bool WIDE, int G>
+template <bool WIDE, int G, bool PARTS = false>
 int launch_g(hc_ctx *ctx, const SearchArgs &a, int grid, uint32_t threads, size_t smem, cudaStream_t st)
 {
     if (G >= 4 && threads > 512) threads = 512;
-    HC_CUDA(ctx, cudaFuncSetAttribute(k_search<WIDE, G>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-    HC_CUDA(ctx, launch_after(k_search<WIDE, G>, (unsigned)grid, threads, smem, st, a));
+    HC_CUDA(ctx, cudaFuncSetAttribute(k_search<WIDE, G, PARTS>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+    HC_CUDA(ctx, launch_after(k_search<WIDE, G, PARTS>, (unsigned)grid, threads, smem, st, a));
     return HC_SUCCESS;
 }
 
@@ -2477,14 +2603,14 @@ static int grow(hc_ctx *ctx, T **p, size_t *cap, size_t need)
 // The windows of a batch: four-way searches in small batches, halving ones in large
 // ones; the two meet between 2,000 and 6,000 spectra of 34 lengths (find_limits).
 static int launch_windows(hc_ctx *ctx, const LenDev *lens, uint32_t nlen, const float *d_prec, const double *d_dM,
-                          uint32_t nspec, int2 *win, cudaStream_t st)
+                          uint32_t nspec, int2 *win, uint32_t *zero, cudaStream_t st)
 {
     const uint64_t nw = (uint64_t)nspec * nlen;
     const unsigned blocks = (unsigned)((nw + 255) / 256);
     if (nw <= kWideWindows * (uint64_t)ctx->sm_count)
-        k_windows<3><<<blocks, 256, 0, st>>>(lens, nlen, d_prec, d_dM, ctx->p.dM, nspec, win);
+        k_windows<3><<<blocks, 256, 0, st>>>(lens, nlen, d_prec, d_dM, ctx->p.dM, nspec, win, zero);
     else
-        k_windows<1><<<blocks, 256, 0, st>>>(lens, nlen, d_prec, d_dM, ctx->p.dM, nspec, win);
+        k_windows<1><<<blocks, 256, 0, st>>>(lens, nlen, d_prec, d_dM, ctx->p.dM, nspec, win, zero);
     HC_CUDA(ctx, cudaGetLastError());
     return HC_SUCCESS;
 }
@@ -2504,6 +2630,29 @@ static int launch_small(hc_ctx *ctx, SearchArgs s, uint32_t nspec, const uint32_
     HC_CUDA(ctx, launch_after(k_search_small, std::min<uint32_t>(nspec, (uint32_t)ctx->sm_count * kSmCtas), kSmThreads,
                               smem, st, s));
     return HC_SUCCESS;
+}
+
+static uint64_t index_entries(const hc_ctx *ctx)
+{
+    uint64_t n = 0;
+    for (const LenHost &lh : ctx->lens) n += lh.built ? lh.n : 0u;
+    return n;
+}
+
+// The CTAs that share a spectrum in k_search, at most. With at most half as many spectra as
+// SMs, in a context whose launch shape nobody chose, the windows are cut so that every SM
+// (one 1024-thread CTA each) has a part, up to kMaxParts: one CTA a spectrum left the
+// others idle. A part costs its CTA some 8 us of set-up, so it holds kPartMin candidates at
+// least, kPartMinFew while one spectrum in eight SMs is all there is. Whole / in parts:
+// +-500 Da against 2 M peptides, 1 spectrum 539 / 71 us, 8 586 / 94, 32 755 / 257, 76 780 /
+// 435; against 500,000, 8 spectra 186 / 66, 76 286 / 175. (Four parts an SM for two 512-thread
+// CTAs: 76 spectra 321 and 165, but 40 spectra of 44 k candidates 137 us against 117 whole,
+// 152 of 54 k 175 against 138.)
+static uint32_t auto_parts(const hc_ctx *ctx, uint32_t nspec)
+{
+    const uint32_t items = std::min((uint32_t)ctx->sm_count, kMaxPartItems);
+    if (!ctx->auto_shape || 2 * (uint64_t)nspec > items || index_entries(ctx) < kAutoAllSmall) return 1;
+    return std::min(items / nspec, kMaxParts);
 }
 
 // The packed search of a batch: with schedule 2 the longest-first order first,
@@ -2530,9 +2679,7 @@ static int launch_packed(hc_ctx *ctx, SearchArgs &a, uint32_t nspec, uint32_t nl
     a.wsplit = 0;
     if (ctx->auto_shape)
     {
-        uint64_t entries = 0;
-        for (const LenHost &lh : ctx->lens) entries += lh.built ? lh.n : 0u;
-        all_small = entries < kAutoAllSmall;
+        all_small = index_entries(ctx) < kAutoAllSmall;
         const uint32_t tile = max_tile_for(ctx, a.dF, 2, 512);
         if (nspec > (uint32_t)ctx->sm_count && tile >= kRowG)
         {
@@ -2552,6 +2699,9 @@ static int launch_packed(hc_ctx *ctx, SearchArgs &a, uint32_t nspec, uint32_t nl
     a.tile = t.tile;
     a.persistent = t.schedule != 1;
     a.obase = a.olim = nullptr;
+    a.arrived = work + kWkArrived;
+    a.part_min = nspec <= (uint32_t)ctx->sm_count / 8 ? kPartMinFew : kPartMin;
+    a.psum = reinterpret_cast<PartSum *>(work + kWkPart);
     const bool split = t.schedule == 2 && t.small_log2 != 0;
     if (t.schedule == 2 && !all_small)
     {
@@ -2573,7 +2723,8 @@ static int launch_packed(hc_ctx *ctx, SearchArgs &a, uint32_t nspec, uint32_t nl
     }
     const size_t smem = search_smem(t.tile, a.dF, false, t.threads);
     const int grid = t.schedule == 1 ? (int)nspec : ctx->sm_count * (int)t.ctas_per_sm;
-    const int rc = launch_search<false>(ctx, a, grid, t.threads, smem, t.pairs_per_warp, st);
+    const int rc = a.parts > 1 ? launch_g<false, 2, true>(ctx, a, grid, t.threads, smem, st)
+                               : launch_search<false>(ctx, a, grid, t.threads, smem, t.pairs_per_warp, st);
     if (rc || !(split || a.wsplit)) return rc;
     launches++;
     return launch_small(ctx, a, nspec, split ? work + kWkSplit : nullptr, work, true, st);
@@ -2609,10 +2760,12 @@ int query_device(hc_ctx *ctx, const uint32_t *d_idx, const uint32_t *d_moz, cons
     if ((rc = grow(ctx, &q.d_fitstart, &q.fit_cap, (size_t)nspec))) return rc;
     if (!q.d_work) HC_CUDA(ctx, cudaMalloc((void **)&q.d_work, 4 * kWorkWords));
     q.d_nwide = q.d_work + kWkNwide;
-    HC_CUDA(ctx, cudaMemsetAsync(q.d_work, 0, 4 * kWorkWords, st));
+    HC_CUDA(ctx, cudaMemsetAsync(q.d_work, 0, 4 * kWkPart, st));
+    const uint32_t parts = auto_parts(ctx, nspec);
 
     if (ctx->profiling) HC_CUDA(ctx, record_stage(ctx, 0, st));
-    if ((rc = launch_windows(ctx, ctx->d_lens, nlen, d_prec, d_dM, nspec, q.d_win, st))) return rc;
+    rc = launch_windows(ctx, ctx->d_lens, nlen, d_prec, d_dM, nspec, q.d_win, parts > 1 ? d_hist : nullptr, st);
+    if (rc) return rc;
 
     SearchArgs a{};
     a.lens = ctx->d_lens;
@@ -2634,6 +2787,7 @@ int query_device(hc_ctx *ctx, const uint32_t *d_idx, const uint32_t *d_moz, cons
     a.wide_list = q.d_wide;
     a.nwide = q.d_nwide;
     a.work = q.d_work;
+    a.parts = parts;
     a.defer_cap = ctx->tuning.defer_cap;
     a.maxz = ctx->p.maxz;
     a.classes = ctx->d_classes;
@@ -2652,6 +2806,7 @@ int query_device(hc_ctx *ctx, const uint32_t *d_idx, const uint32_t *d_moz, cons
     b.nonly_dev = q.d_nwide;
     b.work = q.d_work + kWkWide;
     b.obase = b.olim = nullptr;
+    b.parts = 0;
     b.tile = std::max(kRowG, ctx->tuning.tile / 2 / kRowG * kRowG);  // same shared memory, 16-byte words
     const size_t smem2 = search_smem(b.tile, b.dF, true, ctx->tuning.threads);
     rc2 = launch_search<true>(ctx, b, ctx->sm_count, ctx->tuning.threads, smem2, 2, st);
@@ -2708,6 +2863,7 @@ int preload_query_kernels(hc_ctx *ctx)
     chk(load_one(k_tailfit));
     chk(load_one(k_search<false, 1>));
     chk(load_one(k_search<false, 2>));
+    chk(load_one(k_search<false, 2, true>));
     chk(load_one(k_search<false, 4>));
     chk(load_one(k_search<false, 8>));
     chk(load_one(k_search<true, 2>));
@@ -2748,8 +2904,9 @@ int launch_query_scratch(hc_ctx *ctx, const uint32_t *d_idx, const uint32_t *d_m
     ctx->last_launches = 0;
     if (nspec == 0) return HC_SUCCESS;
     uint32_t *nwide = s.work + kWkNwide;
-    HC_CUDA(ctx, cudaMemsetAsync(s.work, 0, 4 * kWorkWords, st));
-    int rc = launch_windows(ctx, s.lens, nlen, d_prec, d_dM, nspec, s.win, st);
+    HC_CUDA(ctx, cudaMemsetAsync(s.work, 0, 4 * kWkPart, st));
+    const uint32_t parts = auto_parts(ctx, nspec);
+    int rc = launch_windows(ctx, s.lens, nlen, d_prec, d_dM, nspec, s.win, parts > 1 ? d_hist : nullptr, st);
     if (rc) return rc;
     SearchArgs a{};
     a.lens = s.lens;
@@ -2771,6 +2928,7 @@ int launch_query_scratch(hc_ctx *ctx, const uint32_t *d_idx, const uint32_t *d_m
     a.wide_list = s.wide;
     a.nwide = nwide;
     a.work = s.work;
+    a.parts = parts;
     a.defer_cap = ctx->tuning.defer_cap;
     a.maxz = ctx->p.maxz;
     a.classes = ctx->d_classes;
@@ -2784,6 +2942,7 @@ int launch_query_scratch(hc_ctx *ctx, const uint32_t *d_idx, const uint32_t *d_m
     b.nonly_dev = nwide;
     b.work = s.work + kWkWide;
     b.obase = b.olim = nullptr;
+    b.parts = 0;
     b.tile = std::max(kRowG, ctx->tuning.tile / 2 / kRowG * kRowG);  // same shared memory, 16-byte words
     rc = launch_search<true>(ctx, b, ctx->sm_count, ctx->tuning.threads, search_smem(b.tile, b.dF, true, ctx->tuning.threads), 2, st);
     if (rc) return rc;
