@@ -358,6 +358,10 @@ int hc_dslim_load(hc_ctx *ctx, uint32_t L, const uint8_t *seqs, uint32_t npep, c
     uint32_t *d_ids = nullptr;
     HC_CUDA(ctx, dalloc(ctx, &d_ids, M + 1));
     cudaError_t e = cudaMemcpyAsync(d_ids, iA, 4 * M, cudaMemcpyHostToDevice, st);
+    // offsets that do not start at 0: what lies in front of them is in no bucket, and the
+    // build, which places every posting, passes over padding
+    static_assert(kQpostPad == 0xFFFFFFFFu, "written byte by byte");
+    if (e == cudaSuccess && bA[0]) e = cudaMemsetAsync(d_ids, 0xFF, 4ull * bA[0], st);
     if (e == cudaSuccess) e = cudaStreamSynchronize(st);  // the host vectors above go with this call
     lh->npost = M;
     const int rq = e == cudaSuccess ? build_query_postings(ctx, *lh, M ? d_ids : nullptr, nullptr)

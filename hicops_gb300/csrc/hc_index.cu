@@ -745,7 +745,8 @@ __device__ __forceinline__ int y1_charge(uint32_t ion, uint32_t Lm1, uint32_t ha
 // y1 ions hold a large share each, walked by one thread), 0.6 ms so.
 // Every y1 posting of a classed entry must lie in its class's key bucket;
 // bad[e] = 1 marks the entries where one does not (they lose their class).
-// A padding id (kQpostPad) is skipped. qp null: the check only.
+// A padding id (kQpostPad) is skipped: every posting in front of the first bucket is
+// one. qp null: the check only.
 __global__ void k_qpost(const uint32_t *__restrict__ ids, const uint32_t *__restrict__ keys, uint32_t total,
                         const uint32_t *__restrict__ bA, const uint32_t *__restrict__ qA, IdDiv div, uint32_t half,
                         uint32_t Lm1, const uint8_t *__restrict__ cls, const ClassKeys *__restrict__ ck,
@@ -790,7 +791,8 @@ __global__ void k_qpost_pads(const uint32_t *__restrict__ bA, const uint32_t *__
     }
 }
 
-// The last bucket that starts at or before i: start[b] <= i < start[b + 1].
+// The last bucket that starts at or before i: start[b] <= i < start[b + 1]; 0 where i lies in
+// front of every bucket.
 __device__ __forceinline__ uint32_t bucket_of(const uint32_t *__restrict__ start, uint32_t nb, uint32_t i)
 {
     uint32_t lo = 0, hi = nb - 1;
@@ -843,7 +845,8 @@ __global__ void k_check_qpost(const uint32_t *__restrict__ qp, const uint16_t *_
     if (b) atomicAdd(bad, b);
 }
 
-// query postings -> ids (the reference's iA), one thread per posting
+// query postings -> ids (the reference's iA), one thread per posting; 0 in front of the first
+// bucket (such postings are not kept)
 __global__ void k_qpost_ids(const uint32_t *__restrict__ bA, const uint32_t *__restrict__ qA,
                             const uint32_t *__restrict__ qp, const uint16_t *__restrict__ qion, uint32_t nb,
                             uint32_t npost, uint32_t speclen, uint32_t *__restrict__ ids)
@@ -853,8 +856,9 @@ __global__ void k_qpost_ids(const uint32_t *__restrict__ bA, const uint32_t *__r
     const uint32_t qtotal = qA[nb];
     for (uint64_t j = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; j < npost; j += (uint64_t)gridDim.x * blockDim.x)
     {
-        const uint32_t b = bucket_of(bA, nb, (uint32_t)j), q = qA[b] + ((uint32_t)j - bA[b]);
-        if (q < qtotal) ids[j] = (qp[q] >> kQpEntryShift) * speclen + qion[q];
+        const uint32_t b = bucket_of(bA, nb, (uint32_t)j), s = bA[b], q = qA[b] + ((uint32_t)j - s);
+        if ((uint32_t)j < s) ids[j] = 0;
+        else if (q < qtotal) ids[j] = (qp[q] >> kQpEntryShift) * speclen + qion[q];
     }
 }
 
