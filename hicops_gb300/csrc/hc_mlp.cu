@@ -157,7 +157,10 @@ __global__ void __launch_bounds__(256) k_features(const uint32_t *__restrict__ h
 // starts under the end of the one before (16 minibatches of 512: 492 -> 414 us a call).
 constexpr int kGradThreads = 512;
 constexpr int kW2Pitch = kH2 + 4;  // rows 16 bytes apart modulo the banks: a warp reads 32 rows' float4 without conflicts
-constexpr size_t kPartStride = (kParams + 1 + 3) / 4 * 4;  // a CTA's share: gradients, then its loss
+// A CTA's share: gradients, then its loss, in 128-byte lines of its own. A CTA of several
+// tiles adds to its share in place under a successor that has started (see after_predecessor).
+constexpr size_t kPartStride = (kParams + 1 + 31) / 32 * 32;
+static_assert(kPartStride * sizeof(float) % 128 == 0, "no line of two CTAs");
 
 template <int R>
 struct GradSmem
