@@ -320,6 +320,10 @@ __global__ void __launch_bounds__(kScanThreads) k_scan_add(uint32_t *__restrict_
     store4(a, at, n, al, make_uint4(x.x + off, x.y + off, x.z + off, x.w + off));
 }
 
+// Words of one level's sums, to whole 128-byte lines: the next level's lie behind them, and
+// a level is scanned in place under a successor that has started (see after_predecessor).
+constexpr size_t scan_level_words(size_t n) { return (n + 31) / 32 * 32; }
+
 cudaError_t scan_exclusive(uint32_t *a, size_t n, uint32_t *tmp, cudaStream_t st)
 {
     if (n == 0) return cudaSuccess;
@@ -333,7 +337,7 @@ cudaError_t scan_exclusive(uint32_t *a, size_t n, uint32_t *tmp, cudaStream_t st
     const bool raw = nb <= (size_t)kScanTile;
     if (!raw)
     {
-        const cudaError_t e = scan_exclusive(tmp, nb, tmp + nb, st);
+        const cudaError_t e = scan_exclusive(tmp, nb, tmp + scan_level_words(nb), st);
         if (e != cudaSuccess) return e;
     }
     launch_after(k_scan_add, (unsigned)nb, kScanThreads, 0, st, a, n, tmp, raw ? 1 : 0);
@@ -346,7 +350,7 @@ size_t scan_tmp_words(size_t n)
     while (n > (size_t)kScanTile)
     {
         n = (n + kScanTile - 1) / kScanTile;
-        t += n;
+        t += scan_level_words(n);
     }
     return t + 16;
 }
