@@ -30,9 +30,12 @@ cudaError_t pool_alloc(hc_ctx *ctx, void **p, size_t bytes)
 }
 
 // Frees a length's arrays. A search of them may still run on any stream (the
-// frees are ordered on the context's), so a length in use is waited for.
+// frees are ordered on the context's), so a length in use is waited for. The device's
+// length records name them until they are written again, whatever becomes of the call
+// that takes the length's place.
 void free_len(hc_ctx *ctx, LenHost &lh)
 {
+    ctx->lens_dirty = true;
     if (lh.built) cudaDeviceSynchronize();
     dfree(ctx, lh.d_mass);
     dfree(ctx, lh.d_seqid);
