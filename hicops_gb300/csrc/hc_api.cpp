@@ -36,6 +36,7 @@ cudaError_t pool_alloc(hc_ctx *ctx, void **p, size_t bytes)
 void free_len(hc_ctx *ctx, LenHost &lh)
 {
     ctx->lens_dirty = true;
+    ctx->epoch++;
     if (lh.built) cudaDeviceSynchronize();
     dfree(ctx, lh.d_mass);
     dfree(ctx, lh.d_seqid);
@@ -373,6 +374,7 @@ int hc_dslim_load(hc_ctx *ctx, uint32_t L, const uint8_t *seqs, uint32_t npep, c
     if (rq) return rq;
     lh->built = true;
     ctx->lens_dirty = true;
+    ctx->epoch++;
     return HC_SUCCESS;
 }
 

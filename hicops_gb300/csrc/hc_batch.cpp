@@ -52,6 +52,7 @@ static GraphKey make_key(const hc_ctx *ctx, const uint32_t *d_idx, const uint32_
                          hc_result *d_out, uint32_t *d_hist)
 {
     GraphKey key{};
+    key.epoch = ctx->epoch;
     key.idx = d_idx;
     key.moz = d_moz;
     key.inten = d_intensity;
@@ -82,10 +83,10 @@ int hc_dslim_query_graph(hc_ctx *ctx, const uint32_t *d_idx, const uint32_t *d_m
         return set_error(ctx, HC_ERR_INVLD_PTR, "null device buffer");
     cudaSetDevice(ctx->device);
     cudaStream_t st = stream ? (cudaStream_t)stream : ctx->stream;
-    const GraphKey key = make_key(ctx, d_idx, d_moz, d_intensity, d_precurse, d_dM, nspec, npeaks, d_out, d_hist);
     // everything that allocates or copies synchronously happens before capture
     int rc = prepare_query(ctx, nspec);
     if (rc) return rc;
+    const GraphKey key = make_key(ctx, d_idx, d_moz, d_intensity, d_precurse, d_dM, nspec, npeaks, d_out, d_hist);
     rc = replay(ctx, key, st, [&](cudaStream_t cs) {
         return query_device(ctx, d_idx, d_moz, d_intensity, d_precurse, d_dM, nspec, npeaks, d_out, d_hist, cs);
     });
@@ -103,13 +104,13 @@ int hc_dslim_query_learned(hc_ctx *ctx, hc_mlp *mlp, const uint32_t *d_idx, cons
         return set_error(ctx, HC_ERR_INVLD_PTR, "null device buffer");
     cudaSetDevice(ctx->device);
     cudaStream_t st = stream ? (cudaStream_t)stream : ctx->stream;
-    GraphKey key = make_key(ctx, d_idx, d_moz, d_intensity, d_precurse, d_dM, nspec, npeaks, d_out, d_hist);
-    key.mlp = mlp;
-    key.learned = d_learned_log10e;
-    learned_gate(mlp, &key.gate_resid, &key.gate_radius);
     int rc = prepare_query(ctx, nspec);
     if (rc) return rc;
     if ((rc = learned_prepare(mlp, nspec))) return rc;
+    GraphKey key = make_key(ctx, d_idx, d_moz, d_intensity, d_precurse, d_dM, nspec, npeaks, d_out, d_hist);
+    key.mlp = mlp;
+    key.learned = d_learned_log10e;
+    learned_key(mlp, &key);
     rc = replay(ctx, key, st, [&](cudaStream_t cs) {
         int r = query_device(ctx, d_idx, d_moz, d_intensity, d_precurse, d_dM, nspec, npeaks, d_out, d_hist, cs,
                              false);
@@ -242,6 +243,7 @@ int hc_ctx_set_phase_timing(hc_ctx *ctx, int on)
 {
     if (!ctx) return HC_ERR_INVLD_PTR;
     cudaSetDevice(ctx->device);
+    if ((on != 0) != (ctx->d_phase != nullptr)) ctx->epoch++;
     if (on && !ctx->d_phase)
     {
         HC_CUDA(ctx, cudaMalloc((void **)&ctx->d_phase, 8 * 16));

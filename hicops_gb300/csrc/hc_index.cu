@@ -1206,6 +1206,7 @@ int build_length_device(hc_ctx *ctx, LenHost &lh, const hc_entry *h_entries, boo
     }
     lh.built = true;
     ctx->lens_dirty = true;
+    ctx->epoch++;
     ctx->last_launches = launches + 1;
     return HC_SUCCESS;
 }

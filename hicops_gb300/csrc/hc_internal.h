@@ -174,10 +174,13 @@ static_assert(kWkPart % 4 == 0, "16-byte aligned");
 // What a captured query graph was recorded with; a call that differs re-captures.
 struct GraphKey
 {
+    uint64_t epoch;             // of the index and of the scratch that the graph's kernels name
     const void *idx, *moz, *inten, *prec, *dM, *out, *hist;
     const void *mlp, *learned;  // the learned form: network, learned log10 e-values (else null)
     float gate_resid;           // ... and its gate (kernel parameters of the captured graph)
     uint32_t gate_radius;
+    uint64_t net_serial;        // ... and the network's buffers, and its context's scratch
+    uint64_t net_epoch;
     uint32_t nspec, npeaks;
     hc_tuning tuning;
     uint32_t auto_shape;
@@ -227,6 +230,10 @@ struct hc_ctx
     std::string last_error;
     int last_launches = 0;
     bool lens_dirty = true;
+    // Counts what a captured graph does not outlive: a length's arrays freed or built
+    // (a graph holds their addresses, sizes and the launches picked for them), and
+    // every buffer of the pipeline allocated again.
+    uint64_t epoch = 0;
     bool profiling = false;
     bool last_learned = false;  // the last query ran the learned tail (stage 5 recorded)
     cudaEvent_t ev[6] = {};  // windows | search | wide | tailfit | learned tail boundaries
@@ -303,7 +310,7 @@ int launch_query_scratch(hc_ctx *ctx, const uint32_t *d_idx, const uint32_t *d_m
 
 // hc_mlp.cu: the learned tail after a search without tail fit
 int learned_prepare(hc_mlp *m, uint32_t n);
-void learned_gate(const hc_mlp *m, float *max_resid, uint32_t *radius);
+void learned_key(const hc_mlp *m, GraphKey *key);
 int learned_pipeline(hc_mlp *m, const uint32_t *d_hist, hc_result *d_res, uint32_t n, float *lg, cudaStream_t st,
                      int *launches);
 

@@ -26,6 +26,7 @@
 // within FP32 rounding of a point, the spectrum is listed and the FP64
 // expeRT fit (k_tailfit) runs on that list only.
 #include <algorithm>
+#include <atomic>
 #include <cmath>
 #include <cstring>
 #include <vector>
@@ -60,6 +61,7 @@ struct hc_mlp
     float *d_m = nullptr, *d_v = nullptr;
     float *d_loss = nullptr;
     int step = 0;
+    uint64_t serial = 0;        // changes with any buffer that the learned pipeline's kernels name
     // gate of the learned tail: largest predicted RMS residual (log10 units),
     // and how far from the predicted first bin the confirmation looks
     float gate_resid = 0.1f;
@@ -1174,9 +1176,17 @@ static int mlp_step(hc_mlp *m, const float *X, const float *Y, uint32_t n, const
     return HC_SUCCESS;
 }
 
+// of a network's device buffers: a new network may lie where one lay before
+static uint64_t next_serial()
+{
+    static std::atomic<uint64_t> n{0};
+    return ++n;
+}
+
 static int grow_pipe(hc_mlp *m, uint32_t n)
 {
     if (m->pipe_cap >= n) return HC_SUCCESS;
+    m->serial = next_serial();
     cudaFree(m->d_X);
     cudaFree(m->d_net);
     cudaFree(m->d_fb);
@@ -1203,10 +1213,13 @@ static int tail_kernel(hc_ctx *ctx, const TailGate &g, const uint32_t *d_hist, c
 
 static TailGate gate_of(const hc_mlp *m) { return TailGate{m->gate_resid, (int)m->radius}; }
 
-void learned_gate(const hc_mlp *m, float *max_resid, uint32_t *radius)
+// what a graph with this network in it was captured with
+void learned_key(const hc_mlp *m, GraphKey *key)
 {
-    *max_resid = m->gate_resid;
-    *radius = m->radius;
+    key->gate_resid = m->gate_resid;
+    key->gate_radius = m->radius;
+    key->net_serial = m->serial;
+    key->net_epoch = m->ctx->epoch;
 }
 
 // Allocates what the learned pipeline of n spectra needs (before any capture).
@@ -1217,6 +1230,7 @@ int learned_prepare(hc_mlp *m, uint32_t n)
     QueryScratch &q = m->ctx->qs;
     if (q.fit_cap < n)
     {
+        m->ctx->epoch++;
         cudaFree(q.d_fitstart);
         q.d_fitstart = nullptr;
         q.fit_cap = 0;
@@ -1261,6 +1275,7 @@ int hc_mlp_create(hc_ctx *ctx, uint64_t seed, hc_mlp **out)
     cudaSetDevice(ctx->device);
     hc_mlp *m = new hc_mlp();
     m->ctx = ctx;
+    m->serial = next_serial();
     std::vector<float> h(kParams, 0.0f);
     // He-uniform initialisation from a splitmix64 stream
     uint64_t x = seed ? seed : 0x9E3779B97F4A7C15ull;

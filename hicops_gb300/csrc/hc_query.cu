@@ -2592,6 +2592,7 @@ template <class T>
 static int grow(hc_ctx *ctx, T **p, size_t *cap, size_t need)
 {
     if (*cap >= need) return HC_SUCCESS;
+    ctx->epoch++;
     if (*p) cudaFree(*p);
     *p = nullptr;
     *cap = 0;

@@ -197,6 +197,7 @@ extern "C" int hc_dslim_restore(hc_ctx *ctx, const char *path)
         }
         lh.built = true;
         ctx->lens_dirty = true;
+        ctx->epoch++;
     }
     return HC_SUCCESS;
 }

@@ -185,7 +185,7 @@ int hc_dslim_query_device(hc_ctx *ctx, const uint32_t *d_idx, const uint32_t *d_
                           hc_result *d_out, uint32_t *d_hist, void *stream);
 /* Batched form: the same pipeline captured once into a CUDA graph and
  * replayed; a call whose buffers, sizes or tuning differ from the captured
- * one re-captures. Results are identical to hc_dslim_query_device. */
+ * one, or that finds another index or larger scratch, re-captures. Results are identical to hc_dslim_query_device. */
 int hc_dslim_query_graph(hc_ctx *ctx, const uint32_t *d_idx, const uint32_t *d_moz,
                          const uint32_t *d_intensity, const float *d_precurse,
                          const double *d_dM, uint32_t nspec, uint32_t npeaks,
