@@ -789,27 +789,9 @@ const char *next_s_line(const char *base, const char *p, const char *e)
 
 using namespace hc;
 
-extern "C" int hc_ms2_read(const char *path, uint32_t scale_u, hc_ms2 **out, uint32_t *nspec, uint32_t *maxslen)
+// The text [base, end) parsed by all host threads.
+static int parse_host(const char *base, const char *end, double scale, hc_ms2 **out)
 {
-    if (!path || !out) return HC_ERR_INVLD_PTR;
-    *out = nullptr;
-    FILE *f = std::fopen(path, "rb");
-    if (!f) return HC_ERR_FILE_ERROR;
-    std::vector<char> buf;
-    bool rerr = std::fseek(f, 0, SEEK_END) != 0;
-    const long fsz = rerr ? -1 : std::ftell(f);
-    rerr = rerr || fsz < 0 || std::fseek(f, 0, SEEK_SET) != 0;
-    if (!rerr)
-    {
-        buf.resize((size_t)fsz + 1);
-        rerr = std::fread(buf.data(), 1, (size_t)fsz, f) != (size_t)fsz;
-        buf[(size_t)fsz] = 0;
-    }
-    std::fclose(f);
-    if (rerr) return HC_ERR_FILE_ERROR;
-    const char *base = buf.data(), *end = base + (buf.size() - 1);
-    const double scale = (double)scale_u;
-
     // stretches: the first runs from the file start through its first 'S'
     // line; the others start at 'S' lines, about equal in size
     const char *s0 = next_s_line(base, base, end);
@@ -871,9 +853,36 @@ extern "C" int hc_ms2_read(const char *path, uint32_t scale_u, hc_ms2 **out, uin
         return HC_ERR_INVLD_SIZE;
     }
     *out = m;
-    if (nspec) *nspec = (uint32_t)m->prec.size();
-    if (maxslen) *maxslen = m->maxslen;
     return HC_SUCCESS;
+}
+
+// `rc` with what the caller of an open or a read asked for
+static int opened(int rc, hc_ms2 *const *out, uint32_t *nspec, uint32_t *maxslen)
+{
+    if (rc != HC_SUCCESS) return rc;
+    if (nspec) *nspec = (uint32_t)(*out)->prec.size();
+    if (maxslen) *maxslen = (*out)->maxslen;
+    return rc;
+}
+
+extern "C" int hc_ms2_read(const char *path, uint32_t scale_u, hc_ms2 **out, uint32_t *nspec, uint32_t *maxslen)
+{
+    if (!path || !out) return HC_ERR_INVLD_PTR;
+    *out = nullptr;
+    FILE *f = std::fopen(path, "rb");
+    if (!f) return HC_ERR_FILE_ERROR;
+    std::vector<char> buf;
+    bool rerr = std::fseek(f, 0, SEEK_END) != 0;
+    const long fsz = rerr ? -1 : std::ftell(f);
+    rerr = rerr || fsz < 0 || std::fseek(f, 0, SEEK_SET) != 0;
+    if (!rerr)
+    {
+        buf.resize((size_t)fsz);
+        rerr = std::fread(buf.data(), 1, (size_t)fsz, f) != (size_t)fsz;
+    }
+    std::fclose(f);
+    if (rerr) return HC_ERR_FILE_ERROR;
+    return opened(parse_host(buf.data(), buf.data() + buf.size(), (double)scale_u, out), out, nspec, maxslen);
 }
 
 namespace hc {
@@ -884,7 +893,7 @@ namespace {
 // at 28 MB.
 constexpr uint64_t kDeviceText = 1u << 14;
 
-// The whole file, by up to eight threads; false when it cannot be read.
+// The whole file, by up to eight threads; false when it is small or cannot be read.
 bool read_file(const char *path, std::unique_ptr<char[]> &buf, uint64_t &size)
 {
     const int fd = ::open(path, O_RDONLY);
@@ -922,14 +931,11 @@ bool read_file(const char *path, std::unique_ptr<char[]> &buf, uint64_t &size)
     return ok;
 }
 
-// Parses the file on the device: HC_SUCCESS with *out set, an error, or 1 when it
-// is the host parser's (small, unreadable, a peak line that is not plain).
-int read_device(hc_ctx *ctx, const char *path, hc_ms2 **out)
+// Parses the text on the device: HC_SUCCESS with *out set, an error, or 1 when it
+// is the host parser's (4 GB or more, a peak line that is not plain).
+int parse_device(hc_ctx *ctx, const std::unique_ptr<char[]> &buf, uint64_t size, hc_ms2 **out)
 {
-    std::unique_ptr<char[]> buf;
-    uint64_t size = 0;
-    if (!read_file(path, buf, size) || size >= 0xFFFFFFFFull) return 1;
-    HC_CUDA(ctx, cudaSetDevice(ctx->device));
+    if (size >= 0xFFFFFFFFull) return 1;
     cudaStream_t st = ctx->stream;
     const uint32_t nb = (uint32_t)((size + kTxt - 1) / kTxt);
     const uint64_t room = (uint64_t)nb * kTxt + kTxtHalo;
@@ -1041,16 +1047,20 @@ extern "C" int hc_ms2_open(hc_ctx *ctx, const char *path, hc_ms2 **out, uint32_t
 {
     if (!ctx || !path || !out) return HC_ERR_INVLD_PTR;
     *out = nullptr;
-    int rc = read_device(ctx, path, out);
-    if (rc == HC_SUCCESS)
+    std::unique_ptr<char[]> buf;
+    uint64_t size = 0;
+    int rc;
+    if (read_file(path, buf, size))
     {
-        if (nspec) *nspec = (uint32_t)(*out)->prec.size();
-        if (maxslen) *maxslen = (*out)->maxslen;
-        return rc;
+        HC_CUDA(ctx, cudaSetDevice(ctx->device));
+        rc = parse_device(ctx, buf, size, out);
+        if (rc < 0 && rc != HC_ERR_BAD_MEM_ALLOC) return rc;
+        if (rc < 0) cudaGetLastError();  // no room on the device: the host's arrays do
+        if (rc != HC_SUCCESS) rc = parse_host(buf.get(), buf.get() + size, (double)ctx->p.scale, out);
+        rc = opened(rc, out, nspec, maxslen);
     }
-    if (rc < 0 && rc != HC_ERR_BAD_MEM_ALLOC) return rc;
-    if (rc < 0) cudaGetLastError();  // no room on the device: the host's arrays do
-    rc = hc_ms2_read(path, ctx->p.scale, out, nspec, maxslen);
+    else
+        rc = hc_ms2_read(path, ctx->p.scale, out, nspec, maxslen);
     if (rc == HC_ERR_FILE_ERROR) return set_error(ctx, rc, std::string("cannot read ") + path);
     if (rc == HC_ERR_INVLD_SIZE) return set_error(ctx, rc, std::string("no peaks (or 2^32 or more) in ") + path);
     return rc;
