@@ -56,6 +56,26 @@ void free_len(hc_ctx *ctx, LenHost &lh)
     lh.L = L;
 }
 
+int left_running(hc_ctx *ctx, cudaStream_t st)
+{
+    if (st == ctx->stream) return HC_SUCCESS;
+    cudaStreamCaptureStatus cs = cudaStreamCaptureStatusNone;
+    if (cudaStreamIsCapturing(st, &cs) != cudaSuccess || cs != cudaStreamCaptureStatusNone)
+    {
+        cudaGetLastError();
+        return HC_SUCCESS;
+    }
+    HC_CUDA(ctx, cudaEventRecord(ctx->searched, st));
+    return HC_SUCCESS;
+}
+
+bool device_idle(hc_ctx *ctx)
+{
+    const bool idle = cudaStreamQuery(ctx->stream) == cudaSuccess && cudaEventQuery(ctx->searched) == cudaSuccess;
+    if (!idle) cudaGetLastError();
+    return idle;
+}
+
 static int check_params(const hc_params *p)
 {
     if (!p) return HC_ERR_INVLD_PTR;
@@ -125,9 +145,10 @@ int hc_ctx_create(int device, const hc_params *p, hc_ctx **out)
     ctx->smem_sm = prop.sharedMemPerMultiprocessor;
     ctx->smem_reserved = prop.reservedSharedMemPerBlock;
     if (cudaSetDevice(device) != cudaSuccess) { delete ctx; return HC_ERR_NO_DEVICE; }
-    if (cudaStreamCreateWithFlags(&ctx->stream, cudaStreamNonBlocking) != cudaSuccess)
+    if (cudaStreamCreateWithFlags(&ctx->stream, cudaStreamNonBlocking) != cudaSuccess ||
+        cudaEventCreateWithFlags(&ctx->searched, cudaEventDisableTiming) != cudaSuccess)
     {
-        delete ctx;
+        hc_ctx_destroy(ctx);
         return HC_ERR_CUDA;
     }
     {
@@ -214,6 +235,7 @@ int hc_ctx_destroy(hc_ctx *ctx)
     if (ctx->graph_exec) cudaGraphExecDestroy(ctx->graph_exec);
     if (ctx->cap_stream) cudaStreamDestroy(ctx->cap_stream);
     free_stream_stage(ctx->stage);
+    if (ctx->searched) cudaEventDestroy(ctx->searched);
     if (ctx->stream) cudaStreamDestroy(ctx->stream);
     delete ctx;
     return HC_SUCCESS;
@@ -428,7 +450,8 @@ int hc_dslim_query_device(hc_ctx *ctx, const uint32_t *d_idx, const uint32_t *d_
         return set_error(ctx, HC_ERR_INVLD_PTR, "null device buffer");
     cudaSetDevice(ctx->device);
     cudaStream_t st = stream ? (cudaStream_t)stream : ctx->stream;
-    return query_device(ctx, d_idx, d_moz, d_intensity, d_precurse, d_dM, nspec, npeaks, d_out, d_hist, st);
+    const int rc = query_device(ctx, d_idx, d_moz, d_intensity, d_precurse, d_dM, nspec, npeaks, d_out, d_hist, st);
+    return rc ? rc : left_running(ctx, st);
 }
 
 int hc_dslim_query(hc_ctx *ctx, const uint32_t *idx, const uint32_t *moz, const uint32_t *intensity,

@@ -44,7 +44,7 @@ static int replay(hc_ctx *ctx, const GraphKey &key, cudaStream_t st, Body body)
     }
     HC_CUDA(ctx, cudaGraphLaunch(ctx->graph_exec, st));
     ctx->last_launches = ctx->graph_launches;
-    return HC_SUCCESS;
+    return left_running(ctx, st);
 }
 
 static GraphKey make_key(const hc_ctx *ctx, const uint32_t *d_idx, const uint32_t *d_moz, const uint32_t *d_intensity,

@@ -214,6 +214,7 @@ struct hc_ctx
     size_t smem_reserved = 0;  // per CTA, kept by the system
     hc_params p{};
     cudaStream_t stream = nullptr;
+    cudaEvent_t searched = nullptr;  // after the last search on a stream other than `stream`
     hc_tuning tuning{};
     bool auto_shape = true;  // nobody chose a launch shape: picked by what is searched (launch_packed)
     std::vector<hc::LenHost> lens;
@@ -352,6 +353,12 @@ struct PoolScratch
         for (void *p : ptrs) dfree(ctx, p);
     }
 };
+
+// A search was enqueued on st and may be left running there.
+int left_running(hc_ctx *ctx, cudaStream_t st);
+// No search of the context is running (as far as one can see that is not part of a
+// graph of the caller's own).
+bool device_idle(hc_ctx *ctx);
 
 int set_error(hc_ctx *ctx, int code, const std::string &msg);
 int cuda_check(hc_ctx *ctx, cudaError_t e, const char *what);

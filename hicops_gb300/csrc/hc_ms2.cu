@@ -1049,11 +1049,12 @@ extern "C" int hc_ms2_open(hc_ctx *ctx, const char *path, hc_ms2 **out, uint32_t
     *out = nullptr;
     std::unique_ptr<char[]> buf;
     uint64_t size = 0;
-    int rc;
+    int rc = 1;
     if (read_file(path, buf, size))
     {
         HC_CUDA(ctx, cudaSetDevice(ctx->device));
-        rc = parse_device(ctx, buf, size, out);
+        // (a device at work would do it when it has ended what it does)
+        if (device_idle(ctx)) rc = parse_device(ctx, buf, size, out);
         if (rc < 0 && rc != HC_ERR_BAD_MEM_ALLOC) return rc;
         if (rc < 0) cudaGetLastError();  // no room on the device: the host's arrays do
         if (rc != HC_SUCCESS) rc = parse_host(buf.get(), buf.get() + size, (double)ctx->p.scale, out);

@@ -136,5 +136,6 @@ extern "C" int hc_dslim_query_noalloc(hc_ctx *ctx, const uint32_t *d_idx, const 
     s.fitstart = reinterpret_cast<int32_t *>(base + kFitOff);
     s.lens = reinterpret_cast<LenDev *>(base + kLensOff);
     cudaStream_t st = stream ? (cudaStream_t)stream : ctx->stream;
-    return launch_query_scratch(ctx, d_idx, d_moz, d_intensity, d_precurse, d_dM, nspec, d_out, d_hist, s, st);
+    const int rc = launch_query_scratch(ctx, d_idx, d_moz, d_intensity, d_precurse, d_dM, nspec, d_out, d_hist, s, st);
+    return rc ? rc : left_running(ctx, st);
 }

@@ -303,8 +303,10 @@ int hc_write_psms(hc_ctx *ctx, const char *path, const char *file_label, uint32_
  * spectra, *maxslen = largest raw peak count. HC_ERR_FILE_ERROR when the file
  * cannot be opened or read, HC_ERR_INVLD_SIZE when it holds no peak at all
  * (the reference's ERR_INVLD_SIZE). Files of some size are parsed on the
- * context's device and their raw peaks stay there until hc_ms2_close; the
- * values are the same. */
+ * context's device, whose memory then holds their raw peaks (8 bytes each)
+ * until hc_ms2_close. While a search of the context is running, on its stream or
+ * another, the host parses them instead, so that opening the next file overlaps the
+ * search. The values are the same. */
 typedef struct hc_ms2 hc_ms2;
 int hc_ms2_open(hc_ctx *ctx, const char *path, hc_ms2 **out, uint32_t *nspec, uint32_t *maxslen);
 /* The same without a context (host only, no CUDA call): m/z scaled by `scale`.
