@@ -1028,6 +1028,17 @@ int parse_device(hc_ctx *ctx, const std::unique_ptr<char[]> &buf, uint64_t size,
     return HC_SUCCESS;
 }
 
+// Reading a file is a host call to its caller: it may come while a thread of the program
+// captures a graph, in a mode that forbids others most calls until it has ended. What
+// is enqueued here goes to no stream under capture, so those calls are safe.
+struct BesideCapture
+{
+    cudaStreamCaptureMode mode = cudaStreamCaptureModeRelaxed;
+    BesideCapture() { cudaThreadExchangeStreamCaptureMode(&mode); }
+    ~BesideCapture() { cudaThreadExchangeStreamCaptureMode(&mode); }
+    BesideCapture(const BesideCapture &) = delete;
+};
+
 // the raw peaks on the host (for a device other than theirs)
 int peaks_to_host(hc_ctx *ctx, hc_ms2 *m)
 {
@@ -1052,6 +1063,7 @@ extern "C" int hc_ms2_open(hc_ctx *ctx, const char *path, hc_ms2 **out, uint32_t
     int rc = 1;
     if (read_file(path, buf, size))
     {
+        const BesideCapture beside;
         HC_CUDA(ctx, cudaSetDevice(ctx->device));
         // (a device at work would do it when it has ended what it does)
         if (device_idle(ctx)) rc = parse_device(ctx, buf, size, out);
@@ -1078,9 +1090,13 @@ extern "C" int hc_ms2_raw(const hc_ms2 *m, uint32_t first, uint32_t count, uint6
     const uint64_t n = m->off[first + count] - a;
     if (m->d_mz && n && (mz || intensity))
     {
+        const BesideCapture beside;
+        const cudaStream_t st = cudaStreamPerThread;
         cudaError_t e = cudaSetDevice(m->device);
-        if (e == cudaSuccess && mz) e = cudaMemcpy(mz, m->d_mz + a, 4 * n, cudaMemcpyDeviceToHost);
-        if (e == cudaSuccess && intensity) e = cudaMemcpy(intensity, m->d_int + a, 4 * n, cudaMemcpyDeviceToHost);
+        if (e == cudaSuccess && mz) e = cudaMemcpyAsync(mz, m->d_mz + a, 4 * n, cudaMemcpyDeviceToHost, st);
+        if (e == cudaSuccess && intensity)
+            e = cudaMemcpyAsync(intensity, m->d_int + a, 4 * n, cudaMemcpyDeviceToHost, st);
+        if (e == cudaSuccess) e = cudaStreamSynchronize(st);
         if (e != cudaSuccess) return HC_ERR_CUDA;
     }
     else if (n)
@@ -1102,8 +1118,10 @@ extern "C" int hc_ms2_close(hc_ms2 *m)
     if (!m) return HC_SUCCESS;
     if (m->d_mz)
     {
+        // (no call on m leaves work that reads it behind)
+        const BesideCapture beside;
         cudaSetDevice(m->device);
-        cudaFree(m->d_mz);  // (waits for what still reads it)
+        cudaFree(m->d_mz);
     }
     delete m;
     return HC_SUCCESS;
@@ -1129,6 +1147,7 @@ extern "C" int hc_ms2_extract(hc_ctx *ctx, hc_ms2 *m, uint32_t first, uint32_t c
     }
     idx[0] = 0;
     if (n == 0) return HC_SUCCESS;
+    const BesideCapture beside;
     cudaSetDevice(ctx->device);
     cudaStream_t st = ctx->stream;
     const uint64_t r0 = m->off[first], r1 = m->off[first + n];

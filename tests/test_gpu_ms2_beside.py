@@ -76,3 +76,36 @@ def test_open_while_a_search_runs(own, form, tmp_path):
     _same(_batch(r), o)
     r.DeinitQueryFile()
     ix.close()
+
+
+def test_read_while_a_graph_is_captured(tmp_path):
+    """Opening a file, taking its raw and picked peaks and closing it, inside a capture that forbids
+    unsafe calls: the capture ends well, its graph replays, and the file's values are right."""
+    import torch
+    from hicops_gb300 import _lib as L
+    from hicops_gb300 import dslim
+    path, o = _file(tmp_path)
+    p = S.SearchParams(maxz=2, dF=2, dM=100.0)
+    p.base_int, p.min_int = PICK[1], PICK[2]
+    ix = dslim.Index(p)
+    raw = dslim.read_ms2_raw(path, p.scale)
+    off, mz, it = np.zeros_like(raw["off"]), np.zeros_like(raw["mz"]), np.zeros_like(raw["mz"])
+    x = torch.ones(1000, device="cuda")
+    torch.cuda.synchronize()
+    g = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(g, capture_error_mode="global"):
+        y = x + 1
+        r = dslim.MSQuery(ix).initialize(path)
+        assert ix.lib.hc_ms2_raw(r.h, 0, r.QAcount, L.ptr(off), L.ptr(mz), L.ptr(it), None, None, None) == 0
+        other = dslim.MSQuery(ix).initialize(path)
+        within = _batch(other)
+        other.DeinitQueryFile()
+        z = y * 3
+    g.replay()
+    torch.cuda.synchronize()
+    assert (z == 6).all()
+    assert np.array_equal(off, raw["off"]) and np.array_equal(mz, raw["mz"]) and np.array_equal(it, raw["intensity"])
+    _same(within, o)
+    _same(_batch(r), o)
+    r.DeinitQueryFile()
+    ix.close()
