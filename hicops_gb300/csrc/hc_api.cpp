@@ -200,6 +200,7 @@ int hc_ctx_create(int device, const hc_params *p, hc_ctx **out)
     ctx->tuning.schedule = 0;
     ctx->tuning.defer_cap = HC_DEFER_MAX;
     ctx->tuning.small_log2 = 0;
+    ctx->initial = ctx->tuning;
     *out = ctx;
     return HC_SUCCESS;
 }
@@ -256,7 +257,7 @@ int hc_ctx_set_tuning(hc_ctx *ctx, const hc_tuning *t)
     if (t->ctas_per_sm * (need + ctx->smem_reserved) > ctx->smem_sm || need > ctx->smem_optin)
         return set_error(ctx, HC_ERR_INVLD_PARAM, "tile does not fit in shared memory");
     ctx->tuning = *t;
-    ctx->auto_shape = false;
+    ctx->auto_shape = std::memcmp(t, &ctx->initial, sizeof(*t)) == 0;
     return HC_SUCCESS;
 }
 

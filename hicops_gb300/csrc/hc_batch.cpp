@@ -163,6 +163,7 @@ int hc_tune(hc_ctx *ctx, const uint32_t *d_idx, const uint32_t *d_moz, const uin
     std::vector<std::pair<float, hc_tuning>> timed;
     auto run = [&](const hc_tuning &t) {
         if (hc_ctx_set_tuning(ctx, &t) != HC_SUCCESS) return;
+        ctx->auto_shape = false;  // this very shape is timed
         rc = query_device(ctx, d_idx, d_moz, d_intensity, d_precurse, d_dM, nspec, npeaks, d_out, d_hist, st);
         if (rc) return;
         float ms[2];
@@ -234,6 +235,7 @@ int hc_tune(hc_ctx *ctx, const uint32_t *d_idx, const uint32_t *d_moz, const uin
     const auto bestp = *std::min_element(timed.begin(), timed.end(),
                                          [](const auto &a, const auto &b) { return a.first < b.first; });
     ctx->tuning = bestp.second;
+    ctx->auto_shape = false;
     if (best) *best = bestp.second;
     if (best_ms) *best_ms = bestp.first;
     return HC_SUCCESS;

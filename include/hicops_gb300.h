@@ -136,6 +136,10 @@ const char *hc_status_string(int status);
 int hc_ctx_create(int device, const hc_params *p, hc_ctx **out);
 int hc_ctx_destroy(hc_ctx *ctx);
 const char *hc_last_error(const hc_ctx *ctx);
+/* The launch shape. A new context picks one for each call by what is searched (as
+ * hc_ctx_get_tuning cannot report: it gives the shape that the picking starts from).
+ * hc_tune, or any other shape set here, fixes it; setting what a new context
+ * reports turns the picking on again. */
 int hc_ctx_set_tuning(hc_ctx *ctx, const hc_tuning *t);
 int hc_ctx_get_tuning(const hc_ctx *ctx, hc_tuning *t);
 /* Waits at most timeout_s seconds (< 0: no limit) for the device work

@@ -46,3 +46,30 @@ def test_few_spectra_equal_oracle(nspec):
     ores, ohist = orc.query(q, tie_rule=1)
     for _ in range(2):
         compare(*ix.query(q), ores, ohist)
+
+
+def test_shape_read_and_set_back():
+    """Setting back the shape that was read leaves a context as it was: a new one launches what it
+    picks (both searches here), a set one what was set."""
+    p, db, ix, orc = _setup()
+    from hicops_gb300 import dslim
+    q = S.make_queries(db, 300, 5899, p)
+    ores, ohist = orc.query(q, tie_rule=1)
+    new = dslim.Index(p)
+    new.construct_all(db)
+
+    def launches():
+        compare(*new.query(q), ores, ohist)
+        return new.last_launch_count()
+
+    picked, saved = launches(), new.tuning()
+    new.set_tuning(**saved)
+    assert launches() == picked
+    new.set_tuning(tile=4096, threads=512)
+    fixed, shape = launches(), new.tuning()
+    assert fixed == picked - 1
+    new.set_tuning(**shape)
+    assert launches() == fixed
+    new.set_tuning(**saved)
+    assert launches() == picked
+    new.close()
