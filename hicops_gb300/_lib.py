@@ -111,6 +111,7 @@ _SIGS = [
                                         C.c_void_p]),
     ("hc_last_launch_count", C.c_int, [C.c_void_p]),
     ("hc_check_division", C.c_uint64, [C.c_uint32, C.c_uint32]),
+    ("hc_check_tailfit", C.c_int, [C.c_void_p, C.c_void_p, C.c_void_p, C.c_uint32, C.c_int, C.c_void_p]),
     ("hc_ctx_set_phase_timing", C.c_int, [C.c_void_p, C.c_int]),
     ("hc_mlp_create", C.c_int, [C.c_void_p, C.c_uint64, C.POINTER(C.c_void_p)]),
     ("hc_mlp_destroy", C.c_int, [C.c_void_p]),

@@ -2082,6 +2082,19 @@ __device__ void tailfit_one(uint32_t s, hc_result *__restrict__ out, const uint3
     }
 }
 
+// Every spectrum by tailfit_one: what k_tailfit's results are compared with.
+constexpr int kTfPlainWarps = 4;
+
+__global__ void __launch_bounds__(kTfPlainWarps * 32) k_tailfit_plain(hc_result *__restrict__ out,
+                                                                     const uint32_t *__restrict__ hist, uint32_t n,
+                                                                     uint32_t min_cpsm, double expect_max,
+                                                                     int32_t *__restrict__ fitstart)
+{
+    __shared__ double sx[kTfPlainWarps][HC_HIST_BINS + 2];
+    const uint32_t s = blockIdx.x * kTfPlainWarps + (threadIdx.x >> 5);
+    if (s < n) tailfit_one(s, out, hist, min_cpsm, expect_max, fitstart, sx[threadIdx.x >> 5], threadIdx.x & 31);
+}
+
 // k_tailfit. This part's FP64 rate is 1/64 of its FP32 rate (a warp's FP64
 // instruction takes the SM's pipe 16 clocks, whatever its active lanes), so
 // the fit is arranged around it:
@@ -2953,3 +2966,24 @@ int launch_query_scratch(hc_ctx *ctx, const uint32_t *d_idx, const uint32_t *d_m
 }
 
 }  // namespace hc
+
+using namespace hc;
+
+extern "C" int hc_check_tailfit(hc_ctx *ctx, const uint32_t *d_hist, hc_result *d_res, uint32_t n, int plain,
+                                int32_t *d_first)
+{
+    if (!ctx || (n && (!d_hist || !d_res || !d_first))) return HC_ERR_INVLD_PTR;
+    if (n == 0) return HC_SUCCESS;
+    HC_CUDA(ctx, cudaSetDevice(ctx->device));
+    cudaStream_t st = ctx->stream;
+    if (plain)
+    {
+        k_tailfit_plain<<<(n + kTfPlainWarps - 1) / kTfPlainWarps, kTfPlainWarps * 32, 0, st>>>(
+            d_res, d_hist, n, ctx->p.min_cpsm, ctx->p.expect_max, d_first);
+        HC_CUDA(ctx, cudaGetLastError());
+    }
+    else if (const int rc = launch_tailfit(ctx, d_res, d_hist, n, d_first, nullptr, nullptr, st))
+        return rc;
+    HC_CUDA(ctx, cudaStreamSynchronize(st));
+    return HC_SUCCESS;
+}

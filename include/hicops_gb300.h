@@ -366,6 +366,12 @@ int hc_phase_cycles(hc_ctx *ctx, uint64_t out[10]);
  * which the multiply-shift quotient used on the device differs from x / d
  * (0 expected; no device needed). */
 uint64_t hc_check_division(uint32_t d, uint32_t xmax);
+/* Device check of the tail fit: expeRT's fit of n spectra (device histograms and
+ * results, these in place; d_first[n]: the first bin of each regression window, -1:
+ * none) as a search runs it, or, with `plain`, every step of every spectrum in the
+ * reference's order of operations. Both give the same bits. Synchronous. */
+int hc_check_tailfit(hc_ctx *ctx, const uint32_t *d_hist, hc_result *d_res, uint32_t n, int plain,
+                     int32_t *d_first);
 /* Kernel launches made by the last query call (for launch accounting). */
 int hc_last_launch_count(const hc_ctx *ctx);
 /* With profiling on, every query records CUDA events around its kernels on
