@@ -2119,7 +2119,12 @@ __global__ void __launch_bounds__(kTfPlainWarps * 32) k_tailfit_plain(hc_result 
 constexpr int kTfWarps = 16;
 constexpr float kTfNear = 5e-5f;      // FP32 curve and level: together within 5e-6 of FP64's
 constexpr double kTfLevel = 1e-9;     // the short FP64 logarithm: within 1e-14
-constexpr double kTfInteger = 1e-5;   // mu, beta x 1e6: within 5e-6 of tailfit_one's
+// How far the values x 1e6 may be from tailfit_one's. Two logarithms of a point differ by
+// 4e-15 at most (the short one within 2e-15, log10's 2 ulp below 8), the slope of m points by
+// 3 / m times that and twice it for two, so by 8e-15 and its own rounding: below 1.5e-8 x 1e-6.
+// The intercept is a point's value less the slope times the window's middle, up to bin 1000:
+// 8.5e-12 and the roundings of the product, 2.3e-13 each way: below 1e-5 x 1e-6.
+constexpr double kTfSlope = 1e-6, kTfIntercept = 3e-5;
 
 struct TfJob
 {
@@ -2329,8 +2334,8 @@ __device__ __forceinline__ bool tailfit_line(const TfJob &j, hc_result *__restri
         beta_t = (ybar - mu * xbar) * 1e6;
         // (a value that truncates to 0 from either side is not open)
         const bool open = !(fabs(mu_t) < 1e9) || !(fabs(beta_t) < 1e9) ||
-                          (fabs(mu_t) > 0.5 && fabs(mu_t - rint(mu_t)) < kTfInteger) ||
-                          (fabs(beta_t) > 0.5 && fabs(beta_t - rint(beta_t)) < kTfInteger);
+                          (fabs(mu_t) > 0.5 && fabs(mu_t - rint(mu_t)) < kTfSlope) ||
+                          (fabs(beta_t) > 0.5 && fabs(beta_t - rint(beta_t)) < kTfIntercept);
         if (open) return false;
     }
     hc_result r = out[j.s];
