@@ -14,6 +14,8 @@ namespace hc {
 int set_error(hc_ctx *ctx, int code, const std::string &msg)
 {
     if (ctx) ctx->last_error = msg;
+    // reported here: the next call's check of its launches is not to find it again
+    if (code == HC_ERR_CUDA || code == HC_ERR_BAD_MEM_ALLOC) cudaGetLastError();
     return code;
 }
 

@@ -1108,7 +1108,7 @@ try
         // (a device at work would do it when it has ended what it does)
         if (device_idle(ctx)) rc = parse_device(ctx, buf, size, out);
         if (rc < 0 && rc != HC_ERR_BAD_MEM_ALLOC) return rc;
-        if (rc < 0) cudaGetLastError();  // no room on the device: the host's arrays do
+        // (no room on the device: the host's arrays do)
         if (rc != HC_SUCCESS) rc = parse_host(buf.get(), buf.get() + size, (double)ctx->p.scale, out);
         rc = opened(rc, out, nspec, maxslen);
     }
