@@ -309,9 +309,16 @@ __attribute__((optimize("O3"))) static bool residues_ok(const uint8_t *seqs, siz
     return true;
 }
 
+static int check_seqs(hc_ctx *ctx, const LenHost &lh, const uint8_t *seqs, uint32_t npep)
+{
+    if (residues_ok(seqs, (size_t)npep * lh.L)) return HC_SUCCESS;
+    return set_error(ctx, HC_ERR_INVLD_PARAM, "residue outside A-Z");
+}
+
+// Enqueues the copy of the caller's sequences: after the checks, and waited for before a
+// call returns, whatever it returns.
 static int upload_seqs(hc_ctx *ctx, LenHost &lh, const uint8_t *seqs, uint32_t npep)
 {
-    if (!residues_ok(seqs, (size_t)npep * lh.L)) return set_error(ctx, HC_ERR_INVLD_PARAM, "residue outside A-Z");
     HC_CUDA(ctx, dalloc(ctx, &lh.d_seqs, (size_t)npep * lh.L + 1));
     HC_CUDA(ctx, cudaMemcpyAsync(lh.d_seqs, seqs, (size_t)npep * lh.L, cudaMemcpyHostToDevice, ctx->stream));
     lh.npep = npep;
@@ -326,14 +333,20 @@ int hc_dslim_construct(hc_ctx *ctx, uint32_t L, const uint8_t *seqs, uint32_t np
     if (!lh) return set_error(ctx, HC_ERR_INVLD_PARAM, "length outside [min_len, max_len]");
     cudaSetDevice(ctx->device);
     free_len(ctx, *lh);
-    int rc = upload_seqs(ctx, *lh, seqs, npep);
+    int rc = check_seqs(ctx, *lh, seqs, npep);
     if (rc) return rc;
-    if (!order) return build_length_device(ctx, *lh, nullptr, true);  // entries enumerated on the device
-    for (uint32_t i = 0; i < norder; i++)
-        if (order[i].seqid >= npep) return set_error(ctx, HC_ERR_INVLD_INDEX, "entry seqid out of range");
-    if (norder >= (1u << 24)) return set_error(ctx, HC_ERR_INVLD_SIZE, "more than 2^24 entries in one length");
-    lh->n = norder;
-    return build_length_device(ctx, *lh, order, false);
+    if (order)
+    {
+        for (uint32_t i = 0; i < norder; i++)
+            if (order[i].seqid >= npep) return set_error(ctx, HC_ERR_INVLD_INDEX, "entry seqid out of range");
+        if (norder >= (1u << 24)) return set_error(ctx, HC_ERR_INVLD_SIZE, "more than 2^24 entries in one length");
+        lh->n = norder;
+    }
+    rc = upload_seqs(ctx, *lh, seqs, npep);
+    // (without an order the entries are enumerated on the device)
+    if (rc == HC_SUCCESS) rc = build_length_device(ctx, *lh, order, !order);
+    if (rc) cudaStreamSynchronize(ctx->stream);
+    return rc;
 }
 
 int hc_dslim_load(hc_ctx *ctx, uint32_t L, const uint8_t *seqs, uint32_t npep, const hc_entry *entries,
@@ -345,7 +358,7 @@ int hc_dslim_load(hc_ctx *ctx, uint32_t L, const uint8_t *seqs, uint32_t npep, c
     if (n >= (1u << 24)) return set_error(ctx, HC_ERR_INVLD_SIZE, "more than 2^24 entries in one length");
     cudaSetDevice(ctx->device);
     free_len(ctx, *lh);
-    int rc = upload_seqs(ctx, *lh, seqs, npep);
+    int rc = check_seqs(ctx, *lh, seqs, npep);
     if (rc) return rc;
     const uint32_t speclen = 2 * ctx->p.maxz * (L - 1);
     const uint64_t M = (uint64_t)n * speclen;
@@ -374,6 +387,12 @@ int hc_dslim_load(hc_ctx *ctx, uint32_t L, const uint8_t *seqs, uint32_t npep, c
         mo[i] = entries[i].modnum;
     }
     cudaStream_t st = ctx->stream;
+    struct Wait  // for the copies of the arrays above and of the caller's
+    {
+        cudaStream_t st;
+        ~Wait() { cudaStreamSynchronize(st); }
+    } const wait{st};
+    if ((rc = upload_seqs(ctx, *lh, seqs, npep))) return rc;
     HC_CUDA(ctx, dalloc(ctx, &lh->d_mass, (size_t)n + 1));
     HC_CUDA(ctx, dalloc(ctx, &lh->d_seqid, (size_t)n + 1));
     HC_CUDA(ctx, dalloc(ctx, &lh->d_modnum, (size_t)n + 1));
@@ -391,7 +410,6 @@ int hc_dslim_load(hc_ctx *ctx, uint32_t L, const uint8_t *seqs, uint32_t npep, c
     // build, which places every posting, passes over padding
     static_assert(kQpostPad == 0xFFFFFFFFu, "written byte by byte");
     if (e == cudaSuccess && bA[0]) e = cudaMemsetAsync(d_ids, 0xFF, 4ull * bA[0], st);
-    if (e == cudaSuccess) e = cudaStreamSynchronize(st);  // the host vectors above go with this call
     lh->npost = M;
     const int rq = e == cudaSuccess ? build_query_postings(ctx, *lh, M ? d_ids : nullptr, nullptr)
                                     : cuda_check(ctx, e, "hc_dslim_load");
