@@ -68,12 +68,14 @@ int left_running(hc_ctx *ctx, cudaStream_t st)
         return HC_SUCCESS;
     }
     HC_CUDA(ctx, cudaEventRecord(ctx->searched, st));
+    ctx->elsewhere = true;
     return HC_SUCCESS;
 }
 
 bool device_idle(hc_ctx *ctx)
 {
-    const bool idle = cudaStreamQuery(ctx->stream) == cudaSuccess && cudaEventQuery(ctx->searched) == cudaSuccess;
+    if (ctx->elsewhere) ctx->elsewhere = cudaEventQuery(ctx->searched) != cudaSuccess;
+    const bool idle = !ctx->elsewhere && cudaStreamQuery(ctx->stream) == cudaSuccess;
     if (!idle) cudaGetLastError();
     return idle;
 }

@@ -215,6 +215,7 @@ struct hc_ctx
     hc_params p{};
     cudaStream_t stream = nullptr;
     cudaEvent_t searched = nullptr;  // after the last search on a stream other than `stream`
+    bool elsewhere = false;          // ... which has not been seen to have ended
     hc_tuning tuning{}, initial{};  // the shape, and a new context's
     bool auto_shape = true;  // nobody chose a launch shape: picked by what is searched (launch_packed)
     std::vector<hc::LenHost> lens;
