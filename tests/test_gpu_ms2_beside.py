@@ -109,3 +109,24 @@ def test_read_while_a_graph_is_captured(tmp_path):
     _same(_batch(r), o)
     r.DeinitQueryFile()
     ix.close()
+
+
+def test_reader_outlives_its_context(tmp_path):
+    """A file's raw peaks are its own: read and closed after the context that parsed it is gone, and
+    extracted by another context of the device."""
+    from hicops_gb300 import _lib as L
+    from hicops_gb300 import dslim
+    path, o = _file(tmp_path)
+    p = S.SearchParams(maxz=2, dF=2, dM=100.0)
+    p.base_int, p.min_int = PICK[1], PICK[2]
+    a, b = dslim.Index(p), dslim.Index(p)
+    raw = dslim.read_ms2_raw(path, p.scale)
+    r = dslim.MSQuery(a).initialize(path)
+    a.close()
+    off, mz, it = np.zeros_like(raw["off"]), np.zeros_like(raw["mz"]), np.zeros_like(raw["mz"])
+    assert a.lib.hc_ms2_raw(r.h, 0, r.QAcount, L.ptr(off), L.ptr(mz), L.ptr(it), None, None, None) == 0
+    assert np.array_equal(off, raw["off"]) and np.array_equal(mz, raw["mz"]) and np.array_equal(it, raw["intensity"])
+    r.ix = b
+    _same(_batch(r), o)
+    r.DeinitQueryFile()
+    b.close()
