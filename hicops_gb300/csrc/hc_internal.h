@@ -204,8 +204,11 @@ struct hc_ctx
     int device = 0;
     // Index arrays and build scratch come from this pool, ordered on `stream`:
     // building a length takes some 25 buffers, and cudaMalloc / cudaFree at 10-25 us
-    // each were two thirds of a build. What a build gives back is kept for the
-    // next one up to kPoolKeep bytes; the pool goes with the context.
+    // each were two thirds of a build. At a wait for the stream the pool gives free memory
+    // back to the device until it holds kPoolKeep bytes, the index's arrays among them: a
+    // small index keeps a build's scratch for the next length and the next build (45 MB
+    // beside 20,000 peptides' 340 MB, 170 MB beside 660), one past kPoolKeep maps it anew.
+    // The pool goes with the context.
     cudaMemPool_t pool = nullptr;
     void *h_read = nullptr;  // pinned words the build reads counts back through
     int sm_count = 0;
@@ -316,7 +319,7 @@ void learned_key(const hc_mlp *m, GraphKey *key);
 int learned_pipeline(hc_mlp *m, const uint32_t *d_hist, hc_result *d_res, uint32_t n, float *lg, cudaStream_t st,
                      int *launches);
 
-constexpr uint64_t kPoolKeep = 1ull << 30;
+constexpr uint64_t kPoolKeep = 1ull << 30;  // hc_ctx::pool's release threshold
 constexpr size_t kReadBytes = 4096;  // hc_ctx::h_read
 
 // hc_api.cpp: device memory of the index and its builds, n elements (at least one)

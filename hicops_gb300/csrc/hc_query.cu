@@ -744,7 +744,7 @@ __global__ void __launch_bounds__(G >= 4 ? 512 : 1024, G == 4 ? 2 : 1) k_search(
             T.best_shp = 0;
             T.maxbits = 0;
             T.cpsms = 0;
-                T.ndefer = 0;
+            T.ndefer = 0;
             T.flags = WIDE ? HC_FLAG_WIDE : 0u;
             T.overflow = 0;
             T.bytes = 0;

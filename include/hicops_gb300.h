@@ -132,7 +132,10 @@ typedef struct hc_tuning
 int hc_version(void);
 const char *hc_status_string(int status);
 
-/* ---- context (owns the index, the scorecard scratch and a stream) ---- */
+/* ---- context (owns the index, the scorecard scratch and a stream) ----
+ * The index's arrays and its builds' scratch lie in a memory pool of the context,
+ * which may keep freed memory, up to 1 GB with the index itself, until it is
+ * destroyed. */
 int hc_ctx_create(int device, const hc_params *p, hc_ctx **out);
 int hc_ctx_destroy(hc_ctx *ctx);
 const char *hc_last_error(const hc_ctx *ctx);
@@ -161,7 +164,9 @@ int hc_ctx_wait(hc_ctx *ctx, void *stream, double timeout_s);
  * (e.g. the reference's own sorted order); NULL = device sort. */
 int hc_dslim_construct(hc_ctx *ctx, uint32_t L, const uint8_t *seqs, uint32_t npep,
                        const hc_entry *order, uint32_t norder);
-/* Loads a host-built index as-is (bA/iA as DSLIM_Construct lays them out). */
+/* Loads a host-built index as-is (bA/iA as DSLIM_Construct lays them out). Postings in
+ * front of bA[0], which is 0 there, lie in no bucket: they are not searched, and
+ * hc_dslim_export gives 0 in their place. */
 int hc_dslim_load(hc_ctx *ctx, uint32_t L, const uint8_t *seqs, uint32_t npep,
                   const hc_entry *entries, uint32_t n, const uint32_t *bA, const uint32_t *iA);
 int hc_dslim_info(hc_ctx *ctx, uint32_t L, uint32_t *n_entries, uint64_t *n_postings);
