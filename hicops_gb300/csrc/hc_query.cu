@@ -326,6 +326,10 @@ __device__ __forceinline__ uint32_t atom_shared_add(uint32_t addr, uint32_t v)
     return old;
 }
 
+// A word to which an add came with this in it has a count of 128 or more: more than
+// a count byte's compare, and the score's table, hold.
+__device__ __forceinline__ bool count_full(uint32_t before) { return before >= 127u << 24; }
+
 // Bounds of a bucket's postings for candidates [c0, c1), widened to row-table
 // boundaries (multiples of kRowG entries): the postings of entries outside
 // the range are read but fail the scorecard's index test, so no search is
@@ -967,7 +971,7 @@ __global__ void __launch_bounds__(G >= 4 ? 512 : 1024, G == 4 ? 2 : 1) k_search(
             // Visited postings are counted per posting only in a window's end
             // tiles; an interior tile's lists hold exactly the tile's entries,
             // and their lengths were added when its bounds were set.
-            uint32_t ovf = 0;  // OR of the words the atomics returned
+            uint32_t ovf = 0;  // largest word that an atomic returned (see count_full)
             auto stream = [&](auto no_return, auto count) {
             constexpr bool NR = decltype(no_return)::value;
             constexpr bool CNT = decltype(count)::value;
@@ -1059,7 +1063,7 @@ __global__ void __launch_bounds__(G >= 4 ? 512 : 1024, G == 4 ? 2 : 1) k_search(
                             else
                             {
                                 const uint32_t old = atom_shared_add(wa, add);
-                                ovf |= in ? old : 0u;
+                                ovf = max(ovf, in ? old : 0u);
                             }
                             if constexpr (CNT) npass += in ? 1u : 0u;
                         }
@@ -1096,7 +1100,7 @@ __global__ void __launch_bounds__(G >= 4 ? 512 : 1024, G == 4 ? 2 : 1) k_search(
                     else stream(std::false_type{}, std::false_type{});
                 }
             }
-            if (!WIDE && (__reduce_or_sync(0xFFFFFFFFu, ovf) & 0x80000000u) && lane == 0) T.overflow = 1;
+            if (!WIDE && count_full(__reduce_max_sync(0xFFFFFFFFu, ovf)) && lane == 0) T.overflow = 1;
             // ---- the next job's list bounds ----
             if (nj.l != kNoJob)
             {
@@ -1712,7 +1716,7 @@ __global__ void __launch_bounds__(kSmThreads, 4) k_search_small(SearchArgs a)
                     const uint32_t o = xs[e] - g.off;
                     const bool in = o < g.lim;
                     const uint32_t old = atom_shared_add(in ? g.card + o : sink_s, add);
-                    ovf |= in ? old : 0u;
+                    ovf = max(ovf, in ? old : 0u);
                     npass += in ? 1u : 0u;
                 }
             };
@@ -1822,7 +1826,7 @@ __global__ void __launch_bounds__(kSmThreads, 4) k_search_small(SearchArgs a)
             if (fill) pop_score(fill);
             __syncthreads();
         }
-        if ((__reduce_or_sync(0xFFFFFFFFu, ovf) & 0x80000000u) && lane == 0) S.overflow = 1;
+        if (count_full(__reduce_max_sync(0xFFFFFFFFu, ovf)) && lane == 0) S.overflow = 1;
         // ---- candidates whose sign or bin the float estimate left open ----
         for (uint32_t i = tid; i < min(S.ndefer, a.defer_cap); i += nthr)
         {
