@@ -1409,12 +1409,13 @@ int hc_mlp_train(hc_mlp *m, const float *d_X, const float *d_Y, uint32_t n, uint
         for (uint32_t s0 = 0; s0 < n; s0 += batch)
         {
             const uint32_t b = std::min(batch, n - s0);
-            m->step++;
+            const int t = m->step + 1;  // (a step that is refused is none)
             // in double: 1 - 0.999f alone is 5e-5 off 0.001
-            const float c1 = (float)(1.0 - std::pow(0.9, m->step)), c2 = (float)(1.0 - std::pow(0.999, m->step));
+            const float c1 = (float)(1.0 - std::pow(0.9, t)), c2 = (float)(1.0 - std::pow(0.999, t));
             int rc = mlp_step(m, d_X + (size_t)s0 * kIn, d_Y + (size_t)s0 * kOut, b,
                               AdamStep{m->d_params, m->d_m, m->d_v, lr, c1, c2}, st);
             if (rc) return rc;
+            m->step = t;
             nb++;
         }
         HC_CUDA(m->ctx, cudaMemcpyAsync(&loss, m->d_loss, 4, cudaMemcpyDeviceToHost, st));
