@@ -177,7 +177,7 @@ int hc_ctx_create(int device, const hc_params *p, hc_ctx **out)
         std::vector<double> lt(kLog10Tab);
         make_log10_table(lt.data(), kLog10Tab);
         if (cudaMalloc((void **)&ctx->d_log10, sizeof(double) * kLog10Tab) != cudaSuccess ||
-            cudaMemcpy(ctx->d_log10, lt.data(), sizeof(double) * kLog10Tab, cudaMemcpyHostToDevice) != cudaSuccess)
+            upload(ctx, ctx->d_log10, lt.data(), sizeof(double) * kLog10Tab) != cudaSuccess)
         {
             hc_ctx_destroy(ctx);
             return HC_ERR_BAD_MEM_ALLOC;
@@ -186,8 +186,8 @@ int hc_ctx_create(int device, const hc_params *p, hc_ctx **out)
     }
     if (cudaMalloc((void **)&ctx->d_tables, sizeof(IonTables)) != cudaSuccess ||
         cudaMalloc((void **)&ctx->d_qconst, sizeof(QueryConst)) != cudaSuccess ||
-        cudaMemcpy(ctx->d_tables, &ctx->tables, sizeof(IonTables), cudaMemcpyHostToDevice) != cudaSuccess ||
-        cudaMemcpy(ctx->d_qconst, &qc, sizeof(QueryConst), cudaMemcpyHostToDevice) != cudaSuccess)
+        upload(ctx, ctx->d_tables, &ctx->tables, sizeof(IonTables)) != cudaSuccess ||
+        upload(ctx, ctx->d_qconst, &qc, sizeof(QueryConst)) != cudaSuccess)
     {
         hc_ctx_destroy(ctx);
         return HC_ERR_BAD_MEM_ALLOC;

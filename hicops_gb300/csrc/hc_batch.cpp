@@ -249,7 +249,8 @@ int hc_ctx_set_phase_timing(hc_ctx *ctx, int on)
     if (on && !ctx->d_phase)
     {
         HC_CUDA(ctx, cudaMalloc((void **)&ctx->d_phase, 8 * 16));
-        HC_CUDA(ctx, cudaMemset(ctx->d_phase, 0, 8 * 16));
+        HC_CUDA(ctx, cudaMemsetAsync(ctx->d_phase, 0, 8 * 16, ctx->stream));
+        HC_CUDA(ctx, cudaStreamSynchronize(ctx->stream));
     }
     if (!on && ctx->d_phase)
     {
@@ -266,7 +267,8 @@ int hc_phase_cycles(hc_ctx *ctx, uint64_t out[10])
     HC_CUDA(ctx, cudaStreamSynchronize(ctx->stream));
     HC_CUDA(ctx, cudaDeviceSynchronize());
     HC_CUDA(ctx, cudaMemcpy(out, ctx->d_phase, 8 * 10, cudaMemcpyDeviceToHost));
-    HC_CUDA(ctx, cudaMemset(ctx->d_phase, 0, 8 * 16));
+    HC_CUDA(ctx, cudaMemsetAsync(ctx->d_phase, 0, 8 * 16, ctx->stream));
+    HC_CUDA(ctx, cudaStreamSynchronize(ctx->stream));
     return HC_SUCCESS;
 }
 

@@ -1316,8 +1316,8 @@ static int add_classes(hc_ctx *ctx, const uint8_t *used)
     }
     if (changed)
     {
-        HC_CUDA(ctx, cudaMemcpy(ctx->d_classes, &ctx->classes, sizeof(ClassKeys), cudaMemcpyHostToDevice));
-        HC_CUDA(ctx, cudaMemcpy(ctx->d_class_of, ctx->class_of.data(), kCodes, cudaMemcpyHostToDevice));
+        HC_CUDA(ctx, overwrite(ctx->d_classes, &ctx->classes, sizeof(ClassKeys)));
+        HC_CUDA(ctx, overwrite(ctx->d_class_of, ctx->class_of.data(), kCodes));
     }
     return HC_SUCCESS;
 }
@@ -1430,7 +1430,7 @@ int check_query_postings(hc_ctx *ctx, const LenHost &lh, uint64_t qtotal)
     uint32_t *d_bad = nullptr;
     HC_CUDA(ctx, cudaMalloc((void **)&d_bad, 4));
     uint32_t bad = 0;
-    cudaError_t e = cudaMemset(d_bad, 0, 4);
+    cudaError_t e = cudaMemsetAsync(d_bad, 0, 4, ctx->stream);
     if (e == cudaSuccess && qtotal)
     {
         const unsigned blocks = (unsigned)std::min<uint64_t>((qtotal + 255) / 256, (uint64_t)ctx->sm_count * 32);

@@ -336,6 +336,21 @@ void dfree(hc_ctx *ctx, T *&p)
     p = nullptr;
 }
 
+// Copies to the device that have ended, for any stream, when they return. (The runtime's
+// blocking copy of pageable memory may end after the call, on the legacy stream, which neither
+// the context's stream nor a caller's non-blocking one waits for.) upload: to a buffer that
+// nothing has read yet; overwrite: behind what a caller's blocking streams still read there.
+inline cudaError_t upload(hc_ctx *ctx, void *d, const void *h, size_t bytes)
+{
+    const cudaError_t e = cudaMemcpyAsync(d, h, bytes, cudaMemcpyHostToDevice, ctx->stream);
+    return e != cudaSuccess ? e : cudaStreamSynchronize(ctx->stream);
+}
+inline cudaError_t overwrite(void *d, const void *h, size_t bytes)
+{
+    const cudaError_t e = cudaMemcpy(d, h, bytes, cudaMemcpyHostToDevice);
+    return e != cudaSuccess ? e : cudaStreamSynchronize(cudaStreamLegacy);
+}
+
 // Device scratch of one call or build step, given back when it goes out of
 // scope (also on error paths); the work enqueued on the context's stream until
 // then still has it.

@@ -1302,8 +1302,9 @@ int hc_mlp_create(hc_ctx *ctx, uint64_t seed, hc_mlp **out)
         hc_mlp_destroy(m);
         return HC_ERR_BAD_MEM_ALLOC;
     }
-    if (cudaMemcpy(m->d_params, h.data(), 4 * kParams, cudaMemcpyHostToDevice) != cudaSuccess ||
-        cudaMemset(m->d_m, 0, 4 * kParams) != cudaSuccess || cudaMemset(m->d_v, 0, 4 * kParams) != cudaSuccess)
+    if (cudaMemsetAsync(m->d_m, 0, 4 * kParams, ctx->stream) != cudaSuccess ||
+        cudaMemsetAsync(m->d_v, 0, 4 * kParams, ctx->stream) != cudaSuccess ||
+        upload(ctx, m->d_params, h.data(), 4 * kParams) != cudaSuccess)
     {
         hc_mlp_destroy(m);
         return HC_ERR_CUDA;
@@ -1339,7 +1340,7 @@ int hc_mlp_get_params(hc_mlp *m, float *host)
 int hc_mlp_set_params(hc_mlp *m, const float *host)
 {
     if (!m || !host) return HC_ERR_INVLD_PTR;
-    HC_CUDA(m->ctx, cudaMemcpy(m->d_params, host, 4 * kParams, cudaMemcpyHostToDevice));
+    HC_CUDA(m->ctx, overwrite(m->d_params, host, 4 * kParams));
     return HC_SUCCESS;
 }
 

@@ -68,7 +68,7 @@ extern "C" int hc_write_psms(hc_ctx *ctx, const char *path, const char *file_lab
         cudaError_t e = cudaMalloc((void **)&d_hits, sizeof(int2) * n);
         if (e == cudaSuccess) e = cudaMalloc((void **)&d_mass, 4ull * n);
         if (e == cudaSuccess) e = cudaMalloc((void **)&d_seq, (size_t)n * kSeqCap);
-        if (e == cudaSuccess) e = cudaMemcpy(d_hits, hits.data(), sizeof(int2) * n, cudaMemcpyHostToDevice);
+        if (e == cudaSuccess) e = upload(ctx, d_hits, hits.data(), sizeof(int2) * n);
         if (e == cudaSuccess)
         {
             k_psm_rows<<<(n + 127) / 128, 128, 0, ctx->stream>>>(ctx->d_lens, d_hits, n, d_mass, d_seq);

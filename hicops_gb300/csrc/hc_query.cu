@@ -2605,7 +2605,7 @@ int sync_lengths(hc_ctx *ctx)
         fill_lendev(ctx, ctx->lens[i], h[i]);
     }
     if (!ctx->d_lens) HC_CUDA(ctx, cudaMalloc((void **)&ctx->d_lens, sizeof(LenDev) * HC_MAX_LENGTHS));
-    HC_CUDA(ctx, cudaMemcpy(ctx->d_lens, h.data(), sizeof(LenDev) * nlen, cudaMemcpyHostToDevice));
+    HC_CUDA(ctx, overwrite(ctx->d_lens, h.data(), sizeof(LenDev) * nlen));
     ctx->lens_dirty = false;
     return HC_SUCCESS;
 }

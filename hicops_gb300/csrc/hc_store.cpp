@@ -67,14 +67,14 @@ bool put_dev(FILE *f, const void *d, size_t bytes, std::vector<char> &buf)
     return true;
 }
 
-bool get_dev(FILE *f, void *d, size_t bytes, std::vector<char> &buf)
+bool get_dev(hc_ctx *ctx, FILE *f, void *d, size_t bytes, std::vector<char> &buf)
 {
     char *dst = static_cast<char *>(d);
     for (size_t off = 0; off < bytes; off += buf.size())
     {
         const size_t n = std::min(buf.size(), bytes - off);
         if (std::fread(buf.data(), 1, n, f) != n) return false;
-        if (cudaMemcpy(dst + off, buf.data(), n, cudaMemcpyHostToDevice) != cudaSuccess) return false;
+        if (hc::upload(ctx, dst + off, buf.data(), n) != cudaSuccess) return false;
     }
     return true;
 }
@@ -161,18 +161,16 @@ extern "C" int hc_dslim_restore(hc_ctx *ctx, const char *path)
         if (e == cudaSuccess) e = dalloc(ctx, &lh.d_qp, (size_t)qtotal + kIaPad);
         if (e == cudaSuccess) e = cudaMemsetAsync(lh.d_qp + qtotal, 0xFF, 4ull * kIaPad, ctx->stream);
         if (e == cudaSuccess) e = dalloc(ctx, &lh.d_qion, (size_t)qtotal + kIaPad);
-        // the file's arrays are copied on the default stream: the buffers are there first
-        if (e == cudaSuccess) e = cudaStreamSynchronize(ctx->stream);
         if (e != cudaSuccess)
         {
             free_len(ctx, lh);
             return set_error(ctx, HC_ERR_BAD_MEM_ALLOC, cudaGetErrorString(e));
         }
-        bool ok = get_dev(f, lh.d_seqs, (size_t)npep * L, buf);
-        ok = ok && get_dev(f, lh.d_mass, 4ull * n, buf) && get_dev(f, lh.d_seqid, 4ull * n, buf);
-        ok = ok && get_dev(f, lh.d_sites, 8ull * n, buf) && get_dev(f, lh.d_modnum, 4ull * n, buf);
-        ok = ok && get_dev(f, lh.d_bA, 4ull * (nb + 1), buf) && get_dev(f, lh.d_qA, 4ull * (nb + 1), buf);
-        ok = ok && get_dev(f, lh.d_qp, 4ull * qtotal, buf) && get_dev(f, lh.d_qion, 2ull * qtotal, buf);
+        bool ok = get_dev(ctx, f, lh.d_seqs, (size_t)npep * L, buf);
+        ok = ok && get_dev(ctx, f, lh.d_mass, 4ull * n, buf) && get_dev(ctx, f, lh.d_seqid, 4ull * n, buf);
+        ok = ok && get_dev(ctx, f, lh.d_sites, 8ull * n, buf) && get_dev(ctx, f, lh.d_modnum, 4ull * n, buf);
+        ok = ok && get_dev(ctx, f, lh.d_bA, 4ull * (nb + 1), buf) && get_dev(ctx, f, lh.d_qA, 4ull * (nb + 1), buf);
+        ok = ok && get_dev(ctx, f, lh.d_qp, 4ull * qtotal, buf) && get_dev(ctx, f, lh.d_qion, 2ull * qtotal, buf);
         if (!ok)
         {
             free_len(ctx, lh);
