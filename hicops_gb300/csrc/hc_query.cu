@@ -2126,9 +2126,11 @@ constexpr double kTfLevel = 1e-9;     // the short FP64 logarithm: within 1e-14
 // How far the values x 1e6 may be from tailfit_one's. Two logarithms of a point differ by
 // 4e-15 at most (the short one within 2e-15, log10's 2 ulp below 8), the slope of m points by
 // 3 / m times that and twice it for two, so by 8e-15 and its own rounding: below 1.5e-8 x 1e-6.
-// The intercept is a point's value less the slope times the window's middle, up to bin 1000:
-// 8.5e-12 and the roundings of the product, 2.3e-13 each way: below 1e-5 x 1e-6.
-constexpr double kTfSlope = 1e-6, kTfIntercept = 3e-5;
+// The intercept is the points' mean less the slope times the window's middle x: 8.5e-15 x, the
+// product's roundings (2.3e-13 each where x is 1000) and the mean's, below 5e-13: 1.1e-8 x and
+// 5e-7 x 1e-6. Each margin is more than twice its bound, and what is next to an integer is refitted
+// by one warp in 10 us: with 3e-5 for every intercept a batch of 129 spectra had one more often.
+constexpr double kTfSlope = 1e-6, kTfIntercept = 2e-6, kTfMiddle = 3e-8;
 
 struct TfJob
 {
@@ -2339,7 +2341,7 @@ __device__ __forceinline__ bool tailfit_line(const TfJob &j, hc_result *__restri
         // (a value that truncates to 0 from either side is not open)
         const bool open = !(fabs(mu_t) < 1e9) || !(fabs(beta_t) < 1e9) ||
                           (fabs(mu_t) > 0.5 && fabs(mu_t - rint(mu_t)) < kTfSlope) ||
-                          (fabs(beta_t) > 0.5 && fabs(beta_t - rint(beta_t)) < kTfIntercept);
+                          (fabs(beta_t) > 0.5 && fabs(beta_t - rint(beta_t)) < fma(kTfMiddle, xbar, kTfIntercept));
         if (open) return false;
     }
     hc_result r = out[j.s];
