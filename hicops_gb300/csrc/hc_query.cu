@@ -2116,7 +2116,7 @@ __global__ void __launch_bounds__(kTfPlainWarps * 32) k_tailfit_plain(hc_result 
 //     lane per spectrum, sixteen spectra at a time.
 // The line is (mu, beta) x 1e6 truncated to integers, so a result that differs
 // in its last bits is the same result unless a value lies near an integer (or
-// a point on a level): those spectra, about 1 in 10^4, are fitted again by
+// a point on a level): those spectra, about 1 in 10^5, are fitted again by
 // tailfit_one, in the reference's own order of operations. Results are therefore
 // tailfit_one's, bit for bit. 2,000 spectra of an open search: 23 us,
 // against 183 us with every point in FP64 and the sums on one lane.
