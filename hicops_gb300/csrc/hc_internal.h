@@ -351,6 +351,17 @@ inline cudaError_t overwrite(void *d, const void *h, size_t bytes)
     return e != cudaSuccess ? e : cudaStreamSynchronize(cudaStreamLegacy);
 }
 
+// For calls that touch no stream under capture (reading a file is a host call to its
+// caller): they may come while a thread of the program captures a graph, in a mode that
+// forbids all others most calls until it has ended.
+struct BesideCapture
+{
+    cudaStreamCaptureMode mode = cudaStreamCaptureModeRelaxed;
+    BesideCapture() { cudaThreadExchangeStreamCaptureMode(&mode); }
+    ~BesideCapture() { cudaThreadExchangeStreamCaptureMode(&mode); }
+    BesideCapture(const BesideCapture &) = delete;
+};
+
 // Device scratch of one call or build step, given back when it goes out of
 // scope (also on error paths); the work enqueued on the context's stream until
 // then still has it.

@@ -61,6 +61,7 @@ struct hc_mlp
     float *d_m = nullptr, *d_v = nullptr;
     float *d_loss = nullptr;
     int step = 0;
+    bool written = false;       // weights or moments set by copies that may not have ended (settle)
     uint64_t serial = 0;        // changes with any buffer that the learned pipeline's kernels name
     // gate of the learned tail: largest predicted RMS residual (log10 units),
     // and how far from the predicted first bin the confirmation looks
@@ -1112,10 +1113,26 @@ __global__ void __launch_bounds__(kLtWarps * 32, 3) k_learned_tail(const uint32_
 
 }  // namespace
 
+// Before work on st that reads the network: the copies that set it are blocking ones on the
+// legacy stream, which may end after their call and which st need not wait for. They are
+// waited for by the first work after them. (A capture only records, and forbids the wait.)
+static int settle(hc_mlp *m, cudaStream_t st)
+{
+    if (!m->written) return HC_SUCCESS;
+    cudaStreamCaptureStatus cs = cudaStreamCaptureStatusNone;
+    HC_CUDA(m->ctx, cudaStreamIsCapturing(st, &cs));
+    if (cs != cudaStreamCaptureStatusNone) return HC_SUCCESS;
+    const BesideCapture beside;
+    HC_CUDA(m->ctx, cudaStreamSynchronize(cudaStreamLegacy));
+    m->written = false;
+    return HC_SUCCESS;
+}
+
 // the fused inference kernels (no activations kept)
 static int mlp_infer(hc_mlp *m, const float *X, uint32_t n, float *out, cudaStream_t st)
 {
     if (n == 0) return HC_SUCCESS;
+    if (const int rc = settle(m, st)) return rc;
     if (n <= kInferRowsPerSm * (uint32_t)m->ctx->sm_count)
     {
         HC_CUDA(m->ctx, cudaFuncSetAttribute(k_infer_rows, cudaFuncAttributeMaxDynamicSharedMemorySize,
@@ -1152,6 +1169,7 @@ static cudaError_t grad_tile(const float *P, const float *X, const float *Y, uin
 // is applied to the parameters. d_loss grows by the minibatch's loss.
 static int mlp_step(hc_mlp *m, const float *X, const float *Y, uint32_t n, const AdamStep &ad, cudaStream_t st)
 {
+    if (const int rc = settle(m, st)) return rc;
     const uint32_t sms = (uint32_t)m->ctx->sm_count;
     const uint32_t R = n <= 8 * sms ? 8u : (n <= 16 * sms ? 16u : 32u);
     const uint32_t ntiles = (n + R - 1) / R, grid = std::min(ntiles, sms);
@@ -1225,8 +1243,9 @@ void learned_key(const hc_mlp *m, GraphKey *key)
 // Allocates what the learned pipeline of n spectra needs (before any capture).
 int learned_prepare(hc_mlp *m, uint32_t n)
 {
-    int rc = grow_pipe(m, n);
+    int rc = settle(m, m->ctx->stream);
     if (rc) return rc;
+    if ((rc = grow_pipe(m, n))) return rc;
     QueryScratch &q = m->ctx->qs;
     if (q.fit_cap < n)
     {
@@ -1302,9 +1321,9 @@ int hc_mlp_create(hc_ctx *ctx, uint64_t seed, hc_mlp **out)
         hc_mlp_destroy(m);
         return HC_ERR_BAD_MEM_ALLOC;
     }
-    if (cudaMemsetAsync(m->d_m, 0, 4 * kParams, ctx->stream) != cudaSuccess ||
-        cudaMemsetAsync(m->d_v, 0, 4 * kParams, ctx->stream) != cudaSuccess ||
-        upload(ctx, m->d_params, h.data(), 4 * kParams) != cudaSuccess)
+    m->written = true;
+    if (cudaMemcpy(m->d_params, h.data(), 4 * kParams, cudaMemcpyHostToDevice) != cudaSuccess ||
+        cudaMemset(m->d_m, 0, 4 * kParams) != cudaSuccess || cudaMemset(m->d_v, 0, 4 * kParams) != cudaSuccess)
     {
         hc_mlp_destroy(m);
         return HC_ERR_CUDA;
@@ -1340,7 +1359,8 @@ int hc_mlp_get_params(hc_mlp *m, float *host)
 int hc_mlp_set_params(hc_mlp *m, const float *host)
 {
     if (!m || !host) return HC_ERR_INVLD_PTR;
-    HC_CUDA(m->ctx, overwrite(m->d_params, host, 4 * kParams));
+    m->written = true;
+    HC_CUDA(m->ctx, cudaMemcpy(m->d_params, host, 4 * kParams, cudaMemcpyHostToDevice));
     return HC_SUCCESS;
 }
 

@@ -1067,17 +1067,6 @@ int parse_device(hc_ctx *ctx, const std::unique_ptr<char[]> &buf, uint64_t size,
     return HC_SUCCESS;
 }
 
-// Reading a file is a host call to its caller: it may come while a thread of the program
-// captures a graph, in a mode that forbids others most calls until it has ended. What
-// is enqueued here goes to no stream under capture, so those calls are safe.
-struct BesideCapture
-{
-    cudaStreamCaptureMode mode = cudaStreamCaptureModeRelaxed;
-    BesideCapture() { cudaThreadExchangeStreamCaptureMode(&mode); }
-    ~BesideCapture() { cudaThreadExchangeStreamCaptureMode(&mode); }
-    BesideCapture(const BesideCapture &) = delete;
-};
-
 // the raw peaks on the host (for a device other than theirs)
 int peaks_to_host(hc_ctx *ctx, hc_ms2 *m)
 {
